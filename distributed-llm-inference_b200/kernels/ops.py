@@ -1256,12 +1256,28 @@ def conv_state_update(state: torch.Tensor, u: torch.Tensor, col0: int, q_start: 
 SSM_SCAN_MAX_STATE = 512
 
 
+SSM_CHUNK_MAX_STATE = 128  # the tensor-core form keeps a state column block in registers
+# shorter portions are walked token after token (us, walk / tiles, 64 heads, P 64, N 128: one portion of 16 tokens 16.9 / 14.5, of 8
+# 13.5 / 15.7; eight portions of 8 19 / 18, of 16 32 / 18, of 2 13 / 18: the tiles' set-up is worth it from about a quarter tile on)
+SSM_CHUNK_MIN_TOKENS = 17
+
+
+def ssm_scan_form(dtype: torch.dtype, P: int, N: int, max_len: int, aligned: bool = True) -> str:
+    """Which kernel serves a step: ``"chunk"`` (bfloat16 portions, tiles of tokens on the tensor cores) or ``"walk"`` (token after token on
+    the CUDA cores: decode steps, float32, sizes that are not whole 16-byte runs, larger states)."""
+    if dtype == torch.bfloat16 and P % 8 == 0 and N % 8 == 0 and N <= SSM_CHUNK_MAX_STATE and aligned and max_len >= SSM_CHUNK_MIN_TOKENS:
+        return "chunk"
+    return "walk"
+
+
 def ssm_scan(y: torch.Tensor, xbc: torch.Tensor, u: torch.Tensor, dt_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
-             state: torch.Tensor, q_start: torch.Tensor, state_slot: torch.Tensor, groups: int, max_len: int = 1 << 30) -> None:
+             state: torch.Tensor, q_start: torch.Tensor, state_slot: torch.Tensor, groups: int, max_len: int = 1 << 30,
+             form: str | None = None, segments: int = 0) -> None:
     """The selective scan of every sequence's tokens of this step, from and to its slot of ``state`` [slots, heads, P, N]
     (float32; S transposed, so that a column's N values are contiguous).  xbc [n, heads P + 2 groups N] holds x | B | C; dt_raw is column dt_col + head of u.  Per head:
     dt = softplus(dt_raw + dt_bias), S <- exp(-exp(a_log) dt) S + dt B x^T, y = S^T C + d_skip x.  y [n, heads P] float32.
-    ``max_len``: the most tokens a sequence brings, if the host knows (a launch hint: nothing is fetched ahead for single tokens)."""
+    ``max_len``: the most tokens a sequence brings, if the host knows (a launch hint).  ``form``: ``"walk"``, ``"chunk"``, or None (chosen:
+    ``ssm_scan_form``).  ``segments`` (of the form ``"chunk"``; 0: chosen): into how many runs of tiles a sequence is cut."""
     _columns(u, "ssm_scan"), _need(xbc, "xbc", u.dtype), _need(y, "y", torch.float32), _need(state, "state", torch.float32)
     for t, name in ((dt_bias, "dt_bias"), (a_log, "a_log"), (d_skip, "d_skip")):
         _need(t, name, torch.float32)
@@ -1272,6 +1288,24 @@ def ssm_scan(y: torch.Tensor, xbc: torch.Tensor, u: torch.Tensor, dt_col: int, d
             or heads % groups or N > SSM_SCAN_MAX_STATE or dt_bias.numel() != heads or a_log.numel() != heads or d_skip.numel() != heads
             or q_start.numel() != state_slot.numel() + 1):
         raise KernelError(f"ssm_scan: shapes do not agree (or the state size is above {SSM_SCAN_MAX_STATE})")
+    form = form or ssm_scan_form(u.dtype, P, N, max_len, xbc.data_ptr() % 16 == 0)
+    if form == "chunk":
+        if u.dtype != torch.bfloat16 or segments < 0:
+            raise KernelError("ssm_scan: the tensor-core form takes bfloat16")
+        count = state_slot.numel()
+        segments = segments or _fn("ssm_tc.cu", "dli_ssm_segments", [c_int] * 4)(count, heads, P, int(min(max_len, n)))
+        part = part_log = None
+        if segments > 1:
+            part = torch.empty(count * (segments - 1) * heads * P * N, dtype=torch.float32, device=y.device)
+            part_log = torch.empty(count * (segments - 1) * heads, dtype=torch.float32, device=y.device)
+        f = _fn("ssm_tc.cu", "dli_ssm_chunk", [c_void_p, c_void_p, c_void_p, c_longlong, c_int] + [c_void_p] * 6 + [c_int] * 6 + [c_void_p] * 3)
+        _check(f(_ptr(y), _ptr(xbc), _ptr(u), u.stride(0), dt_col, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(q_start),
+                 _ptr(state_slot), count, heads, P, N, groups, segments, _ptr(part), _ptr(part_log), _stream()), "ssm_scan")
+        global launch_count
+        launch_count += segments > 1  # two launches
+        return
+    if form != "walk":
+        raise KernelError("ssm_scan: form is walk or chunk")
     f = _fn("ssm.cu", "dli_ssm_scan", [c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]
             + [c_int] * 7 + [c_void_p])
     _check(f(_ptr(y), _ptr(xbc), _ptr(u), u.stride(0), dt_col, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(q_start),

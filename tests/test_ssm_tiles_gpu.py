@@ -1,0 +1,75 @@
+"""The selective scan over tiles of tokens (csrc/ssm_tc.cu) against the recurrence in float64, at the edges of its tiles, segments and column blocks."""
+
+import pytest
+import torch
+
+from dli_b200.kernels import ops
+
+
+def _exact(xbc, u, dt_col, dt_bias, a_log, d_skip, state, lens, groups):
+    _, H, P, N = state.shape
+    inner, out, t0 = H * P, [], 0
+    state, xbc, u = state.double(), xbc.double(), u.double()
+    for s, n in enumerate(lens):
+        S = state[s]
+        for t in range(t0, t0 + n):
+            x = xbc[t, :inner].view(H, P)
+            B = xbc[t, inner : inner + groups * N].view(groups, N).repeat_interleave(H // groups, 0)
+            C = xbc[t, inner + groups * N :].view(groups, N).repeat_interleave(H // groups, 0)
+            dt = torch.nn.functional.softplus(u[t, dt_col : dt_col + H] + dt_bias.double())
+            S = torch.exp(-torch.exp(a_log.double()) * dt)[:, None, None] * S + (dt[:, None] * x)[:, :, None] * B[:, None, :]
+            out.append(((S @ C[:, :, None])[..., 0] + d_skip.double()[:, None] * x).reshape(-1))
+        state[s] = S
+        t0 += n
+    return torch.stack(out), state
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt_shift", [-5.0, 0.0, 40.0], ids=["long_memory", "short_memory", "no_memory"])
+@pytest.mark.parametrize("H,P,N,groups,lens", [
+    (4, 64, 128, 2, [1, 64, 65, 200]), (2, 8, 8, 1, [16, 17, 63, 129]), (3, 72, 40, 3, [500]), (8, 64, 64, 1, [1, 1, 1, 33]), (2, 136, 16, 2, [128, 2]), (1, 64, 96, 1, [321])])
+def test_tiles_and_segments(H, P, N, groups, lens, dt_shift):
+    g = torch.Generator().manual_seed(len(lens) * 1000 + P + N)
+    n, S, dt_col = sum(lens), len(lens), 3
+    xbc = torch.randn(n, H * P + 2 * groups * N, generator=g).bfloat16()
+    u = torch.randn(n, dt_col + H + 2, generator=g).bfloat16()
+    dt_bias, a_log, d_skip = torch.randn(H, generator=g) + dt_shift, torch.rand(H, generator=g) * 2.5, torch.randn(H, generator=g)
+    state = torch.randn(S, H, P, N, generator=g)
+    y_ref, st_ref = _exact(xbc, u, dt_col, dt_bias, a_log, d_skip, state, lens, groups)
+    q_start = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32, device="cuda")
+    slot = torch.arange(S - 1, -1, -1, dtype=torch.int32, device="cuda")  # slots in another order than the sequences
+    walked = None
+    for form, segments in (("walk", 0), ("chunk", 0), ("chunk", 1), ("chunk", 2), ("chunk", 3), ("chunk", 7)):  # (seven: more than a sequence has tiles)
+        y, st = torch.full((n, H * P), float("nan"), device="cuda"), state.flip(0).cuda()
+        ops.ssm_scan(y, xbc.cuda(), u.cuda(), dt_col, dt_bias.cuda(), a_log.cuda(), d_skip.cuda(), st, q_start, slot, groups, max_len=max(lens), form=form, segments=segments)
+        errors = [float((a.cpu().double() - b).norm() / b.norm()) for a, b in ((y, y_ref), (st.flip(0), st_ref))]
+        if form == "walk":
+            walked = errors
+        else:  # float32 sums of up to a few hundred terms: 2^-24 each, some tens of roundings at full size; and no worse than the walk's by more than its scatter
+            assert all(e <= max(2 * w, 4e-7) for e, w in zip(errors, walked)), (form, segments, errors, walked)
+
+
+@pytest.mark.gpu
+def test_a_tile_may_be_replayed_from_a_graph():
+    H, P, N, lens = 2, 64, 64, [1, 200]
+    xbc, u = torch.randn(201, H * P + 2 * N).bfloat16().cuda(), torch.randn(201, H).bfloat16().cuda()
+    one, q_start, slot = torch.zeros(H).cuda(), torch.tensor([0, 1, 201], dtype=torch.int32).cuda(), torch.tensor([0, 1], dtype=torch.int32).cuda()
+    state = torch.zeros(2, H, P, N).cuda()
+    want, got = torch.empty(201, H * P).cuda(), torch.empty(201, H * P).cuda()
+    ops.ssm_scan(want, xbc, u, 0, one, one, one, state, q_start, slot, 1, max_len=200)
+    end = state.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ops.ssm_scan(got, xbc, u, 0, one, one, one, state, q_start, slot, 1, max_len=200)
+    state.zero_()
+    graph.replay()
+    assert torch.equal(got, want) and torch.equal(state, end)
+
+
+def test_which_form_serves_a_step():
+    form, bf, f32 = ops.ssm_scan_form, torch.bfloat16, torch.float32
+    assert form(bf, 64, 128, 17) == "chunk" and form(bf, 8, 8, 1 << 30) == "chunk"
+    assert form(bf, 64, 128, 16) == "walk"  # a decode step, or a short portion
+    assert form(f32, 64, 128, 4096) == "walk"
+    assert form(bf, 64, 136, 4096) == form(bf, 20, 16, 4096) == form(bf, 64, 10, 4096) == "walk"  # larger states; rows that are not whole 16-byte runs
+    assert form(bf, 64, 128, 4096, aligned=False) == "walk"
