@@ -515,6 +515,7 @@ def device_wait_errors(clear: bool = True) -> dict[str, int]:
     found = {}
     for source, read, forget, defines in (("skinny_gemm.cu", "dli_skinny_gemm_error", "dli_skinny_gemm_clear_error", None),
                                           ("dense_gemm.cu", "dli_dense_gemm_error", "dli_dense_gemm_clear_error", None),
+                                          ("recurrence_tiles.cu", "dli_recurrence_tiles_error", "dli_recurrence_tiles_clear_error", None),
                                           ("attention_tc.cu", "dli_paged_prefill_tc_error", "dli_paged_prefill_tc_clear_error", None),
                                           ("attention_tc.cu", "dli_paged_prefill_tc_error", "dli_paged_prefill_tc_clear_error", _BENT)):
         if not _library_in_use(source, defines):
@@ -1338,17 +1339,50 @@ def gated_group_rmsnorm(out: torch.Tensor, y: torch.Tensor, u: torch.Tensor, z_c
 # ------------------------------------------------------------------ gated delta rule
 
 DELTA_MAX_HEAD_DIM = 512
+TILES_MAX_HEAD_DIM = 128  # of keys and of values, in csrc/recurrence_tiles.cu
+TILES_MIN_TOKENS = 33  # shorter portions are walked
+
+
+def recurrence_form(d: int, dv: int, max_len: int, n: int, num_seqs: int, heads: int, on_gpu: bool = True) -> str:
+    """Which kernels serve a step of a delta rule or of the token-shift recurrence: ``"tiles"`` (portions: tiles of 64 tokens on the tensor
+    cores) or ``"walk"`` (decode steps, short portions, larger heads).
+
+    A walk's time goes with the longest sequence: 17 us and 0.43 us a token while its warps do not crowd the schedulers (two full-length
+    sequences of 16 heads), the tiles' with how often the tiles of all heads fill the GPU: about 30 us a time, once at least.  Measured (us, walk / tiles;
+    16 heads of 128 with a decay per channel): one sequence of 32 tokens 29 / 32, 48 37 / 34, 64 45 / 36, 192 107 / 40; 24 single
+    tokens beside one of 100 77 / 146, beside one of 600 312 / 191; a decay per head: 32 43 / 29, 192 99 / 38."""
+    if not on_gpu or d > TILES_MAX_HEAD_DIM or dv > TILES_MAX_HEAD_DIM or max_len < TILES_MIN_TOKENS:
+        return "walk"
+    longest = min(max_len, n)
+    tiles = 30.0 * max(1.0, (n / 64 + num_seqs) * heads / 148)
+    return "tiles" if tiles <= 17.0 + 0.43 * longest * max(1.0, n / longest * heads / 32) else "walk"
+
+
+def _recurrence_tiles(mode: int, what: str, o: torch.Tensor, qkv: torch.Tensor, u: torch.Tensor | None, b_col: int, a_col: int, a: torch.Tensor | None,
+                      dt_bias: torch.Tensor, a_log: torch.Tensor | None, bonus: torch.Tensor | None, state: torch.Tensor, q_start: torch.Tensor,
+                      state_slot: torch.Tensor, kq: int, unit_eps: float) -> None:
+    _, heads, dv, d = state.shape
+    n, count = o.shape[0], state_slot.numel()
+    size = _fn("recurrence_tiles.cu", "dli_recurrence_tiles_scratch", [c_int] * 5)
+    size.restype = c_longlong
+    scratch = torch.empty(size(n, count, heads, d, dv), dtype=torch.uint8, device=o.device)  # what the first kernel leaves for every tile and head
+    f = _fn("recurrence_tiles.cu", "dli_recurrence_tiles", [c_int, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int] + [c_void_p] * 8 + [c_int] * 6
+            + [c_float, c_int, c_void_p])
+    _check(f(mode, _ptr(o), _ptr(qkv), _ptr(u), 0 if u is None else u.stride(0), b_col, a_col, _ptr(a), _ptr(dt_bias), _ptr(a_log), _ptr(bonus), _ptr(state),
+             _ptr(q_start), _ptr(state_slot), _ptr(scratch), n, count, heads, kq, d, dv, unit_eps, DT_CODE[qkv.dtype], _stream()), what)
+    global launch_count
+    launch_count += 1  # two kernels
 
 
 def delta_rule_scan(o: torch.Tensor, qkv: torch.Tensor, u: torch.Tensor, b_col: int, a_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor,
                     state: torch.Tensor, seq_of_token: torch.Tensor, q_start: torch.Tensor, state_slot: torch.Tensor, kv_heads: int, head_dim: int,
-                    unit_eps: float, max_len: int = 1 << 30) -> None:
+                    unit_eps: float, max_len: int = 1 << 30, form: str | None = None) -> None:
     """The gated delta rule over every sequence's tokens of this step, from and to its slot of ``state``
     [slots, heads, dv, d] (float32; S transposed, so that a value column's d numbers are contiguous).
     qkv [n, 2 kv_heads d + heads dv] holds q | k | v after convolution and activation; b and a are columns b_col + head and
     a_col + head of u.  Per head h (q/k head h // (heads / kv_heads)): q and k are divided by sqrt(sum of squares + unit_eps),
     q also by sqrt(d); beta = sigmoid(b), gamma = exp(-exp(a_log) softplus(a + dt_bias));
-    S <- gamma S, w = beta (v - S^T k), S <- S + k w^T, o = S^T q.  o [n, heads dv] float32."""
+    S <- gamma S, w = beta (v - S^T k), S <- S + k w^T, o = S^T q.  o [n, heads dv] float32.  ``form``: ``"walk"``, ``"tiles"``, or None (chosen)."""
     _columns(u, "delta_rule_scan"), _need(qkv, "qkv", u.dtype), _need(o, "o", torch.float32), _need(state, "state", torch.float32)
     _need(dt_bias, "dt_bias", torch.float32), _need(a_log, "a_log", torch.float32)
     _need(seq_of_token, "seq_of_token", torch.int32), _need(q_start, "q_start", torch.int32), _need(state_slot, "state_slot", torch.int32)
@@ -1358,6 +1392,9 @@ def delta_rule_scan(o: torch.Tensor, qkv: torch.Tensor, u: torch.Tensor, b_col: 
             or u.shape[0] != n or b_col + heads > u.shape[1] or a_col + heads > u.shape[1] or d > DELTA_MAX_HEAD_DIM or seq_of_token.numel() != n
             or dt_bias.numel() != heads or a_log.numel() != heads or q_start.numel() != state_slot.numel() + 1):
         raise KernelError(f"delta_rule_scan: shapes do not agree (or the head size is above {DELTA_MAX_HEAD_DIM})")
+    if (form or recurrence_form(d, dv, max_len, n, state_slot.numel(), heads)) == "tiles":
+        _recurrence_tiles(0, "delta_rule_scan", o, qkv, u, b_col, a_col, None, dt_bias, a_log, None, state, q_start, state_slot, kv_heads, unit_eps)
+        return
     # the float32 rows the recurrence reads, written by the first two of the three kernels: unit vectors, values, four numbers a
     # head, and every token's coefficients with the tokens of its tile of 16 (csrc/delta_rule.cu: row_layout)
     stride = ((2 * kv_heads * d + heads * dv + 3) & ~3) + 4 * heads + 2 * heads * 16
@@ -1712,6 +1749,47 @@ def decay_recurrence(o: torch.Tensor, rows: torch.Tensor, state: torch.Tensor, q
     f = _fn("recurrence.cu", "dli_decay_recurrence", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p] + [c_int] * 7 + [c_void_p])
     _check(f(_ptr(o), _ptr(rows), _ptr(state), _ptr(q_start), _ptr(state_slot), _ptr(bonus), state_slot.numel(), heads, kq_heads, d, dv,
              0 if mode == "bonus" else 1, int(rows_per_lane), _stream()), "decay_recurrence")
+
+
+def shift_decay_scan(o: torch.Tensor, rkvg: torch.Tensor, wz: torch.Tensor, w0: torch.Tensor, bonus: torch.Tensor, state: torch.Tensor, q_start: torch.Tensor,
+                     state_slot: torch.Tensor, max_len: int = 1 << 30, form: str | None = None) -> None:
+    """The token-shift recurrence over every sequence's tokens of this step: ``shift_decay_prep`` and ``decay_recurrence`` ("bonus") in one call, or,
+    for portions, the kernels that take tiles of tokens.  ``form``: ``"walk"``, ``"tiles"``, or None (chosen)."""
+    _, heads, _, d = state.shape
+    n = o.shape[0]
+    if (form or recurrence_form(d, d, max_len, n, state_slot.numel(), heads, o.is_cuda)) != "tiles":
+        rows = torch.empty((n, decay_recurrence_row(heads, heads, d, d)), dtype=torch.float32, device=o.device)
+        shift_decay_prep(rows, rkvg, wz, w0, heads, d)
+        decay_recurrence(o, rows, state, q_start, state_slot, heads, "bonus", bonus, max_len=max_len)
+        return
+    _need(o, "o", torch.float32), _need(rkvg, "rkvg"), _need(wz, "wz", rkvg.dtype), _need(w0, "w0", torch.float32), _need(state, "state", torch.float32)
+    _need(bonus, "bonus", torch.float32), _need(q_start, "q_start", torch.int32), _need(state_slot, "state_slot", torch.int32)
+    if (rkvg.dtype not in DT_CODE or tuple(rkvg.shape) != (4, n, heads * d) or tuple(wz.shape) != (n, heads * d) or w0.numel() != heads * d
+            or tuple(bonus.shape) != (heads, d) or tuple(o.shape) != (n, heads * d) or state.shape[2] != d or q_start.numel() != state_slot.numel() + 1):
+        raise KernelError("shift_decay_scan: shapes or dtype do not agree")
+    _recurrence_tiles(2, "shift_decay_scan", o, rkvg, None, 0, 0, wz, w0, None, bonus, state, q_start, state_slot, heads, 0.0)
+
+
+def channel_delta_scan(o: torch.Tensor, qkv: torch.Tensor, u: torch.Tensor, b_col: int, a: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor,
+                       state: torch.Tensor, q_start: torch.Tensor, state_slot: torch.Tensor, kv_heads: int, unit_eps: float, max_len: int = 1 << 30,
+                       form: str | None = None) -> None:
+    """The delta rule with a decay per channel over every sequence's tokens of this step: ``channel_delta_prep`` and ``decay_recurrence`` ("delta")
+    in one call, or, for portions, the kernels that take tiles of tokens.  ``form``: ``"walk"``, ``"tiles"``, or None (chosen)."""
+    _, heads, dv, d = state.shape
+    n = o.shape[0]
+    if (form or recurrence_form(d, dv, max_len, n, state_slot.numel(), heads, o.is_cuda)) != "tiles":
+        rows = torch.empty((n, decay_recurrence_row(kv_heads, heads, d, dv)), dtype=torch.float32, device=o.device)
+        channel_delta_prep(rows, qkv, u, b_col, a, dt_bias, a_log, heads, kv_heads, d, dv, unit_eps)
+        decay_recurrence(o, rows, state, q_start, state_slot, kv_heads, "delta", None, max_len=max_len)
+        return
+    _columns(u, "channel_delta_scan"), _need(o, "o", torch.float32), _need(qkv, "qkv", u.dtype), _need(a, "a", u.dtype)
+    _need(dt_bias, "dt_bias", torch.float32), _need(a_log, "a_log", torch.float32), _need(state, "state", torch.float32)
+    _need(q_start, "q_start", torch.int32), _need(state_slot, "state_slot", torch.int32)
+    if (kv_heads < 1 or heads % kv_heads or tuple(qkv.shape) != (n, 2 * kv_heads * d + heads * dv) or tuple(a.shape) != (n, heads * d) or u.shape[0] != n
+            or b_col + heads > u.shape[1] or dt_bias.numel() != heads * d or a_log.numel() != heads or tuple(o.shape) != (n, heads * dv)
+            or q_start.numel() != state_slot.numel() + 1):
+        raise KernelError("channel_delta_scan: shapes do not agree")
+    _recurrence_tiles(1, "channel_delta_scan", o, qkv, u, b_col, 0, a, dt_bias, a_log, None, state, q_start, state_slot, kv_heads, unit_eps)
 
 
 # ------------------------------------------------------------------ matrix memory with exponential gates

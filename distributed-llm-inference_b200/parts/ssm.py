@@ -11,6 +11,20 @@ from ..weights.loader import TensorDecl
 from .base import Part, register_part, tensor_name
 
 
+# From this many decoded tokens on beside longer portions, a delta rule takes them apart: single tokens are walked and the portions go by
+# tiles of tokens, of which each single token would fill one (16 heads of 128 beside a portion of 100 tokens: 24 single tokens add 108 us
+# as tiles, a walk of their own some 20).
+SINGLES_APART = 4
+
+
+def singles_apart(batch, d: int, dv: int, heads: int, on_gpu: bool) -> int:
+    """How many of the step's leading single-token sequences a delta rule takes in a call of their own (0: one call for all)."""
+    s = batch.num_single
+    if s < SINGLES_APART or s == batch.num_seqs or ops.recurrence_form(d, dv, batch.max_q_len, batch.n - s, batch.num_seqs - s, heads, on_gpu) != "tiles":
+        return 0
+    return s
+
+
 @register_part("mixer", "mamba2")
 class Mamba2Mixer(Part):
     """Mamba-2 (state-space duality) on any mix of prompt portions and decoded tokens.
@@ -168,8 +182,12 @@ class GatedDeltaRule(Part):
         if self.taps > 1:
             ops.conv_state_update(conv_state, u, 0, batch.q_start, batch.state_slot)
         o = torch.empty((n, self.inner), dtype=torch.float32, device=x.device)
-        ops.delta_rule_scan(o, qkv, u, self.b_col, self.a_col, w["dt_bias"], w["A_log"], state, batch.seq_of_token, batch.q_start, batch.state_slot,
-                            self.kv_heads, self.d, self.unit_eps, max_len=batch.max_q_len)
+        s = singles_apart(batch, self.d, self.dv, self.heads, x.is_cuda)
+        if s:
+            ops.delta_rule_scan(o[:s], qkv[:s], u[:s], self.b_col, self.a_col, w["dt_bias"], w["A_log"], state, batch.seq_of_token[:s], batch.q_start[: s + 1],
+                                batch.state_slot[:s], self.kv_heads, self.d, self.unit_eps, max_len=1)
+        ops.delta_rule_scan(o, qkv, u, self.b_col, self.a_col, w["dt_bias"], w["A_log"], state, batch.seq_of_token, batch.q_start[s:], batch.state_slot[s:],
+                            self.kv_heads, self.d, self.unit_eps, max_len=batch.max_q_len, **({"form": "tiles"} if s else {}))
         gated = torch.empty((n, self.inner), dtype=x.dtype, device=x.device)
         ops.gated_group_rmsnorm(gated, o, u, self.g_col, w["norm"], self.heads, self.eps, gate_after=True)
         return project(gated, w["o"])
@@ -216,11 +234,6 @@ class MinGRU(Part):
         gated = torch.empty((x.shape[0], self.width), dtype=x.dtype, device=x.device)
         ops.mingru_scan(gated, p, self.bz, self.bx, cache.state, batch.q_start, batch.state_slot, max_len=batch.max_q_len)
         return project(gated, self.wo)
-
-
-def _recurrence_row(kq_heads: int, heads: int, d: int, dv: int) -> int:
-    """Floats of a token's row as ``ops.decay_recurrence`` reads it: read vectors | keys | decays | values | betas."""
-    return ops.decay_recurrence_row(kq_heads, heads, d, dv)
 
 
 @register_part("mixer", "shift_decay_recurrence")
@@ -292,10 +305,8 @@ class ShiftDecayRecurrence(Part):
         rkvg = batched_project(blends[:4], w["rkvg"])  # [4, n, I]
         low = ops.activation(project(blends[4], w["w1"]), "tanh")
         wz = project(low, w["w2"])
-        rows = torch.empty((n, _recurrence_row(self.heads, self.heads, self.d, self.d)), dtype=torch.float32, device=x.device)
-        ops.shift_decay_prep(rows, rkvg, wz, w["w0"], self.heads, self.d)
         o = torch.empty((n, self.inner), dtype=torch.float32, device=x.device)
-        ops.decay_recurrence(o, rows, state, batch.q_start, batch.state_slot, self.heads, "bonus", w["u"], max_len=batch.max_q_len)
+        ops.shift_decay_scan(o, rkvg, wz, w["w0"], w["u"], state, batch.q_start, batch.state_slot, max_len=batch.max_q_len)
         gated = torch.empty((n, self.inner), dtype=x.dtype, device=x.device)
         ops.gated_group_rmsnorm(gated, o, rkvg[3], 0, w["norm"], self.heads, self.eps, gate_after=True)
         return project(gated, w["o"])
@@ -385,10 +396,13 @@ class ChannelDeltaRule(Part):
             ops.conv_state_update(conv_state, u, 0, batch.q_start, batch.state_slot)
         a = project(u[:, self.a_cols[0] : self.a_cols[1]], w["a2"])  # [n, heads * head_dim]; the library reads the column slice in place
         g = project(u[:, self.g_cols[0] : self.g_cols[1]], w["g2"])  # [n, heads * value_dim]
-        rows = torch.empty((n, _recurrence_row(self.kv_heads, self.heads, self.d, self.dv)), dtype=torch.float32, device=x.device)
-        ops.channel_delta_prep(rows, qkv, u, self.b_col, a, w["dt_bias"], w["A_log"], self.heads, self.kv_heads, self.d, self.dv, self.unit_eps)
         o = torch.empty((n, self.inner), dtype=torch.float32, device=x.device)
-        ops.decay_recurrence(o, rows, state, batch.q_start, batch.state_slot, self.kv_heads, "delta", None, max_len=batch.max_q_len)
+        s = singles_apart(batch, self.d, self.dv, self.heads, x.is_cuda)
+        if s:
+            ops.channel_delta_scan(o[:s], qkv[:s], u[:s], self.b_col, a[:s], w["dt_bias"], w["A_log"], state, batch.q_start[: s + 1], batch.state_slot[:s],
+                                   self.kv_heads, self.unit_eps, max_len=1)
+        ops.channel_delta_scan(o, qkv, u, self.b_col, a, w["dt_bias"], w["A_log"], state, batch.q_start[s:], batch.state_slot[s:], self.kv_heads,
+                               self.unit_eps, max_len=batch.max_q_len, **({"form": "tiles"} if s else {}))
         gated = torch.empty((n, self.inner), dtype=x.dtype, device=x.device)
         ops.gated_group_rmsnorm(gated, o, g, 0, w["norm"], self.heads, self.eps, gate_after=True, gate="sigmoid")
         return project(gated, w["o"])

@@ -1,0 +1,159 @@
+"""The delta rules and the token-shift recurrence over tiles of tokens (csrc/recurrence_tiles.cu) against the recurrences in float64, at the edges of
+their tiles, blocks and column groups; and which kernels serve which step."""
+
+import types
+
+import pytest
+import torch
+
+from dli_b200.kernels import ops
+from dli_b200.parts import ssm
+
+
+def _unit(v):
+    return v / torch.sqrt((v * v).sum(-1, keepdim=True) + 1e-6)
+
+
+def _starts(lens):
+    return torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32)
+
+
+def _delta(channel, qkv, u, a, dt_bias, a_log, state, lens, G):
+    """u: betas' columns 1 .. heads, then the decays' ones of the rule with a decay per head."""
+    S, H, dv, d = state.shape
+    n, x = qkv.shape[0], qkv.double()
+    q = (_unit(x[:, : G * d].view(n, G, d)) * d**-0.5).repeat_interleave(H // G, 1)
+    k = _unit(x[:, G * d : 2 * G * d].view(n, G, d)).repeat_interleave(H // G, 1)
+    v, beta = x[:, 2 * G * d :].view(n, H, dv), torch.sigmoid(u[:, 1 : 1 + H].double())
+    raw = (a.double() + dt_bias.double()).view(n, H, d) if channel else (u[:, 1 + H : 1 + 2 * H].double() + dt_bias.double())[..., None]
+    keep = torch.exp(-torch.exp(a_log.double())[:, None] * torch.nn.functional.softplus(raw))
+    state, out, t0 = state.double(), [], 0
+    for s, count in enumerate(lens):
+        X = state[s]
+        for t in range(t0, t0 + count):
+            X = X * keep[t, :, None, :]
+            X = X + (beta[t, :, None] * (v[t] - (X @ k[t, :, :, None])[..., 0]))[:, :, None] * k[t, :, None, :]
+            out.append((X @ q[t, :, :, None])[..., 0].reshape(-1))
+        state[s], t0 = X, t0 + count
+    return torch.stack(out), state
+
+
+def _bonus(rkvg, wz, w0, bonus, state, lens):
+    S, H, _, d = state.shape
+    n = wz.shape[0]
+    r, k, v = (rkvg[i].double().view(n, H, d) for i in range(3))
+    keep = torch.exp(-torch.exp(wz.double() + w0.double())).view(n, H, d)
+    state, out, t0 = state.double(), [], 0
+    for s, count in enumerate(lens):
+        X = state[s]
+        for t in range(t0, t0 + count):
+            kv = v[t, :, :, None] * k[t, :, None, :]
+            out.append(((X + kv * bonus.double()[:, None, :]) @ r[t, :, :, None])[..., 0].reshape(-1))
+            X = X * keep[t, :, None, :] + kv
+        state[s], t0 = X, t0 + count
+    return torch.stack(out), state
+
+
+def _check(run, want, shape, state):
+    """Both forms from the same start; the tiles' errors are those of float32 sums of up to a few hundred terms, and no worse than the walk's by
+    more than the scatter between two orders of summation."""
+    S = state.shape[0]
+    slot = torch.arange(S - 1, -1, -1, dtype=torch.int32, device="cuda")  # slots in another order than the sequences
+    errors = {}
+    for form in ("walk", "tiles"):
+        o, st = torch.full(shape, float("nan"), device="cuda"), state.flip(0).cuda()
+        run(o, st, slot, form)
+        errors[form] = [float((x.cpu().double() - y).norm() / y.norm()) for x, y in ((o, want[0]), (st.flip(0), want[1]))]
+    assert all(e <= max(2 * w, 5e-7) for e, w in zip(errors["tiles"], errors["walk"])), errors
+    assert ops.device_wait_errors() == {}
+
+
+SHAPES = [(2, 1, 128, 128, [1, 63, 64, 65]), (4, 2, 64, 64, [130, 17]), (2, 2, 40, 24, [200, 2]), (3, 1, 128, 16, [16, 33]), (2, 1, 13, 9, [70]), (40, 20, 128, 128, [65])]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("decay", [-6.0, 0.0, 30.0], ids=["long_memory", "short_memory", "no_memory"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("channel", [False, True], ids=["decay_per_head", "decay_per_channel"])
+@pytest.mark.parametrize("H,G,d,dv,lens", SHAPES)
+def test_delta_rules(H, G, d, dv, lens, channel, dtype, decay):
+    g = torch.Generator().manual_seed(H * 100 + d + dv)
+    n = sum(lens)
+    qkv, u = torch.randn(n, 2 * G * d + H * dv, generator=g).to(dtype), torch.randn(n, 2 * H + 3, generator=g).to(dtype)
+    a, a_log = torch.randn(n, H * d, generator=g).to(dtype), torch.rand(H, generator=g)
+    dt_bias = torch.randn(H * d if channel else H, generator=g) + decay
+    state = torch.randn(len(lens), H, dv, d, generator=g) * 0.3
+    want = _delta(channel, qkv, u, a, dt_bias, a_log, state, lens, G)
+    q_start, seq = _starts(lens).cuda(), torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens)).int().cuda()
+    x = [t.cuda() for t in (qkv, u, a, dt_bias, a_log)]
+
+    def run(o, st, slot, form):
+        if channel:
+            ops.channel_delta_scan(o, x[0], x[1], 1, x[2], x[3], x[4], st, q_start, slot, G, 1e-6, max_len=max(lens), form=form)
+        else:
+            ops.delta_rule_scan(o, x[0], x[1], 1, 1 + H, x[3], x[4], st, seq, q_start, slot, G, d, 1e-6, max_len=max(lens), form=form)
+
+    _check(run, want, (n, H * dv), state)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shift", [-5.0, 0.0, 5.0], ids=["long_memory", "short_memory", "no_memory"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("H,d,lens", [(2, 64, [1, 63, 64, 65]), (2, 128, [130, 17]), (3, 24, [100]), (1, 9, [33, 1, 70]), (40, 64, [65])])
+def test_bonus(H, d, lens, dtype, shift):
+    g = torch.Generator().manual_seed(H * 100 + d)
+    n = sum(lens)
+    rkvg, wz = torch.randn(4, n, H * d, generator=g).to(dtype), torch.randn(n, H * d, generator=g).to(dtype)
+    w0, bonus, state = torch.randn(H * d, generator=g) + shift, torch.randn(H, d, generator=g), torch.randn(len(lens), H, d, d, generator=g)
+    want = _bonus(rkvg, wz, w0, bonus, state, lens)
+    q_start, x = _starts(lens).cuda(), [t.cuda() for t in (rkvg, wz, w0, bonus)]
+    _check(lambda o, st, slot, form: ops.shift_decay_scan(o, x[0], x[1], x[2], x[3], st, q_start, slot, max_len=max(lens), form=form), want, (n, H * d), state)
+
+
+def test_which_form_serves_a_step():
+    form = ops.recurrence_form
+    assert form(128, 128, 2048, 2048, 1, 16) == form(64, 64, 4096, 4096, 1, 16) == form(128, 128, 2100, 3500, 2, 16) == form(128, 128, 1 << 30, 2048, 1, 32) == "tiles"
+    assert form(128, 128, 1, 64, 64, 16) == form(128, 128, 32, 32, 1, 16) == "walk"  # decode steps, short portions
+    assert form(136, 128, 2048, 2048, 1, 16) == form(128, 136, 2048, 2048, 1, 16) == "walk"  # larger heads
+    assert form(128, 128, 100, 124, 25, 16) == "walk"  # a single portion does not pay for a tile of every single token
+    assert form(128, 128, 2048, 2048, 1, 16, on_gpu=False) == "walk"
+
+
+def test_when_single_tokens_are_taken_apart():
+    def apart(singles, portions, tokens, longest):
+        batch = types.SimpleNamespace(num_single=singles, num_seqs=singles + portions, n=singles + tokens, max_q_len=longest)
+        return ssm.singles_apart(batch, 128, 128, 16, True)
+
+    assert apart(24, 1, 600, 600) == 24 and apart(4, 2, 300, 200) == 4
+    assert apart(3, 1, 600, 600) == 0  # a few ride along
+    assert apart(24, 0, 0, 1) == 0 and apart(24, 1, 20, 20) == 0  # nothing, or nothing long enough, beside them
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["gated_delta", "channel_delta"])
+def test_single_tokens_taken_apart_give_the_same(kind, monkeypatch):
+    from dli_b200.cache.pools import LayerCache
+    from dli_b200.config.spec import PartSpec
+    from dli_b200.engine.batch import StepBatch
+    from dli_b200.parts.base import BuildEnv, build_part
+
+    W, H, G, d = 64, 4, 2, 32
+    params = {"hidden_size": W, "num_heads": H, "num_kv_heads": G, "head_dim": d, "value_dim": d, "conv_taps": 4, "eps": 1e-6, "decay_rank": 8, "gate_rank": 8}
+    part = build_part("mixer", PartSpec(kind, params), BuildEnv(torch.bfloat16, torch.device("cuda")))
+    g = torch.Generator().manual_seed(3)
+    part.load({name: (torch.randn(decl.shape, generator=g) * 0.2).to(torch.bfloat16 if decl.kind == "matrix" else torch.float32).cuda()
+               for name, decl in part.declare().items()})
+    lens = [1] * 6 + [130, 40]
+    n, S = sum(lens), len(lens)
+    x = torch.randn(n, W, generator=g).bfloat16().cuda()
+    starts = [(torch.randn((S, *need.shape), generator=g) * 0.3).to(need.dtype).cuda() for need in part.cache_need()]
+    q_start = _starts(lens).cuda()
+    batch = StepBatch(n=n, num_seqs=S, num_single=6, token_ids=None, positions=None, seq_of_token=torch.repeat_interleave(torch.arange(S), torch.tensor(lens)).int().cuda(),
+                      q_start=q_start, kv_len=None, state_slot=torch.arange(S, dtype=torch.int32, device="cuda"), logit_rows=None, groups=[], max_q_len=130)
+    got = []
+    for limit in (4, 100):
+        monkeypatch.setattr(ssm, "SINGLES_APART", limit)
+        cache = LayerCache(states=tuple(s.clone() for s in starts))
+        got.append([part.forward(x, batch, cache), *cache.states])
+    for a, b in zip(*got):  # bfloat16 outputs of float32 sums that differ in their order; float32 states
+        assert (a.float() - b.float()).norm() <= (1e-2 if a.dtype == torch.bfloat16 else 1e-5) * b.float().norm()
