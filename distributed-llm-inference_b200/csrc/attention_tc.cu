@@ -901,6 +901,330 @@ int launch_tc2(const CUtensorMap& map_k, const CUtensorMap& map_v, const Params&
                          map_k, map_v, p);
 }
 
+#if !BENT_SCORES
+// ================================================================ one pool: a cached row is key and value
+// Prompt portions over rows of 136 to 256 numbers whose leading numbers are the values (attention over a cached latent: many query
+// heads on one KV head).  The products and roles are those of the kernel with two threads per row; a tile of 128 rows comes once, as
+// SLABS slabs of 64 columns, and is the K-major operand of S = Q K^T and the MN-major operand of O += P V (all value columns in
+// one instruction).  Q, two tiles and P fill shared memory (64 + 2 x 64 + 32 KB with 256 columns), S twice and O tensor memory (256 + 256
+// columns).  The thread that issues products takes whichever of S(t + 1) and O += P(t) V(t) is possible first: a tile's stage is only free
+// for the copies once both have read it, so neither should stand behind the other.
+//
+// What bounds it: the copies.  With clocks taken in a CTA (4,096 tokens, 16 heads, rows of 256, 192 value columns), a tile takes 4,320 clocks; 3,900 pass
+// from a tile's request to its arrival (64 KB: all SMs read the same rows from L2 at 4.7 TB/s together, the next stage's request waits for O of
+// the tile before the last), 1,000 are S, 2,200 the softmax threads, 800 to 1,700 O.  Measured against the mma.sync kernel, us: 4,096 tokens 798 -> 177
+// (679 TFLOP/s), with a window of 1,024 358 -> 116, 512 tokens 44 -> 20, 8 tokens behind 2,000 149 -> 47, 2 tokens four times 15 -> 12; 32 heads, 2,048 tokens 420 -> 113.
+struct RowParams {
+  bf16* out;
+  const bf16* q;
+  long long q_stride;
+  const int *block_tables, *q_start, *kv_len;
+  int max_blocks, seq0, nh, nkv, page_size, window;
+  float scale_log2, sink_log2;
+  const float* sink_heads;
+  int tokens_per_tile, heads_per_chunk, head_chunks;
+  int d, dv, out_row;  // columns of a cached row, of the values that are wanted, of the output's rows
+  int* error_flag;
+};
+
+template <int SLABS> struct RowCfg {
+  static constexpr int STAGE = SLABS * TILE_BYTES;  // one tile of rows; also the Q tile
+  static constexpr int AT_P = 3 * STAGE, AT_MAX = AT_P + 2 * TILE_BYTES, AT_BAR = AT_MAX + 4 * ROWS * 4, SMEM = AT_BAR + 128;
+  static_assert(SMEM <= 227 * 1024, "one CTA fits an SM");
+};
+
+__device__ __forceinline__ bool barrier_phase_done(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done;
+}
+
+template <int SLABS>
+__global__ void __launch_bounds__(THREADS, 1) paged_prefill_row_kernel(const __grid_constant__ CUtensorMap map, const RowParams p) {
+  using Cfg = RowCfg<SLABS>;
+  pdl_launch_dependents();
+  extern __shared__ __align__(1024) unsigned char smem[];
+  unsigned char* sQ = smem;
+  unsigned char* sK = sQ + Cfg::STAGE;  // two stages
+  unsigned char* sP = smem + Cfg::AT_P;  // keys 0..63 | keys 64..127
+  float* row_max = (float*)(smem + Cfg::AT_MAX);  // [2 (tile parity)][2 (half)][128]
+  uint64_t* bars = (uint64_t*)(smem + Cfg::AT_BAR);
+  uint32_t* tmem_slot = (uint32_t*)(bars + 8);
+  volatile int* failed = (volatile int*)(tmem_slot + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int r = tid & (ROWS - 1), half = (tid >> 7) & 1;
+  const uint32_t k_full = smem_u32(bars), s_done = smem_u32(bars + 2), o_done = smem_u32(bars + 4), p_ready = smem_u32(bars + 6);
+
+  const int s = p.seq0 + blockIdx.y;
+  const int tile = gridDim.z - 1 - blockIdx.z;  // the tiles that see the most keys start first
+  const int kvh = blockIdx.x / p.head_chunks, hc = blockIdx.x - kvh * p.head_chunks;
+  const int q0 = p.q_start[s], qlen = p.q_start[s + 1] - q0, tok0 = tile * p.tokens_per_tile;
+  if (tok0 >= qlen) return;  // the whole CTA: nothing was set up yet
+  if (smem_u32(smem) & 1023) {  // the swizzled tiles need it; nothing else lies in front of them
+    if (tid == 0) atomicExch(p.error_flag, 21);
+    return;
+  }
+  const int kvlen = p.kv_len[s], ntok = min(p.tokens_per_tile, qlen - tok0);
+  const int G = p.nh / p.nkv, Gc = p.heads_per_chunk, head0 = kvh * G + hc * Gc, nheads = min(Gc, G - hc * Gc);
+  const int pos0 = kvlen - qlen + tok0, rows_used = ntok * Gc;
+  const int* table = p.block_tables + (size_t)s * p.max_blocks;
+  const int hi = pos0 + ntok, lo = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
+  const int t_begin = lo / KEYS, t_end = (hi + KEYS - 1) / KEYS, num_tiles = t_end - t_begin;
+  const int vslabs = (p.dv + 63) >> 6;
+
+  if (tid == 0) {
+    for (int i = 0; i < 6; ++i) mbar_init(k_full + 8 * i, 1);  // k_full, s_done, o_done
+    mbar_init(p_ready, SOFTMAX_THREADS);
+    *failed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  pdl_wait();  // queries and the cache are the work of the kernels before this one
+
+  // ---- Q, swizzled by hand (rows beyond the used ones and columns beyond the row are zero); both stages start as zeros: pages beyond the
+  //      sequence are never fetched, and their (masked) rows must not multiply garbage
+  for (int idx = tid; idx < ROWS * 8 * SLABS; idx += THREADS) {
+    const int rr = idx / (8 * SLABS), c = idx - rr * (8 * SLABS);
+    const int tok = rr / Gc, hd = rr - tok * Gc;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (rr < rows_used && hd < nheads && c * 8 < p.d)
+      v = *reinterpret_cast<const uint4*>(p.q + (size_t)(q0 + tok0 + tok) * p.q_stride + (size_t)(head0 + hd) * p.d + c * 8);
+    *reinterpret_cast<uint4*>(sQ + (c >> 3) * TILE_BYTES + rr * 128 + (((c & 7) ^ (rr & 7)) << 4)) = v;
+  }
+  for (int idx = tid; idx < 2 * Cfg::STAGE / 16; idx += THREADS) reinterpret_cast<uint4*>(sK)[idx] = make_uint4(0, 0, 0, 0);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot, tmem_s = tmem, tmem_o = tmem + 2 * KEYS;
+
+  if (warp == SOFTMAX_THREADS / 32 + 1) {
+    // ================================================================ the warp that copies: a page per lane, all its slabs
+    const int pages = KEYS / p.page_size, page_i = lane & 15;
+    auto lookup = [&](int t) -> int {
+      const int first = t * KEYS + page_i * p.page_size;
+      const bool need = lane < 16 && t < t_end && page_i < pages && first < hi && first + p.page_size > lo;
+      return need ? table[first / p.page_size] : -1;
+    };
+    int page = lookup(t_begin);
+    for (int t = 0; t < num_tiles && !*failed; ++t) {
+      const int st = t & 1, cur = page;
+      page = lookup(t_begin + t + 1);
+      if (t >= 2) {
+        if (lane == 0) wait_or_fail(o_done + 8 * st, ((t - 2) >> 1) & 1, failed, 22, p.error_flag);  // P V(t - 2), the stage's last reader
+        __syncwarp();
+        if (*failed) break;
+      }
+      const int count = __popc(__ballot_sync(0xffffffffu, cur >= 0));
+      if (lane == 0) mbar_expect_tx(k_full + 8 * st, (uint32_t)(count * p.page_size * 128 * SLABS));
+      __syncwarp();
+      if (cur >= 0) {
+#pragma unroll
+        for (int sl = 0; sl < SLABS; ++sl)
+          tma_load_2d(smem_u32(sK + st * Cfg::STAGE + sl * TILE_BYTES + page_i * p.page_size * 128), &map, sl * 64, (cur * p.nkv + kvh) * p.page_size, k_full + 8 * st);
+      }
+    }
+  } else if (warp == SOFTMAX_THREADS / 32) {
+    // ================================================================ the thread that issues the matrix products
+    if (lane == 0) {
+      const uint32_t idesc_s = instr_desc(ROWS, KEYS, 0), idesc_o = instr_desc(ROWS, vslabs * 64, 1);
+      const int k_steps = (p.d + 15) >> 4;
+      const uint64_t next_slab = (uint64_t)(TILE_BYTES >> 4) << 16;  // of the MN-major operand: bytes from 64 columns to the next 64
+      const uint32_t qa = smem_u32(sQ), pa = smem_u32(sP);
+      int s_next = 0, o_next = 0;
+      unsigned idle = 0;
+      while (o_next < num_tiles && !*failed) {
+        bool moved = false;
+        // O += P(t) V(t): the probabilities are written, the output rescaled where a row's maximum grew
+        if (o_next < s_next && barrier_phase_done(p_ready, o_next & 1)) {
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t v = smem_u32(sK + (o_next & 1) * Cfg::STAGE);
+#pragma unroll
+          for (int k = 0; k < KEYS / 16; ++k)
+            umma(tmem_o, smem_desc_sw128(pa + (k >> 2) * TILE_BYTES + (k & 3) * 32), smem_desc_sw128(v + k * 2048) | next_slab, idesc_o, (o_next | k) != 0);
+          umma_commit(o_done + 8 * (o_next & 1));
+          ++o_next;
+          moved = true;
+        }
+        // S(t) = Q K(t)^T: the rows have arrived; the buffer held S(t - 2), which every thread had read when P(t - 2) was handed in
+        if (s_next < num_tiles && s_next <= o_next + 1 && barrier_phase_done(k_full + 8 * (s_next & 1), (s_next >> 1) & 1)) {
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t k = smem_u32(sK + (s_next & 1) * Cfg::STAGE);
+#pragma unroll
+          for (int kk = 0; kk < SLABS * 4; ++kk)
+            if (kk < k_steps)
+              umma(tmem_s + (s_next & 1) * KEYS, smem_desc_sw128(qa + (kk >> 2) * TILE_BYTES + (kk & 3) * 32), smem_desc_sw128(k + (kk >> 2) * TILE_BYTES + (kk & 3) * 32), idesc_s, kk != 0);
+          umma_commit(s_done + 8 * (s_next & 1));
+          ++s_next;
+          moved = true;
+        }
+        if (moved) {
+          idle = 0;
+        } else if (++idle > WAIT_LIMIT) {
+          *failed = 23;
+          atomicExch(p.error_flag, 23);
+        } else {
+          __nanosleep(20);
+        }
+      }
+    }
+    __syncwarp();
+  } else {
+    // ================================================================ softmax threads: two a row, 64 keys and half of the value columns each
+    const int rtok = r / Gc;
+    const bool rvalid = r < rows_used && (r - rtok * Gc) < nheads;
+    const int rpos = pos0 + rtok;
+    const uint32_t lane_bits = (uint32_t)((warp & 3) * 32) << 16;
+    const int col0 = half * 64, half_cols = vslabs * 32;
+    constexpr float RESCALE_STEP = 8.f;
+    float m = -CUDART_INF_F, m_ref = -CUDART_INF_F, l = 0.f;
+    bool ok = true;
+    const int group = r >> 6;
+    const uint32_t my_o = tmem_o + lane_bits + half * half_cols;
+    uint32_t pchunk[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) pchunk[c] = smem_u32(sP) + half * TILE_BYTES + r * 128 + ((c ^ (r & 7)) << 4);
+
+    for (int it = 0; it < num_tiles; ++it) {
+      const int b = it & 1, base = (t_begin + it) * KEYS;
+      ok = wait_or_fail(s_done + 8 * b, (it >> 1) & 1, failed, 24, p.error_flag) && ok;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const bool full = base + KEYS - 1 <= pos0 && base >= lo && p.window <= 0;
+      float sc[64];
+      {
+        uint32_t v0[32], v1[32];
+        tmem_ld32_nowait(tmem_s + b * KEYS + lane_bits + col0, v0);
+        tmem_ld32_nowait(tmem_s + b * KEYS + lane_bits + col0 + 32, v1);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 32; ++j) { sc[j] = __uint_as_float(v0[j]); sc[32 + j] = __uint_as_float(v1[j]); }
+      }
+      if (!full) {
+        const int first = base + col0;
+        const int hi_j = rpos - first, lo_j = p.window > 0 ? rpos - p.window - first : -1;
+#pragma unroll
+        for (int j = 0; j < 64; ++j) sc[j] = (j <= hi_j && j > lo_j) ? sc[j] : -CUDART_INF_F;
+      }
+      float mx[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) mx[j] = max3(sc[j], sc[j + 8], sc[j + 16]);
+#pragma unroll
+      for (int j = 24; j < 56; j += 16)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mx[i] = max3(mx[i], sc[j + i], sc[j + 8 + i]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) mx[i] = fmaxf(mx[i], sc[56 + i]);
+      float* rm = row_max + b * 2 * ROWS;  // by parity: a fast thread's next tile writes the other buffer
+      rm[half * ROWS + r] = max3(max3(mx[0], mx[1], mx[2]), max3(mx[3], mx[4], mx[5]), fmaxf(mx[6], mx[7]));
+      if (group == 0) asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_THREADS / 2) : "memory");  // the two halves of this row's 64-row group
+      else asm volatile("bar.sync 2, %0;" ::"n"(SOFTMAX_THREADS / 2) : "memory");
+      m = max3(m, rm[r], rm[ROWS + r]);
+      float corr = 1.f;
+      const bool grown = (m - m_ref) * p.scale_log2 > RESCALE_STEP;  // also the first finite maximum (m_ref = -inf)
+      if (grown) {
+        corr = (m_ref == -CUDART_INF_F) ? 0.f : ex2((m_ref - m) * p.scale_log2);
+        m_ref = m;
+      }
+      const float neg = (m_ref == -CUDART_INF_F) ? 0.f : -m_ref * p.scale_log2;
+#pragma unroll
+      for (int j = 0; j < 64; ++j) sc[j] = ex2(fmaf(sc[j], p.scale_log2, neg));  // masked: ex2(-inf) = 0
+      // P and O are free once the product of the tile before has finished
+      if (it > 0) {
+        ok = wait_or_fail(o_done + 8 * (b ^ 1), ((it - 1) >> 1) & 1, failed, 22, p.error_flag) && ok;
+        ok = __all_sync(0xffffffffu, ok);
+        if (__any_sync(0xffffffffu, grown)) {
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (ok) {
+            for (int c = 0; c < half_cols; c += 32) {
+              uint32_t v[32];
+              tmem_ld32_nowait(my_o + c, v);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * corr);
+              tmem_st32(my_o + c, v);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          }
+        }
+      }
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 64; j += 8) {
+        uint32_t packed[4];
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) {
+          sum[(e >> 1) & 3] += sc[j + e] + sc[j + e + 1];
+          __nv_bfloat162 b2 = __floats2bfloat162_rn(sc[j + e], sc[j + e + 1]);
+          packed[e >> 1] = *reinterpret_cast<uint32_t*>(&b2);
+        }
+        st_shared_v4(pchunk[j >> 3], packed[0], packed[1], packed[2], packed[3]);
+      }
+      l = l * corr + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
+      if (base + KEYS > kvlen) {  // rows of the last page that hold no token: S has been taken, as values they must not multiply garbage
+        const int from = max(kvlen - base, 0);
+        for (int i = tid; i < (KEYS - from) * 8 * vslabs; i += SOFTMAX_THREADS) {
+          const int row = from + i / (8 * vslabs), c = i % (8 * vslabs);
+          *reinterpret_cast<uint4*>(sK + b * Cfg::STAGE + (c >> 3) * TILE_BYTES + row * 128 + ((c & 7) << 4)) = make_uint4(0, 0, 0, 0);
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // P is read by the tensor cores
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      mbar_arrive(p_ready);  // P is written, the output rescaled and S read
+    }
+    // ---- the finished output, once the last product is done; the row sum is the two halves' sums
+    ok = wait_or_fail(o_done + 8 * ((num_tiles - 1) & 1), ((num_tiles - 1) >> 1) & 1, failed, 22, p.error_flag) && ok;
+    ok = __all_sync(0xffffffffu, ok);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    float* rl = row_max + (num_tiles & 1) * 2 * ROWS;  // not the buffer of the last tile's maxima
+    rl[half * ROWS + r] = l;
+    if (group == 0) asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_THREADS / 2) : "memory");
+    else asm volatile("bar.sync 2, %0;" ::"n"(SOFTMAX_THREADS / 2) : "memory");
+    const int head = head0 + (r - rtok * Gc);
+    const float inv = 1.f / (rl[r] + rl[ROWS + r] + sink_term(rvalid ? sink_of(p.sink_heads, p.sink_log2, head) : -CUDART_INF_F, m_ref * p.scale_log2));
+    const size_t row = (size_t)(q0 + tok0 + rtok) * p.nh + head;
+    for (int c = 0; c < half_cols; c += 32) {
+      uint32_t v[32];
+      if (ok) {
+        tmem_ld32_nowait(my_o + c, v);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      }
+      if (ok && !*failed && rvalid) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 8) {
+          const int col = half * half_cols + c + j;
+          if (col >= p.dv) break;
+          uint4 w;
+          __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&w);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) h2[e] = __floats2bfloat162_rn(__uint_as_float(v[j + 2 * e]) * inv, __uint_as_float(v[j + 2 * e + 1]) * inv);
+          *reinterpret_cast<uint4*>(p.out + row * p.out_row + col) = w;
+        }
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+}
+
+template <int SLABS> int launch_rows(const CUtensorMap& map, const RowParams& p, int num_seqs, int max_q_len, cudaStream_t stream) {
+  using Cfg = RowCfg<SLABS>;
+  static OncePerDevice configured;
+  if (!configured.here()) {
+    cudaError_t e = cudaFuncSetAttribute(paged_prefill_row_kernel<SLABS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
+    if (e != cudaSuccess) return (int)e;
+    configured.here() = true;
+  }
+  const int tiles = (max_q_len + p.tokens_per_tile - 1) / p.tokens_per_tile;
+  if (tiles > 65535 || num_seqs > 65535) return DLI_ERR_UNSUPPORTED;  // the grid's y and z
+  return (int)launch_pdl((paged_prefill_row_kernel<SLABS>), dim3(p.nkv * p.head_chunks, num_seqs, tiles), dim3(THREADS), (size_t)Cfg::SMEM, stream, 1, map, p);
+}
+#endif
+
 }  // namespace
 
 // Sequences [seq0, seq0 + num_seqs) of a batch, each bringing at most max_q_len tokens.
@@ -956,6 +1280,40 @@ DLI_EXPORT int dli_paged_prefill_tc(void* out, const void* q, long long q_stride
   return value_dim <= 64 ? launch_tc2<128, 64>(map_k, map_v, p, num_seqs, max_q_len, stream)
                          : launch_tc2<128, 128>(map_k, map_v, p, num_seqs, max_q_len, stream);
 }
+
+#if !BENT_SCORES
+// One pool whose rows (136 to 256 numbers, a multiple of 8) are keys and, in their first value_dim numbers (a multiple of 8), values; the
+// output's rows have head_dim numbers a head, of which the first value_dim are written.
+DLI_EXPORT int dli_paged_prefill_rows(void* out, const void* q, long long q_stride, const void* pool, long long num_pages, const int* block_tables,
+                                      int max_blocks, const int* q_start, const int* kv_len, int seq0, int num_seqs, int max_q_len, int nh, int nkv,
+                                      int head_dim, int value_dim, int page_size, int window, float scale, float sink, const float* sink_heads,
+                                      cudaStream_t stream) {
+  if (num_seqs == 0) return 0;
+  if (head_dim <= 128 || head_dim > 256 || head_dim % 8 || value_dim < 8 || value_dim > head_dim || value_dim % 8) return DLI_ERR_UNSUPPORTED;
+  if (nkv < 1 || nh % nkv || page_size < 8 || page_size > 128 || (KEYS % page_size) != 0) return DLI_ERR_UNSUPPORTED;
+  if ((((uintptr_t)pool | (uintptr_t)q | (uintptr_t)out) & 15) || q_stride % 8) return DLI_ERR_UNSUPPORTED;
+  if (!error_flag_host) {
+    if (cudaHostAlloc((void**)&error_flag_host, sizeof(int), cudaHostAllocMapped) != cudaSuccess) return (int)cudaGetLastError();
+    *error_flag_host = 0;
+    if (cudaHostGetDevicePointer((void**)&error_flag_device, error_flag_host, 0) != cudaSuccess) return (int)cudaGetLastError();
+  }
+  CUtensorMap map;
+  if (!make_pool_map(&map, pool, num_pages * nkv * page_size, page_size, head_dim)) return DLI_ERR_UNSUPPORTED;
+  RowParams p;
+  p.out = (bf16*)out; p.q = (const bf16*)q; p.q_stride = q_stride; p.block_tables = block_tables; p.max_blocks = max_blocks; p.q_start = q_start;
+  p.kv_len = kv_len; p.seq0 = seq0; p.nh = nh; p.nkv = nkv; p.page_size = page_size; p.window = window;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.sink_log2 = sink * 1.4426950408889634f;
+  p.sink_heads = sink_heads;
+  const int G = nh / nkv;
+  p.heads_per_chunk = G < ROWS ? G : ROWS;
+  p.head_chunks = (G + p.heads_per_chunk - 1) / p.heads_per_chunk;
+  p.tokens_per_tile = ROWS / p.heads_per_chunk;
+  p.d = head_dim; p.dv = value_dim; p.out_row = head_dim;
+  p.error_flag = error_flag_device;
+  return head_dim <= 192 ? launch_rows<3>(map, p, num_seqs, max_q_len, stream) : launch_rows<4>(map, p, num_seqs, max_q_len, stream);
+}
+#endif
 
 
 // ================================================================ single-token sequences, TMA-fed

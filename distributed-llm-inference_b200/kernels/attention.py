@@ -96,12 +96,13 @@ def decode_splits(num_seqs: int, num_heads: int, nkv: int, head_dim: int, page_s
 
 def paged_attention(out: torch.Tensor, qkv: torch.Tensor, cache, batch, num_heads: int, scale: float, window: int | None,
                     splits: int | None = None, sink: float | torch.Tensor | None = None, softcap: float | None = None,
-                    slopes: torch.Tensor | None = None) -> None:
+                    slopes: torch.Tensor | None = None, value_dim: int | None = None) -> None:
     """Attention of every token of the step over its sequence's pages.  ``splits``: key runs per single-token
     sequence, if the caller fixed them (a recorded graph); otherwise chosen from this step's shape.  ``sink``: the
     score of a term that is added to every softmax denominator and carries no value (None: no such term); a float32 tensor
     gives a score per query head.  ``softcap`` c: a score s (after the scale) becomes c tanh(s / c); ``slopes`` (float32, one per
-    query head): then slopes[h] * (position - key position) is taken off (None: neither)."""
+    query head): then slopes[h] * (position - key position) is taken off (None: neither).  ``value_dim``: where keys and values are one pool, how many
+    leading numbers of each head's output the caller reads (a kernel may leave the others as they are)."""
     group = batch.group(cache.group)
     _, nkv, _, d = cache.k.shape
     dv = cache.v.shape[3]  # a value's size may differ from a key's
@@ -126,6 +127,9 @@ def paged_attention(out: torch.Tensor, qkv: torch.Tensor, cache, batch, num_head
     if total > singles and ops.prefill_tc_supported(d, cache.page_size, dv) and _slab_kernels(d, one_pool):
         ops.paged_prefill_tc(out, qkv, cache.k, cache.v, group.block_tables, batch.q_start, batch.kv_len, singles, total - singles,
                              batch.max_q_len, num_heads, scale, window, sink=sink, **bend)
+    elif total > singles and one_pool and not bend and ops.prefill_rows_supported(d, cache.page_size) and (out.data_ptr() | qkv.data_ptr() | cache.k.data_ptr()) % 16 == 0:
+        ops.paged_prefill_rows(out, qkv, cache.k, group.block_tables, batch.q_start, batch.kv_len, singles, total - singles, batch.max_q_len, num_heads, scale,
+                               window, sink=sink, value_dim=value_dim if value_dim and value_dim % 8 == 0 else None)
     elif total > singles:
         ops.paged_attention_mma(out, qkv, cache.k, cache.v, group.block_tables, batch.q_start, batch.kv_len, singles,
                                 total - singles, batch.max_q_len, singles, num_heads, scale, window, sink=sink, **bend)

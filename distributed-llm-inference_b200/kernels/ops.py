@@ -380,6 +380,35 @@ def prefill_tc_supported(head_dim: int, page_size: int, value_dim: int | None = 
     return _tma_rows(head_dim, value_dim) and page_size in (8, 16, 32, 64, 128)
 
 
+def prefill_rows_supported(row: int, page_size: int) -> bool:
+    """Whether portions over one pool of such rows (keys, and values in their leading numbers) have a tcgen05 kernel of their own."""
+    return 128 < row <= 256 and row % 8 == 0 and page_size in (8, 16, 32, 64, 128)
+
+
+def paged_prefill_rows(out: torch.Tensor, q: torch.Tensor, pool: torch.Tensor, block_tables: torch.Tensor, q_start: torch.Tensor, kv_len: torch.Tensor,
+                       seq0: int, num_seqs: int, max_q_len: int, num_heads: int, scale: float, window: int | None = None,
+                       sink: float | torch.Tensor | None = None, value_dim: int | None = None) -> None:
+    """bfloat16 attention for prompt portions over one pool [pages, nkv, page_size, row] whose rows are keys and values, on tcgen05 tensor cores
+    (rows of 136 to 256 numbers).  With ``value_dim`` (a multiple of 8) only that many leading numbers of every head's output are wanted:
+    the others of out [n, nh * row] are left as they are."""
+    for t, name in ((out, "out"), (q, "q"), (pool, "pool")):
+        _need(t, name, torch.bfloat16)
+    _need(block_tables, "block_tables", torch.int32), _need(q_start, "q_start", torch.int32), _need(kv_len, "kv_len", torch.int32)
+    pages, nkv, page_size, row = pool.shape
+    value_dim = row if value_dim is None else value_dim
+    if not prefill_rows_supported(row, page_size):
+        raise KernelError(f"paged_prefill_rows: rows of {row} numbers (136 to 256, multiples of 8) or page size {page_size} (8..128, dividing 128) not supported")
+    if out.shape[1] != num_heads * row or q.shape[0] != out.shape[0] or q.shape[1] < num_heads * row or num_heads % nkv or not 0 < value_dim <= row or value_dim % 8:
+        raise KernelError("paged_prefill_rows: shapes do not agree")
+    if seq0 + num_seqs > kv_len.numel() or q_start.numel() != kv_len.numel() + 1:
+        raise KernelError("paged_prefill_rows: sequence range outside the batch")
+    f = _fn("attention_tc.cu", "dli_paged_prefill_rows", [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p]
+            + [c_int] * 9 + [c_float, c_float, c_void_p, c_void_p])
+    _check(f(_ptr(out), _ptr(q), q.shape[1], _ptr(pool), pages, _ptr(block_tables), block_tables.shape[1], _ptr(q_start), _ptr(kv_len), seq0, num_seqs,
+             max_q_len, num_heads, nkv, row, value_dim, page_size, int(window or 0), scale, _sink(sink), _sink_heads(sink, num_heads), _stream()),
+           "paged_prefill_rows")
+
+
 def paged_prefill_tc(
     out: torch.Tensor,
     qkv: torch.Tensor,

@@ -1,0 +1,85 @@
+"""Portions over one pool of rows that are keys and values (the latent attention's cache) on tcgen05 (csrc/attention_tc.cu: paged_prefill_row_kernel) against
+float64, at the edges of its tiles, slabs and windows, with everything in the pool that no token wrote set to NaN."""
+
+import pytest
+import torch
+
+from dli_b200.kernels import attention, ops
+
+
+def _case(lens, heads, nkv, row, page, seed=0):
+    """lens: (tokens of the step, tokens before them) per sequence; pages scattered over the pool."""
+    g = torch.Generator().manual_seed(seed)
+    blocks = [-(-(q + b) // page) for q, b in lens]
+    order = torch.randperm(sum(blocks) + 2, generator=g).tolist()
+    pool = torch.full((sum(blocks) + 2, nkv, page, row), float("nan"), dtype=torch.bfloat16)
+    tables, rows, at = torch.zeros(len(lens), max(blocks), dtype=torch.int32), [], 0
+    for s, ((q, b), n) in enumerate(zip(lens, blocks)):
+        own = order[at : at + n]
+        at += n
+        tables[s, :n] = torch.tensor(own, dtype=torch.int32)
+        x = torch.randn(q + b, nkv, row, generator=g).bfloat16()
+        rows.append(x)
+        for t in range(q + b):
+            pool[own[t // page], :, t % page] = x[t]
+    n = sum(q for q, _ in lens)
+    q = torch.randn(n, heads * row + 8, generator=g).bfloat16()
+    start = torch.tensor([0, *torch.tensor([q for q, _ in lens]).cumsum(0).tolist()], dtype=torch.int32)
+    return pool, tables, rows, q, start, torch.tensor([a + b for a, b in lens], dtype=torch.int32)
+
+
+def _exact(lens, rows, q, start, heads, nkv, row, dv, scale, window, sink):
+    out = torch.empty(q.shape[0], heads, dv, dtype=torch.float64)
+    for s, (count, before) in enumerate(lens):
+        x = rows[s].double()
+        i, j = torch.arange(before, before + count)[:, None], torch.arange(count + before)[None, :]
+        hidden = (j > i) | ((i - j >= window) if window else torch.zeros_like(j > i))
+        for a in range(heads):
+            k = x[:, a // (heads // nkv)]
+            z = (q[start[s] : start[s + 1], a * row : (a + 1) * row].double() @ k.T) * scale
+            z = z.masked_fill(hidden, float("-inf"))
+            if sink is not None:
+                z = torch.cat([z, torch.full((count, 1), float(sink[a]), dtype=torch.float64)], 1)
+            p = torch.softmax(z, 1)[:, : k.shape[0]]
+            out[start[s] : start[s + 1], a] = p @ k[:, :dv]
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("window,with_sink", [(None, False), (50, False), (200, True)])
+@pytest.mark.parametrize("lens,heads,nkv,row,dv,page", [
+    ([(130, 0)], 16, 1, 256, 192, 16), ([(8, 0), (9, 3), (2, 255)], 16, 1, 256, 256, 8), ([(65, 300)], 3, 1, 192, 128, 64),
+    ([(20, 108), (300, 0)], 32, 2, 136, 72, 128), ([(5, 700)], 130, 1, 200, 8, 32)])
+def test_rows_against_float64(lens, heads, nkv, row, dv, page, window, with_sink):
+    pool, tables, rows, q, start, kv_len = _case(lens, heads, nkv, row, page)
+    scale = row**-0.5
+    sink = torch.randn(heads, generator=torch.Generator().manual_seed(5)) * 2 if with_sink else None
+    want = _exact(lens, rows, q, start, heads, nkv, row, dv, scale, window, sink)
+    n = q.shape[0]
+    out = torch.full((n, heads * row), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.paged_prefill_rows(out, q.cuda(), pool.cuda(), tables.cuda(), start.cuda(), kv_len.cuda(), 0, len(lens), max(c for c, _ in lens), heads, scale, window,
+                           sink=None if sink is None else sink.cuda(), value_dim=dv)
+    got = out.view(n, heads, row).cpu()
+    # probabilities and outputs are rounded to bfloat16 (2^-9 each) on the way, the products' sums are float32
+    assert (got[..., :dv].double() - want).norm() <= 6e-3 * want.norm() and (got[..., :dv].double() - want).abs().max() <= 3e-2 * max(1.0, want.abs().max())
+    written = -(-dv // 8) * 8
+    assert (got[..., written:] == 7.0).all(), "columns that nobody wants were written"
+    assert ops.device_wait_errors() == {}
+
+
+@pytest.mark.gpu
+def test_a_sequence_range_of_a_batch():
+    lens = [(1, 40), (70, 10), (33, 0)]
+    pool, tables, rows, q, start, kv_len = _case(lens, 16, 1, 256, 16, seed=3)
+    want = _exact(lens, rows, q, start, 16, 1, 256, 256, 0.0625, None, None)
+    out = torch.full((q.shape[0], 16 * 256), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.paged_prefill_rows(out, q.cuda(), pool.cuda(), tables.cuda(), start.cuda(), kv_len.cuda(), 1, 2, 70, 16, 0.0625)
+    got = out.view(-1, 16, 256).cpu()
+    assert (got[:1] == 7.0).all() and (got[1:].double() - want[1:]).norm() <= 6e-3 * want[1:].norm()
+
+
+def test_which_rows_have_the_kernel():
+    ok = ops.prefill_rows_supported
+    assert ok(256, 16) and ok(136, 8) and ok(192, 128)
+    assert not ok(128, 16) and not ok(264, 16) and not ok(140, 16) and not ok(256, 4) and not ok(256, 48)
+    assert attention._slab_kernels(64, True) and not attention._slab_kernels(256, True)
