@@ -857,6 +857,370 @@ __global__ void __launch_bounds__(T2Cfg<HD, HV>::THREADS, 1) paged_prefill_tc2_k
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cfg::TMEM) : "memory");
 }
 
+#if !BENT_SCORES
+// ================================================================ differential attention
+// Prompt portions of two maps over shared values (a1 - lambda a2, normed and gated per head; keys of 64 numbers a map, values of up to 128): the
+// kernel with a thread per row and two query tiles, whose tiles are the two maps of the same 128 (token, head) rows.  A tile of keys holds
+// both maps' side by side, so keys, values and their copies are shared; tensor memory holds S and O of both maps (512 columns).  A row's first
+// thread reads both outputs from there at the end.  With a window, the tiles of the kept first tokens come in front of the window's.
+//
+// What bounds it: the softmax threads, as in the kernel it follows (with clocks taken in a CTA, a tile of both maps takes 3,400 clocks: 200 to read a
+// row of scores, 400 its maximum, 1,450 its exponentials in turns, the rest waits; the tensor cores' share is 1,540).  Measured against the
+// mma.sync kernel, 16 heads on 4, values of 128, us: 4,096 tokens 608 -> 150 (689 TFLOP/s), with a window of 1,024 289 -> 110, 1,535 behind 1,024 138 -> 65,
+// 512 tokens 41 -> 19, 128 18.6 -> 15.3, 2 tokens behind 1,000 27.5 -> 24.1.
+struct DiffParams {
+  bf16* out;
+  const bf16* q;
+  long long q_stride;
+  const int *block_tables, *q_start, *kv_len;
+  int max_blocks, seq0, nh, nkv, page_size, window, keep_first;
+  float scale_log2, lambda, post, eps;
+  const bf16* gate;  // [n, nh], gate_stride apart; or null
+  int gate_stride;
+  int tokens_per_tile, heads_per_chunk, head_chunks;
+  int dv;
+  int* error_flag;
+};
+
+constexpr int DIFF_THREADS = 2 * ROWS + 128;
+constexpr int DIFF_SMEM = 14 * TILE_BYTES + 256 + ROWS * 4 + 1024;  // Q x2, K x2 (both maps), V x2 (two slabs), P x2 (two halves), barriers, row sums, alignment
+static_assert(DIFF_SMEM <= 227 * 1024, "one CTA fits an SM");
+
+__global__ void __launch_bounds__(DIFF_THREADS, 1) paged_prefill_diff_kernel(const __grid_constant__ CUtensorMap map_k,
+                                                                             const __grid_constant__ CUtensorMap map_v, const DiffParams p) {
+  constexpr int QT = 2, HV = 128, K_BYTES = 2 * TILE_BYTES, V_BYTES = 2 * TILE_BYTES, D = 64;
+  pdl_launch_dependents();
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* sQ = smem;                     // map 1, map 2
+  unsigned char* sK = sQ + QT * TILE_BYTES;     // two stages of (map 1 | map 2)
+  unsigned char* sV = sK + 2 * K_BYTES;         // two stages
+  unsigned char* sP = sV + 2 * V_BYTES;         // per map (keys 0..63 | keys 64..127)
+  uint64_t* bars = (uint64_t*)(sP + QT * 2 * TILE_BYTES);
+  uint32_t* tmem_slot = (uint32_t*)(bars + 16);
+  volatile int* failed = (volatile int*)(tmem_slot + 1);
+  float* row_sum = (float*)(bars + 32);         // of map 2
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t k_full = smem_u32(bars), v_full = smem_u32(bars + 2), k_free = smem_u32(bars + 4), v_free = smem_u32(bars + 6),
+                 s_done = smem_u32(bars + 8), s_read = smem_u32(bars + 10), p_ready = smem_u32(bars + 12), o_done = smem_u32(bars + 14);
+
+  // the tiles that see the most keys start first
+  const int s = p.seq0 + blockIdx.y;
+  const int tile = gridDim.z - 1 - blockIdx.z;
+  const int kvh = blockIdx.x / p.head_chunks, hc = blockIdx.x - kvh * p.head_chunks;
+  const int q0 = p.q_start[s];
+  const int qlen = p.q_start[s + 1] - q0;
+  const int tpt = p.tokens_per_tile;
+  const int tok0 = tile * tpt;
+  if (tok0 >= qlen) return;  // the whole CTA: nothing was set up yet
+  const int kvlen = p.kv_len[s];
+  const int ntok = min(tpt, qlen - tok0);
+  const int G = p.nh / p.nkv, Gc = p.heads_per_chunk;
+  const int head0 = kvh * G + hc * Gc;
+  const int nheads = min(Gc, G - hc * Gc);
+  const int pos0 = kvlen - qlen + tok0;
+  const int* table = p.block_tables + (size_t)s * p.max_blocks;
+  const int hi = pos0 + ntok;
+  const int lo = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
+  // the tiles of the kept first tokens that lie in front of the window, then the window's
+  const int w_begin = lo / KEYS, t_end = (hi + KEYS - 1) / KEYS;
+  const int kept = p.window > 0 ? min((p.keep_first + KEYS - 1) / KEYS, w_begin) : 0;
+  const int num_tiles = kept + t_end - w_begin;
+
+  if (tid == 0) {
+    for (int i = 0; i < 10; ++i) mbar_init(k_full + 8 * i, (i >= 4 && i < 8) ? QT : 1);  // k_full, v_full, k_free, v_free (one arrival per issuing thread), s_done
+    for (int i = 10; i < 14; ++i) mbar_init(k_full + 8 * i, ROWS);  // s_read, p_ready
+    for (int i = 14; i < 16; ++i) mbar_init(k_full + 8 * i, 1);  // o_done
+    *failed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  pdl_wait();  // queries and the cache are the work of the kernels before this one
+
+  // ---- both Q tiles, swizzled by hand (rows beyond the used ones are zero); the value stages start as zeros
+  for (int idx = tid; idx < QT * ROWS * (D / 8); idx += DIFF_THREADS) {
+    const int rr = idx / (D / 8), c = idx - rr * (D / 8);  // rr: row among those of all tiles; c: 16-byte chunk of the row
+    const int rt = rr & (ROWS - 1), tok = rt / Gc, hd = rt % Gc;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (tok < ntok && hd < nheads)
+      v = *reinterpret_cast<const uint4*>(p.q + (size_t)(q0 + tok0 + tok) * p.q_stride + (size_t)(head0 + hd) * 2 * D + (rr >> 7) * D + c * 8);
+    *reinterpret_cast<uint4*>(sQ + (rr >> 7) * TILE_BYTES + rt * 128 + ((c ^ (rt & 7)) << 4)) = v;
+  }
+  for (int idx = tid; idx < 2 * V_BYTES / 16; idx += DIFF_THREADS) reinterpret_cast<uint4*>(sV)[idx] = make_uint4(0, 0, 0, 0);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem_s = tmem, tmem_o = tmem + QT * KEYS;  // S of each query tile, then O of each
+
+  // The softmax threads hold a row of 128 scores in registers; the third warpgroup needs few and gives its
+  // share away (a scheduler then holds two warps of 224 registers and one of 40).
+  if (warp >= QT * ROWS / 32) {
+    // 384 threads start with 168 registers each; the two softmax warpgroups take 224, which leaves 56 for this one
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+  if (warp == QT * ROWS / 32 + 1 || warp == QT * ROWS / 32 + 3) {
+    // ================================================================ the warps that copy: one the keys, one the values; a page per lane, both its slabs
+    const bool keys = warp == QT * ROWS / 32 + 1;
+    const int pages = KEYS / p.page_size;
+    const int page_i = lane & 15;
+    const uint32_t full = keys ? k_full : v_full, freed = keys ? k_free : v_free;
+    unsigned char* stage0 = keys ? sK : sV;
+    const CUtensorMap* map = keys ? &map_k : &map_v;
+    auto lookup = [&](int t) -> int {
+      const int first = t < num_tiles ? (t < kept ? t : w_begin + t - kept) * KEYS + page_i * p.page_size : 0;
+      const bool need = lane < 16 && t < num_tiles && page_i < pages && first < hi && (first + p.page_size > lo || first < p.keep_first);
+      return need ? table[first / p.page_size] : -1;
+    };
+    int page = lookup(0);
+    for (int t = 0; t < num_tiles && !*failed; ++t) {
+      const int st = t & 1, par = ((t - 2) >> 1) & 1;
+      const int cur = page;
+      page = lookup(t + 1);
+      if (t >= 2) {
+        if (lane == 0) wait_or_fail(freed + 8 * st, par, failed, keys ? 12 : 13, p.error_flag);
+        __syncwarp();
+        if (*failed) break;
+      }
+      const int count = __popc(__ballot_sync(0xffffffffu, cur >= 0));
+      if (lane == 0) mbar_expect_tx(full + 8 * st, (uint32_t)(count * p.page_size * 128 * 2));
+      __syncwarp();
+      if (cur >= 0) {
+#pragma unroll
+        for (int sl = 0; sl < 2; ++sl)
+          tma_load_2d(smem_u32(stage0 + st * K_BYTES + sl * TILE_BYTES + page_i * p.page_size * 128), map, sl * 64, (cur * p.nkv + kvh) * p.page_size, full + 8 * st);
+      }
+    }
+  } else if (warp == QT * ROWS / 32 || warp == QT * ROWS / 32 + 2) {
+    // ================================================================ the warps that issue the matrix products (their first lanes): one per map
+    const int q = warp == QT * ROWS / 32 ? 0 : 1;
+    if (lane == 0) {
+      const uint32_t idesc_s = instr_desc(ROWS, KEYS, 0), idesc_o = instr_desc(ROWS, HV, 1);
+      const uint64_t next_slab = (uint64_t)(TILE_BYTES >> 4) << 16;  // of the MN-major operand: bytes from 64 columns to the next 64
+      const uint32_t qa = smem_u32(sQ + q * TILE_BYTES), pa = smem_u32(sP + q * 2 * TILE_BYTES);
+      auto scores = [&](int t) {  // S_q(t) = Q_q K(t)^T
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t k = smem_u32(sK + (t & 1) * K_BYTES + q * TILE_BYTES);
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk)
+          umma(tmem_s + q * KEYS, smem_desc_sw128(qa + kk * 32), smem_desc_sw128(k + kk * 32), idesc_s, kk != 0);
+        umma_commit(s_done + 8 * q);
+        umma_commit(k_free + 8 * (t & 1));  // this tile's product with K(t) is issued
+      };
+      bool ok = num_tiles > 0 && wait_or_fail(k_full, 0, failed, 17, p.error_flag);
+      if (ok) scores(0);
+      for (int t = 0; t < num_tiles && ok; ++t) {
+        if (t + 1 < num_tiles) {  // the keys are there and the thread of every row has S_q(t) in registers
+          ok = wait_or_fail(k_full + 8 * ((t + 1) & 1), ((t + 1) >> 1) & 1, failed, 17, p.error_flag) && wait_or_fail(s_read + 8 * q, t & 1, failed, 18, p.error_flag);
+          if (!ok) break;
+          scores(t + 1);
+        }
+        // O_q += P_q(t) V(t)
+        ok = wait_or_fail(p_ready + 8 * q, t & 1, failed, 19, p.error_flag) && wait_or_fail(v_full + 8 * (t & 1), (t >> 1) & 1, failed, 20, p.error_flag);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t v = smem_u32(sV + (t & 1) * V_BYTES);
+#pragma unroll
+        for (int k = 0; k < KEYS / 16; ++k)
+          umma(tmem_o + q * HV, smem_desc_sw128(pa + (k >> 2) * TILE_BYTES + (k & 3) * 32), smem_desc_sw128(v + k * 2048) | next_slab, idesc_o, (t | k) != 0);
+        umma_commit(o_done + 8 * q);
+        umma_commit(v_free + 8 * (t & 1));  // this tile's product with V(t) is issued
+      }
+    }
+    __syncwarp();
+  }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    // ================================================================ softmax threads: one per row
+    const int q = warp >> 2;                 // map
+    const int r = tid & (ROWS - 1);          // row of the tile
+    const int rtok = r / Gc;                 // token among the CTA's
+    const bool rvalid = rtok < ntok && (r % Gc) < nheads;
+    const int rpos = pos0 + rtok;
+    const uint32_t lane_bits = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t my_s = tmem_s + q * KEYS + lane_bits, my_o = tmem_o + q * HV + lane_bits;
+    const uint32_t my_s_done = s_done + 8 * q, my_s_read = s_read + 8 * q, my_p_ready = p_ready + 8 * q, my_o_done = o_done + 8 * q;
+    constexpr float RESCALE_STEP = 8.f;
+    float m = -CUDART_INF_F, m_ref = -CUDART_INF_F, l = 0.f;
+    bool ok = true;
+    // chunk 0 of this row's 128-byte slab of P; chunk c lies at the address with c added to bits 4..6 (the swizzle)
+    const uint32_t pchunk = smem_u32(sP) + q * 2 * TILE_BYTES + r * 128 + ((r & 7) << 4);
+    // (what the loop needs of positions is kept in few registers: 356 bytes of spills beside the row of scores took 221 us instead of 150)
+    const int sees_all_from = p.window > 0 ? hi - p.window : 0, sees_all_to = pos0 - KEYS + 1;  // tiles that every row sees whole start in between
+    const int last_whole = kvlen - KEYS;
+    int base = 0;
+    if (q == 1 && num_tiles > 0) asm volatile("bar.arrive 1, %0;" ::"n"(2 * ROWS) : "memory");  // map 1 takes the first turn
+
+    for (int t = 0; t < num_tiles; ++t, base += KEYS) {
+      if (t == kept) base = w_begin * KEYS;
+      ok = wait_or_fail(my_s_done, t & 1, failed, 12, p.error_flag) && ok;
+      ok = __all_sync(0xffffffffu, ok);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // (also after a failed wait: what is read then is never stored, and a second way for the scores to get their
+      // values costs a register move per score on the way that counts: 8,192 tokens took 498 us with it, 455 without)
+      float sc[128];
+#pragma unroll
+      for (int c = 0; c < 128; c += 64) {
+        uint32_t v0[32], v1[32];
+        tmem_ld32_nowait(my_s + c, v0);
+        tmem_ld32_nowait(my_s + c + 32, v1);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 32; ++j) { sc[c + j] = __uint_as_float(v0[j]); sc[c + 32 + j] = __uint_as_float(v1[j]); }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      mbar_arrive(my_s_read);  // S is in registers: the next product of this tile may overwrite it
+      if (base > sees_all_to || base < sees_all_from) {
+        const int hi_j = rpos - base, lo_j = p.window > 0 ? rpos - p.window - base : -1, kept_j = p.window > 0 ? p.keep_first - base : 0;
+#pragma unroll
+        for (int j = 0; j < 128; ++j) sc[j] = (j <= hi_j && (j > lo_j || j < kept_j)) ? sc[j] : -CUDART_INF_F;
+      }
+      float mx[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) mx[j] = max3(sc[j], sc[j + 8], sc[j + 16]);
+#pragma unroll
+      for (int j = 24; j < 120; j += 16)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mx[i] = max3(mx[i], sc[j + i], sc[j + 8 + i]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) mx[i] = fmaxf(mx[i], sc[120 + i]);
+      m = max3(m, max3(mx[0], mx[1], mx[2]), max3(max3(mx[3], mx[4], mx[5]), mx[6], mx[7]));
+      float corr = 1.f;
+      const bool grown = (m - m_ref) * p.scale_log2 > RESCALE_STEP;  // also the first finite maximum (m_ref = -inf)
+      if (grown) {
+        corr = (m_ref == -CUDART_INF_F) ? 0.f : ex2((m_ref - m) * p.scale_log2);
+        m_ref = m;
+      }
+      const float neg = (m_ref == -CUDART_INF_F) ? 0.f : -m_ref * p.scale_log2;
+      // P and O of this tile are free once its product of the key tile before has finished
+      if (t > 0) {
+        ok = wait_or_fail(my_o_done, (t - 1) & 1, failed, 13, p.error_flag) && ok;
+        ok = __all_sync(0xffffffffu, ok);
+        if (__any_sync(0xffffffffu, grown)) {  // the output so far times 2^(old - new) in the rows whose reference moved
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (ok) {
+#pragma unroll
+            for (int c = 0; c < HV; c += 32) {
+              uint32_t v[32];
+              tmem_ld32_nowait(my_o + c, v);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * corr);
+              tmem_st32(my_o + c, v);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          }
+        }
+      }
+      // ---- this group's turn at the exponentials (measured: 562 us at 8,192 tokens with turns, 694 without)
+      {
+        if (q == 0) asm volatile("bar.sync 1, %0;" ::"n"(2 * ROWS) : "memory");
+        else asm volatile("bar.sync 2, %0;" ::"n"(2 * ROWS) : "memory");
+      }
+      // two elements per instruction where there is one for it (fma and add on pairs of float32): the loop is
+      // bound by the number of instructions that one warp gets issued, not by the special-function units alone
+      uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
+      const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), neg2 = pack_f32x2(neg, neg);
+#pragma unroll
+      for (int j = 0; j < 128; j += 8) {
+        uint32_t packed[4];
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) {
+          float x0, x1;
+          unpack_f32x2(fma_f32x2(pack_f32x2(sc[j + e], sc[j + e + 1]), scale2, neg2), x0, x1);
+          const float p0 = ex2(x0), p1 = ex2(x1);  // masked: ex2(-inf) = 0
+          sum2[(e >> 1) & 3] = add_f32x2(sum2[(e >> 1) & 3], pack_f32x2(p0, p1));
+          __nv_bfloat162 b2 = __floats2bfloat162_rn(p0, p1);
+          packed[e >> 1] = *reinterpret_cast<uint32_t*>(&b2);
+        }
+        st_shared_v4((pchunk ^ (((j >> 3) & 7) << 4)) + (j >> 6) * TILE_BYTES, packed[0], packed[1], packed[2], packed[3]);
+      }
+      float sum[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float lo_, hi_;
+        unpack_f32x2(sum2[i], lo_, hi_);
+        sum[i] = lo_ + hi_;
+      }
+      {
+        if (q == 0) asm volatile("bar.arrive 2, %0;" ::"n"(2 * ROWS) : "memory");
+        else if (t + 1 < num_tiles) asm volatile("bar.arrive 1, %0;" ::"n"(2 * ROWS) : "memory");
+      }
+      l = l * corr + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
+      if (base > last_whole) {  // rows of the last page that hold no token must not multiply garbage (either map's threads see to it)
+        ok = wait_or_fail(v_full + 8 * (t & 1), (t >> 1) & 1, failed, 20, p.error_flag) && ok;
+        const int from = max(p.kv_len[s] - base, 0);
+        for (int i = r; i < (KEYS - from) * 16; i += ROWS)
+          *reinterpret_cast<uint4*>(sV + (t & 1) * V_BYTES + ((i >> 3) & 1) * TILE_BYTES + (from + (i >> 4)) * 128 + ((i & 7) << 4)) = make_uint4(0, 0, 0, 0);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // P is read by the tensor cores
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      mbar_arrive(my_p_ready);
+    }
+    // ---- the finished row: map 1's thread reads both maps' outputs from tensor memory (they lie in the same lanes), takes the difference, norms
+    //      the head and applies the gate
+    ok = wait_or_fail(my_o_done, (num_tiles - 1) & 1, failed, 13, p.error_flag) && ok;
+    if (q == 1) {
+      row_sum[r] = l;
+      asm volatile("bar.arrive 3, %0;" ::"n"(2 * ROWS) : "memory");
+    } else {
+      asm volatile("bar.sync 3, %0;" ::"n"(2 * ROWS) : "memory");  // map 2's sums are there and its last product has finished
+      ok = wait_or_fail(o_done + 8, (num_tiles - 1) & 1, failed, 13, p.error_flag) && ok;
+      ok = __all_sync(0xffffffffu, ok);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const float inv1 = 1.f / l, inv2 = p.lambda / row_sum[r];
+      auto read = [&](int c, float (&o)[32]) {  // the difference of 32 columns
+        uint32_t v1[32], v2[32];
+        tmem_ld32_nowait(my_o + c, v1);
+        tmem_ld32_nowait(my_o + HV + c, v2);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 32; ++j) o[j] = fmaf(__uint_as_float(v1[j]), inv1, -__uint_as_float(v2[j]) * inv2);
+      };
+      float ss = 0.f;
+#pragma unroll 1
+      for (int c = 0; c < p.dv; c += 32) {
+        float o[32];
+        read(c, o);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) ss = c + j < p.dv ? fmaf(o[j], o[j], ss) : ss;
+      }
+      const size_t token = q0 + tok0 + rtok;
+      const int head = head0 + (r % Gc);
+      float f = p.post / sqrtf(ss / (float)p.dv + p.eps);
+      if (p.gate && rvalid) f *= 1.f / (1.f + expf(-__bfloat162float(p.gate[token * p.gate_stride + head])));
+#pragma unroll 1
+      for (int c = 0; c < p.dv; c += 32) {
+        float o[32];
+        read(c, o);
+        if (ok && !*failed && rvalid) {
+          uint4* dst = reinterpret_cast<uint4*>(p.out + (token * p.nh + head) * p.dv + c);
+#pragma unroll
+          for (int j = 0; j < 32; j += 8) {
+            if (c + j < p.dv) {
+              uint4 w;
+              __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&w);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) h2[i] = __floats2bfloat162_rn(o[j + 2 * i] * f, o[j + 2 * i + 1] * f);
+              dst[j >> 3] = w;
+            }
+          }
+        }
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+}
+
+#endif
+
 typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1093,7 +1457,7 @@ __global__ void __launch_bounds__(THREADS, 1) paged_prefill_row_kernel(const __g
       const int b = it & 1, base = (t_begin + it) * KEYS;
       ok = wait_or_fail(s_done + 8 * b, (it >> 1) & 1, failed, 24, p.error_flag) && ok;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const bool full = base + KEYS - 1 <= pos0 && base >= lo && p.window <= 0;
+      const bool full = base + KEYS - 1 <= pos0 && (p.window <= 0 || base >= hi - p.window);  // every row sees all of the tile
       float sc[64];
       {
         uint32_t v0[32], v1[32];
@@ -1280,6 +1644,46 @@ DLI_EXPORT int dli_paged_prefill_tc(void* out, const void* q, long long q_stride
   return value_dim <= 64 ? launch_tc2<128, 64>(map_k, map_v, p, num_seqs, max_q_len, stream)
                          : launch_tc2<128, 128>(map_k, map_v, p, num_seqs, max_q_len, stream);
 }
+
+#if !BENT_SCORES
+// Differential attention of sequences [seq0, seq0 + num_seqs): k_pool [pages, nkv, page_size, 128] (two maps of 64), v_pool [.., value_dim].
+DLI_EXPORT int dli_paged_prefill_diff(void* out, const void* q, long long q_stride, const void* k_pool, const void* v_pool, long long num_pages,
+                                      const int* block_tables, int max_blocks, const int* q_start, const int* kv_len, int seq0, int num_seqs,
+                                      int max_q_len, const void* gate, int gate_stride, int nh, int nkv, int value_dim, int page_size, int window,
+                                      int keep_first, float scale, float lambda, float post, float eps, cudaStream_t stream) {
+  if (num_seqs == 0) return 0;
+  if (value_dim < 8 || value_dim > 128 || value_dim % 8 || nkv < 1 || nh % nkv || page_size < 8 || page_size > 128 || (KEYS % page_size) != 0) return DLI_ERR_UNSUPPORTED;
+  if ((((uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)q | (uintptr_t)out) & 15) || q_stride % 8) return DLI_ERR_UNSUPPORTED;
+  if (!error_flag_host) {
+    if (cudaHostAlloc((void**)&error_flag_host, sizeof(int), cudaHostAllocMapped) != cudaSuccess) return (int)cudaGetLastError();
+    *error_flag_host = 0;
+    if (cudaHostGetDevicePointer((void**)&error_flag_device, error_flag_host, 0) != cudaSuccess) return (int)cudaGetLastError();
+  }
+  static OncePerDevice configured;
+  if (!configured.here()) {
+    cudaError_t e = cudaFuncSetAttribute(paged_prefill_diff_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DIFF_SMEM);
+    if (e != cudaSuccess) return (int)e;
+    configured.here() = true;
+  }
+  CUtensorMap map_k, map_v;
+  const long long rows = num_pages * nkv * page_size;
+  if (!make_pool_map(&map_k, k_pool, rows, page_size, 128) || !make_pool_map(&map_v, v_pool, rows, page_size, value_dim)) return DLI_ERR_UNSUPPORTED;
+  DiffParams p;
+  p.out = (bf16*)out; p.q = (const bf16*)q; p.q_stride = q_stride; p.block_tables = block_tables; p.max_blocks = max_blocks; p.q_start = q_start;
+  p.kv_len = kv_len; p.seq0 = seq0; p.nh = nh; p.nkv = nkv; p.page_size = page_size; p.window = window; p.keep_first = keep_first;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.lambda = lambda; p.post = post; p.eps = eps; p.gate = (const bf16*)gate; p.gate_stride = gate_stride;
+  const int G = nh / nkv;
+  p.heads_per_chunk = G < ROWS ? G : ROWS;
+  p.head_chunks = (G + p.heads_per_chunk - 1) / p.heads_per_chunk;
+  p.tokens_per_tile = ROWS / p.heads_per_chunk;
+  p.dv = value_dim;
+  p.error_flag = error_flag_device;
+  const int tiles = (max_q_len + p.tokens_per_tile - 1) / p.tokens_per_tile;
+  if (tiles > 65535 || num_seqs > 65535) return DLI_ERR_UNSUPPORTED;  // the grid's y and z
+  return (int)launch_pdl(paged_prefill_diff_kernel, dim3(nkv * p.head_chunks, num_seqs, tiles), dim3(DIFF_THREADS), (size_t)DIFF_SMEM, stream, 1, map_k, map_v, p);
+}
+#endif
 
 #if !BENT_SCORES
 // One pool whose rows (136 to 256 numbers, a multiple of 8) are keys and, in their first value_dim numbers (a multiple of 8), values; the

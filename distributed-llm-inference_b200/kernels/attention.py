@@ -138,20 +138,28 @@ def paged_attention(out: torch.Tensor, qkv: torch.Tensor, cache, batch, num_head
 def diff_attention(out: torch.Tensor, q: torch.Tensor, cache, batch, gate: torch.Tensor | None, num_heads: int, scale: float,
                    window: int | None, keep_first: int, lam: float, post: float, eps: float) -> None:
     """Differential attention of every token of the step over its sequence's pages (``ops.diff_attention_simt`` says what is
-    computed).  bfloat16 with sizes that are multiples of 16: the tensor-core kernel, one launch for portions and single
-    tokens; float32 and any other size: the CUDA-core kernel."""
+    computed).  bfloat16 with sizes that are multiples of 16: portions of maps of 64 go to a tcgen05 kernel, everything else to the mma.sync
+    kernel (portions and single tokens in one launch); float32 and any other size: the CUDA-core kernel."""
     group = batch.group(cache.group)
     if out.dtype == torch.bfloat16 and ops.diff_attention_tc_supported(cache.k.shape[3] // 2, cache.v.shape[3]):
+        _, nkv, _, d2 = cache.k.shape
+        vdim, singles, seqs, longest, seen = cache.v.shape[3], batch.num_single, batch.num_seqs, batch.max_q_len, batch.max_kv_len
+        if (seqs > singles and ops.prefill_diff_supported(d2 // 2, vdim, cache.page_size)
+                and (out.data_ptr() | q.data_ptr() | cache.k.data_ptr() | cache.v.data_ptr()) % 16 == 0):
+            ops.paged_prefill_diff(out, q, cache.k, cache.v, group.block_tables, batch.q_start, batch.kv_len, singles, seqs - singles, longest, gate, num_heads,
+                                   scale, window, keep_first, lam, post, eps)
+            if not singles:
+                return
+            seqs, longest, seen = singles, 1, batch.max_kv_len_single
         splits, scratch = 1, None
-        if batch.max_q_len == 1 and out.is_cuda:  # few single tokens: their key tiles are divided between CTAs to fill the GPU
-            nkv, vdim = cache.k.shape[1], cache.v.shape[3]
-            seen = min(batch.max_kv_len, window + keep_first + 64) if window else batch.max_kv_len
-            wave = one_wave(ops.diff_attention_tc_ctas_per_sm(cache.k.shape[3] // 2, vdim))
-            splits = choose_splits(batch.num_seqs, nkv * -(-(num_heads // nkv) // 64), seen, wave, fill_last_wave=False, min_tiles=1)
+        if longest == 1 and out.is_cuda:  # few single tokens: their key tiles are divided between CTAs to fill the GPU
+            seen = min(seen, window + keep_first + 64) if window else seen
+            wave = one_wave(ops.diff_attention_tc_ctas_per_sm(d2 // 2, vdim))
+            splits = choose_splits(seqs, nkv * -(-(num_heads // nkv) // 64), seen, wave, fill_last_wave=False, min_tiles=1)
             if splits > 1:
-                scratch = torch.empty(ops.diff_attention_scratch(batch.num_seqs, num_heads, vdim, splits), dtype=torch.float32, device=out.device)
-        ops.diff_attention_tc(out, q, cache.k, cache.v, group.block_tables, batch.q_start, batch.kv_len, batch.num_seqs, batch.max_q_len, gate,
-                              num_heads, scale, window, keep_first, lam, post, eps, splits, scratch)
+                scratch = torch.empty(ops.diff_attention_scratch(seqs, num_heads, vdim, splits), dtype=torch.float32, device=out.device)
+        ops.diff_attention_tc(out, q, cache.k, cache.v, group.block_tables, batch.q_start, batch.kv_len, seqs, longest, gate, num_heads, scale, window,
+                              keep_first, lam, post, eps, splits, scratch)
         return
     ops.diff_attention_simt(out, q, cache.k, cache.v, group.block_tables, batch.seq_of_token, batch.positions, gate, num_heads, scale,
                             window, keep_first, lam, post, eps)

@@ -1,0 +1,89 @@
+"""Portions of differential attention on tcgen05 (csrc/attention_tc.cu: paged_prefill_diff_kernel) against float64, at the edges of its tiles and
+windows, with everything in the pools that no token wrote set to NaN; and beside single tokens, which another kernel serves."""
+
+import pytest
+import torch
+
+from dli_b200.cache.pools import LayerCache
+from dli_b200.engine.batch import GroupView, StepBatch
+from dli_b200.kernels import attention, ops
+
+
+def _case(lens, heads, nkv, dv, page, seed=0):
+    g = torch.Generator().manual_seed(seed)
+    blocks = [-(-(q + b) // page) for q, b in lens]
+    order = torch.randperm(sum(blocks) + 2, generator=g).tolist()
+    k = torch.full((sum(blocks) + 2, nkv, page, 128), float("nan"), dtype=torch.bfloat16)
+    v = torch.full((sum(blocks) + 2, nkv, page, dv), float("nan"), dtype=torch.bfloat16)
+    tables, rows, at = torch.zeros(len(lens), max(blocks), dtype=torch.int32), [], 0
+    for s, ((q, b), n) in enumerate(zip(lens, blocks)):
+        own = order[at : at + n]
+        at += n
+        tables[s, :n] = torch.tensor(own, dtype=torch.int32)
+        x, y = torch.randn(q + b, nkv, 128, generator=g).bfloat16(), torch.randn(q + b, nkv, dv, generator=g).bfloat16()
+        rows.append((x, y))
+        for t in range(q + b):
+            k[own[t // page], :, t % page], v[own[t // page], :, t % page] = x[t], y[t]
+    n = sum(q for q, _ in lens)
+    q, gate = torch.randn(n, heads * 128, generator=g).bfloat16(), torch.randn(n, heads + 3, generator=g).bfloat16()
+    start = torch.tensor([0, *torch.tensor([q for q, _ in lens]).cumsum(0).tolist()], dtype=torch.int32)
+    return k, v, tables, rows, q, gate, start, torch.tensor([a + b for a, b in lens], dtype=torch.int32)
+
+
+def _exact(lens, rows, q, gate, start, heads, nkv, dv, scale, window, keep, lam, post, eps):
+    out = torch.empty(q.shape[0], heads, dv, dtype=torch.float64)
+    for s, (count, before) in enumerate(lens):
+        i, j = torch.arange(before, before + count)[:, None], torch.arange(count + before)[None, :]
+        hidden = j > i
+        if window:
+            hidden |= (i - j >= window) & (j >= keep)
+        for a in range(heads):
+            x, y = (t[:, a // (heads // nkv)].double() for t in rows[s])
+            maps = []
+            for m in range(2):
+                c = a * 128 + m * 64
+                z = (q[start[s] : start[s + 1], c : c + 64].double() @ x[:, m * 64 : m * 64 + 64].T) * scale
+                maps.append(torch.softmax(z.masked_fill(hidden, float("-inf")), 1) @ y)
+            o = maps[0] - lam * maps[1]
+            o = o / torch.sqrt((o * o).mean(1, keepdim=True) + eps) * post
+            out[start[s] : start[s + 1], a] = o * (torch.sigmoid(gate[start[s] : start[s + 1], a : a + 1].double()) if gate is not None else 1.0)
+    return out.view(q.shape[0], -1)
+
+
+def _near(got, want):
+    # probabilities are rounded to bfloat16 (2^-9), the difference of the two maps and the head's norm enlarge that by what cancels, the output is rounded once more
+    assert (got.double() - want).norm() <= 1e-2 * want.norm() and (got.double() - want).abs().max() <= 5e-2 * max(1.0, want.abs().max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("window,keep,gated", [(None, 0, True), (50, 16, False), (130, 5, True), (300, 200, True), (64, 0, True)])
+@pytest.mark.parametrize("lens,heads,nkv,dv,page", [
+    ([(300, 0)], 4, 1, 128, 16), ([(2, 0), (33, 500), (65, 127)], 16, 4, 128, 8), ([(130, 260)], 3, 1, 80, 128), ([(40, 700)], 130, 1, 24, 32)])
+def test_portions_against_float64(lens, heads, nkv, dv, page, window, keep, gated):
+    k, v, tables, rows, q, gate, start, kv_len = _case(lens, heads, nkv, dv, page)
+    want = _exact(lens, rows, q, gate if gated else None, start, heads, nkv, dv, 0.125, window, keep, 0.7, 0.3, 1e-6)
+    out = torch.full((q.shape[0], heads * dv), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.paged_prefill_diff(out, q.cuda(), k.cuda(), v.cuda(), tables.cuda(), start.cuda(), kv_len.cuda(), 0, len(lens), max(c for c, _ in lens),
+                           gate.cuda()[:, :heads] if gated else None, heads, 0.125, window, keep, 0.7, 0.3, 1e-6)
+    _near(out.cpu(), want)
+    assert ops.device_wait_errors() == {}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("window,keep", [(None, 0), (100, 16)])
+def test_portions_beside_single_tokens(window, keep):
+    lens, heads, nkv, dv = [(1, 0), (1, 300), (1, 40), (150, 20), (31, 0)], 8, 2, 128
+    k, v, tables, rows, q, gate, start, kv_len = _case(lens, heads, nkv, dv, 16, seed=4)
+    want = _exact(lens, rows, q, gate, start, heads, nkv, dv, 0.125, window, keep, 0.7, 0.3, 1e-6)
+    n = q.shape[0]
+    batch = StepBatch(n=n, num_seqs=5, num_single=3, token_ids=None, positions=None, seq_of_token=None, q_start=start.cuda(), kv_len=kv_len.cuda(), state_slot=None,
+                      logit_rows=None, groups=[GroupView(tables.cuda(), None)], max_q_len=150, max_kv_len=301, max_kv_len_single=301)
+    out = torch.full((n, heads * dv), float("nan"), dtype=torch.bfloat16, device="cuda")
+    attention.diff_attention(out, q.cuda(), LayerCache(0, k.cuda(), v.cuda(), 16), batch, gate.cuda()[:, :heads], heads, 0.125, window, keep, 0.7, 0.3, 1e-6)
+    _near(out.cpu(), want)
+
+
+def test_which_sizes_have_the_kernel():
+    ok = ops.prefill_diff_supported
+    assert ok(64, 128, 16) and ok(64, 24, 8) and ok(64, 64, 128)
+    assert not ok(128, 128, 16) and not ok(64, 136, 16) and not ok(64, 20, 16) and not ok(64, 128, 4) and not ok(48, 96, 16)
