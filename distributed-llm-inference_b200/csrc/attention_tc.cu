@@ -712,16 +712,14 @@ __global__ void __launch_bounds__(T2Cfg<HD, HV>::THREADS, 1) paged_prefill_tc2_k
 #if BENT_SCORES
     const float slope = rvalid ? bend_slope(p.bend, head0 + (r % Gc)) : 0.f;
 #endif
-    // where this row's eight 16-byte chunks of a 128-byte slab of P lie (the swizzle), as shared-memory addresses: a
-    // store then needs no address arithmetic of its own (through a generic pointer each cost five instructions more;
-    // 8,192 tokens: 455 -> 436 us)
-    uint32_t pchunk[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) pchunk[c] = smem_u32(sP) + q * 2 * TILE_BYTES + r * 128 + ((c ^ (r & 7)) << 4);
+    // where chunk 0 of this row's 128-byte slab of P lies, as a shared-memory address; chunk c lies at the address with c added to bits
+    // 4..6 (the swizzle).  A store then needs one instruction of address arithmetic (through a generic pointer each cost five more)
+    const uint32_t pchunk = smem_u32(sP) + q * 2 * TILE_BYTES + r * 128 + ((r & 7) << 4);
+    const int sees_all_from = p.window > 0 ? hi - p.window : 0, sees_all_to = first_pos - KEYS + 1;  // tiles that every row sees whole start in between
+    int base = t_begin * KEYS;
     if (QT == 2 && q == 1 && num_tiles > 0) asm volatile("bar.arrive 1, %0;" ::"n"(2 * ROWS) : "memory");  // tile A takes the first turn
 
-    for (int t = 0; t < num_tiles; ++t) {
-      const int base = (t_begin + t) * KEYS;
+    for (int t = 0; t < num_tiles; ++t, base += KEYS) {
       ok = wait_or_fail(my_s_done, t & 1, failed, 12, p.error_flag) && ok;
       ok = __all_sync(0xffffffffu, ok);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -742,9 +740,7 @@ __global__ void __launch_bounds__(T2Cfg<HD, HV>::THREADS, 1) paged_prefill_tc2_k
 #if BENT_SCORES
       bend_row(sc, p.bend, slope, rpos - base);
 #endif
-      // a tile that lies wholly at or before the first row's position, inside every row's window, needs no mask
-      const bool full = base + KEYS - 1 <= first_pos && base >= lo && p.window <= 0;
-      if (!full) {
+      if (base > sees_all_to || base < sees_all_from) {
         const int hi_j = rpos - base, lo_j = p.window > 0 ? rpos - p.window - base : -1;
 #pragma unroll
         for (int j = 0; j < 128; ++j) sc[j] = (j <= hi_j && j > lo_j) ? sc[j] : -CUDART_INF_F;
@@ -807,7 +803,7 @@ __global__ void __launch_bounds__(T2Cfg<HD, HV>::THREADS, 1) paged_prefill_tc2_k
           __nv_bfloat162 b2 = __floats2bfloat162_rn(p0, p1);
           packed[e >> 1] = *reinterpret_cast<uint32_t*>(&b2);
         }
-        st_shared_v4(pchunk[(j >> 3) & 7] + (j >> 6) * TILE_BYTES, packed[0], packed[1], packed[2], packed[3]);
+        st_shared_v4((pchunk ^ (((j >> 3) & 7) << 4)) + (j >> 6) * TILE_BYTES, packed[0], packed[1], packed[2], packed[3]);
       }
       float sum[4];
 #pragma unroll
@@ -1449,9 +1445,7 @@ __global__ void __launch_bounds__(THREADS, 1) paged_prefill_row_kernel(const __g
     bool ok = true;
     const int group = r >> 6;
     const uint32_t my_o = tmem_o + lane_bits + half * half_cols;
-    uint32_t pchunk[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) pchunk[c] = smem_u32(sP) + half * TILE_BYTES + r * 128 + ((c ^ (r & 7)) << 4);
+    const uint32_t pchunk = smem_u32(sP) + half * TILE_BYTES + r * 128 + ((r & 7) << 4);  // chunk c: with c added to bits 4..6
 
     for (int it = 0; it < num_tiles; ++it) {
       const int b = it & 1, base = (t_begin + it) * KEYS;
@@ -1525,7 +1519,7 @@ __global__ void __launch_bounds__(THREADS, 1) paged_prefill_row_kernel(const __g
           __nv_bfloat162 b2 = __floats2bfloat162_rn(sc[j + e], sc[j + e + 1]);
           packed[e >> 1] = *reinterpret_cast<uint32_t*>(&b2);
         }
-        st_shared_v4(pchunk[j >> 3], packed[0], packed[1], packed[2], packed[3]);
+        st_shared_v4(pchunk ^ ((j >> 3) << 4), packed[0], packed[1], packed[2], packed[3]);
       }
       l = l * corr + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
       if (base + KEYS > kvlen) {  // rows of the last page that hold no token: S has been taken, as values they must not multiply garbage
