@@ -413,8 +413,66 @@ __global__ void gated_group_rmsnorm_kernel(T* __restrict__ out, const float* __r
   }
 }
 
+// Parts of up to 1,024 numbers (size % 8 == 0, aligned rows): LANES lanes share a part of a token, each with CHUNKS runs of eight columns in
+// registers between the sum and the output; a warp holds 32 / LANES parts, a CTA four warps, and nothing waits at a block's barrier.
+// What bounds it: memory and the exponentials' and divisions' instructions, about alike.  A CTA a part (a warp of which half the lanes
+// were idle at heads of 128, two barriers) took, us, L2 flushed: 4,096 tokens of 16 parts of 128 74 -> 23 (2,900 GB/s), 3,001 of 8 parts of 512 33 -> 31, 501 of
+// 16 parts of 64 in float32 13 -> 8.
+constexpr int NORM_WARPS = 4;
+template <typename T, int LANES, int CHUNKS>
+__global__ void __launch_bounds__(NORM_WARPS * 32) gated_part_rmsnorm_kernel(T* __restrict__ out, const float* __restrict__ y, const T* __restrict__ u,
+                                                                             long long u_stride, int z_col, const float* __restrict__ w,
+                                                                             const float* __restrict__ divisor, long long units, int inner, int parts, float eps,
+                                                                             int gate_after) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & (LANES - 1);
+  const long long unit = ((long long)blockIdx.x * NORM_WARPS * 32 + threadIdx.x) / LANES;  // token * parts + part
+  const bool live = unit < units;
+  const long long t = live ? unit / parts : 0;
+  const int part = live ? (int)(unit - t * parts) : 0, size = inner / parts, c0 = part * size;
+  const float* yrow = y + (size_t)t * inner + c0;
+  const T* zrow = u + (size_t)t * u_stride + z_col + c0;
+  float gv[CHUNKS][8], z[CHUNKS][8];
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c) {
+    const int col = (lane + c * LANES) * 8;
+    if (live && col < size) {
+      load8(yrow + col, gv[c]);
+      load8(zrow + col, z[c]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) gv[c][k] = z[c][k] = 0.f;
+    }
+  }
+  const float f = divisor && live ? 1.f / divisor[unit] : 1.f;  // every number of the part, before anything else
+  float q = 0.f;
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float v = gv[c][k] * f, g = v * norm_gate(z[c][k], gate_after);  // the gate is a factor of the output either way
+      q = gate_after ? fmaf(v, v, q) : fmaf(g, g, q);
+      gv[c][k] = g;
+    }
+#pragma unroll
+  for (int o = LANES / 2; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+  const float r = 1.f / sqrtf(q / (float)size + eps);
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c) {
+    const int col = (lane + c * LANES) * 8;
+    if (live && col < size) {
+      float wv[8], o[8];
+      load8(w + c0 + col, wv);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) o[k] = gv[c][k] * r * wv[k];
+      store8(out + (size_t)t * inner + c0 + col, o);
+    }
+  }
+}
+
 // The same with the part's values in registers between the two passes and 16- and 32-byte accesses: a thread owns
-// CHUNKS runs of eight columns (size % 8 == 0, size <= 8 * THREADS * CHUNKS, aligned rows).
+// CHUNKS runs of eight columns (1,024 < size <= 8 * THREADS * CHUNKS, size % 8 == 0, aligned rows).
 template <typename T, int THREADS, int CHUNKS>
 __global__ void __launch_bounds__(THREADS) gated_group_rmsnorm_vec_kernel(T* __restrict__ out, const float* __restrict__ y,
                                                                           const T* __restrict__ u, long long u_stride, int z_col,
@@ -610,10 +668,17 @@ DLI_EXPORT int dli_gated_group_rmsnorm(void* out, const float* y, const void* u,
 #define DLI_GN_VEC(T, THREADS, CHUNKS)                                                                                               \
   return (int)launch_pdl((gated_group_rmsnorm_vec_kernel<T, THREADS, CHUNKS>), grid, dim3(THREADS), 0, stream, 1, (T*)out, y, (const T*)u, \
                          u_stride, z_col, w, divisor, inner, parts, eps, gate_after)
+#define DLI_GN_PART(T, LANES, CHUNKS)                                                                                                \
+  return (int)launch_pdl((gated_part_rmsnorm_kernel<T, LANES, CHUNKS>), dim3((unsigned)((units * LANES + NORM_WARPS * 32 - 1) / (NORM_WARPS * 32))), \
+                         dim3(NORM_WARPS * 32), 0, stream, 1, (T*)out, y, (const T*)u, u_stride, z_col, w, divisor, units, inner, parts, eps, gate_after)
+    const long long units = (long long)n * parts;
 #define DLI_GN_SIZES(T)                       \
-  if (size <= 256) DLI_GN_VEC(T, 32, 1);      \
-  if (size <= 512) DLI_GN_VEC(T, 64, 1);      \
-  if (size <= 1024) DLI_GN_VEC(T, 128, 1);    \
+  if (size <= 32) DLI_GN_PART(T, 4, 1);       \
+  if (size <= 64) DLI_GN_PART(T, 8, 1);       \
+  if (size <= 128) DLI_GN_PART(T, 16, 1);     \
+  if (size <= 256) DLI_GN_PART(T, 32, 1);     \
+  if (size <= 512) DLI_GN_PART(T, 32, 2);     \
+  if (size <= 1024) DLI_GN_PART(T, 32, 4);    \
   if (size <= 2048) DLI_GN_VEC(T, 256, 1);    \
   if (size <= 4096) DLI_GN_VEC(T, 256, 2);    \
   DLI_GN_VEC(T, 256, 4)
@@ -624,6 +689,7 @@ DLI_EXPORT int dli_gated_group_rmsnorm(void* out, const float* y, const void* u,
     }
 #undef DLI_GN_SIZES
 #undef DLI_GN_VEC
+#undef DLI_GN_PART
   }
   const int threads = size >= 1024 ? 256 : 128;
   if (dtype == DLI_F32)
