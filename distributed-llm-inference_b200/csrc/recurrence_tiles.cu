@@ -17,7 +17,7 @@
 // What bounds it, and what it measured.  (1) takes a CTA an SM (228 KB) about 49,000 cycles a tile and head of 128 (some 85,000 warp instructions at 0.45
 // a cycle and scheduler: exponentials and norms of the inputs 10,000 to 17,000 cycles, the diagonal blocks 6,000, products of decays 6,000 to 8,000,
 // the inverse 5,500, W and U 8,500); (2) 3.7 us a tile, by mma.sync (318 a tile and warp) and its operands' arrival (157 KB by bulk copies; with a
-// cp.async per 16 bytes, 6.5 us).  Against the kernels that walk, us: decay per head, 16 heads of 128, one prompt of 2,048 tokens 771 -> 202; decay per channel,
+// cp.async per 16 bytes, 6.5 us).  Against the kernels that walk, us: decay per head in bfloat16 (kernels of its own, below), 16 heads of 128, one prompt of 2,048 tokens 772 -> 135; decay per channel,
 // prompts of 1,400 and 2,100 1,052 -> 354, 32 heads and 2,048 1,031 -> 382; bonus, 16 heads of 64, float32, prompts of 200 and 301 109 -> 30, 4,096 1,336 -> 214.
 // Errors against 64 bits are the walks' or smaller (decay per channel, 2,048 tokens: o 4.9e-7 and S 5.0e-7, walked 5.4e-7 and 5.4e-7).
 #include "common.cuh"
@@ -82,6 +82,67 @@ __device__ __forceinline__ void mma6(float (&large)[4], float (&small)[4], const
 }
 // bytes of pair c of row r of a 16 x 16 block
 __device__ __forceinline__ int block_at(int r, int c) { return r * 32 + (((c >> 2) ^ ((r >> 2) & 1)) * 16) + (c & 3) * 4; }
+
+// A lower triangular 64 x 64 matrix, value(row, column), in three terms, block by block.
+template <int THREADS, typename F> __device__ __forceinline__ void split_blocks(F&& value, unsigned char* dst, int tid) {
+  for (int e = tid; e < 10 * 128; e += THREADS) {
+    const int b = e >> 7, r = (e >> 3) & 15, pr = e & 7;
+    const int rb = b < 1 ? 0 : (b < 3 ? 1 : (b < 6 ? 2 : 3)), cb = b - rb * (rb + 1) / 2;
+    const int row = rb * 16 + r, col = cb * 16 + pr * 2;
+    uint32_t t[3];
+    dli::split3(value(row, col), value(row, col + 1), t[0], t[1], t[2]);
+#pragma unroll
+    for (int s = 0; s < 3; ++s) *reinterpret_cast<uint32_t*>(dst + s * Q_TERM + b * Q_TILE + block_at(r, pr)) = t[s];
+  }
+}
+
+// T = (I + A)^-1 for a strictly lower triangular A (rows of F_ROW floats; what lies on and above the diagonal is not read), by all threads of a
+// CTA of at least 256, with barriers: the blocks on the diagonal a column a lane, the others block by block away from it,
+// T_ba = -T_bb sum_{a <= e < b} A_be T_ea (the sum is kept above the diagonal meanwhile).
+__device__ __forceinline__ void invert_unit_lower(const float* sA, float* sT, int tid) {
+  const int warp = tid >> 5, lane = tid & 31;
+  if (warp < 4) {
+    const int b0 = warp * 16;
+    if (lane < 16) {
+      float x[16];
+#pragma unroll
+      for (int t = 0; t < 16; ++t) {
+        float s = t == lane ? 1.f : 0.f;
+#pragma unroll
+        for (int j = 0; j < t; ++j) s = fmaf(-sA[(b0 + t) * F_ROW + b0 + j], x[j], s);
+        x[t] = s;
+      }
+#pragma unroll
+      for (int t = 0; t < 16; ++t) sT[(b0 + t) * F_ROW + b0 + lane] = x[t];
+    }
+  }
+  __syncthreads();
+  for (int away = 1; away < 4; ++away) {  // a thread takes four columns of a row
+    const int a = tid >> 6, b = a + away, r = (tid >> 2) & 15, cc = (tid & 3) * 4;
+    if (b < 4) {
+      float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+      for (int j = a * 16; j < b * 16; ++j) {
+        const float x = sA[(b * 16 + r) * F_ROW + j];
+        const float4 y = *reinterpret_cast<const float4*>(sT + j * F_ROW + a * 16 + cc);
+        s[0] = fmaf(x, y.x, s[0]); s[1] = fmaf(x, y.y, s[1]); s[2] = fmaf(x, y.z, s[2]); s[3] = fmaf(x, y.w, s[3]);
+      }
+      *reinterpret_cast<float4*>(sT + (a * 16 + r) * F_ROW + b * 16 + cc) = make_float4(s[0], s[1], s[2], s[3]);
+    }
+    __syncthreads();
+    if (b < 4) {
+      float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float x = sT[(b * 16 + r) * F_ROW + b * 16 + j];
+        const float4 y = *reinterpret_cast<const float4*>(sT + (a * 16 + j) * F_ROW + b * 16 + cc);
+        s[0] = fmaf(x, y.x, s[0]); s[1] = fmaf(x, y.y, s[1]); s[2] = fmaf(x, y.z, s[2]); s[3] = fmaf(x, y.w, s[3]);
+      }
+      *reinterpret_cast<float4*>(sT + (b * 16 + r) * F_ROW + a * 16 + cc) = make_float4(-s[0], -s[1], -s[2], -s[3]);
+    }
+    __syncthreads();
+  }
+}
 
 // ---------------------------------------------------------------- (1) what does not depend on the state
 
@@ -415,17 +476,6 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
   __syncthreads();
 
   // ---- Q leaves in three terms, block by block
-  auto split_blocks = [&](auto&& value, unsigned char* dst) {  // value(row, column) of a lower triangular 64 x 64 matrix
-    for (int e = tid; e < 10 * 128; e += Z::THREADS) {
-      const int b = e >> 7, r = (e >> 3) & 15, pr = e & 7;
-      const int rb = b < 1 ? 0 : (b < 3 ? 1 : (b < 6 ? 2 : 3)), cb = b - rb * (rb + 1) / 2;
-      const int row = rb * 16 + r, col = cb * 16 + pr * 2;
-      uint32_t t[3];
-      dli::split3(value(row, col), value(row, col + 1), t[0], t[1], t[2]);
-#pragma unroll
-      for (int s = 0; s < 3; ++s) *reinterpret_cast<uint32_t*>(dst + s * Q_TERM + b * Q_TILE + block_at(r, pr)) = t[s];
-    }
-  };
   float vv[DELTA ? ROWS : 1][4];  // this warp's rows of V, requested ahead of what comes in between
   if constexpr (DELTA) {
 #pragma unroll
@@ -436,7 +486,7 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
       for (int m = 0; m < 4; ++m) vv[e][m] = r < len && lane + 32 * m < dv ? to_float(v[lane + 32 * m]) : 0.f;
     }
   }
-  split_blocks([&](int r, int cc) { return *reinterpret_cast<const float*>(sQm + r * F_ROW + cc); }, left + L::Q);
+  split_blocks<Z::THREADS>([&](int r, int cc) { return sQm[r * F_ROW + cc]; }, left + L::Q, tid);
   if constexpr (DELTA) {
     // ---- P o K and V as operands, in the place of the blocks' operands
     unsigned char* sKg = smem;
@@ -461,50 +511,8 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
         }
       }
     }
-    // ---- (I + A)^-1: the blocks on the diagonal a column a lane, the others block by block away from it,
-    // T_ba = -T_bb sum_{a <= e < b} A_be T_ea (the sum is kept above the diagonal meanwhile)
-    if (warp < 4) {
-      const int b0 = warp * 16;
-      if (lane < 16) {
-        float x[16];
-#pragma unroll
-        for (int t = 0; t < 16; ++t) {
-          float s = t == lane ? 1.f : 0.f;
-#pragma unroll
-          for (int j = 0; j < t; ++j) s = fmaf(-sA[(b0 + t) * F_ROW + b0 + j], x[j], s);
-          x[t] = s;
-        }
-#pragma unroll
-        for (int t = 0; t < 16; ++t) sT[(b0 + t) * F_ROW + b0 + lane] = x[t];
-      }
-    }
-    __syncthreads();
-    for (int away = 1; away < 4; ++away) {  // a thread takes four columns of a row
-      const int a = tid >> 6, b = a + away, r = (tid >> 2) & 15, cc = (tid & 3) * 4;
-      if (b < 4) {
-        float s[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-        for (int j = a * 16; j < b * 16; ++j) {
-          const float x = sA[(b * 16 + r) * F_ROW + j];
-          const float4 y = *reinterpret_cast<const float4*>(sT + j * F_ROW + a * 16 + cc);
-          s[0] = fmaf(x, y.x, s[0]); s[1] = fmaf(x, y.y, s[1]); s[2] = fmaf(x, y.z, s[2]); s[3] = fmaf(x, y.w, s[3]);
-        }
-        *reinterpret_cast<float4*>(sT + (a * 16 + r) * F_ROW + b * 16 + cc) = make_float4(s[0], s[1], s[2], s[3]);
-      }
-      __syncthreads();
-      if (b < 4) {
-        float s[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const float x = sT[(b * 16 + r) * F_ROW + b * 16 + j];
-          const float4 y = *reinterpret_cast<const float4*>(sT + (a * 16 + j) * F_ROW + b * 16 + cc);
-          s[0] = fmaf(x, y.x, s[0]); s[1] = fmaf(x, y.y, s[1]); s[2] = fmaf(x, y.z, s[2]); s[3] = fmaf(x, y.w, s[3]);
-        }
-        *reinterpret_cast<float4*>(sT + (b * 16 + r) * F_ROW + a * 16 + cc) = make_float4(-s[0], -s[1], -s[2], -s[3]);
-      }
-      __syncthreads();
-    }
-    split_blocks([&](int r, int cc) { return cc <= r ? sT[r * F_ROW + cc] * sBeta[cc] : 0.f; }, sTt);
+    invert_unit_lower(sA, sT, tid);
+    split_blocks<Z::THREADS>([&](int r, int cc) { return cc <= r ? sT[r * F_ROW + cc] * sBeta[cc] : 0.f; }, sTt, tid);
     __syncthreads();
     // ---- W = T (P o K) and U = T V: a warp takes sixteen columns and two of the four blocks of rows (0 and 3, or 1 and 2)
     unsigned char* sW = sV + Z::V_TERMS * Z::V_TERM;
@@ -817,6 +825,462 @@ __global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const Params p) 
   each([&](float& x, bool in, size_t at) { if (in) S0[at] = x; });
 }
 
+// ---------------------------------------------------------------- a decay per head, bfloat16
+// Here queries and keys are bfloat16 numbers times a float32 factor of their token (the unit vector's, the decays'), so they go into products as they
+// came, in one term, and the factors move to the other operand's rows or to the sums: A and Q are plain products of bfloat16 rows times
+// factors, W = T diag(P fk) K, (P fq) o (Q S0), S = P_last S + ((P_last / P) fk o w)^T K.  222 mma.sync a tile and warp instead of 318, 87 KB of operands
+// instead of 157, and no operand is split in the first kernel but T and Q.  Decays between two tokens are powers of differences of sums of
+// logarithms, the sums in double and kept as two floats.  Measured against the general kernels, 16 heads of 128, one prompt of 2,048 tokens: 202 -> 135 us (300
+// tokens 36, 64 tokens 25; 32 heads 233); errors against 64 bits o 1.8e-7 and S 1.3e-7 (the tiles of sixteen tokens on the CUDA cores 3.2e-7 and 3.5e-7).
+template <int KD> struct HeadLeft {
+  static constexpr int TERM = Left<KD>::TERM, MATRIX = Left<KD>::MATRIX;
+  static constexpr int FACTORS = 576;  // bytes: P fq [64] | (P_last / P) fk [64] | P_last, rounded up
+  static constexpr int W = 0, QB = MATRIX, KB = QB + TERM, Q = KB + TERM, F = Q + 3 * Q_TERM, U = F + FACTORS;
+  __host__ __device__ static size_t bytes(int dv, int cols) { return (size_t)U + (size_t)((dv + cols - 1) / cols) * TOKENS * (cols + 4) * 4; }
+};
+
+template <int KD> struct HeadPrep {
+  static constexpr int THREADS = 256, WARPS = 8;
+  static constexpr int ROW = Left<KD>::ROW, TERM = Left<KD>::TERM, V_ROW = 128 * 2 + 16, SQUARE = TOKENS * F_ROW * 4;
+  static constexpr int SECOND = TERM > TOKENS * V_ROW ? TERM : TOKENS * V_ROW;  // queries, then values
+  static constexpr int AT_Q = TERM, AT_A = AT_Q + SECOND, AT_QM = AT_A + SQUARE, AT_T = AT_QM + SQUARE, AT_TT = AT_T + SQUARE, AT_F = AT_TT + 3 * Q_TERM,
+                       SMEM = AT_F + 8 * TOKENS * 4;
+  static_assert(3 * Q_TERM <= SQUARE && 2 * (SMEM + 1024) <= 227 * 1024, "two CTAs an SM");
+};
+
+template <int KD>
+__global__ void __launch_bounds__(256, 2) head_prep_kernel(const Params p, int vec) {
+  pdl_launch_dependents();
+  pdl_wait();
+  using Z = HeadPrep<KD>;
+  using L = HeadLeft<KD>;
+  extern __shared__ __align__(128) unsigned char smem[];
+  unsigned char* sK = smem;
+  unsigned char* sQ = smem + Z::AT_Q;
+  float* sA = reinterpret_cast<float*>(smem + Z::AT_A);
+  float* sQm = reinterpret_cast<float*>(smem + Z::AT_QM);
+  float* sT = reinterpret_cast<float*>(smem + Z::AT_T);
+  unsigned char* sTt = smem + Z::AT_TT;       // T diag(beta), in three terms
+  unsigned char* sTk = smem + Z::AT_QM;       // T diag(beta P fk), in the place of Q
+  float* fk = reinterpret_cast<float*>(smem + Z::AT_F);  // per token: factor of the key, of the query, beta, sums of log decays (two terms), P, P_last / P, a scratch
+  float *fq = fk + TOKENS, *beta = fq + TOKENS, *lh = beta + TOKENS, *lm = lh + TOKENS, *up = lm + TOKENS, *behind = up + TOKENS, *raw = behind + TOKENS;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, head = blockIdx.y, place = blockIdx.x;
+  int seq = -1;
+  for (int s0 = 0; s0 < p.num_seqs; s0 += Z::THREADS) {
+    const int s = s0 + tid;
+    seq += __syncthreads_count(s < p.num_seqs && first_tile(p.q_start[s < p.num_seqs ? s : 0], s) <= place);
+  }
+  if (seq < 0) return;
+  const int first = p.q_start[seq] + (place - first_tile(p.q_start[seq], seq)) * TOKENS, len = min(TOKENS, p.q_start[seq + 1] - first);
+  if (len <= 0) return;
+  const int d = p.d, dv = p.dv, kqh = head / (p.heads / p.kq), dvp = padded_columns(dv), width = 2 * p.kq * d + p.heads * dv;
+  unsigned char* left = p.left + ((size_t)place * p.heads + head) * L::bytes(dv, p.cols);
+  float* left_u = reinterpret_cast<float*>(left + L::U);
+  float* left_f = reinterpret_cast<float*>(left + L::F);
+  const bf16* rows = (const bf16*)p.qkv + (size_t)first * width;
+  const bf16* u = (const bf16*)p.u + (size_t)first * p.u_stride + head;
+
+  auto load_rows = [&](unsigned char* dst, const bf16* src, int size, int row, int columns) {  // 64 rows of `columns` numbers, zeros where there is nothing
+    if (vec) {
+      const int runs = columns >> 3;
+      for (int e = tid; e < TOKENS * runs; e += Z::THREADS) {
+        const int r = e / runs, c = e - r * runs;
+        const bool ok = r < len && c * 8 < size;
+        cp_async16(smem_u32(dst + r * row + c * 16), ok ? src + (size_t)r * width + c * 8 : src, ok ? 16 : 0);
+      }
+    } else {
+      for (int e = tid; e < TOKENS * columns; e += Z::THREADS) {
+        const int r = e / columns, c = e - r * columns;
+        *reinterpret_cast<bf16*>(dst + r * row + c * 2) = r < len && c < size ? src[(size_t)r * width + c] : __float2bfloat16_rn(0.f);
+      }
+    }
+    cp_async_commit();
+  };
+  load_rows(sQ, rows + kqh * d, d, Z::ROW, KD);
+  load_rows(sK, rows + (p.kq + kqh) * d, d, Z::ROW, KD);
+  if (tid < TOKENS) {
+    const bool ok = tid < len;
+    beta[tid] = ok ? 1.f / (1.f + expf(-to_float(u[(size_t)(ok ? tid : 0) * p.u_stride + p.b_col]))) : 0.f;
+    raw[tid] = ok ? -expf(p.a_log[head]) * softplus(to_float(u[(size_t)(ok ? tid : 0) * p.u_stride + p.a_col]) + p.dt_bias[head]) : 0.f;
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+
+  // ---- the tokens' factors: four threads a row for the unit vectors, a warp for the sums of log decays
+  {
+    const int r = tid >> 2, part = tid & 3;
+    float sq = 0.f, sk = 0.f;
+#pragma unroll
+    for (int c = 0; c < KD / 8; c += 4) {
+      float q[8], k[8];
+      load8(reinterpret_cast<const bf16*>(sQ + r * Z::ROW + (c + part) * 16), q);
+      load8(reinterpret_cast<const bf16*>(sK + r * Z::ROW + (c + part) * 16), k);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { sq = fmaf(q[i], q[i], sq); sk = fmaf(k[i], k[i], sk); }
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) { sq += __shfl_xor_sync(0xffffffffu, sq, o); sk += __shfl_xor_sync(0xffffffffu, sk, o); }
+    if (part == 0) {
+      fk[r] = r < len ? 1.f / sqrtf(sk + p.unit_eps) : 0.f;
+      fq[r] = r < len ? (1.f / sqrtf((float)d)) / sqrtf(sq + p.unit_eps) : 0.f;
+    }
+  }
+  if (warp == 0) {
+    double l[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) l[k] = (double)fmaxf(raw[2 * lane + k], -1e4f);  // (a decay below that is 0, and its sums stay finite)
+    l[1] += l[0];
+    double incl = l[1];
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const double other = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += other;
+    }
+    const double before = incl - l[1], end = __shfl_sync(0xffffffffu, incl, 31);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const double lt = before + l[k], l2 = lt * 1.4426950408889634074;
+      const float hi = (float)l2;
+      lh[2 * lane + k] = hi;
+      lm[2 * lane + k] = (float)(l2 - (double)hi);
+      up[2 * lane + k] = expf((float)lt);
+      behind[2 * lane + k] = expf((float)(end - lt));
+    }
+    if (lane == 0) left_f[2 * TOKENS] = expf((float)end);
+  }
+  for (int e = tid; e < TOKENS * (KD / 8); e += Z::THREADS) {  // queries and keys as the second kernel wants them
+    const int at = e / (KD / 8) * Z::ROW + e % (KD / 8) * 16;
+    *reinterpret_cast<uint4*>(left + L::QB + at) = *reinterpret_cast<const uint4*>(sQ + at);
+    *reinterpret_cast<uint4*>(left + L::KB + at) = *reinterpret_cast<const uint4*>(sK + at);
+  }
+  __syncthreads();
+  if (tid < TOKENS) {
+    left_f[tid] = up[tid] * fq[tid];
+    left_f[TOKENS + tid] = behind[tid] * fk[tid];
+  }
+
+  // ---- A and Q: a warp takes sixteen rows of one of them
+  const int kcol = (lane & 3) * 2;
+  {
+    const int is_q = warp >> 2, mt = warp & 3;
+    if (mt * 16 < len) {
+      float sum[2][8][4];  // the two halves of k apart: an mma.sync addition cuts off, a plain one rounds
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sum[0][j][e] = sum[1][j][e] = 0.f;
+      const uint32_t a_addr = smem_u32(is_q ? sQ : sK) + (mt * 16 + (lane & 15)) * Z::ROW + (lane >> 4) * 16;
+      const uint32_t b_addr = smem_u32(sK) + ((lane & 7) + (lane >> 4) * 8) * Z::ROW + ((lane >> 3) & 1) * 16;
+#pragma unroll
+      for (int k16 = 0; k16 < KD / 16; ++k16) {
+        uint32_t a[4];
+        ldsm_x4(a, a_addr + k16 * 32);
+#pragma unroll
+        for (int jp = 0; jp < 4; ++jp)
+          if (jp <= mt) {
+            uint32_t b[4];
+            ldsm_x4(b, b_addr + jp * 16 * Z::ROW + k16 * 32);
+            mma16816(sum[k16 & 1][2 * jp], a, b[0], b[1]);
+            mma16816(sum[k16 & 1][2 * jp + 1], a, b[2], b[3]);
+          }
+      }
+      float* dst = is_q ? sQm : sA;
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        const int r = mt * 16 + (lane >> 2) + hf * 8;
+        const float h = lh[r], m = lm[r], f = is_q ? fq[r] : fk[r] * beta[r];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (j < 2 * (mt + 1)) {
+            const int col = j * 8 + kcol;
+            const float2 ch = *reinterpret_cast<const float2*>(lh + col), cm = *reinterpret_cast<const float2*>(lm + col), cf = *reinterpret_cast<const float2*>(fk + col);
+            const float x = (sum[0][j][2 * hf] + sum[1][j][2 * hf]) * f * cf.x * ex2((h - ch.x) + (m - cm.x));
+            const float y = (sum[0][j][2 * hf + 1] + sum[1][j][2 * hf + 1]) * f * cf.y * ex2((h - ch.y) + (m - cm.y));
+            *reinterpret_cast<float2*>(dst + r * F_ROW + col) = make_float2(col <= r ? x : 0.f, col + 1 <= r ? y : 0.f);
+          }
+      }
+    } else {
+      float* dst = is_q ? sQm : sA;
+      for (int e = lane; e < 16 * (mt + 1) * 16; e += 32) dst[(mt * 16 + e / ((mt + 1) * 16)) * F_ROW + e % ((mt + 1) * 16)] = 0.f;
+    }
+  }
+  __syncthreads();
+  load_rows(sQ, rows + 2 * p.kq * d + head * dv, dv, Z::V_ROW, dvp);  // the values, in the queries' place
+  split_blocks<Z::THREADS>([&](int r, int c) { return c <= r ? sQm[r * F_ROW + c] : 0.f; }, left + L::Q, tid);
+  invert_unit_lower(sA, sT, tid);
+  split_blocks<Z::THREADS>([&](int r, int c) { return c <= r ? sT[r * F_ROW + c] * beta[c] : 0.f; }, sTt, tid);
+  split_blocks<Z::THREADS>([&](int r, int c) { return c <= r ? sT[r * F_ROW + c] * (beta[c] * up[c] * fk[c]) : 0.f; }, sTk, tid);
+  cp_async_wait<0>();
+  __syncthreads();
+
+  // ---- W = T diag(beta P fk) K and U = T diag(beta) V: a warp takes sixteen columns and two of the four blocks of rows (0 and 3, or 1 and 2)
+  const int w_tasks = KD / 16 * 2, tasks = w_tasks + dvp / 16 * 2;
+  auto columns16 = [&](auto mt0_, auto mt1_, bool is_w, int col0) {
+    constexpr int mts[2] = {decltype(mt0_)::value, decltype(mt1_)::value};
+    const int row = is_w ? Z::ROW : Z::V_ROW;
+    const uint32_t b_addr = smem_u32(is_w ? sK : sQ) + (uint32_t)(((lane & 7) + ((lane >> 3) & 1) * 8) * row) + (col0 + (lane >> 4) * 8) * 2;
+    const uint32_t t_addr = smem_u32(is_w ? sTk : sTt) + (lane & 15) * 32 + ((lane >> 4) ^ ((lane >> 2) & 1)) * 16;
+    float large[2][2][4], small[2][2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) large[i][0][e] = large[i][1][e] = small[i][0][e] = small[i][1][e] = 0.f;
+#pragma unroll
+    for (int k16 = 0; k16 <= mts[1]; ++k16) {
+      uint32_t b[4];
+      ldsm_x4_trans(b, b_addr + k16 * 16 * row);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (k16 <= mts[i]) {
+#pragma unroll
+          for (int s = 2; s >= 0; --s) {
+            uint32_t a[4];
+            ldsm_x4(a, t_addr + s * Q_TERM + (mts[i] * (mts[i] + 1) / 2 + k16) * Q_TILE);
+            mma16816(s ? small[i][0] : large[i][0], a, b[0], b[1]);
+            mma16816(s ? small[i][1] : large[i][1], a, b[2], b[3]);
+          }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          const int r = mts[i] * 16 + (lane >> 2) + hf * 8, col = col0 + nt * 8 + kcol;
+          const float x = large[i][nt][2 * hf] + small[i][nt][2 * hf], y = large[i][nt][2 * hf + 1] + small[i][nt][2 * hf + 1];
+          if (is_w) {
+            uint32_t t[3];
+            dli::split3(x, y, t[0], t[1], t[2]);
+#pragma unroll
+            for (int s = 0; s < 3; ++s) *reinterpret_cast<uint32_t*>(left + L::W + s * Z::TERM + r * Z::ROW + col * 2) = t[s];
+          } else if (col < (dv + p.cols - 1) / p.cols * p.cols) {
+            *reinterpret_cast<float2*>(left_u + (col / p.cols) * TOKENS * (p.cols + 4) + r * (p.cols + 4) + col % p.cols) = make_float2(x, y);
+          }
+        }
+  };
+  for (int task = warp; task < tasks; task += Z::WARPS) {
+    const bool is_w = task < w_tasks;
+    const int col0 = (is_w ? task : task - w_tasks) / 2 * 16;
+    if (task & 1) columns16(std::integral_constant<int, 1>(), std::integral_constant<int, 2>(), is_w, col0);
+    else columns16(std::integral_constant<int, 0>(), std::integral_constant<int, 3>(), is_w, col0);
+  }
+}
+
+template <int KD, int COLS> struct HeadWalk {
+  static constexpr int THREADS = COLS * 8;  // warps as in the walk above
+  static constexpr int ROW = Left<KD>::ROW, TERM = Left<KD>::TERM, MATRIX = Left<KD>::MATRIX;
+  static constexpr int S_TERM = COLS * ROW, W_ROW = COLS * 2 + 16, W_TERM = TOKENS * W_ROW, U_ROW = COLS + 4, U_BYTES = TOKENS * U_ROW * 4;
+  static constexpr int BEFORE = MATRIX + TERM, BEHIND = TERM + 3 * Q_TERM + HeadLeft<KD>::FACTORS;  // bytes: W and Q rows; K rows, Q, factors
+  static constexpr int AT_W = 0, AT_QB = MATRIX, AT_KB = BEFORE, AT_Q = AT_KB + TERM, AT_F = AT_Q + 3 * Q_TERM, AT_U = AT_F + HeadLeft<KD>::FACTORS,
+                       AT_S = AT_U + U_BYTES, AT_w = AT_S + 3 * S_TERM, AT_BAR = AT_w + 6 * W_TERM, SMEM = AT_BAR + 32;
+  static_assert(SMEM <= 227 * 1024, "shared memory");
+};
+
+template <int KD, int COLS>
+__global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const Params p) {
+  pdl_launch_dependents();
+  pdl_wait();
+  using Z = HeadWalk<KD, COLS>;
+  using L = HeadLeft<KD>;
+  constexpr int SLICE = KD / 4, NT = SLICE / 8;
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int seq = p.num_seqs - 1 - blockIdx.z, head = blockIdx.y, col0 = blockIdx.x * COLS;
+  const int first = p.q_start[seq], last = p.q_start[seq + 1];
+  if (last <= first) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, mt = warp & 3, half = warp >> 2;
+  const int d = p.d, dv = p.dv, inner = p.heads * dv;
+  const size_t bytes = L::bytes(dv, COLS);
+  const unsigned char* left = p.left + ((size_t)first_tile(first, seq) * p.heads + head) * bytes;
+  const float* sU = reinterpret_cast<const float*>(smem + Z::AT_U);
+  const float* sF = reinterpret_cast<const float*>(smem + Z::AT_F);
+  const uint32_t bar_before = smem_u32(smem + Z::AT_BAR), bar_behind = bar_before + 8;
+  volatile int* failed = reinterpret_cast<volatile int*>(smem + Z::AT_BAR + 16);
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_before));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_behind));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    *failed = 0;
+  }
+  __syncthreads();
+  auto load_before = [&](const unsigned char* src) {
+    if (tid == 0) {
+      expect_bytes(bar_before, Z::BEFORE + Z::U_BYTES);
+      bulk_load(smem_u32(smem + Z::AT_W), src + L::W, Z::BEFORE, bar_before);
+      bulk_load(smem_u32(smem + Z::AT_U), src + L::U + (size_t)blockIdx.x * Z::U_BYTES, Z::U_BYTES, bar_before);
+    }
+  };
+  auto load_behind = [&](const unsigned char* src) {
+    if (tid == 0) {
+      expect_bytes(bar_behind, Z::BEHIND);
+      bulk_load(smem_u32(smem + Z::AT_KB), src + L::KB, Z::BEHIND, bar_behind);
+    }
+  };
+  load_before(left);
+
+  // ---- S: rows = value columns of this warp's half, columns = its quarter of the channels
+  const int kcol = (lane & 3) * 2, c_lo = half * 16 + (lane >> 2), slice0 = mt * SLICE;
+  float S[NT][4];
+  float* S0 = p.state + ((size_t)p.state_slot[seq] * p.heads + head) * dv * d;
+  auto each = [&](auto&& fn) {
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int col = col0 + c_lo + (e >> 1) * 8, i = slice0 + j * 8 + kcol + (e & 1);
+        fn(S[j][e], col < dv && i < d, (size_t)col * d + i);
+      }
+  };
+  each([&](float& x, bool in, size_t at) { x = in ? S0[at] : 0.f; });
+
+  const uint32_t row_a = (mt * 16 + (lane & 15)) * Z::ROW + (lane >> 4) * 16;
+  const uint32_t w_addr = smem_u32(smem + Z::AT_W) + row_a, qb_addr = smem_u32(smem + Z::AT_QB) + row_a;
+  const uint32_t s_addr = smem_u32(smem + Z::AT_S) + (half * 16 + (lane & 7) + (lane >> 4) * 8) * Z::ROW + ((lane >> 3) & 1) * 16;
+  const uint32_t q_addr = smem_u32(smem + Z::AT_Q) + (lane & 15) * 32 + ((lane >> 4) ^ ((lane >> 2) & 1)) * 16;
+  const uint32_t wb_addr = smem_u32(smem + Z::AT_w) + ((lane & 7) + ((lane >> 3) & 1) * 8) * Z::W_ROW + (half * 16 + (lane >> 4) * 8) * 2;
+  const uint32_t wa_addr = smem_u32(smem + Z::AT_w) + 3 * Z::W_TERM + ((lane & 7) + (lane >> 4) * 8) * Z::W_ROW + (half * 16 + ((lane >> 3) & 1) * 8) * 2;  // with the factors
+  const uint32_t kb_addr = smem_u32(smem + Z::AT_KB) + ((lane & 7) + ((lane >> 3) & 1) * 8) * Z::ROW + (slice0 + (lane >> 4) * 8) * 2;
+
+  uint32_t parity = 0;
+  for (int base = first; base < last; base += TOKENS, parity ^= 1) {
+    const int len = min(TOKENS, last - base);
+    const bool active = mt * 16 < len;
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        uint32_t t[3];
+        dli::split3(S[j][2 * hf], S[j][2 * hf + 1], t[0], t[1], t[2]);
+#pragma unroll
+        for (int s = 0; s < 3; ++s)
+          *reinterpret_cast<uint32_t*>(smem + Z::AT_S + s * Z::S_TERM + (c_lo + hf * 8) * Z::ROW + (slice0 + j * 8 + kcol) * 2) = t[s];
+      }
+    __syncthreads();  // S0 is there; the operands behind (of the tile before) have been read
+    load_behind(left);
+    wait_copies(bar_before, parity, failed, p.error_flag);
+    float O[2][4], w[2][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) O[0][e] = O[1][e] = w[0][e] = w[1][e] = 0.f;
+    if (active) {
+      float yl[2][2][4], ys[2][4], ol[2][2][4], os[2][4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        yl[0][0][e] = yl[0][1][e] = yl[1][0][e] = yl[1][1][e] = ys[0][e] = ys[1][e] = 0.f;
+        ol[0][0][e] = ol[0][1][e] = ol[1][0][e] = ol[1][1][e] = os[0][e] = os[1][e] = 0.f;
+      }
+#pragma unroll
+      for (int k16 = 0; k16 < KD / 16; ++k16) {
+        uint32_t b[3][4], a[3][4], q[4];
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+          ldsm_x4(b[s], s_addr + s * Z::S_TERM + k16 * 32);
+          ldsm_x4(a[s], w_addr + s * Z::TERM + k16 * 32);
+        }
+        ldsm_x4(q, qb_addr + k16 * 32);
+        mma6(yl[k16 & 1][0], ys[0], a, b[0][0], b[0][1], b[1][0], b[1][1], b[2][0], b[2][1]);
+        mma6(yl[k16 & 1][1], ys[1], a, b[0][2], b[0][3], b[1][2], b[1][3], b[2][2], b[2][3]);
+#pragma unroll
+        for (int s = 2; s >= 0; --s) {
+          mma16816(s ? os[0] : ol[k16 & 1][0], q, b[s][0], b[s][1]);
+          mma16816(s ? os[1] : ol[k16 & 1][1], q, b[s][2], b[s][3]);
+        }
+      }
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          O[nt][e] = (os[nt][e] + ol[1][nt][e]) + ol[0][nt][e];
+          w[nt][e] = sU[(mt * 16 + (lane >> 2) + (e >> 1) * 8) * Z::U_ROW + half * 16 + nt * 8 + kcol + (e & 1)] - ((ys[nt][e] + yl[1][nt][e]) + yl[0][nt][e]);
+        }
+      }
+    }
+    wait_copies(bar_behind, parity, failed, p.error_flag);
+    if (active) {
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          const int r = mt * 16 + (lane >> 2) + hf * 8, col = half * 16 + nt * 8 + kcol;
+          const float f = sF[TOKENS + r];
+          uint32_t t[3], g[3];
+          dli::split3(w[nt][2 * hf], w[nt][2 * hf + 1], t[0], t[1], t[2]);
+          dli::split3(w[nt][2 * hf] * f, w[nt][2 * hf + 1] * f, g[0], g[1], g[2]);
+#pragma unroll
+          for (int s = 0; s < 3; ++s) {
+            *reinterpret_cast<uint32_t*>(smem + Z::AT_w + s * Z::W_TERM + r * Z::W_ROW + col * 2) = t[s];
+            *reinterpret_cast<uint32_t*>(smem + Z::AT_w + (3 + s) * Z::W_TERM + r * Z::W_ROW + col * 2) = g[s];
+          }
+        }
+    }
+    __syncthreads();  // w is there; S0 and the operands in front have been read
+    left += (size_t)p.heads * bytes;
+    if (base + TOKENS < last) load_before(left);
+    // ---- the read-outs
+    if (active) {
+      float ql[2][4], qs[2][4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) ql[0][e] = ql[1][e] = qs[0][e] = qs[1][e] = 0.f;
+      for (int k16 = 0; k16 <= mt; ++k16) {
+        uint32_t a[3][4], b[3][4];
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+          ldsm_x4(a[s], q_addr + s * Q_TERM + (mt * (mt + 1) / 2 + k16) * Q_TILE);
+          ldsm_x4_trans(b[s], wb_addr + s * Z::W_TERM + k16 * 16 * Z::W_ROW);
+        }
+        mma6(ql[0], qs[0], a, b[0][0], b[0][1], b[1][0], b[1][1], b[2][0], b[2][1]);
+        mma6(ql[1], qs[1], a, b[0][2], b[0][3], b[1][2], b[1][3], b[2][2], b[2][3]);
+      }
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          const int r = mt * 16 + (lane >> 2) + hf * 8, col = col0 + half * 16 + nt * 8 + kcol;
+          if (r < len) {
+            const float f = sF[r];
+            float* dst = p.o + (size_t)(base + r) * inner + (size_t)head * dv + col;
+            const float x = fmaf(f, O[nt][2 * hf], qs[nt][2 * hf] + ql[nt][2 * hf]), y = fmaf(f, O[nt][2 * hf + 1], qs[nt][2 * hf + 1] + ql[nt][2 * hf + 1]);
+            if ((dv & 1) == 0) {
+              if (col < dv) *reinterpret_cast<float2*>(dst) = make_float2(x, y);
+            } else {
+              if (col < dv) dst[0] = x;
+              if (col + 1 < dv) dst[1] = y;
+            }
+          }
+        }
+    }
+    // ---- the state at the tile's end
+    float dl[NT][4], ds[NT][4];
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) dl[j][e] = ds[j][e] = 0.f;
+#pragma unroll
+    for (int k16 = 0; k16 < TOKENS / 16; ++k16) {
+      if (k16 * 16 < len) {
+        uint32_t a[3][4];
+#pragma unroll
+        for (int s = 0; s < 3; ++s) ldsm_x4_trans(a[s], wa_addr + s * Z::W_TERM + k16 * 16 * Z::W_ROW);
+#pragma unroll
+        for (int jp = 0; jp < NT / 2; ++jp) {
+          uint32_t b[4];
+          ldsm_x4_trans(b, kb_addr + k16 * 16 * Z::ROW + jp * 32);
+#pragma unroll
+          for (int s = 2; s >= 0; --s) {
+            mma16816(s ? ds[2 * jp] : dl[2 * jp], a[s], b[0], b[1]);
+            mma16816(s ? ds[2 * jp + 1] : dl[2 * jp + 1], a[s], b[2], b[3]);
+          }
+        }
+      }
+    }
+    const float g = sF[2 * TOKENS];
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) S[j][e] = fmaf(g, S[j][e], ds[j][e] + dl[j][e]);
+  }
+  each([&](float& x, bool in, size_t at) { if (in) S0[at] = x; });
+}
+
 template <typename K> cudaError_t allow(K kernel, int smem, OncePerDevice& done) {
   if (done.here()) return cudaSuccess;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -849,11 +1313,32 @@ template <typename T, int MODE, int KD> int launch(const Params& p, cudaStream_t
   if (e == cudaSuccess) e = p.cols == 16 ? launch_walk<KD, 16, MODE != BONUS>(p, stream) : launch_walk<KD, 32, MODE != BONUS>(p, stream);
   return (int)e;
 }
+template <int KD, int COLS> cudaError_t launch_head_walk(const Params& p, cudaStream_t stream) {
+  using Z = HeadWalk<KD, COLS>;
+  static OncePerDevice done;
+  const cudaError_t e = allow(head_walk_kernel<KD, COLS>, Z::SMEM, done);
+  if (e != cudaSuccess) return e;
+  return launch_pdl((head_walk_kernel<KD, COLS>), dim3((p.dv + COLS - 1) / COLS, p.heads, p.num_seqs), dim3(Z::THREADS), (size_t)Z::SMEM, stream, 1, p);
+}
+template <int KD> int launch_head(const Params& p, cudaStream_t stream) {
+  using Z = HeadPrep<KD>;
+  static OncePerDevice done;
+  cudaError_t e = allow(head_prep_kernel<KD>, Z::SMEM, done);
+  const int width = 2 * p.kq * p.d + p.heads * p.dv, vec = width % 8 == 0 && p.d % 8 == 0 && p.dv % 8 == 0 && ((uintptr_t)p.qkv & 15) == 0;  // 16-byte runs
+  if (e == cudaSuccess) e = launch_pdl((head_prep_kernel<KD>), dim3(places(p.n, p.num_seqs), p.heads), dim3(Z::THREADS), (size_t)Z::SMEM, stream, 1, p, vec);
+  if (e == cudaSuccess) e = p.cols == 16 ? launch_head_walk<KD, 16>(p, stream) : launch_head_walk<KD, 32>(p, stream);
+  return (int)e;
+}
+
 template <typename T, int MODE> int launch_sized(const Params& p, cudaStream_t stream) {
   return p.d <= 64 ? launch<T, MODE, 64>(p, stream) : launch<T, MODE, 128>(p, stream);
 }
 template <typename T> int launch_mode(int mode, const Params& p, cudaStream_t stream) {
-  if (mode == HEAD_DELTA) return launch_sized<T, HEAD_DELTA>(p, stream);
+  if constexpr (sizeof(T) == 2) {
+    if (mode == HEAD_DELTA) return p.d <= 64 ? launch_head<64>(p, stream) : launch_head<128>(p, stream);
+  } else {
+    if (mode == HEAD_DELTA) return launch_sized<T, HEAD_DELTA>(p, stream);
+  }
   if (mode == CHANNEL_DELTA) return launch_sized<T, CHANNEL_DELTA>(p, stream);
   return launch_sized<T, BONUS>(p, stream);
 }

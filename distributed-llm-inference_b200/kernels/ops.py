@@ -1379,7 +1379,7 @@ def recurrence_form(d: int, dv: int, max_len: int, n: int, num_seqs: int, heads:
     A walk's time goes with the longest sequence: 17 us and 0.43 us a token while its warps do not crowd the schedulers (two full-length
     sequences of 16 heads), the tiles' with how often the tiles of all heads fill the GPU: about 30 us a time, once at least.  Measured (us, walk / tiles;
     16 heads of 128 with a decay per channel): one sequence of 32 tokens 29 / 32, 48 37 / 34, 64 45 / 36, 192 107 / 40; 24 single
-    tokens beside one of 100 77 / 146, beside one of 600 312 / 191; a decay per head: 32 43 / 29, 192 99 / 38."""
+    tokens beside one of 100 77 / 146, beside one of 600 312 / 191; a decay per head: 33 43 / 24, 128 75 / 28."""
     if not on_gpu or d > TILES_MAX_HEAD_DIM or dv > TILES_MAX_HEAD_DIM or max_len < TILES_MIN_TOKENS:
         return "walk"
     longest = min(max_len, n)
