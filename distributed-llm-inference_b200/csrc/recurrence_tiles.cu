@@ -59,6 +59,8 @@ struct Params {
   int n, num_seqs, heads, kq, d, dv;
   float unit_eps;
   int cols;  // value columns of a CTA of the second kernel: 16 or 32
+  int vec;   // rows of queries, keys and decays are whole (d = KD) and aligned: a lane's channels come in one load
+  int vec_v; // rows of values lie in 16-byte runs
   unsigned char* left;
   int* error_flag;
 };
@@ -80,6 +82,25 @@ __device__ __forceinline__ void mma6(float (&large)[4], float (&small)[4], const
   mma16816(small, a[1], b00, b01);
   mma16816(small, a[0], b10, b11);
 }
+// N (2 or 4) numbers side by side, aligned to all of them
+template <int N> __device__ __forceinline__ void load_run(const float* p, float (&v)[N]) {
+  if constexpr (N == 4) { const float4 x = *reinterpret_cast<const float4*>(p); v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; }
+  else { const float2 x = *reinterpret_cast<const float2*>(p); v[0] = x.x; v[1] = x.y; }
+}
+template <int N> __device__ __forceinline__ void load_run(const bf16* p, float (&v)[N]) {
+  uint32_t w[N / 2];
+  if constexpr (N == 4) { const uint2 x = *reinterpret_cast<const uint2*>(p); w[0] = x.x; w[1] = x.y; }
+  else w[0] = *reinterpret_cast<const uint32_t*>(p);
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) {
+    v[2 * i] = __uint_as_float(w[i] << 16);
+    v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+template <int N> __device__ __forceinline__ void store_run(float* p, const float (&v)[N]) {
+  if constexpr (N == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  else *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+}
 // bytes of pair c of row r of a 16 x 16 block
 __device__ __forceinline__ int block_at(int r, int c) { return r * 32 + (((c >> 2) ^ ((r >> 2) & 1)) * 16) + (c & 3) * 4; }
 
@@ -97,9 +118,13 @@ template <int THREADS, typename F> __device__ __forceinline__ void split_blocks(
 }
 
 // T = (I + A)^-1 for a strictly lower triangular A (rows of F_ROW floats; what lies on and above the diagonal is not read), by all threads of a
-// CTA of at least 256, with barriers: the blocks on the diagonal a column a lane, the others block by block away from it,
+// CTA of at least 256 or (OWN_BARRIER) by the first 256, with barriers: the blocks on the diagonal a column a lane, the others block by block away from it,
 // T_ba = -T_bb sum_{a <= e < b} A_be T_ea (the sum is kept above the diagonal meanwhile).
-__device__ __forceinline__ void invert_unit_lower(const float* sA, float* sT, int tid) {
+template <bool OWN_BARRIER = false> __device__ __forceinline__ void invert_unit_lower(const float* sA, float* sT, int tid) {
+  auto sync = [] {
+    if (OWN_BARRIER) asm volatile("bar.sync 1, 256;" ::: "memory");
+    else __syncthreads();
+  };
   const int warp = tid >> 5, lane = tid & 31;
   if (warp < 4) {
     const int b0 = warp * 16;
@@ -116,7 +141,7 @@ __device__ __forceinline__ void invert_unit_lower(const float* sA, float* sT, in
       for (int t = 0; t < 16; ++t) sT[(b0 + t) * F_ROW + b0 + lane] = x[t];
     }
   }
-  __syncthreads();
+  sync();
   for (int away = 1; away < 4; ++away) {  // a thread takes four columns of a row
     const int a = tid >> 6, b = a + away, r = (tid >> 2) & 15, cc = (tid & 3) * 4;
     if (b < 4) {
@@ -129,7 +154,7 @@ __device__ __forceinline__ void invert_unit_lower(const float* sA, float* sT, in
       }
       *reinterpret_cast<float4*>(sT + (a * 16 + r) * F_ROW + b * 16 + cc) = make_float4(s[0], s[1], s[2], s[3]);
     }
-    __syncthreads();
+    sync();
     if (b < 4) {
       float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -140,7 +165,7 @@ __device__ __forceinline__ void invert_unit_lower(const float* sA, float* sT, in
       }
       *reinterpret_cast<float4*>(sT + (b * 16 + r) * F_ROW + a * 16 + cc) = make_float4(-s[0], -s[1], -s[2], -s[3]);
     }
-    __syncthreads();
+    sync();
   }
 }
 
@@ -177,7 +202,7 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
   unsigned char* sTt = smem + Z::REGION + 3 * Z::SQUARE;         // (DELTA)
   float* sB = reinterpret_cast<float*>(smem + Z::REGION + (DELTA ? 3 * Z::SQUARE + 3 * Q_TERM : Z::SQUARE));  // [8][KD]: products of the decays of eight tokens
   float* sBeta = sB + 8 * KD;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, head = blockIdx.y, place = blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, head = blockIdx.x % p.heads, place = blockIdx.x / p.heads;  // (the heads of a tile read the same rows)
 
   // ---- which sequence's tile this is: the last one that begins at or in front of this place
   int seq = -1;
@@ -201,11 +226,31 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
     sQm[i] = 0.f;
     if (DELTA) sA[i] = 0.f;
   }
+  // V's rows come now, into the place of T, when they lie in 16-byte runs (p.vec_v): asked for behind the stores of the decays' products
+  // they took 5,000 clocks.
+  constexpr bool V_AHEAD = DELTA && sizeof(T) == 2;
+  if constexpr (V_AHEAD) {
+    if (p.vec_v) {
+      for (int i = tid; i < TOKENS * (dv / 8); i += Z::THREADS) {
+        const int r = i / (dv / 8), part = i % (dv / 8);
+        const uint32_t dst = smem_u32(sT) + (r * 128 + part * 8) * 2;
+        const T* src = qkv + (size_t)(first + (r < len ? r : 0)) * width + 2 * p.kq * d + head * dv + part * 8;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(r < len ? 16 : 0) : "memory");
+      }
+    }
+  }
   const float rate = MODE == BONUS ? 0.f : expf(p.a_log[head]);
-  constexpr int ROWS = TOKENS / Z::WARPS, GROUP = ROWS < 4 ? ROWS : 4;  // rows of a warp; those whose loads are under way together
+  // A lane has PER channels side by side.  Where rows are whole and aligned (p.vec) they come in one load each: a load per number, a division
+  // and a square root per lane and row, and forty shuffles a row's two norms made this part 16,700 of a tile's 61,300 clocks.
+  constexpr int ROWS = TOKENS / Z::WARPS, GROUP = 4;  // rows of a warp; those whose loads are under way together
+  static_assert(ROWS % GROUP == 0, "rows");
+  const int c0 = lane * PER;
+  float bias[PER];
+#pragma unroll
+  for (int m = 0; m < PER; ++m) bias[m] = MODE != HEAD_DELTA && c0 + m < d ? p.dt_bias[head * d + c0 + m] : 0.f;
 #pragma unroll 1
   for (int r0 = 0; r0 < ROWS; r0 += GROUP) {
-    float qv[GROUP][PER], kv[GROUP][PER], gv[GROUP][PER], beta[GROUP];
+    float qv[GROUP][PER], kv[GROUP][PER], gv[GROUP][PER], beta = 0.f;
 #pragma unroll
     for (int e = 0; e < GROUP; ++e) {
       const int r = warp + (r0 + e) * Z::WARPS;
@@ -215,19 +260,53 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
       const T* k = MODE == BONUS ? q + slab : q + p.kq * d;
       const T* a = (const T*)p.a + t * p.heads * d + head * d;
       const T* ut = (const T*)p.u + t * p.u_stride + head;
+      if (p.vec) {
+        load_run<PER>(q + c0, qv[e]);
+        load_run<PER>(k + c0, kv[e]);
+        if (MODE != HEAD_DELTA) load_run<PER>(a + c0, gv[e]);
+      } else {
 #pragma unroll
-      for (int m = 0; m < PER; ++m) {
-        const int i = lane + 32 * m;
-        const bool in = ok && i < d;
-        qv[e][m] = in ? to_float(q[i]) : 0.f;
-        kv[e][m] = in ? to_float(k[i]) : 0.f;
-        if (MODE != HEAD_DELTA) gv[e][m] = in ? to_float(a[i]) : 0.f;
+        for (int m = 0; m < PER; ++m) {
+          const bool in = c0 + m < d;
+          qv[e][m] = in ? to_float(q[c0 + m]) : 0.f;
+          kv[e][m] = in ? to_float(k[c0 + m]) : 0.f;
+          if (MODE != HEAD_DELTA) gv[e][m] = in ? to_float(a[c0 + m]) : 0.f;
+        }
       }
       if (MODE == HEAD_DELTA) gv[e][0] = to_float(ut[p.a_col]);
-      if (DELTA) beta[e] = to_float(ut[p.b_col]);
+      if (DELTA && lane == e) beta = to_float(ut[p.b_col]);
       if (!DELTA) {
         const T* v = qkv + 2 * slab + t * p.heads * d + head * d;
         for (int i = lane; i < (dv + p.cols - 1) / p.cols * p.cols; i += 32) *u_at(r, i) = ok && i < dv ? to_float(v[i]) : 0.f;
+      }
+    }
+    float factor = 0.f;  // lane 8 e + i: row e's factor, of the query (i < 4) or of the key
+    if (DELTA) {
+      float sum[2 * GROUP];  // eight sums over the lanes: a lane keeps the half of its numbers that its bit names
+#pragma unroll
+      for (int e = 0; e < GROUP; ++e) {
+        sum[2 * e] = sum[2 * e + 1] = 0.f;
+#pragma unroll
+        for (int m = 0; m < PER; ++m) {
+          sum[2 * e] = fmaf(qv[e][m], qv[e][m], sum[2 * e]);
+          sum[2 * e + 1] = fmaf(kv[e][m], kv[e][m], sum[2 * e + 1]);
+        }
+      }
+#pragma unroll
+      for (int half = 4, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
+        const bool upper = (lane & bit) != 0;
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+          const float give = upper ? sum[i] : sum[i + half], keep = upper ? sum[i + half] : sum[i];
+          sum[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+        }
+      }
+      sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 2);
+      sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 1);
+      factor = ((lane & 4) ? 1.f : 1.f / sqrtf((float)d)) / sqrtf(sum[0] + p.unit_eps);
+      if (lane < GROUP) {
+        const int r = warp + (r0 + lane) * Z::WARPS;
+        sBeta[r] = r < len ? 1.f / (1.f + expf(-beta)) : 0.f;
       }
     }
 #pragma unroll
@@ -240,29 +319,18 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
         for (int m = 0; m < PER; ++m) gv[e][m] = g;
       } else {
 #pragma unroll
-        for (int m = 0; m < PER; ++m) {
-          const int i = lane + 32 * m;
-          const float b = i < d ? p.dt_bias[head * d + i] : 0.f;
-          gv[e][m] = MODE == BONUS ? expf(-expf(gv[e][m] + b)) : expf(-rate * softplus(gv[e][m] + b));
-        }
+        for (int m = 0; m < PER; ++m) gv[e][m] = MODE == BONUS ? expf(-expf(gv[e][m] + bias[m])) : expf(-rate * softplus(gv[e][m] + bias[m]));
       }
-      if (DELTA) {
-        float sq = 0.f, sk = 0.f;
+      const float fq = DELTA ? __shfl_sync(0xffffffffu, factor, 8 * e) : 1.f, fk = DELTA ? __shfl_sync(0xffffffffu, factor, 8 * e + 4) : 1.f;
 #pragma unroll
-        for (int m = 0; m < PER; ++m) { sq = fmaf(qv[e][m], qv[e][m], sq); sk = fmaf(kv[e][m], kv[e][m], sk); }
-        sq = warp_sum(sq); sk = warp_sum(sk);
-        const float fq = (1.f / sqrtf((float)d)) / sqrtf(sq + p.unit_eps), fk = 1.f / sqrtf(sk + p.unit_eps);
-#pragma unroll
-        for (int m = 0; m < PER; ++m) { qv[e][m] *= fq; kv[e][m] *= fk; }
-        if (lane == 0) sBeta[r] = ok ? 1.f / (1.f + expf(-beta[e])) : 0.f;
+      for (int m = 0; m < PER; ++m) {  // (0 / sqrt(0 + 0) of a row that is not there must not get through)
+        qv[e][m] = ok ? qv[e][m] * fq : 0.f;
+        kv[e][m] = ok ? kv[e][m] * fk : 0.f;
+        gv[e][m] = ok ? gv[e][m] : 1.f;
       }
-#pragma unroll
-      for (int m = 0; m < PER; ++m) {
-        const int i = lane + 32 * m;
-        sQ[r * KD + i] = ok ? qv[e][m] : 0.f;  // (0 / sqrt(0 + 0) of a row that is not there must not get through)
-        sK[r * KD + i] = ok ? kv[e][m] : 0.f;
-        sG[r * KD + i] = ok ? gv[e][m] : 1.f;
-      }
+      store_run<PER>(sQ + r * KD + c0, qv[e]);
+      store_run<PER>(sK + r * KD + c0, kv[e]);
+      store_run<PER>(sG + r * KD + c0, gv[e]);
     }
   }
   __syncthreads();
@@ -437,6 +505,7 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
   }
   __syncthreads();
 
+  if (V_AHEAD) asm volatile("cp.async.wait_all;" ::: "memory");  // (seen by everybody behind the barrier below)
   // ---- the six blocks below the diagonal: (1, 0) and (3, 2) across their common border, (2, 0), (2, 1), (3, 0), (3, 1) across the tile's middle
   const int kcol = (lane & 3) * 2;
   for (int task = warp; task < (DELTA ? 12 : 6); task += Z::WARPS) {
@@ -475,43 +544,62 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
   }
   __syncthreads();
 
-  // ---- Q leaves in three terms, block by block
-  float vv[DELTA ? ROWS : 1][4];  // this warp's rows of V, requested ahead of what comes in between
+  auto q_leaves = [&](auto threads, int id) {  // Q in three terms, block by block
+    split_blocks<decltype(threads)::value>([&](int r, int cc) { return sQm[r * F_ROW + cc]; }, left + L::Q, id);
+  };
+  if constexpr (!DELTA) q_leaves(std::integral_constant<int, Z::THREADS>(), tid);
   if constexpr (DELTA) {
-#pragma unroll
-    for (int e = 0; e < ROWS; ++e) {
-      const int r = warp + e * Z::WARPS;
-      const T* v = qkv + (size_t)(first + (r < len ? r : 0)) * width + 2 * p.kq * d + head * dv;
-#pragma unroll
-      for (int m = 0; m < 4; ++m) vv[e][m] = r < len && lane + 32 * m < dv ? to_float(v[lane + 32 * m]) : 0.f;
-    }
-  }
-  split_blocks<Z::THREADS>([&](int r, int cc) { return sQm[r * F_ROW + cc]; }, left + L::Q, tid);
-  if constexpr (DELTA) {
-    // ---- P o K and V as operands, in the place of the blocks' operands
+    // ---- P o K and V as operands, in the place of the blocks' operands.  With sixteen warps, eight make the inverse, a chain of short steps,
+    // while the others see to V and Q (one after the other 14,700 of the 61,300 clocks).
+    constexpr bool APART = Z::WARPS == 16;
+    constexpr int V_WARPS = APART ? Z::WARPS / 2 : Z::WARPS, V_ROWS = TOKENS / V_WARPS;
     unsigned char* sKg = smem;
     unsigned char* sV = smem + Z::MATRIX;
 #pragma unroll
     for (int t = 0; t < 8; ++t) put(sKg, grp * 8 + t, kg[t]);
+    if (V_AHEAD && p.vec_v) {
+      for (int i = tid; i < TOKENS * (dvp / 8); i += Z::THREADS) {
+        const int r = i / (dvp / 8), part = i % (dvp / 8);
+        *reinterpret_cast<uint4*>(sV + r * Z::V_ROW + part * 16) = part * 8 < dv ? reinterpret_cast<const uint4*>(sT)[r * 16 + part] : make_uint4(0, 0, 0, 0);
+      }
+      __syncthreads();  // the place is T's from here on
+    }
+    if (APART && warp < 8) {
+      invert_unit_lower<true>(sA, sT, tid);
+    } else {
+      const int w0 = APART ? warp - 8 : warp;
+      const bool from_rows = !(V_AHEAD && p.vec_v);
+      float vv[V_ROWS][4];
 #pragma unroll
-    for (int e = 0; e < ROWS; ++e) {
+      for (int e = 0; e < V_ROWS; ++e) {
+        const int r = w0 + e * V_WARPS;
+        const T* v = qkv + (size_t)(first + (r < len ? r : 0)) * width + 2 * p.kq * d + head * dv;
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        if (lane + 32 * m < dvp) {
-          unsigned char* at = sV + (warp + e * Z::WARPS) * Z::V_ROW + (lane + 32 * m) * 2;
-          if (Z::V_TERMS == 1) {
-            *reinterpret_cast<bf16*>(at) = __float2bfloat16_rn(vv[e][m]);
-          } else {
-            bf16 h, mid, l;
-            split3(vv[e][m], h, mid, l);
-            *reinterpret_cast<bf16*>(at) = h;
-            *reinterpret_cast<bf16*>(at + Z::V_TERM) = mid;
-            *reinterpret_cast<bf16*>(at + 2 * Z::V_TERM) = l;
+        for (int m = 0; m < 4; ++m) vv[e][m] = from_rows && r < len && lane + 32 * m < dv ? to_float(v[lane + 32 * m]) : 0.f;
+      }
+      q_leaves(std::integral_constant<int, V_WARPS * 32>(), w0 * 32 + lane);
+#pragma unroll
+      for (int e = 0; e < V_ROWS; ++e) {
+        if (!from_rows) break;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          if (lane + 32 * m < dvp) {
+            unsigned char* at = sV + (w0 + e * V_WARPS) * Z::V_ROW + (lane + 32 * m) * 2;
+            if (Z::V_TERMS == 1) {
+              *reinterpret_cast<bf16*>(at) = __float2bfloat16_rn(vv[e][m]);
+            } else {
+              bf16 h, mid, l;
+              split3(vv[e][m], h, mid, l);
+              *reinterpret_cast<bf16*>(at) = h;
+              *reinterpret_cast<bf16*>(at + Z::V_TERM) = mid;
+              *reinterpret_cast<bf16*>(at + 2 * Z::V_TERM) = l;
+            }
           }
         }
       }
+      if (!APART) invert_unit_lower(sA, sT, tid);
     }
-    invert_unit_lower(sA, sT, tid);
+    if (APART) __syncthreads();
     split_blocks<Z::THREADS>([&](int r, int cc) { return cc <= r ? sT[r * F_ROW + cc] * sBeta[cc] : 0.f; }, sTt, tid);
     __syncthreads();
     // ---- W = T (P o K) and U = T V: a warp takes sixteen columns and two of the four blocks of rows (0 and 3, or 1 and 2)
@@ -864,7 +952,7 @@ __global__ void __launch_bounds__(256, 2) head_prep_kernel(const Params p, int v
   unsigned char* sTk = smem + Z::AT_QM;       // T diag(beta P fk), in the place of Q
   float* fk = reinterpret_cast<float*>(smem + Z::AT_F);  // per token: factor of the key, of the query, beta, sums of log decays (two terms), P, P_last / P, a scratch
   float *fq = fk + TOKENS, *beta = fq + TOKENS, *lh = beta + TOKENS, *lm = lh + TOKENS, *up = lm + TOKENS, *behind = up + TOKENS, *raw = behind + TOKENS;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, head = blockIdx.y, place = blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, head = blockIdx.x % p.heads, place = blockIdx.x / p.heads;  // (the heads of a tile read the same rows)
   int seq = -1;
   for (int s0 = 0; s0 < p.num_seqs; s0 += Z::THREADS) {
     const int s = s0 + tid;
@@ -1305,11 +1393,16 @@ template <int KD, int COLS, bool DELTA> cudaError_t launch_walk(const Params& p,
   return launch_pdl((tile_walk_kernel<KD, COLS, DELTA>), dim3((p.dv + COLS - 1) / COLS, p.heads, p.num_seqs), dim3(Z::THREADS), (size_t)Z::SMEM, stream, 1, p);
 }
 
-template <typename T, int MODE, int KD> int launch(const Params& p, cudaStream_t stream) {
+template <typename T, int MODE, int KD> int launch(const Params& params, cudaStream_t stream) {
   using Z = Prep<T, MODE, KD>;
+  constexpr int PER = KD / 32, RUN = PER * sizeof(T);
+  Params p = params;
+  const int width = MODE == BONUS ? p.d : 2 * p.kq * p.d + p.heads * p.dv;  // (BONUS: every row of every head begins at a multiple of d numbers)
+  p.vec = p.d == KD && width % PER == 0 && (((uintptr_t)p.qkv | (MODE == HEAD_DELTA ? 0 : (uintptr_t)p.a)) & (RUN - 1)) == 0;
+  p.vec_v = width % 8 == 0 && (2 * p.kq * p.d) % 8 == 0 && p.dv % 8 == 0 && ((uintptr_t)p.qkv & 15) == 0;
   static OncePerDevice prep;
   cudaError_t e = allow(tile_prep_kernel<T, MODE, KD>, Z::SMEM, prep);
-  if (e == cudaSuccess) e = launch_pdl((tile_prep_kernel<T, MODE, KD>), dim3(places(p.n, p.num_seqs), p.heads), dim3(Z::THREADS), (size_t)Z::SMEM, stream, 1, p);
+  if (e == cudaSuccess) e = launch_pdl((tile_prep_kernel<T, MODE, KD>), dim3((unsigned)places(p.n, p.num_seqs) * p.heads), dim3(Z::THREADS), (size_t)Z::SMEM, stream, 1, p);
   if (e == cudaSuccess) e = p.cols == 16 ? launch_walk<KD, 16, MODE != BONUS>(p, stream) : launch_walk<KD, 32, MODE != BONUS>(p, stream);
   return (int)e;
 }
@@ -1325,7 +1418,7 @@ template <int KD> int launch_head(const Params& p, cudaStream_t stream) {
   static OncePerDevice done;
   cudaError_t e = allow(head_prep_kernel<KD>, Z::SMEM, done);
   const int width = 2 * p.kq * p.d + p.heads * p.dv, vec = width % 8 == 0 && p.d % 8 == 0 && p.dv % 8 == 0 && ((uintptr_t)p.qkv & 15) == 0;  // 16-byte runs
-  if (e == cudaSuccess) e = launch_pdl((head_prep_kernel<KD>), dim3(places(p.n, p.num_seqs), p.heads), dim3(Z::THREADS), (size_t)Z::SMEM, stream, 1, p, vec);
+  if (e == cudaSuccess) e = launch_pdl((head_prep_kernel<KD>), dim3((unsigned)places(p.n, p.num_seqs) * p.heads), dim3(Z::THREADS), (size_t)Z::SMEM, stream, 1, p, vec);
   if (e == cudaSuccess) e = p.cols == 16 ? launch_head_walk<KD, 16>(p, stream) : launch_head_walk<KD, 32>(p, stream);
   return (int)e;
 }
@@ -1370,7 +1463,7 @@ DLI_EXPORT int dli_recurrence_tiles(int mode, float* o, const void* qkv, const v
   Params p;
   p.o = o; p.qkv = qkv; p.u = u; p.a = a; p.u_stride = u_stride; p.b_col = b_col; p.a_col = a_col; p.dt_bias = dt_bias; p.a_log = a_log; p.bonus = bonus;
   p.state = state; p.q_start = q_start; p.state_slot = state_slot; p.n = n; p.num_seqs = num_seqs; p.heads = heads; p.kq = kq; p.d = d; p.dv = dv;
-  p.unit_eps = unit_eps; p.cols = columns(heads, num_seqs, dv); p.left = (unsigned char*)scratch; p.error_flag = error_flag_device;
+  p.unit_eps = unit_eps; p.vec = p.vec_v = 0; p.cols = columns(heads, num_seqs, dv); p.left = (unsigned char*)scratch; p.error_flag = error_flag_device;
   return dtype == DLI_F32 ? launch_mode<float>(mode, p, stream) : launch_mode<bf16>(mode, p, stream);
 }
 
