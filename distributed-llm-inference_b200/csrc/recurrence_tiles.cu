@@ -14,11 +14,13 @@
 // Products of decays are only ever multiplied together (at most 1, underflow to zero is right): for tokens t and j in different blocks of 16
 // the decays behind j are split at a border between the blocks, those behind it go with t, those in front of it with j; blocks of 16 are
 // taken on the CUDA cores, split at their middle, and the halves of 8 by running products.
-// What bounds it, and what it measured.  (1) takes a CTA an SM (228 KB) about 49,000 cycles a tile and head of 128 (some 85,000 warp instructions at 0.45
-// a cycle and scheduler: exponentials and norms of the inputs 10,000 to 17,000 cycles, the diagonal blocks 6,000, products of decays 6,000 to 8,000,
-// the inverse 5,500, W and U 8,500); (2) 3.7 us a tile, by mma.sync (318 a tile and warp) and its operands' arrival (157 KB by bulk copies; with a
-// cp.async per 16 bytes, 6.5 us).  Against the kernels that walk, us: decay per head in bfloat16 (kernels of its own, below), 16 heads of 128, one prompt of 2,048 tokens 772 -> 135; decay per channel,
-// prompts of 1,400 and 2,100 1,052 -> 354, 32 heads and 2,048 1,031 -> 382; bonus, 16 heads of 64, float32, prompts of 200 and 301 109 -> 30, 4,096 1,336 -> 214.
+// What bounds it, and what it measured.  (1) takes a CTA an SM (228 KB) about 50,000 clocks a tile and head of 128 with a decay per channel, in
+// steps that wait on one another: 14,000 until the rows are there as unit vectors and decays (their loads 5,000, the exponentials 4,800), the diagonal
+// blocks 5,600, products of decays 7,700, blocks below the diagonal 3,300, the inverse 6,100, W and U 7,600, W's way out 2,200.  (2) takes 3.7 us a
+// tile (5 with 32 columns a CTA), by mma.sync (318 a tile and warp) and its operands' arrival (157 KB by bulk copies; with a cp.async per 16 bytes, 6.5 us).
+// Against the kernels that walk, us: decay per head in bfloat16 (kernels of its own, below), 16 heads of 128, one prompt of 2,048 tokens 772 -> 134;
+// decay per channel, prompts of 1,400 and 2,100 1,050 -> 324, one of 2,048 1,008 -> 206; bonus, 16 heads of 64, float32, prompts of 200 and 301 109 -> 30,
+// 4,096 1,336 -> 214.
 // Errors against 64 bits are the walks' or smaller (decay per channel, 2,048 tokens: o 4.9e-7 and S 5.0e-7, walked 5.4e-7 and 5.4e-7).
 #include "common.cuh"
 #include "mma_split.cuh"
@@ -202,7 +204,7 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
   unsigned char* sTt = smem + Z::REGION + 3 * Z::SQUARE;         // (DELTA)
   float* sB = reinterpret_cast<float*>(smem + Z::REGION + (DELTA ? 3 * Z::SQUARE + 3 * Q_TERM : Z::SQUARE));  // [8][KD]: products of the decays of eight tokens
   float* sBeta = sB + 8 * KD;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, head = blockIdx.x % p.heads, place = blockIdx.x / p.heads;  // (the heads of a tile read the same rows)
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, head = blockIdx.y, place = blockIdx.x;
 
   // ---- which sequence's tile this is: the last one that begins at or in front of this place
   int seq = -1;
@@ -240,8 +242,8 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
     }
   }
   const float rate = MODE == BONUS ? 0.f : expf(p.a_log[head]);
-  // A lane has PER channels side by side.  Where rows are whole and aligned (p.vec) they come in one load each: a load per number, a division
-  // and a square root per lane and row, and forty shuffles a row's two norms made this part 16,700 of a tile's 61,300 clocks.
+  // A lane has PER channels side by side, which come in one load each where rows are whole and aligned (p.vec).  A warp's eight norms share five
+  // rounds of shuffles and one root and division (with a load per number and these per row this part took 16,700 clocks, now 12,000).
   constexpr int ROWS = TOKENS / Z::WARPS, GROUP = 4;  // rows of a warp; those whose loads are under way together
   static_assert(ROWS % GROUP == 0, "rows");
   const int c0 = lane * PER;
@@ -250,7 +252,10 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
   for (int m = 0; m < PER; ++m) bias[m] = MODE != HEAD_DELTA && c0 + m < d ? p.dt_bias[head * d + c0 + m] : 0.f;
 #pragma unroll 1
   for (int r0 = 0; r0 < ROWS; r0 += GROUP) {
-    float qv[GROUP][PER], kv[GROUP][PER], gv[GROUP][PER], beta = 0.f;
+    float qv[GROUP][PER], kv[GROUP][PER], gv[GROUP][PER];
+    const int own = warp + (r0 + (lane & (GROUP - 1))) * Z::WARPS;  // the row whose beta this lane makes (all lanes load: a branch would wait for its load)
+    T beta = T(0.f);
+    if (DELTA) beta = ((const T*)p.u)[(size_t)(first + (own < len ? own : 0)) * p.u_stride + p.b_col + head];
 #pragma unroll
     for (int e = 0; e < GROUP; ++e) {
       const int r = warp + (r0 + e) * Z::WARPS;
@@ -259,7 +264,6 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
       const T* q = MODE == BONUS ? qkv + t * p.heads * d + head * d : qkv + t * width + kqh * d;
       const T* k = MODE == BONUS ? q + slab : q + p.kq * d;
       const T* a = (const T*)p.a + t * p.heads * d + head * d;
-      const T* ut = (const T*)p.u + t * p.u_stride + head;
       if (p.vec) {
         load_run<PER>(q + c0, qv[e]);
         load_run<PER>(k + c0, kv[e]);
@@ -273,8 +277,7 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
           if (MODE != HEAD_DELTA) gv[e][m] = in ? to_float(a[c0 + m]) : 0.f;
         }
       }
-      if (MODE == HEAD_DELTA) gv[e][0] = to_float(ut[p.a_col]);
-      if (DELTA && lane == e) beta = to_float(ut[p.b_col]);
+      if (MODE == HEAD_DELTA) gv[e][0] = to_float(((const T*)p.u)[t * p.u_stride + p.a_col + head]);
       if (!DELTA) {
         const T* v = qkv + 2 * slab + t * p.heads * d + head * d;
         for (int i = lane; i < (dv + p.cols - 1) / p.cols * p.cols; i += 32) *u_at(r, i) = ok && i < dv ? to_float(v[i]) : 0.f;
@@ -304,10 +307,7 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
       sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 2);
       sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 1);
       factor = ((lane & 4) ? 1.f : 1.f / sqrtf((float)d)) / sqrtf(sum[0] + p.unit_eps);
-      if (lane < GROUP) {
-        const int r = warp + (r0 + lane) * Z::WARPS;
-        sBeta[r] = r < len ? 1.f / (1.f + expf(-beta)) : 0.f;
-      }
+      if (lane < GROUP) sBeta[own] = own < len ? 1.f / (1.f + expf(-to_float(beta))) : 0.f;
     }
 #pragma unroll
     for (int e = 0; e < GROUP; ++e) {
@@ -952,7 +952,7 @@ __global__ void __launch_bounds__(256, 2) head_prep_kernel(const Params p, int v
   unsigned char* sTk = smem + Z::AT_QM;       // T diag(beta P fk), in the place of Q
   float* fk = reinterpret_cast<float*>(smem + Z::AT_F);  // per token: factor of the key, of the query, beta, sums of log decays (two terms), P, P_last / P, a scratch
   float *fq = fk + TOKENS, *beta = fq + TOKENS, *lh = beta + TOKENS, *lm = lh + TOKENS, *up = lm + TOKENS, *behind = up + TOKENS, *raw = behind + TOKENS;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, head = blockIdx.x % p.heads, place = blockIdx.x / p.heads;  // (the heads of a tile read the same rows)
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, head = blockIdx.y, place = blockIdx.x;
   int seq = -1;
   for (int s0 = 0; s0 < p.num_seqs; s0 += Z::THREADS) {
     const int s = s0 + tid;
@@ -1402,7 +1402,7 @@ template <typename T, int MODE, int KD> int launch(const Params& params, cudaStr
   p.vec_v = width % 8 == 0 && (2 * p.kq * p.d) % 8 == 0 && p.dv % 8 == 0 && ((uintptr_t)p.qkv & 15) == 0;
   static OncePerDevice prep;
   cudaError_t e = allow(tile_prep_kernel<T, MODE, KD>, Z::SMEM, prep);
-  if (e == cudaSuccess) e = launch_pdl((tile_prep_kernel<T, MODE, KD>), dim3((unsigned)places(p.n, p.num_seqs) * p.heads), dim3(Z::THREADS), (size_t)Z::SMEM, stream, 1, p);
+  if (e == cudaSuccess) e = launch_pdl((tile_prep_kernel<T, MODE, KD>), dim3(places(p.n, p.num_seqs), p.heads), dim3(Z::THREADS), (size_t)Z::SMEM, stream, 1, p);
   if (e == cudaSuccess) e = p.cols == 16 ? launch_walk<KD, 16, MODE != BONUS>(p, stream) : launch_walk<KD, 32, MODE != BONUS>(p, stream);
   return (int)e;
 }
@@ -1418,7 +1418,7 @@ template <int KD> int launch_head(const Params& p, cudaStream_t stream) {
   static OncePerDevice done;
   cudaError_t e = allow(head_prep_kernel<KD>, Z::SMEM, done);
   const int width = 2 * p.kq * p.d + p.heads * p.dv, vec = width % 8 == 0 && p.d % 8 == 0 && p.dv % 8 == 0 && ((uintptr_t)p.qkv & 15) == 0;  // 16-byte runs
-  if (e == cudaSuccess) e = launch_pdl((head_prep_kernel<KD>), dim3((unsigned)places(p.n, p.num_seqs) * p.heads), dim3(Z::THREADS), (size_t)Z::SMEM, stream, 1, p, vec);
+  if (e == cudaSuccess) e = launch_pdl((head_prep_kernel<KD>), dim3(places(p.n, p.num_seqs), p.heads), dim3(Z::THREADS), (size_t)Z::SMEM, stream, 1, p, vec);
   if (e == cudaSuccess) e = p.cols == 16 ? launch_head_walk<KD, 16>(p, stream) : launch_head_walk<KD, 32>(p, stream);
   return (int)e;
 }
