@@ -1809,17 +1809,19 @@ def decay_recurrence(o: torch.Tensor, rows: torch.Tensor, state: torch.Tensor, q
              0 if mode == "bonus" else 1, int(rows_per_lane), _stream()), "decay_recurrence")
 
 
-def shift_decay_scan(o: torch.Tensor, rkvg: torch.Tensor, wz: torch.Tensor, w0: torch.Tensor, bonus: torch.Tensor, state: torch.Tensor, q_start: torch.Tensor,
-                     state_slot: torch.Tensor, max_len: int = 1 << 30, form: str | None = None) -> None:
-    """The token-shift recurrence over every sequence's tokens of this step: ``shift_decay_prep`` and ``decay_recurrence`` ("bonus") in one call, or,
-    for portions, the kernels that take tiles of tokens.  ``form``: ``"walk"``, ``"tiles"``, or None (chosen)."""
+def shift_decay_scan(o: torch.Tensor, rkvg: torch.Tensor, wz: torch.Tensor, w0: torch.Tensor, mode: str, bonus: torch.Tensor, state: torch.Tensor,
+                     q_start: torch.Tensor, state_slot: torch.Tensor, max_len: int = 1 << 30, form: str | None = None) -> None:
+    """The token-shift recurrence over every sequence's tokens of this step: ``shift_decay_prep`` and ``decay_recurrence`` (``mode``: its update, "bonus") in one
+    call, or, for portions, the kernels that take tiles of tokens.  ``form``: ``"walk"``, ``"tiles"``, or None (chosen)."""
     _, heads, _, d = state.shape
     n = o.shape[0]
     if (form or recurrence_form(d, d, max_len, n, state_slot.numel(), heads, o.is_cuda)) != "tiles":
         rows = torch.empty((n, decay_recurrence_row(heads, heads, d, d)), dtype=torch.float32, device=o.device)
         shift_decay_prep(rows, rkvg, wz, w0, heads, d)
-        decay_recurrence(o, rows, state, q_start, state_slot, heads, "bonus", bonus, max_len=max_len)
+        decay_recurrence(o, rows, state, q_start, state_slot, heads, mode, bonus, max_len=max_len)
         return
+    if mode != "bonus":
+        raise KernelError(f"shift_decay_scan: no tiles for the update {mode!r}")
     _need(o, "o", torch.float32), _need(rkvg, "rkvg"), _need(wz, "wz", rkvg.dtype), _need(w0, "w0", torch.float32), _need(state, "state", torch.float32)
     _need(bonus, "bonus", torch.float32), _need(q_start, "q_start", torch.int32), _need(state_slot, "state_slot", torch.int32)
     if (rkvg.dtype not in DT_CODE or tuple(rkvg.shape) != (4, n, heads * d) or tuple(wz.shape) != (n, heads * d) or w0.numel() != heads * d

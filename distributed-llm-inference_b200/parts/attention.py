@@ -530,7 +530,7 @@ class LatentAttention(Part):
                       q.view(n, self.nh, self.row)[:, :, : self.rank])
         latent = torch.empty((n, self.nh * self.row), dtype=x.dtype, device=x.device)
         attn_kernels.paged_attention(latent, q, cache, batch, self.nh, self.scale, self.window, splits=batch.launch_keys.get(id(self)),
-                                     sink=self.sinks, value_dim=self.rank)
+                                     value_dim=self.rank, sink=self.sinks)
         out = torch.empty((n, self.nh * self.dv), dtype=x.dtype, device=x.device)
         heads_product(latent.view(n, self.nh, self.row)[:, :, : self.rank], self.w_uv, out.view(n, self.nh, self.dv),
                       gate=proj[:, self.gate_col : self.gate_col + self.nh * self.dv] if self.gated else None)

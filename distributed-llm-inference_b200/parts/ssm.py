@@ -25,6 +25,14 @@ def singles_apart(batch, d: int, dv: int, heads: int, on_gpu: bool) -> int:
     return s
 
 
+def scan_calls(batch, s: int) -> list[tuple]:
+    """A delta rule's calls for a step whose first ``s`` single tokens are taken apart: (rows, q_start, state_slot, options) of each."""
+    if not s:
+        return [(batch.n, batch.q_start, batch.state_slot, {"max_len": batch.max_q_len})]
+    return [(s, batch.q_start[: s + 1], batch.state_slot[:s], {"max_len": 1}),
+            (batch.n, batch.q_start[s:], batch.state_slot[s:], {"max_len": batch.max_q_len, "form": "tiles"})]
+
+
 @register_part("mixer", "mamba2")
 class Mamba2Mixer(Part):
     """Mamba-2 (state-space duality) on any mix of prompt portions and decoded tokens.
@@ -182,12 +190,9 @@ class GatedDeltaRule(Part):
         if self.taps > 1:
             ops.conv_state_update(conv_state, u, 0, batch.q_start, batch.state_slot)
         o = torch.empty((n, self.inner), dtype=torch.float32, device=x.device)
-        s = singles_apart(batch, self.d, self.dv, self.heads, x.is_cuda)
-        if s:
-            ops.delta_rule_scan(o[:s], qkv[:s], u[:s], self.b_col, self.a_col, w["dt_bias"], w["A_log"], state, batch.seq_of_token[:s], batch.q_start[: s + 1],
-                                batch.state_slot[:s], self.kv_heads, self.d, self.unit_eps, max_len=1)
-        ops.delta_rule_scan(o, qkv, u, self.b_col, self.a_col, w["dt_bias"], w["A_log"], state, batch.seq_of_token, batch.q_start[s:], batch.state_slot[s:],
-                            self.kv_heads, self.d, self.unit_eps, max_len=batch.max_q_len, **({"form": "tiles"} if s else {}))
+        for rows, q_start, slots, options in scan_calls(batch, singles_apart(batch, self.d, self.dv, self.heads, x.is_cuda)):
+            ops.delta_rule_scan(o[:rows], qkv[:rows], u[:rows], self.b_col, self.a_col, w["dt_bias"], w["A_log"], state, batch.seq_of_token[:rows], q_start,
+                                slots, self.kv_heads, self.d, self.unit_eps, **options)
         gated = torch.empty((n, self.inner), dtype=x.dtype, device=x.device)
         ops.gated_group_rmsnorm(gated, o, u, self.g_col, w["norm"], self.heads, self.eps, gate_after=True)
         return project(gated, w["o"])
@@ -306,7 +311,7 @@ class ShiftDecayRecurrence(Part):
         low = ops.activation(project(blends[4], w["w1"]), "tanh")
         wz = project(low, w["w2"])
         o = torch.empty((n, self.inner), dtype=torch.float32, device=x.device)
-        ops.shift_decay_scan(o, rkvg, wz, w["w0"], w["u"], state, batch.q_start, batch.state_slot, max_len=batch.max_q_len)
+        ops.shift_decay_scan(o, rkvg, wz, w["w0"], "bonus", w["u"], state, batch.q_start, batch.state_slot, max_len=batch.max_q_len)
         gated = torch.empty((n, self.inner), dtype=x.dtype, device=x.device)
         ops.gated_group_rmsnorm(gated, o, rkvg[3], 0, w["norm"], self.heads, self.eps, gate_after=True)
         return project(gated, w["o"])
@@ -397,12 +402,9 @@ class ChannelDeltaRule(Part):
         a = project(u[:, self.a_cols[0] : self.a_cols[1]], w["a2"])  # [n, heads * head_dim]; the library reads the column slice in place
         g = project(u[:, self.g_cols[0] : self.g_cols[1]], w["g2"])  # [n, heads * value_dim]
         o = torch.empty((n, self.inner), dtype=torch.float32, device=x.device)
-        s = singles_apart(batch, self.d, self.dv, self.heads, x.is_cuda)
-        if s:
-            ops.channel_delta_scan(o[:s], qkv[:s], u[:s], self.b_col, a[:s], w["dt_bias"], w["A_log"], state, batch.q_start[: s + 1], batch.state_slot[:s],
-                                   self.kv_heads, self.unit_eps, max_len=1)
-        ops.channel_delta_scan(o, qkv, u, self.b_col, a, w["dt_bias"], w["A_log"], state, batch.q_start[s:], batch.state_slot[s:], self.kv_heads,
-                               self.unit_eps, max_len=batch.max_q_len, **({"form": "tiles"} if s else {}))
+        for rows, q_start, slots, options in scan_calls(batch, singles_apart(batch, self.d, self.dv, self.heads, x.is_cuda)):
+            ops.channel_delta_scan(o[:rows], qkv[:rows], u[:rows], self.b_col, a[:rows], w["dt_bias"], w["A_log"], state, q_start, slots, self.kv_heads,
+                                   self.unit_eps, **options)
         gated = torch.empty((n, self.inner), dtype=x.dtype, device=x.device)
         ops.gated_group_rmsnorm(gated, o, g, 0, w["norm"], self.heads, self.eps, gate_after=True, gate="sigmoid")
         return project(gated, w["o"])

@@ -107,7 +107,7 @@ def test_bonus(H, d, lens, dtype, shift):
     w0, bonus, state = torch.randn(H * d, generator=g) + shift, torch.randn(H, d, generator=g), torch.randn(len(lens), H, d, d, generator=g)
     want = _bonus(rkvg, wz, w0, bonus, state, lens)
     q_start, x = _starts(lens).cuda(), [t.cuda() for t in (rkvg, wz, w0, bonus)]
-    _check(lambda o, st, slot, form: ops.shift_decay_scan(o, x[0], x[1], x[2], x[3], st, q_start, slot, max_len=max(lens), form=form), want, (n, H * d), state)
+    _check(lambda o, st, slot, form: ops.shift_decay_scan(o, x[0], x[1], x[2], "bonus", x[3], st, q_start, slot, max_len=max(lens), form=form), want, (n, H * d), state)
 
 
 def test_which_form_serves_a_step():
