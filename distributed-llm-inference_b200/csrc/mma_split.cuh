@@ -27,6 +27,8 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// the logarithm of a decay, not below `lowest`, where the decay is 0 and sums of logarithms stay finite; a NaN stays one (fmaxf would drop it)
+__device__ __forceinline__ float log_decay(float x, float lowest) { return x < lowest ? lowest : x; }
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&v);

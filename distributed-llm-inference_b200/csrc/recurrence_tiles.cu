@@ -1016,7 +1016,7 @@ __global__ void __launch_bounds__(256, 2) head_prep_kernel(const Params p, int v
   if (warp == 0) {
     double l[2];
 #pragma unroll
-    for (int k = 0; k < 2; ++k) l[k] = (double)fmaxf(raw[2 * lane + k], -1e4f);  // (a decay below that is 0, and its sums stay finite)
+    for (int k = 0; k < 2; ++k) l[k] = (double)log_decay(raw[2 * lane + k], -1e4f);
     l[1] += l[0];
     double incl = l[1];
 #pragma unroll

@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) ssm_chunk_kernel(const Params p
     for (int k = 0; k < 2; ++k) {
       const bool ok = base + 2 * lane + k < t1;
       dt[k] = ok ? softplus(raw[k] + bias) : 0.f;
-      l[k] = ok ? (double)fmaxf(-A * dt[k], LOG_FLOOR) : 0.0;
+      l[k] = ok ? (double)log_decay(-A * dt[k], LOG_FLOOR) : 0.0;
     }
     l[1] += l[0];
     double incl = l[1];

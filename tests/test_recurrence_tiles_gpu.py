@@ -110,6 +110,27 @@ def test_bonus(H, d, lens, dtype, shift):
     _check(lambda o, st, slot, form: ops.shift_decay_scan(o, x[0], x[1], x[2], "bonus", x[3], st, q_start, slot, max_len=max(lens), form=form), want, (n, H * d), state)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("channel", [False, True], ids=["decay_per_head", "decay_per_channel"])
+def test_a_gate_that_is_not_a_number_stays_one(channel, dtype):
+    """Such a decay is not taken for 0: outputs and state are NaN from its token on, as token after token."""
+    H, d, n, bad = 2, 16, 150, 70
+    g = torch.Generator().manual_seed(9)
+    qkv, u, a = (torch.randn(n, c, generator=g).to(dtype) for c in (3 * H * d, 2 * H, H * d))
+    (a if channel else u)[bad, d if channel else H + 1] = float("nan")  # of head 1
+    q_start, slot, seq = torch.tensor([0, n], dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda(), torch.zeros(n, dtype=torch.int32).cuda()
+    zero, qkv, u, a = torch.zeros(H).cuda(), qkv.cuda(), u.cuda(), a.cuda()
+    for form in ("walk", "tiles"):
+        o, state = torch.zeros(n, H, d).cuda(), torch.full((1, H, d, d), 0.1).cuda()
+        if channel:
+            ops.channel_delta_scan(o.view(n, -1), qkv, u, 0, a, torch.zeros(H * d).cuda(), zero, state, q_start, slot, H, 1e-6, max_len=n, form=form)
+        else:
+            ops.delta_rule_scan(o.view(n, -1), qkv, u, 0, H, zero, zero, state, seq, q_start, slot, H, d, 1e-6, max_len=n, form=form)
+        assert o[bad:, 1].isnan().all() and state[:, 1].isnan().all(), form
+        assert o[:64].isfinite().all() and o[:, 0].isfinite().all() and state[:, 0].isfinite().all(), form
+
+
 def test_which_form_serves_a_step():
     form = ops.recurrence_form
     assert form(128, 128, 2048, 2048, 1, 16) == form(64, 64, 4096, 4096, 1, 16) == form(128, 128, 2100, 3500, 2, 16) == form(128, 128, 1 << 30, 2048, 1, 32) == "tiles"

@@ -50,6 +50,26 @@ def test_tiles_and_segments(H, P, N, groups, lens, dt_shift):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("where", ["step size", "A_log"])
+def test_a_gate_that_is_not_a_number_stays_one(where):
+    """Such a decay is not taken for 0: outputs and state are NaN from its token on, as token after token."""
+    H, P, N, n, bad = 2, 16, 16, 200, 70 if where == "step size" else 0
+    g = torch.Generator().manual_seed(9)
+    xbc, u, zero = torch.randn(n, H * P + 2 * N, generator=g).bfloat16().cuda(), torch.randn(n, H, generator=g).bfloat16(), torch.zeros(H)
+    a_log = zero.clone()
+    if where == "A_log":
+        a_log[1] = float("nan")
+    else:
+        u[bad, 1] = float("nan")
+    q_start, slot = torch.tensor([0, n], dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda()
+    for form, segments in (("walk", 0), ("chunk", 1), ("chunk", 3)):
+        y, state = torch.zeros(n, H, P).cuda(), torch.zeros(1, H, P, N).cuda()
+        ops.ssm_scan(y.view(n, -1), xbc, u.cuda(), 0, zero.cuda(), a_log.cuda(), zero.cuda(), state, q_start, slot, 1, max_len=n, form=form, segments=segments)
+        assert y[bad:, 1].isnan().all() and state[:, 1].isnan().all(), (form, segments)
+        assert y[:bad].isfinite().all() and y[:, 0].isfinite().all() and state[:, 0].isfinite().all(), (form, segments)
+
+
+@pytest.mark.gpu
 def test_a_tile_may_be_replayed_from_a_graph():
     H, P, N, lens = 2, 64, 64, [1, 200]
     xbc, u = torch.randn(201, H * P + 2 * N).bfloat16().cuda(), torch.randn(201, H).bfloat16().cuda()
