@@ -17,6 +17,10 @@
 // zero, without read-outs; the second starts every later segment from exp(sum of its log decays) S + what was added, segment
 // after segment, and walks them side by side.  A segment without read-outs costs 0.45 of one with, so segment 0 is that much shorter.
 //
+// A masked weight is 0, and 0 times an infinity or a NaN is a NaN; an infinity in three terms is one too.  So a CTA looks at what it
+// computed: where a read-out or the state is not finite, it walks its columns again token after token (walk_again), and infinities and
+// NaNs appear where ssm.cu has them.  Looking costs a multiply-add for each result.
+//
 // What bounds it: the latency of a warp's instructions (ncu, one prompt of 1,024 tokens, a CTA an SM: 3,500 warp instructions a tile and
 // warp, an instruction every 4.3 cycles, tensor pipe active 26 %); registers and shared memory hold two CTAs an SM.  Measured, us, against
 // the walk of ssm.cu (64 heads, P 64, N 128): prompts of 666, 1,000 and 1,335 tokens 772 -> 159, one of 4,096 1,405 -> 213, one
@@ -74,9 +78,55 @@ __device__ __forceinline__ void segment_tiles(int tiles, int segments, int seg, 
   to = min(tiles, head + seg * share);
 }
 
+// The scan of a CTA's columns token after token: from the state `from` in front of token t_from, with read-outs of tokens t_emit .. t_end - 1, the
+// state behind them to `to` (or null).  A warp takes sixteen columns, four at a time; a lane holds every 32nd number of them.
+__device__ __noinline__ void walk_again(const Params& p, int head, int col0, const float* from, int t_from, int t_emit, int t_end, float* to) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, N = p.N, P = p.P, inner = p.heads * P, width = inner + 2 * p.groups * N;
+  const float A = expf(p.A_log[head]), bias = p.dt_bias[head], Dh = p.D[head];
+  const int g = head / (p.heads / p.groups);
+  for (int c0 = col0 + warp * 16; c0 < min(P, col0 + warp * 16 + 16); c0 += 4) {  // (P is a multiple of 8)
+    float S[4][4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int m = 0; m < 4; ++m) S[c][m] = lane + 32 * m < N ? from[(size_t)(c0 + c) * N + lane + 32 * m] : 0.f;
+    for (int t = t_from; t < t_end; ++t) {
+      const bf16* row = p.xbc + (size_t)t * width;
+      const float dt = softplus(to_float(p.u[(size_t)t * p.u_stride + p.dt_col + head]) + bias), decay = expf(-A * dt);
+      float B[4], C[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const bool in = lane + 32 * m < N;
+        B[m] = in ? to_float(row[inner + g * N + lane + 32 * m]) : 0.f;
+        C[m] = in ? to_float(row[inner + (p.groups + g) * N + lane + 32 * m]) : 0.f;
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float x = to_float(row[head * P + c0 + c]), dtx = dt * x;
+        float sum = 0.f;
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+          if (lane + 32 * m < N) {  // (0 times an infinity of a number that is not there must not get through)
+            S[c][m] = fmaf(decay, S[c][m], B[m] * dtx);
+            sum = fmaf(S[c][m], C[m], sum);
+          }
+        sum = warp_sum(sum);
+        if (t >= t_emit && lane == 0) p.y[(size_t)t * inner + head * P + c0 + c] = fmaf(Dh, x, sum);
+      }
+    }
+    if (to) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+          if (lane + 32 * m < N) to[(size_t)(c0 + c) * N + lane + 32 * m] = S[c][m];
+    }
+  }
+}
+
 // SECOND: the second of the two launches over segments.
 template <int NK, bool SECOND>
-__global__ void __launch_bounds__(WARPS * 32, 2) ssm_chunk_kernel(const Params p) {
+__global__ void __launch_bounds__(WARPS * 32, 2) ssm_chunk_kernel(const __grid_constant__ Params p) {
   pdl_launch_dependents();
   pdl_wait();
   using Z = Shape<NK>;
@@ -220,6 +270,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) ssm_chunk_kernel(const Params p
     }
   }
 
+  float finite = 0.f;  // 0 while every result was finite, NaN from the first one on that was not
   int stage = 0;
   for (int base = t0; base < t1; base += TOKENS, stage ^= 1) {
     const int len = min(TOKENS, t1 - base);
@@ -363,6 +414,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) ssm_chunk_kernel(const Params p
                   v.y = fmaf(O[mt][nt][2 * hf + 1], e, (T[2][nt][2 * hf + 1] + T[1][nt][2 * hf + 1]) + T[0][nt][2 * hf + 1]);
                   v.x = fmaf(Dh, x.x, v.x);
                   v.y = fmaf(Dh, x.y, v.y);
+                  finite = fmaf(v.x, 0.f, fmaf(v.y, 0.f, finite));
                   *reinterpret_cast<float2*>(p.y + (size_t)(base + r) * inner + head * P + col0 + col) = v;
                 }
               }
@@ -409,9 +461,17 @@ __global__ void __launch_bounds__(WARPS * 32, 2) ssm_chunk_kernel(const Params p
       }
     }
   }
-  float* dst = t1 == last ? slot_state : p.part + pbase(seg) * block;
-  if (SECOND && t1 != last) return;
-  each([&](int j, int e, size_t at) { *reinterpret_cast<float2*>(dst + at) = make_float2(S[j][e], S[j][e + 1]); });
+  float* dst = t1 == last ? slot_state : (SECOND ? nullptr : p.part + pbase(seg) * block);
+  if (emit) {
+    if (dst) each([&](int j, int e, size_t) { finite = fmaf(S[j][e], 0.f, fmaf(S[j][e + 1], 0.f, finite)); });
+    if (__syncthreads_or(finite != 0.f)) {  // (also: nobody writes a read-out behind this)
+      int second = 0, end = 0;              // segments behind the first start again from the state behind it, the last one that was walked from the slot's
+      if (SECOND) segment_tiles((last - first + TOKENS - 1) / TOKENS, p.segments, 1, second, end);
+      walk_again(p, head, col0, SECOND ? p.part + pbase(0) * block : slot_state, first + second * TOKENS, t0, t1, dst);
+      dst = nullptr;
+    }
+  }
+  if (dst) each([&](int j, int e, size_t at) { *reinterpret_cast<float2*>(dst + at) = make_float2(S[j][e], S[j][e + 1]); });
   if (!SECOND && t1 != last && tid == 0 && blockIdx.x == 0) p.part_log[pbase(seg)] = (float)total;
 }
 

@@ -69,6 +69,43 @@ def test_a_gate_that_is_not_a_number_stays_one(where):
         assert y[:bad].isfinite().all() and y[:, 0].isfinite().all() and state[:, 0].isfinite().all(), (form, segments)
 
 
+def _same_kind(got, want, tol):
+    """Infinities and NaNs in the same places, and what is finite near."""
+    got, fine = got.cpu().double(), want.isfinite()
+    return bool((got.isnan() == want.isnan()).all() and (got.isinf() == want.isinf()).all() and (got[want.isinf()] == want[want.isinf()]).all()
+                and (got[fine] - want[fine]).norm() <= tol * want[fine].norm())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.0e38], ids=["inf", "-inf", "nan", "3e38"])
+@pytest.mark.parametrize("where", ["x", "B", "C", "dt", "state"])
+@pytest.mark.parametrize("bad", [0, 5, 71, 140, 199])
+def test_infinities_and_nans_stay_where_the_recurrence_has_them(where, value, bad):
+    """A number that is not finite reaches its own and later tokens of its own columns, and no other."""
+    H, P, N, n = 2, 72, 24, 200
+    g = torch.Generator().manual_seed(11)
+    xbc, u, state = torch.randn(n, H * P + 2 * N, generator=g).bfloat16(), torch.randn(n, H, generator=g).bfloat16(), torch.randn(1, H, P, N, generator=g)
+    if where == "state":
+        state[0, 1, bad % P, 3] = value
+    elif where == "dt":
+        u[bad, 1] = value
+    else:
+        xbc[bad, {"x": P + bad % P, "B": H * P + 3, "C": H * P + N + 3}[where]] = value
+    vec = torch.randn(3, H, generator=g)
+    vec[0] -= 3.0  # small steps: no decay of the whole sequence underflows in float32
+    want = _exact(xbc, u, 0, vec[0], vec[1] * 0.1, vec[2], state.clone(), [n], 1)
+    if value == 3.0e38:  # what float32 does not hold is infinite there
+        want = [w.float().double() for w in want]
+    q_start, slot, vec = torch.tensor([0, n], dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda(), vec.cuda()
+    for segments in (1, 3):
+        y, st = torch.zeros(n, H * P).cuda(), state.cuda()
+        ops.ssm_scan(y, xbc.cuda(), u.cuda(), 0, vec[0], vec[1] * 0.1, vec[2], st, q_start, slot, 1, max_len=n, form="chunk", segments=segments)
+        if value == 3.0e38:  # (sums of such numbers may leave float32 on the way in one order and not in another: only tokens in front of it are compared)
+            assert where == "state" or _same_kind(y[:bad], want[0][:bad], 1e-6)
+        else:
+            assert _same_kind(y, want[0], 1e-6) and _same_kind(st, want[1], 1e-6)
+
+
 @pytest.mark.gpu
 def test_a_tile_may_be_replayed_from_a_graph():
     H, P, N, lens = 2, 64, 64, [1, 200]
