@@ -14,6 +14,10 @@
 // Products of decays are only ever multiplied together (at most 1, underflow to zero is right): for tokens t and j in different blocks of 16
 // the decays behind j are split at a border between the blocks, those behind it go with t, those in front of it with j; blocks of 16 are
 // taken on the CUDA cores, split at their middle, and the halves of 8 by running products.
+// A masked weight is 0, and 0 times an infinity or a NaN is a NaN; an infinity in three terms is one too.  So a CTA of the second kernel looks
+// at what it computed: where a read-out or the state is not finite, it walks its columns again token after token (walk_again), and infinities
+// and NaNs appear where the recurrence has them.  Looking costs a multiply-add for each result.
+//
 // What bounds it, and what it measured.  (1) takes a CTA an SM (228 KB) about 50,000 clocks a tile and head of 128 with a decay per channel, in
 // steps that wait on one another: 14,000 until the rows are there as unit vectors and decays (their loads 5,000, the exponentials 4,800), the diagonal
 // blocks 5,600, products of decays 7,700, blocks below the diagonal 3,300, the inverse 6,100, W and U 7,600, W's way out 2,200.  (2) takes 3.7 us a
@@ -51,6 +55,7 @@ __host__ __device__ inline int padded_columns(int dv) { return (dv + 31) / 32 * 
 __host__ __device__ inline int first_tile(int q_start, int seq) { return q_start / TOKENS + seq; }
 
 struct Params {
+  int mode, f32;  // f32: qkv, u and a are float32, else bfloat16
   float* o;
   const void *qkv, *u, *a;  // BONUS: qkv holds the slabs r | k | v, a the decays' products
   long long u_stride;
@@ -685,6 +690,89 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
 
 // ---------------------------------------------------------------- (2) the walk over the tiles
 
+// Tokens first .. last - 1 of a head token after token, for 4 columns a warp from col0 on, from and to the state in memory.  A lane holds every
+// 32nd channel.
+__device__ __noinline__ void walk_again(const Params& p, int head, int col0, int first, int last, float* S0) {
+  const int lane = threadIdx.x & 31, d = p.d, dv = p.dv, kqh = head / (p.heads / p.kq), width = 2 * p.kq * d + p.heads * dv;
+  const size_t slab = (size_t)p.n * p.heads * d;  // BONUS
+  auto number = [&](const void* base, size_t i) { return p.f32 ? static_cast<const float*>(base)[i] : to_float(static_cast<const bf16*>(base)[i]); };
+  const int c0 = col0 + (threadIdx.x >> 5) * 4;
+  if (c0 >= dv) return;
+  float S[4][4], bias[4], own[4];
+  bool in[4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const int i = lane + 32 * m;
+    in[m] = i < d;
+    bias[m] = in[m] && p.mode != HEAD_DELTA ? p.dt_bias[head * d + i] : 0.f;
+    own[m] = in[m] && p.mode == BONUS ? p.bonus[head * d + i] : 0.f;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) S[c][m] = in[m] && c0 + c < dv ? S0[(size_t)(c0 + c) * d + i] : 0.f;
+  }
+  const float rate = p.mode == BONUS ? 0.f : expf(p.a_log[head]);
+  for (size_t t = first; t < (size_t)last; ++t) {
+    const size_t q_at = p.mode == BONUS ? (t * p.heads + head) * d : t * width + kqh * d, k_at = p.mode == BONUS ? q_at + slab : q_at + p.kq * d;
+    const size_t v_at = p.mode == BONUS ? q_at + 2 * slab : t * width + 2 * p.kq * d + head * dv;
+    float q[4], k[4], g[4], beta = 0.f;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const int i = lane + 32 * m;
+      q[m] = in[m] ? number(p.qkv, q_at + i) : 0.f;
+      k[m] = in[m] ? number(p.qkv, k_at + i) : 0.f;
+      if (p.mode != HEAD_DELTA) {
+        const float a = in[m] ? number(p.a, (t * p.heads + head) * d + i) + bias[m] : 0.f;
+        g[m] = p.mode == BONUS ? expf(-expf(a)) : expf(-rate * softplus(a));
+      }
+    }
+    if (p.mode != BONUS) {
+      float sq = 0.f, sk = 0.f;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) { sq = fmaf(q[m], q[m], sq); sk = fmaf(k[m], k[m], sk); }
+      const float fq = (1.f / sqrtf((float)d)) / sqrtf(warp_sum(sq) + p.unit_eps), fk = 1.f / sqrtf(warp_sum(sk) + p.unit_eps);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) { q[m] *= fq; k[m] *= fk; }
+      beta = 1.f / (1.f + expf(-number(p.u, t * p.u_stride + p.b_col + head)));
+      if (p.mode == HEAD_DELTA) g[0] = g[1] = g[2] = g[3] = expf(-rate * softplus(number(p.u, t * p.u_stride + p.a_col + head) + p.dt_bias[head]));
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float v = c0 + c < dv ? number(p.qkv, v_at + c0 + c) : 0.f;
+      float out = 0.f;
+      if (p.mode == BONUS) {
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+          if (in[m]) {  // (0 times an infinity of a number that is not there must not get through)
+            const float kv = k[m] * v;
+            out = fmaf(q[m], fmaf(own[m], kv, S[c][m]), out);
+            S[c][m] = fmaf(g[m], S[c][m], kv);
+          }
+      } else {
+        float sum = 0.f;
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+          if (in[m]) {
+            S[c][m] *= g[m];
+            sum = fmaf(k[m], S[c][m], sum);
+          }
+        const float w = beta * (v - warp_sum(sum));
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+          if (in[m]) {
+            S[c][m] = fmaf(k[m], w, S[c][m]);
+            out = fmaf(q[m], S[c][m], out);
+          }
+      }
+      out = warp_sum(out);
+      if (lane == 0 && c0 + c < dv) p.o[t * p.heads * dv + (size_t)head * dv + c0 + c] = out;
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+      if (in[m] && c0 + c < dv) S0[(size_t)(c0 + c) * d + lane + 32 * m] = S[c][m];
+}
+
 template <int KD, int COLS> struct Walk {
   static constexpr int THREADS = COLS * 8;  // warps: (block of 16 tokens, 16 of the columns) of the products with S0; (quarter of the channels, 16 columns) of S
   static constexpr int ROW = Left<KD>::ROW, TERM = Left<KD>::TERM, MATRIX = Left<KD>::MATRIX;
@@ -718,7 +806,7 @@ __device__ __forceinline__ void wait_copies(uint32_t bar, uint32_t parity, volat
 }
 
 template <int KD, int COLS, bool DELTA>
-__global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const Params p) {
+__global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const __grid_constant__ Params p) {
   pdl_launch_dependents();
   pdl_wait();
   using Z = Walk<KD, COLS>;
@@ -782,6 +870,7 @@ __global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const Params p) 
   const uint32_t wa_addr = smem_u32(smem + Z::AT_w) + ((lane & 7) + (lane >> 4) * 8) * Z::W_ROW + (half * 16 + ((lane >> 3) & 1) * 8) * 2;  // m = column, k = token
   const uint32_t pk_addr = smem_u32(smem + Z::AT_PK) + ((lane & 7) + ((lane >> 3) & 1) * 8) * Z::ROW + (slice0 + (lane >> 4) * 8) * 2;
 
+  float finite = 0.f;  // 0 while every result was finite, NaN from the first one on that was not
   uint32_t parity = 0;
   for (int base = first; base < last; base += TOKENS, parity ^= 1) {
     const int len = min(TOKENS, last - base);
@@ -872,6 +961,7 @@ __global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const Params p) 
           if (r < len) {
             float* dst = p.o + (size_t)(base + r) * inner + (size_t)head * dv + col;
             const float x = O[nt][2 * hf] + (qs[nt][2 * hf] + ql[nt][2 * hf]), y = O[nt][2 * hf + 1] + (qs[nt][2 * hf + 1] + ql[nt][2 * hf + 1]);
+            finite = fmaf(x, 0.f, fmaf(y, 0.f, finite));
             if ((dv & 1) == 0) {
               if (col < dv) *reinterpret_cast<float2*>(dst) = make_float2(x, y);
             } else {
@@ -909,6 +999,11 @@ __global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const Params p) 
 #pragma unroll
       for (int e = 0; e < 4; ++e) S[j][e] = fmaf((e & 1) ? g.y : g.x, S[j][e], ds[j][e] + dl[j][e]);
     }
+  }
+  each([&](float& x, bool, size_t) { finite = fmaf(x, 0.f, finite); });
+  if (__syncthreads_or(finite != 0.f)) {  // (also: nobody writes a read-out behind this)
+    walk_again(p, head, col0, first, last, S0);
+    return;
   }
   each([&](float& x, bool in, size_t at) { if (in) S0[at] = x; });
 }
@@ -1166,7 +1261,7 @@ template <int KD, int COLS> struct HeadWalk {
 };
 
 template <int KD, int COLS>
-__global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const Params p) {
+__global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const __grid_constant__ Params p) {
   pdl_launch_dependents();
   pdl_wait();
   using Z = HeadWalk<KD, COLS>;
@@ -1229,6 +1324,7 @@ __global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const Params p) 
   const uint32_t wa_addr = smem_u32(smem + Z::AT_w) + 3 * Z::W_TERM + ((lane & 7) + (lane >> 4) * 8) * Z::W_ROW + (half * 16 + ((lane >> 3) & 1) * 8) * 2;  // with the factors
   const uint32_t kb_addr = smem_u32(smem + Z::AT_KB) + ((lane & 7) + ((lane >> 3) & 1) * 8) * Z::ROW + (slice0 + (lane >> 4) * 8) * 2;
 
+  float finite = 0.f;  // 0 while every result was finite, NaN from the first one on that was not
   uint32_t parity = 0;
   for (int base = first; base < last; base += TOKENS, parity ^= 1) {
     const int len = min(TOKENS, last - base);
@@ -1327,6 +1423,7 @@ __global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const Params p) 
             const float f = sF[r];
             float* dst = p.o + (size_t)(base + r) * inner + (size_t)head * dv + col;
             const float x = fmaf(f, O[nt][2 * hf], qs[nt][2 * hf] + ql[nt][2 * hf]), y = fmaf(f, O[nt][2 * hf + 1], qs[nt][2 * hf + 1] + ql[nt][2 * hf + 1]);
+            finite = fmaf(x, 0.f, fmaf(y, 0.f, finite));
             if ((dv & 1) == 0) {
               if (col < dv) *reinterpret_cast<float2*>(dst) = make_float2(x, y);
             } else {
@@ -1365,6 +1462,11 @@ __global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const Params p) 
     for (int j = 0; j < NT; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) S[j][e] = fmaf(g, S[j][e], ds[j][e] + dl[j][e]);
+  }
+  each([&](float& x, bool, size_t) { finite = fmaf(x, 0.f, finite); });
+  if (__syncthreads_or(finite != 0.f)) {  // (also: nobody writes a read-out behind this)
+    walk_again(p, head, col0, first, last, S0);
+    return;
   }
   each([&](float& x, bool in, size_t at) { if (in) S0[at] = x; });
 }
@@ -1461,6 +1563,7 @@ DLI_EXPORT int dli_recurrence_tiles(int mode, float* o, const void* qkv, const v
     if (cudaHostGetDevicePointer((void**)&error_flag_device, error_flag_host, 0) != cudaSuccess) return (int)cudaGetLastError();
   }
   Params p;
+  p.mode = mode; p.f32 = dtype == DLI_F32;
   p.o = o; p.qkv = qkv; p.u = u; p.a = a; p.u_stride = u_stride; p.b_col = b_col; p.a_col = a_col; p.dt_bias = dt_bias; p.a_log = a_log; p.bonus = bonus;
   p.state = state; p.q_start = q_start; p.state_slot = state_slot; p.n = n; p.num_seqs = num_seqs; p.heads = heads; p.kq = kq; p.d = d; p.dv = dv;
   p.unit_eps = unit_eps; p.vec = p.vec_v = 0; p.cols = columns(heads, num_seqs, dv); p.left = (unsigned char*)scratch; p.error_flag = error_flag_device;

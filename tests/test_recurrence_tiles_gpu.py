@@ -131,6 +131,51 @@ def test_a_gate_that_is_not_a_number_stays_one(channel, dtype):
         assert o[:64].isfinite().all() and o[:, 0].isfinite().all() and state[:, 0].isfinite().all(), form
 
 
+def _same_kind(got, want, tol):
+    """Infinities and NaNs in the same places, and what is finite near."""
+    got, fine = got.cpu().double(), want.isfinite()
+    return bool((got.isnan() == want.isnan()).all() and (got.isinf() == want.isinf()).all() and (got[want.isinf()] == want[want.isinf()]).all()
+                and (got[fine] - want[fine]).norm() <= tol * want[fine].norm())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")], ids=["inf", "-inf", "nan"])
+@pytest.mark.parametrize("where", ["q", "k", "v", "gate", "beta", "state"])
+@pytest.mark.parametrize("bad", [0, 5, 71, 149])
+@pytest.mark.parametrize("kind,dtype,d,dv", [("head", torch.bfloat16, 24, 40), ("head", torch.float32, 24, 17), ("channel", torch.bfloat16, 128, 20), ("channel", torch.float32, 30, 8),
+                                             ("bonus", torch.bfloat16, 40, 40), ("bonus", torch.float32, 9, 9)])
+def test_infinities_and_nans_stay_where_the_recurrence_has_them(kind, dtype, d, dv, where, value, bad):
+    """A number that is not finite reaches its own and later tokens, of a value or a state its own columns only, and no other."""
+    H, n = 2, 150
+    if kind == "bonus" and where == "beta":
+        pytest.skip("no beta")
+    g = torch.Generator().manual_seed(13)
+    qkv = torch.randn(4, n, H * d, generator=g) if kind == "bonus" else torch.randn(n, 2 * H * d + H * dv, generator=g)
+    u, a, state = torch.randn(n, 2 * H + 1, generator=g), torch.randn(n, H * d, generator=g), torch.randn(1, H, dv, d, generator=g)
+    bias, a_log, bonus = torch.randn(H if kind == "head" else H * d, generator=g) - 4.0, torch.zeros(H), torch.randn(H, d, generator=g)
+    if where == "state":
+        state[0, 1, bad % dv, 3] = value
+    elif where == "beta":
+        u[bad, 2] = value
+    elif where == "gate":
+        (u if kind == "head" else a)[bad, 1 + H + 1 if kind == "head" else d + 3] = value
+    elif kind == "bonus":
+        qkv["qkv".index(where), bad, d + bad % d] = value
+    else:
+        qkv[bad, {"q": d + 3, "k": H * d + d + 3, "v": 2 * H * d + dv + bad % dv}[where]] = value
+    qkv, u, a = qkv.to(dtype), u.to(dtype), a.to(dtype)
+    want = _bonus(qkv, a, bias, bonus, state, [n]) if kind == "bonus" else _delta(kind == "channel", qkv, u, a, bias, a_log, state, [n], H)
+    q_start, slot, seq = torch.tensor([0, n], dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda(), torch.zeros(n, dtype=torch.int32).cuda()
+    o, st, x = torch.zeros(n, H * dv).cuda(), state.cuda(), [t.cuda() for t in (qkv, u, a, bias, a_log, bonus)]
+    if kind == "bonus":
+        ops.shift_decay_scan(o, x[0], x[2], x[3], "bonus", x[5], st, q_start, slot, max_len=n, form="tiles")
+    elif kind == "channel":
+        ops.channel_delta_scan(o, x[0], x[1], 1, x[2], x[3], x[4], st, q_start, slot, H, 1e-6, max_len=n, form="tiles")
+    else:
+        ops.delta_rule_scan(o, x[0], x[1], 1, 1 + H, x[3], x[4], st, seq, q_start, slot, H, d, 1e-6, max_len=n, form="tiles")
+    assert _same_kind(o, want[0], 2e-6) and _same_kind(st, want[1], 2e-6)
+
+
 def test_which_form_serves_a_step():
     form = ops.recurrence_form
     assert form(128, 128, 2048, 2048, 1, 16) == form(64, 64, 4096, 4096, 1, 16) == form(128, 128, 2100, 3500, 2, 16) == form(128, 128, 1 << 30, 2048, 1, 32) == "tiles"
