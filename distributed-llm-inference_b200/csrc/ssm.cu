@@ -413,11 +413,13 @@ __global__ void gated_group_rmsnorm_kernel(T* __restrict__ out, const float* __r
   }
 }
 
-// Parts of up to 1,024 numbers (size % 8 == 0, aligned rows): LANES lanes share a part of a token, each with CHUNKS runs of eight columns in
+// Parts of up to 512 numbers (size % 8 == 0, aligned rows): LANES lanes share a part of a token, each with CHUNKS runs of eight columns in
 // registers between the sum and the output; a warp holds 32 / LANES parts, a CTA four warps, and nothing waits at a block's barrier.
-// What bounds it: memory and the exponentials' and divisions' instructions, about alike.  A CTA a part (a warp of which half the lanes
-// were idle at heads of 128, two barriers) took, us, L2 flushed: 4,096 tokens of 16 parts of 128 74 -> 23 (2,900 GB/s), 3,001 of 8 parts of 512 33 -> 31, 501 of
-// 16 parts of 64 in float32 13 -> 8.
+// What bounds it: memory and the exponentials' and divisions' instructions, about alike.  In place of a CTA a part (a warp of which half the lanes
+// were idle at heads of 128, two barriers), us, one launch behind another: 3,001 tokens of 16 parts of 128 50 -> 12, of 72 50 -> 12, of 264 51 -> 37;
+// 24 rows of 16 parts of up to 256 2.6 both.  Where every lane has two runs a few parts take 3.1 to 3.6 us instead of 2.6 (twice the exponentials and
+// divisions in a row): from 2,048 parts on it is as fast (4.6) and then faster.  With four runs (parts of 513 to 1,024) it is slower at every
+// number of parts (8 rows 4.6 against 2.6, 3,001 tokens of 8 parts of 1,024 44 against 41), so a CTA takes such a part.
 constexpr int NORM_WARPS = 4;
 template <typename T, int LANES, int CHUNKS>
 __global__ void __launch_bounds__(NORM_WARPS * 32) gated_part_rmsnorm_kernel(T* __restrict__ out, const float* __restrict__ y, const T* __restrict__ u,
@@ -435,16 +437,18 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) gated_part_rmsnorm_kernel(T* 
   const T* zrow = u + (size_t)t * u_stride + z_col + c0;
   float gv[CHUNKS][8], z[CHUNKS][8];
 #pragma unroll
-  for (int c = 0; c < CHUNKS; ++c) {
-    const int col = (lane + c * LANES) * 8;
-    if (live && col < size) {
-      load8(yrow + col, gv[c]);
-      load8(zrow + col, z[c]);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) gv[c][k] = z[c][k] = 0.f;
-    }
+  for (int c = 0; c < CHUNKS; ++c) {  // every lane loads (the part's last run where it has none of its own): a branch would wait for its loads
+    const int col = min((lane + c * LANES) * 8, size - 8);
+    load8(yrow + col, gv[c]);
+    load8(zrow + col, z[c]);
   }
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      gv[c][k] = (lane + c * LANES) * 8 < size ? gv[c][k] : 0.f;
+      z[c][k] = (lane + c * LANES) * 8 < size ? z[c][k] : 1.f;  // (a finite gate; 0 would take the division's slow way)
+    }
   const float f = divisor && live ? 1.f / divisor[unit] : 1.f;  // every number of the part, before anything else
   float q = 0.f;
 #pragma unroll
@@ -472,7 +476,7 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) gated_part_rmsnorm_kernel(T* 
 }
 
 // The same with the part's values in registers between the two passes and 16- and 32-byte accesses: a thread owns
-// CHUNKS runs of eight columns (1,024 < size <= 8 * THREADS * CHUNKS, size % 8 == 0, aligned rows).
+// CHUNKS runs of eight columns (256 < size <= 8 * THREADS * CHUNKS, size % 8 == 0, aligned rows).
 template <typename T, int THREADS, int CHUNKS>
 __global__ void __launch_bounds__(THREADS) gated_group_rmsnorm_vec_kernel(T* __restrict__ out, const float* __restrict__ y,
                                                                           const T* __restrict__ u, long long u_stride, int z_col,
@@ -677,8 +681,9 @@ DLI_EXPORT int dli_gated_group_rmsnorm(void* out, const float* y, const void* u,
   if (size <= 64) DLI_GN_PART(T, 8, 1);       \
   if (size <= 128) DLI_GN_PART(T, 16, 1);     \
   if (size <= 256) DLI_GN_PART(T, 32, 1);     \
-  if (size <= 512) DLI_GN_PART(T, 32, 2);     \
-  if (size <= 1024) DLI_GN_PART(T, 32, 4);    \
+  if (size <= 512 && units >= 2048) DLI_GN_PART(T, 32, 2); \
+  if (size <= 512) DLI_GN_VEC(T, 64, 1);      \
+  if (size <= 1024) DLI_GN_VEC(T, 128, 1);    \
   if (size <= 2048) DLI_GN_VEC(T, 256, 1);    \
   if (size <= 4096) DLI_GN_VEC(T, 256, 2);    \
   DLI_GN_VEC(T, 256, 4)
