@@ -1438,8 +1438,7 @@ __global__ void __launch_bounds__(THREADS, 1) paged_prefill_row_kernel(const __g
     const int rpos = pos0 + rtok;
     const uint32_t lane_bits = (uint32_t)((warp & 3) * 32) << 16;
     const int col0 = half * 64, half_cols = vslabs * 32;
-    constexpr float RESCALE_STEP = 8.f;
-    float m = -CUDART_INF_F, m_ref = -CUDART_INF_F, l = 0.f;
+    float m = -CUDART_INF_F, l = 0.f;
     bool ok = true;
     const int group = r >> 6;
     const uint32_t my_o = tmem_o + lane_bits + half * half_cols;
@@ -1478,14 +1477,13 @@ __global__ void __launch_bounds__(THREADS, 1) paged_prefill_row_kernel(const __g
       rm[half * ROWS + r] = max3(max3(mx[0], mx[1], mx[2]), max3(mx[3], mx[4], mx[5]), fmaxf(mx[6], mx[7]));
       if (group == 0) asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_THREADS / 2) : "memory");  // the two halves of this row's 64-row group
       else asm volatile("bar.sync 2, %0;" ::"n"(SOFTMAX_THREADS / 2) : "memory");
+      // probabilities are relative to the exact maximum so far: the largest one is then 1 and bfloat16 holds it as it is (following the maximum
+      // only when it has grown by 2^8 took 175 us instead of 185 for 4,096 tokens, but an error 2 to 23 % larger)
+      const float before = m;
       m = max3(m, rm[r], rm[ROWS + r]);
-      float corr = 1.f;
-      const bool grown = (m - m_ref) * p.scale_log2 > RESCALE_STEP;  // also the first finite maximum (m_ref = -inf)
-      if (grown) {
-        corr = (m_ref == -CUDART_INF_F) ? 0.f : ex2((m_ref - m) * p.scale_log2);
-        m_ref = m;
-      }
-      const float neg = (m_ref == -CUDART_INF_F) ? 0.f : -m_ref * p.scale_log2;
+      const bool grown = m > before;  // also the first finite maximum (before = -inf)
+      const float corr = grown ? ex2((before - m) * p.scale_log2) : 1.f;
+      const float neg = (m == -CUDART_INF_F) ? 0.f : -m * p.scale_log2;
 #pragma unroll
       for (int j = 0; j < 64; ++j) sc[j] = ex2(fmaf(sc[j], p.scale_log2, neg));  // masked: ex2(-inf) = 0
       // P and O are free once the product of the tile before has finished
@@ -1513,9 +1511,9 @@ __global__ void __launch_bounds__(THREADS, 1) paged_prefill_row_kernel(const __g
         uint32_t packed[4];
 #pragma unroll
         for (int e = 0; e < 8; e += 2) {
-          sum[(e >> 1) & 3] += sc[j + e] + sc[j + e + 1];
           __nv_bfloat162 b2 = __floats2bfloat162_rn(sc[j + e], sc[j + e + 1]);
           packed[e >> 1] = *reinterpret_cast<uint32_t*>(&b2);
+          sum[(e >> 1) & 3] += __uint_as_float(packed[e >> 1] << 16) + __uint_as_float(packed[e >> 1] & 0xffff0000u);  // of the rounded numbers, the weights the values get
         }
         st_shared_v4(pchunk ^ ((j >> 3) << 4), packed[0], packed[1], packed[2], packed[3]);
       }
@@ -1540,7 +1538,7 @@ __global__ void __launch_bounds__(THREADS, 1) paged_prefill_row_kernel(const __g
     if (group == 0) asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_THREADS / 2) : "memory");
     else asm volatile("bar.sync 2, %0;" ::"n"(SOFTMAX_THREADS / 2) : "memory");
     const int head = head0 + (r - rtok * Gc);
-    const float inv = 1.f / (rl[r] + rl[ROWS + r] + sink_term(rvalid ? sink_of(p.sink_heads, p.sink_log2, head) : -CUDART_INF_F, m_ref * p.scale_log2));
+    const float inv = 1.f / (rl[r] + rl[ROWS + r] + sink_term(rvalid ? sink_of(p.sink_heads, p.sink_log2, head) : -CUDART_INF_F, m * p.scale_log2));
     const size_t row = (size_t)(q0 + tok0 + rtok) * p.nh + head;
     for (int c = 0; c < half_cols; c += 32) {
       uint32_t v[32];
