@@ -53,6 +53,7 @@ class StepBatch:
     max_q_len: int = 0
     max_kv_len: int = 0
     max_kv_len_single: int = 0  # longest context among the single-token sequences
+    max_kv_len_portion: int = 0  # .. among the sequences that bring more tokens (0: not known)
     # id(part) -> what that part answered to ``decode_launch_key`` when this step's shape was fixed ahead of its
     # data (a captured graph); a part not named here decides its launches from the step itself
     launch_keys: dict = field(default_factory=dict)
@@ -269,7 +270,7 @@ def build_batch(entries: Sequence[StepEntry], manager, device, vocab_size: int, 
         n=n, num_seqs=S, num_single=sum(1 for q in q_lens if q == 1), token_ids=b_tokens, positions=b_pos,
         seq_of_token=b_seq, q_start=b_qstart, kv_len=b_kvlen, state_slot=b_slot, logit_rows=b_rows, groups=views,
         q_lens=q_lens, starts=h["starts"].tolist(), state_slots=h["state_slot"].tolist(), max_q_len=max(q_lens), max_kv_len=max(kv),
-        max_kv_len_single=max((k for k, q in zip(kv, q_lens) if q == 1), default=0),
+        max_kv_len_single=max((k for k, q in zip(kv, q_lens) if q == 1), default=0), max_kv_len_portion=max((k for k, q in zip(kv, q_lens) if q > 1), default=0),
         logits_all_rows=h["logit_rows"].size == n and bool((h["logit_rows"] == np.arange(n)).all()),
         token_src=b_src,
     )

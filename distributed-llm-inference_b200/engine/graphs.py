@@ -152,6 +152,7 @@ class MixedGraph:
             kv_len=self.ints[o["kv_len"] : o["kv_len"] + S], state_slot=self.ints[o["state_slot"] : o["state_slot"] + S],
             logit_rows=self.ints[o["logit_rows"] : o["logit_rows"] + S - 1], groups=views, q_lens=[1] * singles + [0] * (portions + 1),
             starts=[0] * S, state_slots=[0] * S, max_q_len=tokens, max_kv_len=width * page_size, max_kv_len_single=width * page_size,
+            max_kv_len_portion=width * page_size,
             launch_keys=launch_keys, logits_all_rows=False,
         )
         side = torch.cuda.Stream(device=dev)

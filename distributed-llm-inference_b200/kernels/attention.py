@@ -94,6 +94,16 @@ def decode_splits(num_seqs: int, num_heads: int, nkv: int, head_dim: int, page_s
     return splits
 
 
+ONE_KEY_TILE = 64  # keys that one tile of the mma.sync kernels holds
+
+
+def portions_pay_for_tiles_of_rows(batch) -> bool:
+    """Whether portions over one pool of rows go to the tcgen05 kernel: from the second key tile of the mma.sync kernel on.  Measured (us, mma.sync /
+    tcgen05, 16 heads, rows of 256): 2 tokens alone 9.3 / 9.9, 64 tokens 11.8 / 13.4, 16 portions of 16 tokens 11.9 / 14.0, 2 tokens behind 64 12.6 / 9.9,
+    80 tokens 15.2 / 13.6, 128 tokens 16.0 / 13.9; 8 heads, rows of 192: 2 tokens 7.1 / 9.2, 2 behind 64 10.5 / 9.2."""
+    return not 0 < (batch.max_kv_len_portion or batch.max_kv_len) <= ONE_KEY_TILE
+
+
 def paged_attention(out: torch.Tensor, qkv: torch.Tensor, cache, batch, num_heads: int, scale: float, window: int | None,
                     splits: int | None = None, sink: float | torch.Tensor | None = None, softcap: float | None = None,
                     slopes: torch.Tensor | None = None, value_dim: int | None = None) -> None:
@@ -127,7 +137,8 @@ def paged_attention(out: torch.Tensor, qkv: torch.Tensor, cache, batch, num_head
     if total > singles and ops.prefill_tc_supported(d, cache.page_size, dv) and _slab_kernels(d, one_pool):
         ops.paged_prefill_tc(out, qkv, cache.k, cache.v, group.block_tables, batch.q_start, batch.kv_len, singles, total - singles,
                              batch.max_q_len, num_heads, scale, window, sink=sink, **bend)
-    elif total > singles and one_pool and not bend and ops.prefill_rows_supported(d, cache.page_size) and (out.data_ptr() | qkv.data_ptr() | cache.k.data_ptr()) % 16 == 0:
+    elif (total > singles and one_pool and not bend and ops.prefill_rows_supported(d, cache.page_size) and portions_pay_for_tiles_of_rows(batch)
+          and (out.data_ptr() | qkv.data_ptr() | cache.k.data_ptr()) % 16 == 0):
         ops.paged_prefill_rows(out, qkv, cache.k, group.block_tables, batch.q_start, batch.kv_len, singles, total - singles, batch.max_q_len, num_heads, scale,
                                window, sink=sink, value_dim=value_dim if value_dim and value_dim % 8 == 0 else None)
     elif total > singles:
