@@ -97,11 +97,16 @@ def decode_splits(num_seqs: int, num_heads: int, nkv: int, head_dim: int, page_s
 ONE_KEY_TILE = 64  # keys that one tile of the mma.sync kernels holds
 
 
+def _portion_keys(batch) -> int:
+    """The most keys that a portion of the step sees; where the step does not say, its longest sequence bounds it."""
+    return getattr(batch, "max_kv_len_portion", 0) or batch.max_kv_len
+
+
 def portions_pay_for_tiles_of_rows(batch) -> bool:
     """Whether portions over one pool of rows go to the tcgen05 kernel: from the second key tile of the mma.sync kernel on.  Measured (us, mma.sync /
     tcgen05, 16 heads, rows of 256): 2 tokens alone 9.3 / 9.9, 64 tokens 11.8 / 13.4, 16 portions of 16 tokens 11.9 / 14.0, 2 tokens behind 64 12.6 / 9.9,
     80 tokens 15.2 / 13.6, 128 tokens 16.0 / 13.9; 8 heads, rows of 192: 2 tokens 7.1 / 9.2, 2 behind 64 10.5 / 9.2."""
-    return not 0 < (batch.max_kv_len_portion or batch.max_kv_len) <= ONE_KEY_TILE
+    return not 0 < _portion_keys(batch) <= ONE_KEY_TILE
 
 
 def paged_attention(out: torch.Tensor, qkv: torch.Tensor, cache, batch, num_heads: int, scale: float, window: int | None,
@@ -146,16 +151,41 @@ def paged_attention(out: torch.Tensor, qkv: torch.Tensor, cache, batch, num_head
                                 total - singles, batch.max_q_len, singles, num_heads, scale, window, sink=sink, **bend)
 
 
+def diff_portions_apart(batch, tokens: int, num_heads: int, nkv: int, window: int | None, keep_first: int) -> bool:
+    """Whether the portions of a step of ``tokens`` rows of differential attention go to the tcgen05 kernel, single tokens following in a launch of their own, or everything to
+    one launch of the mma.sync kernel.
+
+    Estimates of both, us, fitted to 800 steps (16 and 32 heads on 4 and 8, 8 on 2, 16 on 16; with and without a window of 1,024; 0 to 64 single tokens
+    at 200 to 3,000 keys; portions of 2 to 1,024 tokens behind 0 to 3,000).  One launch takes as long as its slowest part: 23 us for 1,000 keys of a
+    single token, 13 to 53 of a portion (the more of its 64 rows are queries), more where CTAs queue.  Two launches add up: 12 us and 17 for
+    1,000 keys, and behind them 11 us and some 5 for 1,000 keys.  The new kernel is taken where it promises 15 % or more: then 5 of the 800 steps took over 5 %
+    longer than in one launch (29 % at most), with two launches throughout 359 did.  Measured, us, one / two launches: 2 tokens 6.1 / 12.1,
+    64 tokens 16 / 14, 1,024 76 / 29; 24 single tokens at 200 keys beside 16 tokens 16 / 30, beside 512 behind 512 80 / 44; at 3,000 keys 82 / 65, 106 / 80."""
+    singles, portions = batch.num_single, batch.num_seqs - batch.num_single
+    tokens -= singles
+
+    def seen(keys: int) -> float:  # thousands of keys that a query reads
+        return (min(keys, window + keep_first + 64) if window else keys) / 1000
+
+    group, sms = num_heads // nkv, sm_count()
+    keys, single_keys = seen(_portion_keys(batch)), seen(batch.max_kv_len_single) if singles else 0.0
+    rows = min(1.0, batch.max_q_len * group / 64)
+    portion = 9 * rows + keys * (13 + 40 * rows) * max(1.0, nkv * max(portions, tokens * group / 64) / (1.3 * sms))
+    one = 6 + max(portion, single_keys * 23 * max(1.0, singles * nkv / sms))
+    two = 12 + keys * 17 * max(1.0, nkv * max(portions, tokens * group / 128) / sms) + (11 + single_keys * 20 * max(0.26, singles * nkv / sms) if singles else 0)
+    return two <= 0.85 * one
+
+
 def diff_attention(out: torch.Tensor, q: torch.Tensor, cache, batch, gate: torch.Tensor | None, num_heads: int, scale: float,
                    window: int | None, keep_first: int, lam: float, post: float, eps: float) -> None:
     """Differential attention of every token of the step over its sequence's pages (``ops.diff_attention_simt`` says what is
-    computed).  bfloat16 with sizes that are multiples of 16: portions of maps of 64 go to a tcgen05 kernel, everything else to the mma.sync
-    kernel (portions and single tokens in one launch); float32 and any other size: the CUDA-core kernel."""
+    computed).  bfloat16 with sizes that are multiples of 16: portions of maps of 64 go to a tcgen05 kernel where that pays (``diff_portions_apart``),
+    everything else to the mma.sync kernel (portions and single tokens in one launch); float32 and any other size: the CUDA-core kernel."""
     group = batch.group(cache.group)
     if out.dtype == torch.bfloat16 and ops.diff_attention_tc_supported(cache.k.shape[3] // 2, cache.v.shape[3]):
         _, nkv, _, d2 = cache.k.shape
         vdim, singles, seqs, longest, seen = cache.v.shape[3], batch.num_single, batch.num_seqs, batch.max_q_len, batch.max_kv_len
-        if (seqs > singles and ops.prefill_diff_supported(d2 // 2, vdim, cache.page_size)
+        if (seqs > singles and ops.prefill_diff_supported(d2 // 2, vdim, cache.page_size) and diff_portions_apart(batch, q.shape[0], num_heads, nkv, window, keep_first)
                 and (out.data_ptr() | q.data_ptr() | cache.k.data_ptr() | cache.v.data_ptr()) % 16 == 0):
             ops.paged_prefill_diff(out, q, cache.k, cache.v, group.block_tables, batch.q_start, batch.kv_len, singles, seqs - singles, longest, gate, num_heads,
                                    scale, window, keep_first, lam, post, eps)

@@ -12,3 +12,14 @@ from dli_b200.kernels import attention
 def test_portions_over_one_pool_of_rows(portion, step, tiles):
     """One key tile of the mma.sync kernel: that kernel.  What the step does not say of its portions, its longest sequence bounds; 0: not known."""
     assert attention.portions_pay_for_tiles_of_rows(types.SimpleNamespace(max_kv_len_portion=portion, max_kv_len=step)) == tiles
+
+
+@pytest.mark.parametrize("portions,singles,context,apart", [
+    ([(2, 0)], 0, 0, False), ([(2, 300)], 0, 0, False), ([(64, 0)], 0, 0, True), ([(300, 0)], 0, 0, True), ([(1024, 0)], 0, 0, True), ([(128, 3000)], 0, 0, True),
+    ([(16, 0)], 24, 200, False), ([(3, 200)] * 8, 64, 300, False), ([(512, 512)], 24, 200, True), ([(16, 0)], 24, 3000, True), ([(128, 0)], 64, 2000, False),
+    ([(128, 3000)], 64, 2000, True), ([(1535, 1024)], 9, 1500, True)])
+def test_portions_of_differential_attention(portions, singles, context, apart):
+    """Few tokens beside single tokens go with them in one launch; portions that make up a launch go to the tcgen05 kernel."""
+    longest = max(q + before for q, before in portions)
+    batch = types.SimpleNamespace(num_single=singles, num_seqs=singles + len(portions), max_q_len=max(q for q, _ in portions), max_kv_len=max(longest, context), max_kv_len_single=context, max_kv_len_portion=longest)
+    assert attention.diff_portions_apart(batch, singles + sum(q for q, _ in portions), 16, 4, None, 0) == apart

@@ -103,6 +103,16 @@ def test_portions_beside_single_tokens(window, keep):
     _near(out.cpu(), want)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("apart", [False, True], ids=["one_launch", "two_launches"])
+def test_both_routes_of_a_mixed_step(apart, monkeypatch):
+    monkeypatch.setattr(attention, "diff_portions_apart", lambda *a: apart)
+    calls, kernel = [], ops.paged_prefill_diff
+    monkeypatch.setattr(ops, "paged_prefill_diff", lambda *a, **k: (calls.append(1), kernel(*a, **k)))
+    test_portions_beside_single_tokens(100, 16)
+    assert len(calls) == apart
+
+
 def test_which_sizes_have_the_kernel():
     ok = ops.prefill_diff_supported
     assert ok(64, 128, 16) and ok(64, 24, 8) and ok(64, 64, 128)
