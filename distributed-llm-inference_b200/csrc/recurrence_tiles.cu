@@ -42,17 +42,20 @@ constexpr int F_ROW = TOKENS + 4;     // floats of a row of a 64 x 64 matrix in 
 
 enum Mode { HEAD_DELTA = 0, CHANNEL_DELTA = 1, BONUS = 2 };
 
-// What the first kernel leaves for a (tile, head), in bytes, laid out as the second one wants it in shared memory (rows padded so that
-// ldmatrix reads different banks), so that a bulk copy brings a whole part: three matrices of 64 x KD in three terms, U in runs of
-// the columns of a CTA of the second kernel, Q in blocks, P_last.
-template <int KD> struct Left {
+template <int KD> struct Rows {  // a matrix of 64 x KD in three terms, in bytes, rows padded so that ldmatrix reads different banks
   static constexpr int ROW = KD * 2 + 16, TERM = TOKENS * ROW, MATRIX = 3 * TERM;
-  static constexpr int W = 0, PQ = MATRIX, PK = 2 * MATRIX, Q = 3 * MATRIX, P_LAST = Q + 3 * Q_TERM, U = P_LAST + KD * 4;
+};
+// What the first kernel leaves for a (tile, head), in bytes, laid out as the second one wants it in shared memory, so that a bulk copy brings
+// a whole part: the matrices (W of the delta rules only), U in runs of the columns of a CTA of the second kernel, Q in blocks, P_last.
+template <int KD, bool DELTA> struct Left : Rows<KD> {
+  static constexpr int MATRIX = Rows<KD>::MATRIX;
+  static constexpr int W = 0, PQ = DELTA ? MATRIX : 0, PK = PQ + MATRIX, Q = PK + MATRIX, P_LAST = Q + 3 * Q_TERM, U = P_LAST + KD * 4;
   __host__ __device__ static size_t bytes(int dv, int cols) { return (size_t)U + (size_t)((dv + cols - 1) / cols) * TOKENS * (cols + 4) * 4; }
 };
 __host__ __device__ inline int padded_columns(int dv) { return (dv + 31) / 32 * 32; }
 // A sequence's tiles lie behind one another from this place on; the places of different sequences do not meet.
 __host__ __device__ inline int first_tile(int q_start, int seq) { return q_start / TOKENS + seq; }
+inline int places(int n, int num_seqs) { return n / TOKENS + num_seqs + 1; }
 
 struct Params {
   int mode, f32;  // f32: qkv, u and a are float32, else bfloat16
@@ -68,7 +71,8 @@ struct Params {
   int cols;  // value columns of a CTA of the second kernel: 16 or 32
   int vec;   // rows of queries, keys and decays are whole (d = KD) and aligned: a lane's channels come in one load
   int vec_v; // rows of values lie in 16-byte runs
-  unsigned char* left;
+  int place0, num_places;  // the places that this pass takes; a sequence's state waits in its slot between two passes
+  unsigned char* left;     // what the first kernel leaves, from place0 on
   int* error_flag;
 };
 
@@ -181,7 +185,7 @@ template <bool OWN_BARRIER = false> __device__ __forceinline__ void invert_unit_
 template <typename T, int MODE, int KD> struct Prep {
   static constexpr int THREADS = KD * 4, WARPS = THREADS / 32;
   static constexpr bool DELTA = MODE != BONUS;
-  static constexpr int ROW = Left<KD>::ROW, TERM = Left<KD>::TERM, MATRIX = Left<KD>::MATRIX;
+  static constexpr int ROW = Rows<KD>::ROW, TERM = Rows<KD>::TERM, MATRIX = Rows<KD>::MATRIX;
   static constexpr int V_TERMS = sizeof(T) == 2 ? 1 : 3, V_ROW = 128 * 2 + 16, V_TERM = TOKENS * V_ROW;
   static constexpr int RAW = 3 * TOKENS * KD * 4;  // k, q, decays as float32
   static constexpr int LATER = DELTA ? 2 * MATRIX + V_TERMS * V_TERM : 0;  // P o K | V | W on its way out
@@ -196,7 +200,7 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
   pdl_launch_dependents();
   pdl_wait();
   using Z = Prep<T, MODE, KD>;
-  using L = Left<KD>;
+  using L = Left<KD, Prep<T, MODE, KD>::DELTA>;
   constexpr bool DELTA = Z::DELTA;
   constexpr int PER = KD / 32;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -209,7 +213,7 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
   unsigned char* sTt = smem + Z::REGION + 3 * Z::SQUARE;         // (DELTA)
   float* sB = reinterpret_cast<float*>(smem + Z::REGION + (DELTA ? 3 * Z::SQUARE + 3 * Q_TERM : Z::SQUARE));  // [8][KD]: products of the decays of eight tokens
   float* sBeta = sB + 8 * KD;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, head = blockIdx.y, place = blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, head = blockIdx.y, place = p.place0 + blockIdx.x;
 
   // ---- which sequence's tile this is: the last one that begins at or in front of this place
   int seq = -1;
@@ -221,7 +225,7 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
   const int first = p.q_start[seq] + (place - first_tile(p.q_start[seq], seq)) * TOKENS, len = min(TOKENS, p.q_start[seq + 1] - first);
   if (len <= 0) return;
   const int d = p.d, dv = p.dv, kqh = head / (p.heads / p.kq), dvp = padded_columns(dv);
-  unsigned char* left = p.left + ((size_t)place * p.heads + head) * L::bytes(dv, p.cols);
+  unsigned char* left = p.left + ((size_t)blockIdx.x * p.heads + head) * L::bytes(dv, p.cols);
   float* left_u = reinterpret_cast<float*>(left + L::U);
   auto u_at = [&](int r, int col) { return left_u + (col / p.cols) * TOKENS * (p.cols + 4) + r * (p.cols + 4) + col % p.cols; };
   const T* qkv = (const T*)p.qkv;
@@ -775,7 +779,7 @@ __device__ __noinline__ void walk_again(const Params& p, int head, int col0, int
 
 template <int KD, int COLS> struct Walk {
   static constexpr int THREADS = COLS * 8;  // warps: (block of 16 tokens, 16 of the columns) of the products with S0; (quarter of the channels, 16 columns) of S
-  static constexpr int ROW = Left<KD>::ROW, TERM = Left<KD>::TERM, MATRIX = Left<KD>::MATRIX;
+  static constexpr int ROW = Rows<KD>::ROW, TERM = Rows<KD>::TERM, MATRIX = Rows<KD>::MATRIX;
   static constexpr int S_TERM = COLS * ROW;
   static constexpr int W_ROW = COLS * 2 + 16, W_TERM = TOKENS * W_ROW;
   static constexpr int U_ROW = COLS + 4, U_BYTES = TOKENS * U_ROW * 4;
@@ -783,6 +787,16 @@ template <int KD, int COLS> struct Walk {
                        AT_w = AT_S + 3 * S_TERM, AT_BAR = AT_w + 3 * W_TERM, SMEM = AT_BAR + 32;
   static_assert(SMEM <= 227 * 1024, "shared memory");
 };
+
+// The tokens of a sequence's tiles that lie in this pass; false: none.
+__device__ __forceinline__ bool tokens_of_pass(const Params& p, int seq, int& first, int& last) {
+  const int begin = p.q_start[seq], end = p.q_start[seq + 1], at = first_tile(begin, seq);
+  first = begin + max(0, p.place0 - at) * TOKENS;
+  last = min(end, begin + (p.place0 + p.num_places - at) * TOKENS);
+  return first < last;
+}
+// .. and where in p.left they begin
+__device__ __forceinline__ int place_of_pass(const Params& p, int seq) { return max(0, first_tile(p.q_start[seq], seq) - p.place0); }
 
 constexpr unsigned WAIT_LIMIT = 1u << 24;
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, int bytes, uint32_t bar) {
@@ -810,16 +824,16 @@ __global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const __grid_con
   pdl_launch_dependents();
   pdl_wait();
   using Z = Walk<KD, COLS>;
-  using L = Left<KD>;
+  using L = Left<KD, DELTA>;
   constexpr int SLICE = KD / 4, NT = SLICE / 8;  // channels of S of a warp, in accumulators of 16 x 8
   extern __shared__ __align__(128) unsigned char smem[];
   const int seq = p.num_seqs - 1 - blockIdx.z, head = blockIdx.y, col0 = blockIdx.x * COLS;  // (single tokens come first in a step: long portions start first)
-  const int first = p.q_start[seq], last = p.q_start[seq + 1];
-  if (last <= first) return;
+  int first, last;
+  if (!tokens_of_pass(p, seq, first, last)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, mt = warp & 3, half = warp >> 2;
   const int d = p.d, dv = p.dv, inner = p.heads * dv;
   const size_t bytes = L::bytes(dv, COLS);
-  const unsigned char* left = p.left + ((size_t)first_tile(first, seq) * p.heads + head) * bytes;
+  const unsigned char* left = p.left + ((size_t)place_of_pass(p, seq) * p.heads + head) * bytes;
   const float* sU = reinterpret_cast<const float*>(smem + Z::AT_U);
   const float* sP = reinterpret_cast<const float*>(smem + Z::AT_P);
   const uint32_t bar_before = smem_u32(smem + Z::AT_BAR), bar_behind = bar_before + 8;
@@ -1016,7 +1030,7 @@ __global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const __grid_con
 // logarithms, the sums in double and kept as two floats.  Measured against the general kernels, 16 heads of 128, one prompt of 2,048 tokens: 202 -> 135 us (300
 // tokens 36, 64 tokens 25; 32 heads 233); errors against 64 bits o 1.8e-7 and S 1.3e-7 (the tiles of sixteen tokens on the CUDA cores 3.2e-7 and 3.5e-7).
 template <int KD> struct HeadLeft {
-  static constexpr int TERM = Left<KD>::TERM, MATRIX = Left<KD>::MATRIX;
+  static constexpr int TERM = Rows<KD>::TERM, MATRIX = Rows<KD>::MATRIX;
   static constexpr int FACTORS = 576;  // bytes: P fq [64] | (P_last / P) fk [64] | P_last, rounded up
   static constexpr int W = 0, QB = MATRIX, KB = QB + TERM, Q = KB + TERM, F = Q + 3 * Q_TERM, U = F + FACTORS;
   __host__ __device__ static size_t bytes(int dv, int cols) { return (size_t)U + (size_t)((dv + cols - 1) / cols) * TOKENS * (cols + 4) * 4; }
@@ -1024,7 +1038,7 @@ template <int KD> struct HeadLeft {
 
 template <int KD> struct HeadPrep {
   static constexpr int THREADS = 256, WARPS = 8;
-  static constexpr int ROW = Left<KD>::ROW, TERM = Left<KD>::TERM, V_ROW = 128 * 2 + 16, SQUARE = TOKENS * F_ROW * 4;
+  static constexpr int ROW = Rows<KD>::ROW, TERM = Rows<KD>::TERM, V_ROW = 128 * 2 + 16, SQUARE = TOKENS * F_ROW * 4;
   static constexpr int SECOND = TERM > TOKENS * V_ROW ? TERM : TOKENS * V_ROW;  // queries, then values
   static constexpr int AT_Q = TERM, AT_A = AT_Q + SECOND, AT_QM = AT_A + SQUARE, AT_T = AT_QM + SQUARE, AT_TT = AT_T + SQUARE, AT_F = AT_TT + 3 * Q_TERM,
                        SMEM = AT_F + 8 * TOKENS * 4;
@@ -1047,7 +1061,7 @@ __global__ void __launch_bounds__(256, 2) head_prep_kernel(const Params p, int v
   unsigned char* sTk = smem + Z::AT_QM;       // T diag(beta P fk), in the place of Q
   float* fk = reinterpret_cast<float*>(smem + Z::AT_F);  // per token: factor of the key, of the query, beta, sums of log decays (two terms), P, P_last / P, a scratch
   float *fq = fk + TOKENS, *beta = fq + TOKENS, *lh = beta + TOKENS, *lm = lh + TOKENS, *up = lm + TOKENS, *behind = up + TOKENS, *raw = behind + TOKENS;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, head = blockIdx.y, place = blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, head = blockIdx.y, place = p.place0 + blockIdx.x;
   int seq = -1;
   for (int s0 = 0; s0 < p.num_seqs; s0 += Z::THREADS) {
     const int s = s0 + tid;
@@ -1057,7 +1071,7 @@ __global__ void __launch_bounds__(256, 2) head_prep_kernel(const Params p, int v
   const int first = p.q_start[seq] + (place - first_tile(p.q_start[seq], seq)) * TOKENS, len = min(TOKENS, p.q_start[seq + 1] - first);
   if (len <= 0) return;
   const int d = p.d, dv = p.dv, kqh = head / (p.heads / p.kq), dvp = padded_columns(dv), width = 2 * p.kq * d + p.heads * dv;
-  unsigned char* left = p.left + ((size_t)place * p.heads + head) * L::bytes(dv, p.cols);
+  unsigned char* left = p.left + ((size_t)blockIdx.x * p.heads + head) * L::bytes(dv, p.cols);
   float* left_u = reinterpret_cast<float*>(left + L::U);
   float* left_f = reinterpret_cast<float*>(left + L::F);
   const bf16* rows = (const bf16*)p.qkv + (size_t)first * width;
@@ -1252,7 +1266,7 @@ __global__ void __launch_bounds__(256, 2) head_prep_kernel(const Params p, int v
 
 template <int KD, int COLS> struct HeadWalk {
   static constexpr int THREADS = COLS * 8;  // warps as in the walk above
-  static constexpr int ROW = Left<KD>::ROW, TERM = Left<KD>::TERM, MATRIX = Left<KD>::MATRIX;
+  static constexpr int ROW = Rows<KD>::ROW, TERM = Rows<KD>::TERM, MATRIX = Rows<KD>::MATRIX;
   static constexpr int S_TERM = COLS * ROW, W_ROW = COLS * 2 + 16, W_TERM = TOKENS * W_ROW, U_ROW = COLS + 4, U_BYTES = TOKENS * U_ROW * 4;
   static constexpr int BEFORE = MATRIX + TERM, BEHIND = TERM + 3 * Q_TERM + HeadLeft<KD>::FACTORS;  // bytes: W and Q rows; K rows, Q, factors
   static constexpr int AT_W = 0, AT_QB = MATRIX, AT_KB = BEFORE, AT_Q = AT_KB + TERM, AT_F = AT_Q + 3 * Q_TERM, AT_U = AT_F + HeadLeft<KD>::FACTORS,
@@ -1269,12 +1283,12 @@ __global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const __grid_con
   constexpr int SLICE = KD / 4, NT = SLICE / 8;
   extern __shared__ __align__(128) unsigned char smem[];
   const int seq = p.num_seqs - 1 - blockIdx.z, head = blockIdx.y, col0 = blockIdx.x * COLS;
-  const int first = p.q_start[seq], last = p.q_start[seq + 1];
-  if (last <= first) return;
+  int first, last;
+  if (!tokens_of_pass(p, seq, first, last)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, mt = warp & 3, half = warp >> 2;
   const int d = p.d, dv = p.dv, inner = p.heads * dv;
   const size_t bytes = L::bytes(dv, COLS);
-  const unsigned char* left = p.left + ((size_t)first_tile(first, seq) * p.heads + head) * bytes;
+  const unsigned char* left = p.left + ((size_t)place_of_pass(p, seq) * p.heads + head) * bytes;
   const float* sU = reinterpret_cast<const float*>(smem + Z::AT_U);
   const float* sF = reinterpret_cast<const float*>(smem + Z::AT_F);
   const uint32_t bar_before = smem_u32(smem + Z::AT_BAR), bar_behind = bar_before + 8;
@@ -1478,8 +1492,6 @@ template <typename K> cudaError_t allow(K kernel, int smem, OncePerDevice& done)
   return e;
 }
 
-inline int places(int n, int num_seqs) { return n / TOKENS + num_seqs + 1; }
-
 int* error_flag_device = nullptr;
 int* error_flag_host = nullptr;
 
@@ -1504,7 +1516,7 @@ template <typename T, int MODE, int KD> int launch(const Params& params, cudaStr
   p.vec_v = width % 8 == 0 && (2 * p.kq * p.d) % 8 == 0 && p.dv % 8 == 0 && ((uintptr_t)p.qkv & 15) == 0;
   static OncePerDevice prep;
   cudaError_t e = allow(tile_prep_kernel<T, MODE, KD>, Z::SMEM, prep);
-  if (e == cudaSuccess) e = launch_pdl((tile_prep_kernel<T, MODE, KD>), dim3(places(p.n, p.num_seqs), p.heads), dim3(Z::THREADS), (size_t)Z::SMEM, stream, 1, p);
+  if (e == cudaSuccess) e = launch_pdl((tile_prep_kernel<T, MODE, KD>), dim3(p.num_places, p.heads), dim3(Z::THREADS), (size_t)Z::SMEM, stream, 1, p);
   if (e == cudaSuccess) e = p.cols == 16 ? launch_walk<KD, 16, MODE != BONUS>(p, stream) : launch_walk<KD, 32, MODE != BONUS>(p, stream);
   return (int)e;
 }
@@ -1520,7 +1532,7 @@ template <int KD> int launch_head(const Params& p, cudaStream_t stream) {
   static OncePerDevice done;
   cudaError_t e = allow(head_prep_kernel<KD>, Z::SMEM, done);
   const int width = 2 * p.kq * p.d + p.heads * p.dv, vec = width % 8 == 0 && p.d % 8 == 0 && p.dv % 8 == 0 && ((uintptr_t)p.qkv & 15) == 0;  // 16-byte runs
-  if (e == cudaSuccess) e = launch_pdl((head_prep_kernel<KD>), dim3(places(p.n, p.num_seqs), p.heads), dim3(Z::THREADS), (size_t)Z::SMEM, stream, 1, p, vec);
+  if (e == cudaSuccess) e = launch_pdl((head_prep_kernel<KD>), dim3(p.num_places, p.heads), dim3(Z::THREADS), (size_t)Z::SMEM, stream, 1, p, vec);
   if (e == cudaSuccess) e = p.cols == 16 ? launch_head_walk<KD, 16>(p, stream) : launch_head_walk<KD, 32>(p, stream);
   return (int)e;
 }
@@ -1540,21 +1552,27 @@ template <typename T> int launch_mode(int mode, const Params& p, cudaStream_t st
 
 }  // namespace
 
-// Bytes of scratch for a step of n tokens in num_seqs sequences.
-DLI_EXPORT long long dli_recurrence_tiles_scratch(int n, int num_seqs, int heads, int d, int dv) {
+// Places of a step of n tokens in num_seqs sequences, and the bytes of scratch that a place takes with all heads.  A step whose places do not fit
+// the caller's scratch goes in several passes, one call for each.
+DLI_EXPORT int dli_recurrence_tiles_places(int n, int num_seqs) { return places(n, num_seqs); }
+DLI_EXPORT long long dli_recurrence_tiles_place_bytes(int mode, int num_seqs, int heads, int d, int dv, int dtype) {
   const int cols = columns(heads, num_seqs, dv);
-  const size_t each = d <= 64 ? Left<64>::bytes(dv, cols) : Left<128>::bytes(dv, cols);
-  return (long long)((size_t)places(n, num_seqs) * heads * each);
+  size_t each;
+  if (mode == HEAD_DELTA && dtype != DLI_F32) each = d <= 64 ? HeadLeft<64>::bytes(dv, cols) : HeadLeft<128>::bytes(dv, cols);
+  else if (mode == BONUS) each = d <= 64 ? Left<64, false>::bytes(dv, cols) : Left<128, false>::bytes(dv, cols);
+  else each = d <= 64 ? Left<64, true>::bytes(dv, cols) : Left<128, true>::bytes(dv, cols);
+  return (long long)(each * heads);
 }
 
 // mode 0: gated delta rule (qkv, u with b_col and a_col, dt_bias and a_log per head); 1: a decay per channel (a [n][heads d], dt_bias [heads d]);
-// 2: bonus (qkv: the slabs r | k | v, a: the decays' products, dt_bias: w0, bonus [heads][d]; kq = heads, dv = d).
+// 2: bonus (qkv: the slabs r | k | v, a: the decays' products, dt_bias: w0, bonus [heads][d]; kq = heads, dv = d).  Takes the tiles at places
+// place0 .. place0 + num_places - 1; scratch has room for num_places.
 DLI_EXPORT int dli_recurrence_tiles(int mode, float* o, const void* qkv, const void* u, long long u_stride, int b_col, int a_col, const void* a,
                                     const float* dt_bias, const float* a_log, const float* bonus, float* state, const int* q_start,
-                                    const int* state_slot, void* scratch, int n, int num_seqs, int heads, int kq, int d, int dv, float unit_eps,
-                                    int dtype, cudaStream_t stream) {
+                                    const int* state_slot, void* scratch, int place0, int num_places, int n, int num_seqs, int heads, int kq, int d, int dv,
+                                    float unit_eps, int dtype, cudaStream_t stream) {
   if (num_seqs == 0 || n == 0) return 0;
-  if (mode < 0 || mode > 2 || heads < 1 || heads > 65535 || kq < 1 || heads % kq || d < 1 || d > 128 || dv < 1 || dv > 128 || num_seqs > 65535 || !scratch ||
+  if (mode < 0 || mode > 2 || heads < 1 || heads > 65535 || kq < 1 || heads % kq || d < 1 || d > 128 || dv < 1 || dv > 128 || num_seqs > 65535 || !scratch || place0 < 0 || num_places < 1 ||
       ((uintptr_t)scratch & 15) || ((uintptr_t)o & 7) || (mode == BONUS && (dv != d || kq != heads || !bonus)))
     return DLI_ERR_UNSUPPORTED;
   if (!error_flag_host) {
@@ -1563,6 +1581,7 @@ DLI_EXPORT int dli_recurrence_tiles(int mode, float* o, const void* qkv, const v
     if (cudaHostGetDevicePointer((void**)&error_flag_device, error_flag_host, 0) != cudaSuccess) return (int)cudaGetLastError();
   }
   Params p;
+  p.place0 = place0; p.num_places = num_places;
   p.mode = mode; p.f32 = dtype == DLI_F32;
   p.o = o; p.qkv = qkv; p.u = u; p.a = a; p.u_stride = u_stride; p.b_col = b_col; p.a_col = a_col; p.dt_bias = dt_bias; p.a_log = a_log; p.bonus = bonus;
   p.state = state; p.q_start = q_start; p.state_slot = state_slot; p.n = n; p.num_seqs = num_seqs; p.heads = heads; p.kq = kq; p.d = d; p.dv = dv;

@@ -1370,6 +1370,9 @@ def gated_group_rmsnorm(out: torch.Tensor, y: torch.Tensor, u: torch.Tensor, z_c
 DELTA_MAX_HEAD_DIM = 512
 TILES_MAX_HEAD_DIM = 128  # of keys and of values, in csrc/recurrence_tiles.cu
 TILES_MIN_TOKENS = 33  # shorter portions are walked
+# Bytes that the tiles of one pass may leave for the kernel that walks them; a longer step goes in several passes.  A tile and head of 128 takes 209 KB
+# with a decay per channel, 140 with a decay per head in bfloat16, 157 with a bonus: 8,192 tokens of 32 heads are one pass of the first kind.
+TILES_SCRATCH_LIMIT = 1 << 30
 
 
 def recurrence_form(d: int, dv: int, max_len: int, n: int, num_seqs: int, heads: int, on_gpu: bool = True) -> str:
@@ -1391,16 +1394,20 @@ def _recurrence_tiles(mode: int, what: str, o: torch.Tensor, qkv: torch.Tensor, 
                       dt_bias: torch.Tensor, a_log: torch.Tensor | None, bonus: torch.Tensor | None, state: torch.Tensor, q_start: torch.Tensor,
                       state_slot: torch.Tensor, kq: int, unit_eps: float) -> None:
     _, heads, dv, d = state.shape
-    n, count = o.shape[0], state_slot.numel()
-    size = _fn("recurrence_tiles.cu", "dli_recurrence_tiles_scratch", [c_int] * 5)
+    n, count, dtype = o.shape[0], state_slot.numel(), DT_CODE[qkv.dtype]
+    places = _fn("recurrence_tiles.cu", "dli_recurrence_tiles_places", [c_int] * 2)(n, count)
+    size = _fn("recurrence_tiles.cu", "dli_recurrence_tiles_place_bytes", [c_int] * 6)
     size.restype = c_longlong
-    scratch = torch.empty(size(n, count, heads, d, dv), dtype=torch.uint8, device=o.device)  # what the first kernel leaves for every tile and head
-    f = _fn("recurrence_tiles.cu", "dli_recurrence_tiles", [c_int, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int] + [c_void_p] * 8 + [c_int] * 6
+    each = size(mode, count, heads, d, dv, dtype)
+    run = max(1, min(places, TILES_SCRATCH_LIMIT // each))
+    scratch = torch.empty(run * each, dtype=torch.uint8, device=o.device)  # what the first kernel leaves for every tile and head
+    f = _fn("recurrence_tiles.cu", "dli_recurrence_tiles", [c_int, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int] + [c_void_p] * 8 + [c_int] * 8
             + [c_float, c_int, c_void_p])
-    _check(f(mode, _ptr(o), _ptr(qkv), _ptr(u), 0 if u is None else u.stride(0), b_col, a_col, _ptr(a), _ptr(dt_bias), _ptr(a_log), _ptr(bonus), _ptr(state),
-             _ptr(q_start), _ptr(state_slot), _ptr(scratch), n, count, heads, kq, d, dv, unit_eps, DT_CODE[qkv.dtype], _stream()), what)
     global launch_count
-    launch_count += 1  # two kernels
+    for place in range(0, places, run):
+        _check(f(mode, _ptr(o), _ptr(qkv), _ptr(u), 0 if u is None else u.stride(0), b_col, a_col, _ptr(a), _ptr(dt_bias), _ptr(a_log), _ptr(bonus), _ptr(state),
+                 _ptr(q_start), _ptr(state_slot), _ptr(scratch), place, min(run, places - place), n, count, heads, kq, d, dv, unit_eps, dtype, _stream()), what)
+        launch_count += 1  # two kernels
 
 
 def delta_rule_scan(o: torch.Tensor, qkv: torch.Tensor, u: torch.Tensor, b_col: int, a_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor,

@@ -176,6 +176,37 @@ def test_infinities_and_nans_stay_where_the_recurrence_has_them(kind, dtype, d, 
     assert _same_kind(o, want[0], 2e-6) and _same_kind(st, want[1], 2e-6)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,dtype,least", [("head", torch.bfloat16, 140e3), ("channel", torch.bfloat16, 210e3), ("bonus", torch.bfloat16, 158e3), ("head", torch.float32, 210e3)])
+def test_a_step_whose_tiles_outgrow_the_scratch_goes_in_passes(kind, dtype, least, monkeypatch):
+    """The scratch is that of the tiles' kind and no larger than its limit; the state between two passes waits in its slot, so nothing changes."""
+    H, d, lens = 4, 128, [1, 200, 0, 64, 0, 130]
+    g, n = torch.Generator().manual_seed(17), sum(lens)
+    qkv = torch.randn(4, n, H * d, generator=g) if kind == "bonus" else torch.randn(n, 3 * H * d, generator=g)
+    u, a = torch.randn(n, 2 * H, generator=g).to(dtype).cuda(), torch.randn(n, H * d, generator=g).to(dtype).cuda()
+    qkv, start = qkv.to(dtype).cuda(), torch.randn(len(lens), H, d, d, generator=g).cuda()
+    bias, a_log, bonus = (torch.randn(H if kind == "head" else H * d, generator=g) - 3.0).cuda(), torch.zeros(H).cuda(), torch.randn(H, d, generator=g).cuda()
+    q_start, slot = _starts(lens).cuda(), torch.arange(len(lens), dtype=torch.int32, device="cuda")
+    seq, got, calls = torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens)).int().cuda(), [], []
+    for limit in (1 << 30, 1):
+        monkeypatch.setattr(ops, "TILES_SCRATCH_LIMIT", limit)
+        o, state = torch.zeros(n, H * d).cuda(), start.clone()
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before, launched = torch.cuda.memory_allocated(), ops.launch_count
+        if kind == "bonus":
+            ops.shift_decay_scan(o, qkv, a, bias, "bonus", bonus, state, q_start, slot, max_len=200, form="tiles")
+        elif kind == "channel":
+            ops.channel_delta_scan(o, qkv, u, 0, a, bias, a_log, state, q_start, slot, H, 1e-6, max_len=200, form="tiles")
+        else:
+            ops.delta_rule_scan(o, qkv, u, 0, H, bias, a_log, state, seq, q_start, slot, H, d, 1e-6, max_len=200, form="tiles")
+        places = n // 64 + len(lens) + 1
+        assert torch.cuda.max_memory_allocated() - before <= (places if limit > 1 else 1) * H * least + (1 << 20)  # (the allocator may hand out a block up to 1 MiB larger)
+        calls.append(ops.launch_count - launched)
+        got.append((o, state))
+    assert calls[1] == places * calls[0] and all(torch.equal(x, y) for x, y in zip(*got))
+
+
 def test_which_form_serves_a_step():
     form = ops.recurrence_form
     assert form(128, 128, 2048, 2048, 1, 16) == form(64, 64, 4096, 4096, 1, 16) == form(128, 128, 2100, 3500, 2, 16) == form(128, 128, 1 << 30, 2048, 1, 32) == "tiles"
