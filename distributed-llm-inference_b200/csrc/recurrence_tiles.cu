@@ -71,6 +71,7 @@ struct Params {
   int cols;  // value columns of a CTA of the second kernel: 16 or 32
   int vec;   // rows of queries, keys and decays are whole (d = KD) and aligned: a lane's channels come in one load
   int vec_v; // rows of values lie in 16-byte runs
+  int pairs; // two read-outs side by side lie on an 8-byte boundary
   int place0, num_places;  // the places that this pass takes; a sequence's state waits in its slot between two passes
   unsigned char* left;     // what the first kernel leaves, from place0 on
   int* error_flag;
@@ -976,7 +977,7 @@ __global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const __grid_con
             float* dst = p.o + (size_t)(base + r) * inner + (size_t)head * dv + col;
             const float x = O[nt][2 * hf] + (qs[nt][2 * hf] + ql[nt][2 * hf]), y = O[nt][2 * hf + 1] + (qs[nt][2 * hf + 1] + ql[nt][2 * hf + 1]);
             finite = fmaf(x, 0.f, fmaf(y, 0.f, finite));
-            if ((dv & 1) == 0) {
+            if (p.pairs) {
               if (col < dv) *reinterpret_cast<float2*>(dst) = make_float2(x, y);
             } else {
               if (col < dv) dst[0] = x;
@@ -1438,7 +1439,7 @@ __global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const __grid_con
             float* dst = p.o + (size_t)(base + r) * inner + (size_t)head * dv + col;
             const float x = fmaf(f, O[nt][2 * hf], qs[nt][2 * hf] + ql[nt][2 * hf]), y = fmaf(f, O[nt][2 * hf + 1], qs[nt][2 * hf + 1] + ql[nt][2 * hf + 1]);
             finite = fmaf(x, 0.f, fmaf(y, 0.f, finite));
-            if ((dv & 1) == 0) {
+            if (p.pairs) {
               if (col < dv) *reinterpret_cast<float2*>(dst) = make_float2(x, y);
             } else {
               if (col < dv) dst[0] = x;
@@ -1573,7 +1574,7 @@ DLI_EXPORT int dli_recurrence_tiles(int mode, float* o, const void* qkv, const v
                                     float unit_eps, int dtype, cudaStream_t stream) {
   if (num_seqs == 0 || n == 0) return 0;
   if (mode < 0 || mode > 2 || heads < 1 || heads > 65535 || kq < 1 || heads % kq || d < 1 || d > 128 || dv < 1 || dv > 128 || num_seqs > 65535 || !scratch || place0 < 0 || num_places < 1 ||
-      ((uintptr_t)scratch & 15) || ((uintptr_t)o & 7) || (mode == BONUS && (dv != d || kq != heads || !bonus)))
+      ((uintptr_t)scratch & 15) || (mode == BONUS && (dv != d || kq != heads || !bonus)))
     return DLI_ERR_UNSUPPORTED;
   if (!error_flag_host) {
     if (cudaHostAlloc((void**)&error_flag_host, sizeof(int), cudaHostAllocMapped) != cudaSuccess) return (int)cudaGetLastError();
@@ -1585,7 +1586,7 @@ DLI_EXPORT int dli_recurrence_tiles(int mode, float* o, const void* qkv, const v
   p.mode = mode; p.f32 = dtype == DLI_F32;
   p.o = o; p.qkv = qkv; p.u = u; p.a = a; p.u_stride = u_stride; p.b_col = b_col; p.a_col = a_col; p.dt_bias = dt_bias; p.a_log = a_log; p.bonus = bonus;
   p.state = state; p.q_start = q_start; p.state_slot = state_slot; p.n = n; p.num_seqs = num_seqs; p.heads = heads; p.kq = kq; p.d = d; p.dv = dv;
-  p.unit_eps = unit_eps; p.vec = p.vec_v = 0; p.cols = columns(heads, num_seqs, dv); p.left = (unsigned char*)scratch; p.error_flag = error_flag_device;
+  p.unit_eps = unit_eps; p.vec = p.vec_v = 0; p.pairs = dv % 2 == 0 && ((uintptr_t)o & 7) == 0; p.cols = columns(heads, num_seqs, dv); p.left = (unsigned char*)scratch; p.error_flag = error_flag_device;
   return dtype == DLI_F32 ? launch_mode<float>(mode, p, stream) : launch_mode<bf16>(mode, p, stream);
 }
 

@@ -1318,7 +1318,8 @@ def ssm_scan(y: torch.Tensor, xbc: torch.Tensor, u: torch.Tensor, dt_col: int, d
             or heads % groups or N > SSM_SCAN_MAX_STATE or dt_bias.numel() != heads or a_log.numel() != heads or d_skip.numel() != heads
             or q_start.numel() != state_slot.numel() + 1):
         raise KernelError(f"ssm_scan: shapes do not agree (or the state size is above {SSM_SCAN_MAX_STATE})")
-    form = form or ssm_scan_form(u.dtype, P, N, max_len, xbc.data_ptr() % 16 == 0)
+    # (a state off its 16-byte boundary is not walked either: the tensor-core form refuses it)
+    form = form or ssm_scan_form(u.dtype, P, N, max_len, xbc.data_ptr() % 16 == 0 and y.data_ptr() % 8 == 0)
     if form == "chunk":
         if u.dtype != torch.bfloat16 or segments < 0:
             raise KernelError("ssm_scan: the tensor-core form takes bfloat16")

@@ -177,6 +177,24 @@ def test_infinities_and_nans_stay_where_the_recurrence_has_them(kind, dtype, d, 
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("channel,dtype", [(False, torch.bfloat16), (False, torch.float32), (True, torch.bfloat16)])
+def test_read_outs_off_an_8_byte_boundary(channel, dtype):
+    H, d, n = 2, 16, 100
+    g = torch.Generator().manual_seed(3)
+    qkv, u, a = (torch.randn(n, c, generator=g).to(dtype) for c in (3 * H * d, 2 * H + 1, H * d))
+    bias, a_log, state = torch.randn(H * d if channel else H, generator=g), torch.zeros(H), torch.randn(1, H, d, d, generator=g)
+    want = _delta(channel, qkv, u, a, bias, a_log, state, [n], H)
+    room, st = torch.zeros(n * H * d + 1).cuda(), state.cuda()
+    o, q_start, slot = room[1:].view(n, H * d), torch.tensor([0, n], dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda()
+    qkv, u, a, bias, a_log = (x.cuda() for x in (qkv, u, a, bias, a_log))
+    if channel:
+        ops.channel_delta_scan(o, qkv, u, 1, a, bias, a_log, st, q_start, slot, H, 1e-6, max_len=n, form="tiles")
+    else:
+        ops.delta_rule_scan(o, qkv, u, 1, 1 + H, bias, a_log, st, torch.zeros(n, dtype=torch.int32).cuda(), q_start, slot, H, d, 1e-6, max_len=n, form="tiles")
+    assert all((x.cpu().double() - y).norm() <= 2e-6 * y.norm() for x, y in ((o, want[0]), (st, want[1]))) and room[0] == 0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("kind,dtype,least", [("head", torch.bfloat16, 140e3), ("channel", torch.bfloat16, 210e3), ("bonus", torch.bfloat16, 158e3), ("head", torch.float32, 210e3)])
 def test_a_step_whose_tiles_outgrow_the_scratch_goes_in_passes(kind, dtype, least, monkeypatch):
     """The scratch is that of the tiles' kind and no larger than its limit; the state between two passes waits in its slot, so nothing changes."""

@@ -107,6 +107,20 @@ def test_infinities_and_nans_stay_where_the_recurrence_has_them(where, value, ba
 
 
 @pytest.mark.gpu
+def test_read_outs_off_an_8_byte_boundary_are_walked():
+    H, P, N, n = 2, 16, 16, 100
+    g = torch.Generator().manual_seed(3)
+    xbc, u, state = torch.randn(n, H * P + 2 * N, generator=g).bfloat16(), torch.randn(n, H, generator=g).bfloat16(), torch.randn(1, H, P, N, generator=g)
+    zero = torch.zeros(H)
+    want = _exact(xbc, u, 0, zero, zero, zero, state.clone(), [n], 1)
+    room, st = torch.zeros(n * H * P + 1).cuda(), state.cuda()
+    y = room[1:].view(n, H * P)
+    ops.ssm_scan(y, xbc.cuda(), u.cuda(), 0, zero.cuda(), zero.cuda(), zero.cuda(), st, torch.tensor([0, n], dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda(), 1,
+                 max_len=n)
+    assert all((a.cpu().double() - b).norm() <= 2e-6 * b.norm() for a, b in ((y, want[0]), (st, want[1]))) and room[0] == 0
+
+
+@pytest.mark.gpu
 def test_a_tile_may_be_replayed_from_a_graph():
     H, P, N, lens = 2, 64, 64, [1, 200]
     xbc, u = torch.randn(201, H * P + 2 * N).bfloat16().cuda(), torch.randn(201, H).bfloat16().cuda()
