@@ -157,6 +157,16 @@ __device__ __forceinline__ bool wait_or_fail(uint32_t bar, uint32_t parity, vola
   return false;
 }
 
+// For a kernel that gives up: what it still has under way on this barrier may not land in shared or tensor memory that is no longer its own.
+__device__ __forceinline__ void wait_for_last(uint32_t bar, uint32_t parity) {
+  for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    if (done) return;
+  }
+}
+
 // 320 threads, one CTA per SM.  Warps 0..7 do the softmax: thread t works on row (t & 127); its half
 // (t >> 7) owns 64 of the tile's 128 key columns and 32 of the 64 output columns (warps w and w + 4
 // read the same 32 lanes of tensor memory: the lane group is the warp index modulo 4).  Warp 8 issues
@@ -973,7 +983,7 @@ __global__ void __launch_bounds__(DIFF_THREADS, 1) paged_prefill_diff_kernel(con
       const bool need = lane < 16 && t < num_tiles && page_i < pages && first < hi && (first + p.page_size > lo || first < p.keep_first);
       return need ? table[first / p.page_size] : -1;
     };
-    int page = lookup(0);
+    int page = lookup(0), asked = 0;  // tiles whose copies were asked for
     for (int t = 0; t < num_tiles && !*failed; ++t) {
       const int st = t & 1, par = ((t - 2) >> 1) & 1;
       const int cur = page;
@@ -991,7 +1001,10 @@ __global__ void __launch_bounds__(DIFF_THREADS, 1) paged_prefill_diff_kernel(con
         for (int sl = 0; sl < 2; ++sl)
           tma_load_2d(smem_u32(stage0 + st * K_BYTES + sl * TILE_BYTES + page_i * p.page_size * 128), map, sl * 64, (cur * p.nkv + kvh) * p.page_size, full + 8 * st);
       }
+      ++asked;
     }
+    if (*failed && lane == 0)
+      for (int t = max(0, asked - 2); t < asked; ++t) wait_for_last(full + 8 * (t & 1), (t >> 1) & 1);
   } else if (warp == QT * ROWS / 32 || warp == QT * ROWS / 32 + 2) {
     // ================================================================ the warps that issue the matrix products (their first lanes): one per map
     const int q = warp == QT * ROWS / 32 ? 0 : 1;
@@ -1009,12 +1022,14 @@ __global__ void __launch_bounds__(DIFF_THREADS, 1) paged_prefill_diff_kernel(con
         umma_commit(k_free + 8 * (t & 1));  // this tile's product with K(t) is issued
       };
       bool ok = num_tiles > 0 && wait_or_fail(k_full, 0, failed, 17, p.error_flag);
-      if (ok) scores(0);
+      int scored = 0, summed = 0;  // tiles whose products were issued
+      if (ok) { scores(0); ++scored; }
       for (int t = 0; t < num_tiles && ok; ++t) {
         if (t + 1 < num_tiles) {  // the keys are there and the thread of every row has S_q(t) in registers
           ok = wait_or_fail(k_full + 8 * ((t + 1) & 1), ((t + 1) >> 1) & 1, failed, 17, p.error_flag) && wait_or_fail(s_read + 8 * q, t & 1, failed, 18, p.error_flag);
           if (!ok) break;
           scores(t + 1);
+          ++scored;
         }
         // O_q += P_q(t) V(t)
         ok = wait_or_fail(p_ready + 8 * q, t & 1, failed, 19, p.error_flag) && wait_or_fail(v_full + 8 * (t & 1), (t >> 1) & 1, failed, 20, p.error_flag);
@@ -1026,6 +1041,11 @@ __global__ void __launch_bounds__(DIFF_THREADS, 1) paged_prefill_diff_kernel(con
           umma(tmem_o + q * HV, smem_desc_sw128(pa + (k >> 2) * TILE_BYTES + (k & 3) * 32), smem_desc_sw128(v + k * 2048) | next_slab, idesc_o, (t | k) != 0);
         umma_commit(o_done + 8 * q);
         umma_commit(v_free + 8 * (t & 1));  // this tile's product with V(t) is issued
+        ++summed;
+      }
+      if (!ok) {
+        if (scored > 0) wait_for_last(s_done + 8 * q, (scored - 1) & 1);
+        if (summed > 0) wait_for_last(o_done + 8 * q, (summed - 1) & 1);
       }
     }
     __syncwarp();
@@ -1368,7 +1388,7 @@ __global__ void __launch_bounds__(THREADS, 1) paged_prefill_row_kernel(const __g
       const bool need = lane < 16 && t < t_end && page_i < pages && first < hi && first + p.page_size > lo;
       return need ? table[first / p.page_size] : -1;
     };
-    int page = lookup(t_begin);
+    int page = lookup(t_begin), asked = 0;  // tiles whose copies were asked for
     for (int t = 0; t < num_tiles && !*failed; ++t) {
       const int st = t & 1, cur = page;
       page = lookup(t_begin + t + 1);
@@ -1385,7 +1405,10 @@ __global__ void __launch_bounds__(THREADS, 1) paged_prefill_row_kernel(const __g
         for (int sl = 0; sl < SLABS; ++sl)
           tma_load_2d(smem_u32(sK + st * Cfg::STAGE + sl * TILE_BYTES + page_i * p.page_size * 128), &map, sl * 64, (cur * p.nkv + kvh) * p.page_size, k_full + 8 * st);
       }
+      ++asked;
     }
+    if (*failed && lane == 0)
+      for (int t = max(0, asked - 2); t < asked; ++t) wait_for_last(k_full + 8 * (t & 1), (t >> 1) & 1);
   } else if (warp == SOFTMAX_THREADS / 32) {
     // ================================================================ the thread that issues the matrix products
     if (lane == 0) {
@@ -1428,6 +1451,10 @@ __global__ void __launch_bounds__(THREADS, 1) paged_prefill_row_kernel(const __g
         } else {
           __nanosleep(20);
         }
+      }
+      if (o_next < num_tiles) {
+        for (int t = max(0, s_next - 2); t < s_next; ++t) wait_for_last(s_done + 8 * (t & 1), (t >> 1) & 1);
+        for (int t = max(0, o_next - 2); t < o_next; ++t) wait_for_last(o_done + 8 * (t & 1), (t >> 1) & 1);
       }
     }
     __syncwarp();

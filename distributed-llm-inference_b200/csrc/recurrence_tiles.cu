@@ -806,18 +806,26 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, int byt
 __device__ __forceinline__ void expect_bytes(uint32_t bar, int bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Waits for copies, WAIT_LIMIT polls at most: then the kernel says so in *error_flag and goes on with what is there (the step's results
-// are not to be trusted); once one wait has run out, the later ones are short.
-__device__ __forceinline__ void wait_copies(uint32_t bar, uint32_t parity, volatile int* failed, int* error_flag) {
+__device__ __forceinline__ bool copies_arrived(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done;
+}
+// Waits for copies, WAIT_LIMIT polls at most; false: they did not arrive, here or for another thread, and *error_flag says so.
+__device__ __forceinline__ bool wait_copies(uint32_t bar, uint32_t parity, volatile int* failed, int* error_flag) {
   for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
-    uint32_t done;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    if (done) return;
-    if ((i & 1023) == 1023 && *failed) return;
+    if (copies_arrived(bar, parity)) return true;
+    if ((i & 1023) == 1023 && *failed) return false;
   }
   *failed = 1;
   atomicExch(error_flag, 1);
+  return false;
+}
+// For a CTA that gives up: the copies that it still has under way (`issued` so far on this barrier) may not land in shared memory that is no longer its own.
+__device__ __noinline__ void wait_for_last(uint32_t bar, int issued) {
+  for (unsigned i = 0; issued > 0 && i < WAIT_LIMIT; ++i)
+    if (copies_arrived(bar, (issued - 1) & 1)) return;
 }
 
 template <int KD, int COLS, bool DELTA>
@@ -886,6 +894,8 @@ __global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const __grid_con
   const uint32_t pk_addr = smem_u32(smem + Z::AT_PK) + ((lane & 7) + ((lane >> 3) & 1) * 8) * Z::ROW + (slice0 + (lane >> 4) * 8) * 2;
 
   float finite = 0.f;  // 0 while every result was finite, NaN from the first one on that was not
+  bool ok = true;      // every copy has arrived
+  int before = 1, behind = 0;  // loads so far
   uint32_t parity = 0;
   for (int base = first; base < last; base += TOKENS, parity ^= 1) {
     const int len = min(TOKENS, last - base);
@@ -901,9 +911,10 @@ __global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const __grid_con
         for (int s = 0; s < 3; ++s)
           *reinterpret_cast<uint32_t*>(smem + Z::AT_S + s * Z::S_TERM + (c_lo + hf * 8) * Z::ROW + (slice0 + j * 8 + kcol) * 2) = t[s];
       }
-    __syncthreads();  // S0 is there; the operands behind (of the tile before) have been read
+    if (__syncthreads_or(!ok)) break;  // S0 is there; the operands behind (of the tile before) have been read
     load_behind(left);
-    wait_copies(bar_before, parity, failed, p.error_flag);
+    ++behind;
+    ok = wait_copies(bar_before, parity, failed, p.error_flag);
     float O[2][4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) O[0][e] = O[1][e] = 0.f;
@@ -949,10 +960,10 @@ __global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const __grid_con
         }
       }
     }
-    __syncthreads();  // w is there; S0 and the operands in front have been read
+    if (__syncthreads_or(!ok)) break;  // w is there; S0 and the operands in front have been read
     left += (size_t)p.heads * bytes;
-    if (base + TOKENS < last) load_before(left);
-    wait_copies(bar_behind, parity, failed, p.error_flag);
+    if (base + TOKENS < last) { load_before(left); ++before; }
+    ok = wait_copies(bar_behind, parity, failed, p.error_flag);
     // ---- the read-outs
     if (active) {
       float ql[2][4], qs[2][4];
@@ -1014,6 +1025,13 @@ __global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const __grid_con
 #pragma unroll
       for (int e = 0; e < 4; ++e) S[j][e] = fmaf((e & 1) ? g.y : g.x, S[j][e], ds[j][e] + dl[j][e]);
     }
+  }
+  if (__syncthreads_or(!ok)) {  // (the state stays as it was)
+    if (tid == 0) {
+      wait_for_last(bar_before, before);
+      wait_for_last(bar_behind, behind);
+    }
+    return;
   }
   each([&](float& x, bool, size_t) { finite = fmaf(x, 0.f, finite); });
   if (__syncthreads_or(finite != 0.f)) {  // (also: nobody writes a read-out behind this)
@@ -1340,6 +1358,8 @@ __global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const __grid_con
   const uint32_t kb_addr = smem_u32(smem + Z::AT_KB) + ((lane & 7) + ((lane >> 3) & 1) * 8) * Z::ROW + (slice0 + (lane >> 4) * 8) * 2;
 
   float finite = 0.f;  // 0 while every result was finite, NaN from the first one on that was not
+  bool ok = true;      // every copy has arrived
+  int before = 1, behind = 0;  // loads so far
   uint32_t parity = 0;
   for (int base = first; base < last; base += TOKENS, parity ^= 1) {
     const int len = min(TOKENS, last - base);
@@ -1354,9 +1374,10 @@ __global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const __grid_con
         for (int s = 0; s < 3; ++s)
           *reinterpret_cast<uint32_t*>(smem + Z::AT_S + s * Z::S_TERM + (c_lo + hf * 8) * Z::ROW + (slice0 + j * 8 + kcol) * 2) = t[s];
       }
-    __syncthreads();  // S0 is there; the operands behind (of the tile before) have been read
+    if (__syncthreads_or(!ok)) break;  // S0 is there; the operands behind (of the tile before) have been read
     load_behind(left);
-    wait_copies(bar_before, parity, failed, p.error_flag);
+    ++behind;
+    ok = wait_copies(bar_before, parity, failed, p.error_flag);
     float O[2][4], w[2][4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) O[0][e] = O[1][e] = w[0][e] = w[1][e] = 0.f;
@@ -1393,7 +1414,7 @@ __global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const __grid_con
         }
       }
     }
-    wait_copies(bar_behind, parity, failed, p.error_flag);
+    ok = wait_copies(bar_behind, parity, failed, p.error_flag) && ok;
     if (active) {
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt)
@@ -1411,9 +1432,9 @@ __global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const __grid_con
           }
         }
     }
-    __syncthreads();  // w is there; S0 and the operands in front have been read
+    if (__syncthreads_or(!ok)) break;  // w is there; S0 and the operands in front have been read
     left += (size_t)p.heads * bytes;
-    if (base + TOKENS < last) load_before(left);
+    if (base + TOKENS < last) { load_before(left); ++before; }
     // ---- the read-outs
     if (active) {
       float ql[2][4], qs[2][4];
@@ -1477,6 +1498,13 @@ __global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const __grid_con
     for (int j = 0; j < NT; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) S[j][e] = fmaf(g, S[j][e], ds[j][e] + dl[j][e]);
+  }
+  if (__syncthreads_or(!ok)) {  // (the state stays as it was)
+    if (tid == 0) {
+      wait_for_last(bar_before, before);
+      wait_for_last(bar_behind, behind);
+    }
+    return;
   }
   each([&](float& x, bool, size_t) { finite = fmaf(x, 0.f, finite); });
   if (__syncthreads_or(finite != 0.f)) {  // (also: nobody writes a read-out behind this)
