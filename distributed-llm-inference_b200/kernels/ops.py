@@ -1376,16 +1376,43 @@ TILES_MIN_TOKENS = 33  # shorter portions are walked
 TILES_SCRATCH_LIMIT = 1 << 30
 
 
-def recurrence_form(d: int, dv: int, max_len: int, n: int, num_seqs: int, heads: int, on_gpu: bool = True) -> str:
-    """Which kernels serve a step of a delta rule or of the token-shift recurrence: ``"tiles"`` (portions: tiles of 64 tokens on the tensor
-    cores) or ``"walk"`` (decode steps, short portions, larger heads).
+# What a step of a recurrence costs, us, fitted to 570 measured steps of each kind (4 to 64 heads of 64 and 128; 1 to 32 portions of 33 to 1,500 tokens
+# beside 0 to 64 single tokens).  Walk: a launch or two, a chain of tokens as long as the longest sequence, and all tokens of all heads; the
+# exponents say how the last two go with the head size over 128.  Tiles: preparing all tiles (a CTA an SM), then a chain of tiles, or as
+# many chains as SMs have to take one after the other; the exponent as before.  Singles: what a walk of single tokens adds to tiles of the portions, a launch or
+# two and 2^20 numbers of state.
+RECURRENCE_COSTS = {"channel": {"walk": (10.0, 0.41, 0.28, 1.2, 2.3), "tiles": (0.0, 25.0, 1.2, 4.6, 0.45), "singles": (10.7, 3.9)},
+                    "bonus": {"walk": (6.5, 0.45, 0.54, 1.2, 2.5), "tiles": (5.2, 14.0, 0.0, 3.8, 0.59)}}
+TILES_AHEAD = 0.9  # the tiles are taken where they promise a tenth: then two of the 1,144 steps took over 5 % longer than the walk (13 %)
 
-    A walk's time goes with the longest sequence: 17 us and 0.43 us a token while its warps do not crowd the schedulers (two full-length
-    sequences of 16 heads), the tiles' with how often the tiles of all heads fill the GPU: about 30 us a time, once at least.  Measured (us, walk / tiles;
-    16 heads of 128 with a decay per channel): one sequence of 32 tokens 29 / 32, 48 37 / 34, 64 45 / 36, 192 107 / 40; 24 single
-    tokens beside one of 100 77 / 146, beside one of 600 312 / 191; a decay per head: 33 43 / 24, 128 75 / 28."""
+
+def recurrence_costs(kind: str, d: int, dv: int, max_len: int, n: int, num_seqs: int, heads: int, singles: int = 0) -> tuple[float, float]:
+    """Estimates (us) of a step of ``n`` tokens in ``num_seqs`` sequences, the first ``singles`` of them single tokens: walked, and in tiles."""
+    costs, longest, sms = RECURRENCE_COSTS[kind], min(max_len, n), 148
+    base, token, token_exp, every, every_exp = costs["walk"]
+    walk = base + longest * token * (d / 128) ** token_exp + n * heads / sms * every * (d / 128) ** every_exp
+    base, prepare, chain, tile, exp = costs["tiles"]
+    size, portions = (d / 128) ** exp, num_seqs - singles
+    tiles = singles + (max(portions, (n - singles) / 64 + portions / 2) if portions else 0)
+    chains = max(chain + tile * size * (longest / 64 + 0.5), num_seqs * heads * dv / 32 / sms * (chain + tile * size * tiles / num_seqs))
+    return walk, base + max(1.0, tiles * heads / sms) * prepare * size + chains
+
+
+def recurrence_form(d: int, dv: int, max_len: int, n: int, num_seqs: int, heads: int, on_gpu: bool = True, kind: str = "head", singles: int = 0) -> str:
+    """Which kernels serve a step of a delta rule (``kind`` "head" or "channel": a decay per head or per channel) or of the token-shift recurrence ("bonus"):
+    ``"tiles"`` (portions: tiles of 64 tokens on the tensor cores) or ``"walk"`` (decode steps, short portions, larger heads).
+
+    "channel" and "bonus" go by ``recurrence_costs``.  Measured, us, walk / tiles: decay per channel, 16 heads of 128: one sequence of 33 tokens 27 / 28, of 48
+    34 / 28, of 192 107 / 40; 8 heads: 33 24 / 27; 32 sequences of 33 tokens 167 / 195; 24 single tokens beside one of 100 70 / 131.  Bonus, heads of 64:
+    16 heads, one of 33 16.0 / 15.6, of 128 47 / 19; 64 heads, 32 sequences of 33 126 / 244, of 200 beside 15 others 340 / 457.
+    "head": its tiles won in every measured step of 33 tokens or more without many single tokens (33 tokens 43 / 26, 16 sequences of 40 126 / 63), so the line
+    is drawn wide of that: a walk at 17 us and 0.43 us a token while its warps do not crowd the schedulers, the tiles at 30 us for every time that
+    they fill the GPU."""
     if not on_gpu or d > TILES_MAX_HEAD_DIM or dv > TILES_MAX_HEAD_DIM or max_len < TILES_MIN_TOKENS:
         return "walk"
+    if kind != "head":
+        walk, tiles = recurrence_costs(kind, d, dv, max_len, n, num_seqs, heads, singles)
+        return "tiles" if tiles <= TILES_AHEAD * walk else "walk"
     longest = min(max_len, n)
     tiles = 30.0 * max(1.0, (n / 64 + num_seqs) * heads / 148)
     return "tiles" if tiles <= 17.0 + 0.43 * longest * max(1.0, n / longest * heads / 32) else "walk"
@@ -1823,7 +1850,7 @@ def shift_decay_scan(o: torch.Tensor, rkvg: torch.Tensor, wz: torch.Tensor, w0: 
     call, or, for portions, the kernels that take tiles of tokens.  ``form``: ``"walk"``, ``"tiles"``, or None (chosen)."""
     _, heads, _, d = state.shape
     n = o.shape[0]
-    if (form or recurrence_form(d, d, max_len, n, state_slot.numel(), heads, o.is_cuda)) != "tiles":
+    if (form or recurrence_form(d, d, max_len, n, state_slot.numel(), heads, o.is_cuda, "bonus")) != "tiles":
         rows = torch.empty((n, decay_recurrence_row(heads, heads, d, d)), dtype=torch.float32, device=o.device)
         shift_decay_prep(rows, rkvg, wz, w0, heads, d)
         decay_recurrence(o, rows, state, q_start, state_slot, heads, mode, bonus, max_len=max_len)
@@ -1845,7 +1872,7 @@ def channel_delta_scan(o: torch.Tensor, qkv: torch.Tensor, u: torch.Tensor, b_co
     in one call, or, for portions, the kernels that take tiles of tokens.  ``form``: ``"walk"``, ``"tiles"``, or None (chosen)."""
     _, heads, dv, d = state.shape
     n = o.shape[0]
-    if (form or recurrence_form(d, dv, max_len, n, state_slot.numel(), heads, o.is_cuda)) != "tiles":
+    if (form or recurrence_form(d, dv, max_len, n, state_slot.numel(), heads, o.is_cuda, "channel")) != "tiles":
         rows = torch.empty((n, decay_recurrence_row(kv_heads, heads, d, dv)), dtype=torch.float32, device=o.device)
         channel_delta_prep(rows, qkv, u, b_col, a, dt_bias, a_log, heads, kv_heads, d, dv, unit_eps)
         decay_recurrence(o, rows, state, q_start, state_slot, kv_heads, "delta", None, max_len=max_len)

@@ -11,24 +11,33 @@ from ..weights.loader import TensorDecl
 from .base import Part, register_part, tensor_name
 
 
-# From this many decoded tokens on beside longer portions, a delta rule takes them apart: single tokens are walked and the portions go by
-# tiles of tokens, of which each single token would fill one (16 heads of 128 beside a portion of 100 tokens: 24 single tokens add 108 us
-# as tiles, a walk of their own some 20).
+# From this many decoded tokens on beside longer portions, a delta rule may take them apart: single tokens are walked and the portions go by
+# tiles of tokens, of which each single token would fill one (a decay per head, 16 heads of 128 beside a portion of 100 tokens: 24 single tokens
+# add 68 us as tiles, a walk of their own 17).
 SINGLES_APART = 4
 
 
-def singles_apart(batch, d: int, dv: int, heads: int, on_gpu: bool) -> int:
-    """How many of the step's leading single-token sequences a delta rule takes in a call of their own (0: one call for all)."""
-    s = batch.num_single
-    if s < SINGLES_APART or s == batch.num_seqs or ops.recurrence_form(d, dv, batch.max_q_len, batch.n - s, batch.num_seqs - s, heads, on_gpu) != "tiles":
+def singles_apart(batch, d: int, dv: int, heads: int, on_gpu: bool, kind: str = "head") -> int:
+    """How many of the step's leading single-token sequences a delta rule takes in a call of their own (0: one call for all).  With a decay per channel
+    only where that promises a tenth over a walk of everything: its walk of single tokens is two launches, 11 us (8 of them beside 64 tokens, 16 heads
+    of 128, us, walk / tiles / apart: 45 / 47 / 48, beside 100 62 / 68 / 49)."""
+    s, portions = batch.num_single, batch.num_seqs - batch.num_single
+    if s < SINGLES_APART or not portions or ops.recurrence_form(d, dv, batch.max_q_len, batch.n - s, portions, heads, on_gpu, kind) != "tiles":
         return 0
+    if kind != "head":
+        launches, numbers = ops.RECURRENCE_COSTS[kind]["singles"]
+        walk = ops.recurrence_costs(kind, d, dv, batch.max_q_len, batch.n, batch.num_seqs, heads, s)[0]
+        tiles = ops.recurrence_costs(kind, d, dv, batch.max_q_len, batch.n - s, portions, heads)[1]
+        if tiles + launches + numbers * s * heads * d * dv / 2**20 > ops.TILES_AHEAD * walk:
+            return 0
     return s
 
 
-def scan_calls(batch, s: int) -> list[tuple]:
-    """A delta rule's calls for a step whose first ``s`` single tokens are taken apart: (rows, q_start, state_slot, options) of each."""
+def scan_calls(batch, s: int, form: str | None = None) -> list[tuple]:
+    """A delta rule's calls for a step whose first ``s`` single tokens are taken apart: (rows, q_start, state_slot, options) of each.  ``form``: of a
+    single call."""
     if not s:
-        return [(batch.n, batch.q_start, batch.state_slot, {"max_len": batch.max_q_len})]
+        return [(batch.n, batch.q_start, batch.state_slot, {"max_len": batch.max_q_len, "form": form})]
     return [(s, batch.q_start[: s + 1], batch.state_slot[:s], {"max_len": 1}),
             (batch.n, batch.q_start[s:], batch.state_slot[s:], {"max_len": batch.max_q_len, "form": "tiles"})]
 
@@ -311,7 +320,8 @@ class ShiftDecayRecurrence(Part):
         low = ops.activation(project(blends[4], w["w1"]), "tanh")
         wz = project(low, w["w2"])
         o = torch.empty((n, self.inner), dtype=torch.float32, device=x.device)
-        ops.shift_decay_scan(o, rkvg, wz, w["w0"], "bonus", w["u"], state, batch.q_start, batch.state_slot, max_len=batch.max_q_len)
+        form = ops.recurrence_form(self.d, self.d, batch.max_q_len, n, batch.num_seqs, self.heads, x.is_cuda, "bonus", batch.num_single)
+        ops.shift_decay_scan(o, rkvg, wz, w["w0"], "bonus", w["u"], state, batch.q_start, batch.state_slot, max_len=batch.max_q_len, form=form)
         gated = torch.empty((n, self.inner), dtype=x.dtype, device=x.device)
         ops.gated_group_rmsnorm(gated, o, rkvg[3], 0, w["norm"], self.heads, self.eps, gate_after=True)
         return project(gated, w["o"])
@@ -402,7 +412,8 @@ class ChannelDeltaRule(Part):
         a = project(u[:, self.a_cols[0] : self.a_cols[1]], w["a2"])  # [n, heads * head_dim]; the library reads the column slice in place
         g = project(u[:, self.g_cols[0] : self.g_cols[1]], w["g2"])  # [n, heads * value_dim]
         o = torch.empty((n, self.inner), dtype=torch.float32, device=x.device)
-        for rows, q_start, slots, options in scan_calls(batch, singles_apart(batch, self.d, self.dv, self.heads, x.is_cuda)):
+        form = ops.recurrence_form(self.d, self.dv, batch.max_q_len, n, batch.num_seqs, self.heads, x.is_cuda, "channel", batch.num_single)
+        for rows, q_start, slots, options in scan_calls(batch, singles_apart(batch, self.d, self.dv, self.heads, x.is_cuda, "channel"), form):
             ops.channel_delta_scan(o[:rows], qkv[:rows], u[:rows], self.b_col, a[:rows], w["dt_bias"], w["A_log"], state, q_start, slots, self.kv_heads,
                                    self.unit_eps, **options)
         gated = torch.empty((n, self.inner), dtype=x.dtype, device=x.device)

@@ -4,7 +4,8 @@ import types
 
 import pytest
 
-from dli_b200.kernels import attention
+from dli_b200.kernels import attention, ops
+from dli_b200.parts import ssm
 
 
 @pytest.mark.parametrize("portion,step,tiles", [(64, 64, False), (2, 2, False), (65, 65, True), (4096, 4096, True), (64, 3000, False), (3000, 3000, True), (0, 64, False),
@@ -23,3 +24,18 @@ def test_portions_of_differential_attention(portions, singles, context, apart):
     longest = max(q + before for q, before in portions)
     batch = types.SimpleNamespace(num_single=singles, num_seqs=singles + len(portions), max_q_len=max(q for q, _ in portions), max_kv_len=max(longest, context), max_kv_len_single=context, max_kv_len_portion=longest)
     assert attention.diff_portions_apart(batch, singles + sum(q for q, _ in portions), 16, 4, None, 0) == apart
+
+
+@pytest.mark.parametrize("kind,heads,d,singles,portions,route", [
+    ("channel", 16, 128, 0, [2048], "tiles"), ("channel", 16, 128, 0, [48], "tiles"), ("channel", 8, 128, 0, [33], "walk"), ("channel", 4, 64, 0, [33], "walk"),
+    ("channel", 16, 128, 0, [33] * 32, "walk"), ("channel", 16, 64, 0, [100] * 32, "walk"), ("channel", 8, 128, 3, [33], "walk"), ("channel", 16, 128, 8, [64], "walk"),
+    ("channel", 16, 128, 8, [100], "apart"), ("channel", 16, 128, 24, [300], "apart"), ("channel", 4, 64, 64, [33], "walk"), ("channel", 16, 128, 64, [], "walk"),
+    ("bonus", 16, 64, 0, [250, 251], "tiles"), ("bonus", 64, 64, 0, [33] * 32, "walk"), ("bonus", 64, 64, 0, [200] * 16, "walk"), ("bonus", 16, 64, 4, [33], "walk"),
+    ("bonus", 16, 64, 0, [1500], "tiles"), ("bonus", 16, 64, 24, [300], "tiles"), ("head", 16, 128, 0, [33], "tiles"), ("head", 16, 128, 24, [64], "apart")])
+def test_steps_of_the_recurrences(kind, heads, d, singles, portions, route):
+    """Every kind by its own costs: short portions, and many portions of wide models, are walked where that was measured to be faster."""
+    batch = types.SimpleNamespace(num_single=singles, num_seqs=singles + len(portions), n=singles + sum(portions), max_q_len=max(portions, default=1))
+    if kind != "bonus" and ssm.singles_apart(batch, d, d, heads, True, kind):
+        assert route == "apart"
+    else:
+        assert ops.recurrence_form(d, d, batch.max_q_len, batch.n, batch.num_seqs, heads, True, kind, singles) == route
