@@ -33,13 +33,24 @@ def singles_apart(batch, d: int, dv: int, heads: int, on_gpu: bool, kind: str = 
     return s
 
 
-def scan_calls(batch, s: int, form: str | None = None) -> list[tuple]:
-    """A delta rule's calls for a step whose first ``s`` single tokens are taken apart: (rows, q_start, state_slot, options) of each.  ``form``: of a
-    single call."""
+def scan_singles_apart(batch, P: int, N: int, heads: int, dtype: torch.dtype) -> int:
+    """How many of the step's leading single-token sequences a selective scan takes in a call of their own (0: one call for all): where portions of one
+    tile stand beside so many that their tiles, one each, queue for the SMs (two CTAs each) more than twice over.  Measured, us, walk / tiles / apart,
+    64 heads, N 128: 24 single tokens beside 16 tokens 30 / 50 / 27, 64 of them 74 / 126 / 68, 8 of them 19 / 19 / 18; 128 heads, 4 beside 33 36 / 26 / 22.
+    (Longer portions take their time meanwhile: 16 beside 300 tokens 149 / 48 / 62.)"""
+    s = batch.num_single
+    if s < SINGLES_APART or s == batch.num_seqs or batch.max_q_len > 64 or ops.ssm_scan_form(dtype, P, N, batch.max_q_len) == "walk":
+        return 0
+    return s if batch.num_seqs * heads * -(-P // 64) > 4 * 148 else 0
+
+
+def scan_calls(batch, s: int, form: str | None = None, tiles: str = "tiles") -> list[tuple]:
+    """A recurrence's calls for a step whose first ``s`` single tokens are taken apart: (rows, q_start, state_slot, options) of each.  ``form``: of a
+    single call; ``tiles``: of the portions' one."""
     if not s:
         return [(batch.n, batch.q_start, batch.state_slot, {"max_len": batch.max_q_len, "form": form})]
     return [(s, batch.q_start[: s + 1], batch.state_slot[:s], {"max_len": 1}),
-            (batch.n, batch.q_start[s:], batch.state_slot[s:], {"max_len": batch.max_q_len, "form": "tiles"})]
+            (batch.n, batch.q_start[s:], batch.state_slot[s:], {"max_len": batch.max_q_len, "form": tiles})]
 
 
 @register_part("mixer", "mamba2")
@@ -111,8 +122,9 @@ class Mamba2Mixer(Part):
         if self.taps > 1:
             ops.conv_state_update(conv_state, u, self.inner, batch.q_start, batch.state_slot)
         y = torch.empty((n, self.inner), dtype=torch.float32, device=x.device)
-        ops.ssm_scan(y, xbc, u, self.inner + self.channels, w["dt_bias"], w["A_log"], w["D"], ssm_state, batch.q_start, batch.state_slot,
-                     self.groups, max_len=batch.max_q_len)
+        for rows, q_start, slots, options in scan_calls(batch, scan_singles_apart(batch, self.P, self.N, self.heads, x.dtype), tiles=None):
+            ops.ssm_scan(y[:rows], xbc[:rows], u[:rows], self.inner + self.channels, w["dt_bias"], w["A_log"], w["D"], ssm_state, q_start, slots, self.groups,
+                         **options)
         gated = torch.empty((n, self.inner), dtype=x.dtype, device=x.device)
         ops.gated_group_rmsnorm(gated, y, u, 0, w["norm"], self.parts, self.eps)
         return project(gated, w["o"])

@@ -3,6 +3,7 @@
 import types
 
 import pytest
+import torch
 
 from dli_b200.kernels import attention, ops
 from dli_b200.parts import ssm
@@ -39,3 +40,12 @@ def test_steps_of_the_recurrences(kind, heads, d, singles, portions, route):
         assert route == "apart"
     else:
         assert ops.recurrence_form(d, d, batch.max_q_len, batch.n, batch.num_seqs, heads, True, kind, singles) == route
+
+
+@pytest.mark.parametrize("heads,singles,portions,apart", [(64, 24, [17], 24), (64, 64, [64], 64), (128, 4, [33], 4), (64, 4, [33], 0), (64, 8, [17], 0), (64, 16, [300], 0),
+                                                          (64, 24, [16], 0), (64, 24, [], 0), (128, 0, [33] * 16, 0), (128, 3, [33] * 16, 0), (16, 24, [33], 0)])
+def test_single_tokens_beside_a_scan(heads, singles, portions, apart):
+    """They are walked by themselves where their tiles would queue behind one another while portions of one tile wait for them."""
+    batch = types.SimpleNamespace(num_single=singles, num_seqs=singles + len(portions), n=singles + sum(portions), max_q_len=max(portions, default=1))
+    assert ssm.scan_singles_apart(batch, 64, 128, heads, torch.bfloat16) == apart
+    assert ssm.scan_singles_apart(batch, 64, 128, heads, torch.float32) == 0
