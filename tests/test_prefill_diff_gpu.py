@@ -113,6 +113,34 @@ def test_both_routes_of_a_mixed_step(apart, monkeypatch):
     assert len(calls) == apart
 
 
+@pytest.mark.gpu
+def test_a_recorded_step_takes_other_sequences():
+    """Recorded once for the largest and replayed with other portions and contexts, an empty one among them."""
+    heads, nkv, dv, width = 8, 2, 128, 20
+    steps = [[(130, 20), (31, 0), (1, 7)], [(0, 5), (63, 200), (65, 1)], [(2, 60), (0, 1), (129, 128)]]
+    cases = [_case(lens, heads, nkv, dv, 16, seed=i) for i, lens in enumerate(steps)]
+    pages, rows = max(c[0].shape[0] for c in cases), max(c[4].shape[0] for c in cases)
+    k, v = (torch.zeros(pages, nkv, 16, w, dtype=torch.bfloat16, device="cuda") for w in (128, dv))
+    q, out = torch.zeros(rows, heads * 128, dtype=torch.bfloat16, device="cuda"), torch.zeros(rows, heads * dv, dtype=torch.bfloat16, device="cuda")
+    tables, start, kv_len = torch.zeros(3, width, dtype=torch.int32).cuda(), torch.zeros(4, dtype=torch.int32).cuda(), torch.ones(3, dtype=torch.int32).cuda()
+
+    def run():
+        ops.paged_prefill_diff(out, q, k, v, tables, start, kv_len, 0, 3, 130, None, heads, 0.125, 100, 16, 0.7, 0.3, 1e-6)
+
+    run()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run()
+    for lens, (k1, v1, tables1, data, q1, _, start1, kv1) in zip(steps, cases):
+        n = q1.shape[0]
+        k[: k1.shape[0]], v[: v1.shape[0]], q[:n], tables[:, : tables1.shape[1]] = k1.cuda(), v1.cuda(), q1.cuda(), tables1.cuda()
+        start.copy_(start1), kv_len.copy_(kv1), out.fill_(7.0)
+        graph.replay()
+        _near(out[:n].cpu(), _exact(lens, data, q1, None, start1, heads, nkv, dv, 0.125, 100, 16, 0.7, 0.3, 1e-6))
+        assert (out[n:] == 7.0).all()
+    assert ops.device_wait_errors() == {}
+
+
 def test_which_sizes_have_the_kernel():
     ok = ops.prefill_diff_supported
     assert ok(64, 128, 16) and ok(64, 24, 8) and ok(64, 64, 128)

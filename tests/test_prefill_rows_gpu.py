@@ -98,6 +98,34 @@ def test_a_sequence_range_of_a_batch():
     assert (got[:1] == 7.0).all() and (got[1:].double() - want[1:]).norm() <= 6e-3 * want[1:].norm()
 
 
+@pytest.mark.gpu
+def test_a_recorded_step_takes_other_sequences():
+    """Recorded once for the largest and replayed with other portions and contexts, an empty one among them."""
+    heads, row, width = 4, 192, 20
+    steps = [[(130, 20), (31, 0), (1, 7)], [(0, 5), (63, 200), (65, 1)], [(2, 60), (0, 1), (129, 128)]]
+    cases = [_case(lens, heads, 1, row, 16, seed=i) for i, lens in enumerate(steps)]
+    pages, count = max(c[0].shape[0] for c in cases), max(c[3].shape[0] for c in cases)
+    pool, q = torch.zeros(pages, 1, 16, row, dtype=torch.bfloat16, device="cuda"), torch.zeros(count, heads * row + 8, dtype=torch.bfloat16, device="cuda")
+    out = torch.zeros(count, heads * row, dtype=torch.bfloat16, device="cuda")
+    tables, start, kv_len = torch.zeros(3, width, dtype=torch.int32).cuda(), torch.zeros(4, dtype=torch.int32).cuda(), torch.ones(3, dtype=torch.int32).cuda()
+
+    def run():
+        ops.paged_prefill_rows(out, q, pool, tables, start, kv_len, 0, 3, 130, heads, row**-0.5, 100)
+
+    run()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run()
+    for lens, (pool1, tables1, data, q1, start1, kv1) in zip(steps, cases):
+        n = q1.shape[0]
+        pool[: pool1.shape[0]], q[:n], tables[:, : tables1.shape[1]] = pool1.cuda(), q1.cuda(), tables1.cuda()
+        start.copy_(start1), kv_len.copy_(kv1), out.fill_(7.0)
+        graph.replay()
+        got, want = out[:n].view(n, heads, row).cpu().double(), _exact(lens, data, q1, start1, heads, 1, row, row, row**-0.5, 100, None)
+        assert (got - want).norm() <= 6e-3 * want.norm() and (out[n:] == 7.0).all(), lens
+    assert ops.device_wait_errors() == {}
+
+
 def test_which_rows_have_the_kernel():
     ok = ops.prefill_rows_supported
     assert ok(256, 16) and ok(136, 8) and ok(192, 128)
