@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
 
 // Tokens first .. last - 1 of a head token after token, for 4 columns a warp from col0 on, from and to the state in memory.  A lane holds every
 // 32nd channel.
-__device__ __noinline__ void walk_again(const Params& p, int head, int col0, int first, int last, float* S0) {
+__device__ __forceinline__ void walk_again(const Params& p, int head, int col0, int first, int last, float* S0) {
   const int lane = threadIdx.x & 31, d = p.d, dv = p.dv, kqh = head / (p.heads / p.kq), width = 2 * p.kq * d + p.heads * dv;
   const size_t slab = (size_t)p.n * p.heads * d;  // BONUS
   auto number = [&](const void* base, size_t i) { return p.f32 ? static_cast<const float*>(base)[i] : to_float(static_cast<const bf16*>(base)[i]); };
@@ -823,7 +823,7 @@ __device__ __forceinline__ bool wait_copies(uint32_t bar, uint32_t parity, volat
   return false;
 }
 // For a CTA that gives up: the copies that it still has under way (`issued` so far on this barrier) may not land in shared memory that is no longer its own.
-__device__ __noinline__ void wait_for_last(uint32_t bar, int issued) {
+__device__ __forceinline__ void wait_for_last(uint32_t bar, int issued) {
   for (unsigned i = 0; issued > 0 && i < WAIT_LIMIT; ++i)
     if (copies_arrived(bar, (issued - 1) & 1)) return;
 }
@@ -911,10 +911,12 @@ __global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const __grid_con
         for (int s = 0; s < 3; ++s)
           *reinterpret_cast<uint32_t*>(smem + Z::AT_S + s * Z::S_TERM + (c_lo + hf * 8) * Z::ROW + (slice0 + j * 8 + kcol) * 2) = t[s];
       }
-    if (__syncthreads_or(!ok)) break;  // S0 is there; the operands behind (of the tile before) have been read
-    load_behind(left);
-    ++behind;
-    ok = wait_copies(bar_before, parity, failed, p.error_flag);
+    __syncthreads();  // S0 is there; the operands behind (of the tile before) have been read
+    if (ok) {         // (the thread that asks for copies asks again on a barrier only when it has seen the last ones arrive)
+      load_behind(left);
+      ++behind;
+    }
+    ok = wait_copies(bar_before, parity, failed, p.error_flag) && ok;
     float O[2][4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) O[0][e] = O[1][e] = 0.f;
@@ -960,7 +962,8 @@ __global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const __grid_con
         }
       }
     }
-    if (__syncthreads_or(!ok)) break;  // w is there; S0 and the operands in front have been read
+    __syncthreads();  // w is there; S0 and the operands in front have been read
+    if (*failed) break;
     left += (size_t)p.heads * bytes;
     if (base + TOKENS < last) { load_before(left); ++before; }
     ok = wait_copies(bar_behind, parity, failed, p.error_flag);
@@ -1374,10 +1377,12 @@ __global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const __grid_con
         for (int s = 0; s < 3; ++s)
           *reinterpret_cast<uint32_t*>(smem + Z::AT_S + s * Z::S_TERM + (c_lo + hf * 8) * Z::ROW + (slice0 + j * 8 + kcol) * 2) = t[s];
       }
-    if (__syncthreads_or(!ok)) break;  // S0 is there; the operands behind (of the tile before) have been read
-    load_behind(left);
-    ++behind;
-    ok = wait_copies(bar_before, parity, failed, p.error_flag);
+    __syncthreads();  // S0 is there; the operands behind (of the tile before) have been read
+    if (ok) {         // (the thread that asks for copies asks again on a barrier only when it has seen the last ones arrive)
+      load_behind(left);
+      ++behind;
+    }
+    ok = wait_copies(bar_before, parity, failed, p.error_flag) && ok;
     float O[2][4], w[2][4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) O[0][e] = O[1][e] = w[0][e] = w[1][e] = 0.f;
@@ -1432,7 +1437,8 @@ __global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const __grid_con
           }
         }
     }
-    if (__syncthreads_or(!ok)) break;  // w is there; S0 and the operands in front have been read
+    __syncthreads();  // w is there; S0 and the operands in front have been read
+    if (*failed) break;
     left += (size_t)p.heads * bytes;
     if (base + TOKENS < last) { load_before(left); ++before; }
     // ---- the read-outs

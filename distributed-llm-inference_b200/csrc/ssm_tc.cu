@@ -80,7 +80,7 @@ __device__ __forceinline__ void segment_tiles(int tiles, int segments, int seg, 
 
 // The scan of a CTA's columns token after token: from the state `from` in front of token t_from, with read-outs of tokens t_emit .. t_end - 1, the
 // state behind them to `to` (or null).  A warp takes sixteen columns, four at a time; a lane holds every 32nd number of them.
-__device__ __noinline__ void walk_again(const Params& p, int head, int col0, const float* from, int t_from, int t_emit, int t_end, float* to) {
+__device__ __forceinline__ void walk_again(const Params& p, int head, int col0, const float* from, int t_from, int t_emit, int t_end, float* to) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, N = p.N, P = p.P, inner = p.heads * P, width = inner + 2 * p.groups * N;
   const float A = expf(p.A_log[head]), bias = p.dt_bias[head], Dh = p.D[head];
   const int g = head / (p.heads / p.groups);
