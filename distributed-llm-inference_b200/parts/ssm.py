@@ -47,10 +47,12 @@ def scan_singles_apart(batch, P: int, N: int, heads: int, dtype: torch.dtype) ->
 def scan_calls(batch, s: int, form: str | None = None, tiles: str = "tiles") -> list[tuple]:
     """A recurrence's calls for a step whose first ``s`` single tokens are taken apart: (rows, q_start, state_slot, options) of each.  ``form``: of a
     single call; ``tiles``: of the portions' one."""
+    def options(form):
+        return {"max_len": batch.max_q_len, **({"form": form} if form else {})}
+
     if not s:
-        return [(batch.n, batch.q_start, batch.state_slot, {"max_len": batch.max_q_len, "form": form})]
-    return [(s, batch.q_start[: s + 1], batch.state_slot[:s], {"max_len": 1}),
-            (batch.n, batch.q_start[s:], batch.state_slot[s:], {"max_len": batch.max_q_len, "form": tiles})]
+        return [(batch.n, batch.q_start, batch.state_slot, options(form))]
+    return [(s, batch.q_start[: s + 1], batch.state_slot[:s], {"max_len": 1}), (batch.n, batch.q_start[s:], batch.state_slot[s:], options(tiles))]
 
 
 @register_part("mixer", "mamba2")
