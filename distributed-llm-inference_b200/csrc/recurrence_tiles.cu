@@ -21,10 +21,10 @@
 // What bounds it, and what it measured.  (1) takes a CTA an SM (228 KB) about 50,000 clocks a tile and head of 128 with a decay per channel, in
 // steps that wait on one another: 14,000 until the rows are there as unit vectors and decays (their loads 5,000, the exponentials 4,800), the diagonal
 // blocks 5,600, products of decays 7,700, blocks below the diagonal 3,300, the inverse 6,100, W and U 7,600, W's way out 2,200.  (2) takes 3.7 us a
-// tile (5 with 32 columns a CTA), by mma.sync (318 a tile and warp) and its operands' arrival (157 KB by bulk copies; with a cp.async per 16 bytes, 6.5 us).
-// Against the kernels that walk, us: decay per head in bfloat16 (kernels of its own, below), 16 heads of 128, one prompt of 2,048 tokens 772 -> 134;
-// decay per channel, prompts of 1,400 and 2,100 1,050 -> 324, one of 2,048 1,008 -> 206; bonus, 16 heads of 64, float32, prompts of 200 and 301 109 -> 30,
-// 4,096 1,336 -> 214.
+// tile (4.9 with 32 columns a CTA), by mma.sync (318 a tile and warp) and its operands' arrival (157 KB by bulk copies; with a cp.async per 16 bytes, 6.5 us).
+// Against the kernels that walk, us: decay per head in bfloat16 (kernels of its own, below), 16 heads of 128, one prompt of 2,048 tokens 773 -> 134;
+// decay per channel, prompts of 1,400 and 2,100 1,050 -> 320, one of 2,048 1,005 -> 204; bonus, 16 heads of 64, float32, prompts of 200 and 301 108 -> 28,
+// 4,096 1,333 -> 207.  Short portions, and many of them in a wide model, are walked (ops.recurrence_form says where the line lies).
 // Errors against 64 bits are the walks' or smaller (decay per channel, 2,048 tokens: o 4.9e-7 and S 5.0e-7, walked 5.4e-7 and 5.4e-7).
 #include "common.cuh"
 #include "mma_split.cuh"
@@ -198,7 +198,6 @@ template <typename T, int MODE, int KD> struct Prep {
 
 template <typename T, int MODE, int KD>
 __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) tile_prep_kernel(const Params p) {
-  pdl_launch_dependents();
   pdl_wait();
   using Z = Prep<T, MODE, KD>;
   using L = Left<KD, Prep<T, MODE, KD>::DELTA>;
@@ -253,7 +252,7 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
   }
   const float rate = MODE == BONUS ? 0.f : expf(p.a_log[head]);
   // A lane has PER channels side by side, which come in one load each where rows are whole and aligned (p.vec).  A warp's eight norms share five
-  // rounds of shuffles and one root and division (with a load per number and these per row this part took 16,700 clocks, now 12,000).
+  // rounds of shuffles and one root and division (with a load per number and these per row this part took 16,700 clocks, now 13,900).
   constexpr int ROWS = TOKENS / Z::WARPS, GROUP = 4;  // rows of a warp; those whose loads are under way together
   static_assert(ROWS % GROUP == 0, "rows");
   const int c0 = lane * PER;
@@ -557,7 +556,10 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
   auto q_leaves = [&](auto threads, int id) {  // Q in three terms, block by block
     split_blocks<decltype(threads)::value>([&](int r, int cc) { return sQm[r * F_ROW + cc]; }, left + L::Q, id);
   };
-  if constexpr (!DELTA) q_leaves(std::integral_constant<int, Z::THREADS>(), tid);
+  if constexpr (!DELTA) {
+    pdl_launch_dependents();
+    q_leaves(std::integral_constant<int, Z::THREADS>(), tid);
+  }
   if constexpr (DELTA) {
     // ---- P o K and V as operands, in the place of the blocks' operands.  With sixteen warps, eight make the inverse, a chain of short steps,
     // while the others see to V and Q (one after the other 14,700 of the 61,300 clocks).
@@ -683,6 +685,9 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
         if (task & 1) columns16(v, m1, m2, col0); else columns16(v, m0, m3, col0);
       }
     }
+    // The walk's CTAs come only now: waiting on SMs that the last round leaves free, they slowed that round by 12 us (16 heads of 128, 2,048 tokens: both
+    // kernels 220 us with them there from the start, 199 so).
+    pdl_launch_dependents();
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     if (tid == 0) {  // W leaves in one piece
@@ -1530,7 +1535,7 @@ template <typename K> cudaError_t allow(K kernel, int smem, OncePerDevice& done)
 int* error_flag_device = nullptr;
 int* error_flag_host = nullptr;
 
-// Value columns of a CTA of the second kernel: 16 while that leaves every CTA an SM of its own (a tile takes 3.7 us instead of 6.0 with 32), else 32
+// Value columns of a CTA of the second kernel: 16 while that leaves every CTA an SM of its own (a tile takes 3.7 us instead of 4.9 with 32), else 32
 // (half the copies of the operands).
 inline int columns(int heads, int num_seqs, int dv) { return (long long)heads * num_seqs * ((dv + 15) / 16) <= sm_count() ? 16 : 32; }
 
