@@ -870,10 +870,11 @@ __global__ void __launch_bounds__(T2Cfg<HD, HV>::THREADS, 1) paged_prefill_tc2_k
 // both maps' side by side, so keys, values and their copies are shared; tensor memory holds S and O of both maps (512 columns).  A row's first
 // thread reads both outputs from there at the end.  With a window, the tiles of the kept first tokens come in front of the window's.
 //
-// What bounds it: the softmax threads, as in the kernel it follows (with clocks taken in a CTA, a tile of both maps takes 3,400 clocks: 200 to read a
-// row of scores, 400 its maximum, 1,450 its exponentials in turns, the rest waits; the tensor cores' share is 1,540).  Measured against the
-// mma.sync kernel, 16 heads on 4, values of 128, us: 4,096 tokens 608 -> 150 (689 TFLOP/s), with a window of 1,024 289 -> 110, 1,535 behind 1,024 138 -> 65,
-// 512 tokens 41 -> 19, 128 18.6 -> 15.3, 2 tokens behind 1,000 27.5 -> 24.1.
+// What bounds it: the softmax threads, as in the kernel it follows (with clocks taken in a CTA while the maximum was followed in steps of 2^8, a tile of both
+// maps took 3,400 clocks: 200 to read a row of scores, 400 its maximum, 1,450 its exponentials in turns, the rest waits; the tensor cores' share is
+// 1,540; the exact maximum rescales the outputs more often, 3,700).  Measured against the mma.sync kernel, 16 heads on 4, values of 128, us: 4,096 tokens
+// 600 -> 165 (625 TFLOP/s), with a window of 1,024 283 -> 116, 1,535 behind 1,024 with it 136 -> 72, 1,000 tokens 72 -> 29, 128 18.2 -> 13.7; short
+// portions and steps with many single tokens go by one launch of the other kernel (diff_portions_apart in kernels/attention.py).
 struct DiffParams {
   bf16* out;
   const bf16* q;
@@ -1065,7 +1066,7 @@ __global__ void __launch_bounds__(DIFF_THREADS, 1) paged_prefill_diff_kernel(con
     bool ok = true;
     // chunk 0 of this row's 128-byte slab of P; chunk c lies at the address with c added to bits 4..6 (the swizzle)
     const uint32_t pchunk = smem_u32(sP) + q * 2 * TILE_BYTES + r * 128 + ((r & 7) << 4);
-    // (what the loop needs of positions is kept in few registers: 356 bytes of spills beside the row of scores took 221 us instead of 150)
+    // (what the loop needs of positions is kept in few registers: 356 bytes of spills beside the row of scores took 221 us where 100 took 150)
     const int sees_all_from = p.window > 0 ? hi - p.window : 0, sees_all_to = pos0 - KEYS + 1;  // tiles that every row sees whole start in between
     const int last_whole = kvlen - KEYS;
     int base = 0;
@@ -1290,8 +1291,9 @@ int launch_tc2(const CUtensorMap& map_k, const CUtensorMap& map_v, const Params&
 //
 // What bounds it: the copies.  With clocks taken in a CTA (4,096 tokens, 16 heads, rows of 256, 192 value columns), a tile takes 4,320 clocks; 3,900 pass
 // from a tile's request to its arrival (64 KB: all SMs read the same rows from L2 at 4.7 TB/s together, the next stage's request waits for O of
-// the tile before the last), 1,000 are S, 2,200 the softmax threads, 800 to 1,700 O.  Measured against the mma.sync kernel, us: 4,096 tokens 798 -> 177
-// (679 TFLOP/s), with a window of 1,024 358 -> 116, 512 tokens 44 -> 20, 8 tokens behind 2,000 149 -> 47, 2 tokens four times 15 -> 12; 32 heads, 2,048 tokens 420 -> 113.
+// the tile before the last), 1,000 are S, 2,200 the softmax threads, 800 to 1,700 O.  Measured against the mma.sync kernel, us: 4,096 tokens 797 -> 185
+// (650 TFLOP/s), with a window of 1,024 355 -> 115, 512 tokens 43 -> 21, 8 tokens behind 2,000 four times 149 -> 50, 2 behind 2,000 141 -> 46; portions that see one
+// key tile of the other kernel stay there (portions_pay_for_tiles_of_rows in kernels/attention.py).
 struct RowParams {
   bf16* out;
   const bf16* q;

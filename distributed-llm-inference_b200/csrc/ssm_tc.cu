@@ -23,8 +23,8 @@
 //
 // What bounds it: the latency of a warp's instructions (ncu, one prompt of 1,024 tokens, a CTA an SM: 3,500 warp instructions a tile and
 // warp, an instruction every 4.3 cycles, tensor pipe active 26 %); registers and shared memory hold two CTAs an SM.  Measured, us, against
-// the walk of ssm.cu (64 heads, P 64, N 128): prompts of 666, 1,000 and 1,335 tokens 772 -> 159, one of 4,096 1,405 -> 213, one
-// of 600 210 -> 54; 128 heads, one of 2,048 880 -> 192; 32 heads, N 64, one of 2,048 524 -> 52.  The errors of y and S against 64 bits
+// the walk of ssm.cu (64 heads, P 64, N 128): prompts of 666, 1,000 and 1,335 tokens 772 -> 165, one of 4,096 1,409 -> 215, one
+// of 600 214 -> 51; 128 heads, one of 2,048 880 -> 204; 32 heads, N 64, one of 2,048 490 -> 48.  The errors of y and S against 64 bits
 // are the walk's or smaller (4,096 tokens: 1.7e-7 and 1.7e-7, the walk 2.1e-7 and 2.2e-7): a sum of mma.sync cuts off where a plain
 // addition rounds, so long sums are kept apart and added by the CUDA cores.
 #include "common.cuh"

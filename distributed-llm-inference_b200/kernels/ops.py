@@ -1287,8 +1287,9 @@ SSM_SCAN_MAX_STATE = 512
 
 
 SSM_CHUNK_MAX_STATE = 128  # the tensor-core form keeps a state column block in registers
-# shorter portions are walked token after token (us, walk / tiles, 64 heads, P 64, N 128: one portion of 16 tokens 16.9 / 14.5, of 8
-# 13.5 / 15.7; eight portions of 8 19 / 18, of 16 32 / 18, of 2 13 / 18: the tiles' set-up is worth it from about a quarter tile on)
+# Portions of up to a quarter tile are walked token after token.  That is on the safe side: us, walk / tiles, 64 heads, P 64, N 128: one portion of 4 tokens
+# 7.2 / 8.5, of 8 10.1 / 8.5, of 12 14.1 / 8.4, of 16 16.9 / 8.5; sixteen portions of 4 21 / 34, of 8 31 / 34, of 12 42 / 35, of 16 51 / 35; single tokens beside
+# them: scan_singles_apart in parts/ssm.py.
 SSM_CHUNK_MIN_TOKENS = 17
 
 
