@@ -72,6 +72,7 @@ struct Params {
   int vec;   // rows of queries, keys and decays are whole (d = KD) and aligned: a lane's channels come in one load
   int vec_v; // rows of values lie in 16-byte runs
   int pairs; // two read-outs side by side lie on an 8-byte boundary
+  int one_wave;            // every (tile, head) has an SM of its own
   int place0, num_places;  // the places that this pass takes; a sequence's state waits in its slot between two passes
   unsigned char* left;     // what the first kernel leaves, from place0 on
   int* error_flag;
@@ -198,6 +199,10 @@ template <typename T, int MODE, int KD> struct Prep {
 
 template <typename T, int MODE, int KD>
 __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) tile_prep_kernel(const Params p) {
+  // The walk's CTAs may come from the start on where all tiles have an SM each (their launch then costs nothing: 2 to 3 us of 26 in short steps), otherwise
+  // at the end: waiting on SMs that the last wave of tiles leaves free, they slow that wave by 12 us (16 heads of 128, 2,048 tokens: both kernels
+  // 220 us with them there from the start, 199 so).
+  if (p.one_wave) pdl_launch_dependents();
   pdl_wait();
   using Z = Prep<T, MODE, KD>;
   using L = Left<KD, Prep<T, MODE, KD>::DELTA>;
@@ -557,7 +562,7 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
     split_blocks<decltype(threads)::value>([&](int r, int cc) { return sQm[r * F_ROW + cc]; }, left + L::Q, id);
   };
   if constexpr (!DELTA) {
-    pdl_launch_dependents();
+    if (!p.one_wave) pdl_launch_dependents();
     q_leaves(std::integral_constant<int, Z::THREADS>(), tid);
   }
   if constexpr (DELTA) {
@@ -685,9 +690,7 @@ __global__ void __launch_bounds__(KD * 4, KD == 64 && MODE == BONUS ? 2 : 1) til
         if (task & 1) columns16(v, m1, m2, col0); else columns16(v, m0, m3, col0);
       }
     }
-    // The walk's CTAs come only now: waiting on SMs that the last round leaves free, they slowed that round by 12 us (16 heads of 128, 2,048 tokens: both
-    // kernels 220 us with them there from the start, 199 so).
-    pdl_launch_dependents();
+    if (!p.one_wave) pdl_launch_dependents();
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     if (tid == 0) {  // W leaves in one piece
@@ -1034,16 +1037,14 @@ __global__ void __launch_bounds__(COLS * 8, 1) tile_walk_kernel(const __grid_con
       for (int e = 0; e < 4; ++e) S[j][e] = fmaf((e & 1) ? g.y : g.x, S[j][e], ds[j][e] + dl[j][e]);
     }
   }
-  if (__syncthreads_or(!ok)) {  // (the state stays as it was)
-    if (tid == 0) {
+  each([&](float& x, bool, size_t) { finite = fmaf(x, 0.f, finite); });
+  if (__syncthreads_or(!ok || finite != 0.f)) {  // (also: nobody writes a read-out behind this)
+    if (!__syncthreads_or(!ok)) {
+      walk_again(p, head, col0, first, last, S0);
+    } else if (tid == 0) {  // (the state stays as it was)
       wait_for_last(bar_before, before);
       wait_for_last(bar_behind, behind);
     }
-    return;
-  }
-  each([&](float& x, bool, size_t) { finite = fmaf(x, 0.f, finite); });
-  if (__syncthreads_or(finite != 0.f)) {  // (also: nobody writes a read-out behind this)
-    walk_again(p, head, col0, first, last, S0);
     return;
   }
   each([&](float& x, bool in, size_t at) { if (in) S0[at] = x; });
@@ -1510,16 +1511,14 @@ __global__ void __launch_bounds__(COLS * 8, 1) head_walk_kernel(const __grid_con
 #pragma unroll
       for (int e = 0; e < 4; ++e) S[j][e] = fmaf(g, S[j][e], ds[j][e] + dl[j][e]);
   }
-  if (__syncthreads_or(!ok)) {  // (the state stays as it was)
-    if (tid == 0) {
+  each([&](float& x, bool, size_t) { finite = fmaf(x, 0.f, finite); });
+  if (__syncthreads_or(!ok || finite != 0.f)) {  // (also: nobody writes a read-out behind this)
+    if (!__syncthreads_or(!ok)) {
+      walk_again(p, head, col0, first, last, S0);
+    } else if (tid == 0) {  // (the state stays as it was)
       wait_for_last(bar_before, before);
       wait_for_last(bar_behind, behind);
     }
-    return;
-  }
-  each([&](float& x, bool, size_t) { finite = fmaf(x, 0.f, finite); });
-  if (__syncthreads_or(finite != 0.f)) {  // (also: nobody writes a read-out behind this)
-    walk_again(p, head, col0, first, last, S0);
     return;
   }
   each([&](float& x, bool in, size_t at) { if (in) S0[at] = x; });
@@ -1621,7 +1620,7 @@ DLI_EXPORT int dli_recurrence_tiles(int mode, float* o, const void* qkv, const v
     if (cudaHostGetDevicePointer((void**)&error_flag_device, error_flag_host, 0) != cudaSuccess) return (int)cudaGetLastError();
   }
   Params p;
-  p.place0 = place0; p.num_places = num_places;
+  p.place0 = place0; p.num_places = num_places; p.one_wave = (long long)num_places * heads <= sm_count();
   p.mode = mode; p.f32 = dtype == DLI_F32;
   p.o = o; p.qkv = qkv; p.u = u; p.a = a; p.u_stride = u_stride; p.b_col = b_col; p.a_col = a_col; p.dt_bias = dt_bias; p.a_log = a_log; p.bonus = bonus;
   p.state = state; p.q_start = q_start; p.state_slot = state_slot; p.n = n; p.num_seqs = num_seqs; p.heads = heads; p.kq = kq; p.d = d; p.dv = dv;
