@@ -116,12 +116,26 @@ def last_product(x: torch.Tensor, weight: torch.Tensor, defer: bool):
     return project(x, weight)
 
 
+# From this many tokens and this inner size on a float32 product goes to the engine's own kernel on the tensor cores (csrc/float_gemm.cu: three
+# bfloat16 terms a number, true float32 results).  Library / own, us: 2,048 x 2,048, 1 / 4 / 8 / 100 / 512 tokens 12/21, 32/23, 32/22, 57/27, 94/45; 8,192 x 2,048
+# 23/35, 37/35, 57/35, 94/49, 315/137; K 192, 8 / 512 tokens 12/12, 18/14; K 64 8/10 up to 200 tokens.
+FLOAT_MIN_TOKENS, FLOAT_MIN_K = 8, 256
+
+
+def float_product(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether x [.., n, in] times weight [.., out, in] transposed goes to the engine's float32 product."""
+    return (x.dtype == torch.float32 and x.is_cuda and x.dim() in (2, 3) and x.shape[-2] >= FLOAT_MIN_TOKENS and x.shape[-1] >= FLOAT_MIN_K
+            and ops.float_gemm_supported(x, weight))
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     """x [n, in] times weight [out, in] transposed; float32 accumulation in both dtypes."""
     if not x.is_cuda:
         raise RuntimeError("linear: the engine has no CPU path")
     if torch.backends.cuda.matmul.allow_tf32:
         raise RuntimeError("linear: TF32 was switched on; the float32 path must stay true 32-bit")
+    if out is None and float_product(x, weight):
+        return ops.float_gemm(x, weight)
     return torch.matmul(x, weight.t(), out=out)
 
 
@@ -159,6 +173,8 @@ def batched_project(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     _need_device(x, "batched_project")
     if torch.backends.cuda.matmul.allow_tf32:
         raise RuntimeError("batched_project: TF32 was switched on; the float32 path must stay true 32-bit")
+    if float_product(x, weight.transpose(1, 2)):
+        return ops.float_gemm(x, weight.transpose(1, 2))
     return torch.bmm(x, weight)
 
 

@@ -544,6 +544,7 @@ def device_wait_errors(clear: bool = True) -> dict[str, int]:
     found = {}
     for source, read, forget, defines in (("skinny_gemm.cu", "dli_skinny_gemm_error", "dli_skinny_gemm_clear_error", None),
                                           ("dense_gemm.cu", "dli_dense_gemm_error", "dli_dense_gemm_clear_error", None),
+                                          ("float_gemm.cu", "dli_float_gemm_error", "dli_float_gemm_clear_error", None),
                                           ("recurrence_tiles.cu", "dli_recurrence_tiles_error", "dli_recurrence_tiles_clear_error", None),
                                           ("attention_tc.cu", "dli_paged_prefill_tc_error", "dli_paged_prefill_tc_clear_error", None),
                                           ("attention_tc.cu", "dli_paged_prefill_tc_error", "dli_paged_prefill_tc_clear_error", _BENT)):
@@ -976,6 +977,39 @@ def dense_gemm_error() -> int:
 def skinny_gemm_error() -> int:
     """0, or which bounded wait of the decode matrix product ran out since the library was loaded."""
     return _fn("skinny_gemm.cu", "dli_skinny_gemm_error", [])()
+
+
+# ------------------------------------------------------------------ float32 products on the tensor cores
+
+
+def float_gemm_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether ``float_gemm`` takes these operands: float32, rows of a multiple of 4 numbers that start on 16-byte boundaries."""
+    if x.dtype != torch.float32 or weight.dtype != torch.float32 or x.dim() != weight.dim() or x.dim() not in (2, 3):
+        return False
+    if x.shape[-1] != weight.shape[-1] or x.shape[-1] < 4 or x.shape[-1] % 4 or (x.dim() == 3 and x.shape[0] != weight.shape[0]):
+        return False
+    return all(t.stride(-1) == 1 and t.data_ptr() % 16 == 0 and all(s % 4 == 0 for s in t.stride()[:-1]) for t in (x, weight))
+
+
+def float_gemm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None = None, tile: int = 0, splits: int = 0) -> torch.Tensor:
+    """x [tokens, K] times weight [features, K] transposed (or a batch of such products, [batch, ...]), float32 in, out and sums: every operand goes
+    to the tcgen05 tensor cores as the three bfloat16 numbers whose sum it is.  ``tile`` (tokens) and ``splits`` (of K): the caller's choice, 0 the
+    kernel's own."""
+    if not (x.is_cuda and weight.is_cuda):
+        raise KernelError("float_gemm: the engine has no CPU path")
+    if not float_gemm_supported(x, weight):
+        raise KernelError("float_gemm: float32 rows of a multiple of 4 numbers on 16-byte boundaries are needed, and shapes that agree")
+    shape = (*x.shape[:-1], weight.shape[-2])
+    if out is None:
+        out = torch.empty(shape, dtype=torch.float32, device=x.device)
+    elif tuple(out.shape) != shape or out.dtype != torch.float32 or out.stride(-1) != 1 or out.device != x.device:
+        raise KernelError("float_gemm: out has the wrong shape, type or layout")
+    batches = x.shape[0] if x.dim() == 3 else 1
+    between = [t.stride(0) if t.dim() == 3 else 0 for t in (x, weight, out)]
+    f = _fn("float_gemm.cu", "dli_float_gemm", [c_void_p] * 3 + [c_int] * 4 + [c_longlong] * 6 + [c_int] * 2 + [c_void_p])
+    _check(f(_ptr(out), _ptr(x), _ptr(weight), batches, x.shape[-2], weight.shape[-2], x.shape[-1], x.stride(-2), weight.stride(-2), out.stride(-2),
+             *between, tile, splits, _stream()), "float_gemm")
+    return out
 
 
 # ------------------------------------------------------------------ layer norm around the residual stream

@@ -312,7 +312,9 @@ class ShiftDecayRecurrence(Part):
         t = {role: tensors[name] for role, name in self.names.items()}
         self.w = {
             "mu": torch.stack([t["mu_" + s] for s in "rkvgw"], 0).contiguous(),  # [5, H]
-            "rkvg": torch.stack([t[r].t() for r in ("r", "k", "v", "g")], 0).contiguous(),  # [4, H, I]: the four products are one batched product
+            # [4, H, I]: the four products are one batched product (float32: a column's H numbers lie together, for the engine's own)
+            "rkvg": torch.stack([t[r] for r in ("r", "k", "v", "g")], 0).transpose(1, 2) if self.env.dtype == torch.float32
+            else torch.stack([t[r].t() for r in ("r", "k", "v", "g")], 0).contiguous(),
             "w1": t["w1"], "w2": t["w2"], "w0": t["w0"], "u": t["u"].contiguous(), "norm": t["norm"], "o": t["o"],
         }
 

@@ -1,0 +1,47 @@
+"""The float32 product on the tensor cores (csrc/float_gemm.cu) against float64, at the edges of its tiles, steps and splits."""
+
+import pytest
+import torch
+
+from dli_b200.kernels import gemm, ops
+
+
+def _error(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tile,splits", [(0, 0), (32, 1), (32, 8), (64, 1), (64, 2), (128, 1), (128, 4)])
+@pytest.mark.parametrize("batch,tokens,features,K", [(0, 1, 1, 4), (0, 31, 127, 60), (3, 33, 129, 68), (0, 64, 128, 128), (2, 65, 8, 192), (0, 127, 257, 516), (0, 129, 100, 1028)])
+def test_products_at_the_edges_of_tiles(batch, tokens, features, K, tile, splits):
+    g = torch.Generator().manual_seed(tokens + K)
+    x, w = ([torch.randn(*([batch] if batch else []), rows, K, generator=g).cuda() for rows in (tokens, features)])
+    want = x.double() @ w.double().transpose(-1, -2)
+    # exact products, sums of at most 8 truncated additions (2^-23 each, with one sign) and of K / 64 rounded ones: 5e-7 for these K
+    assert _error(ops.float_gemm(x, w, tile=tile, splits=splits), want) <= 5e-7
+
+
+@pytest.mark.gpu
+def test_rows_of_a_wider_tensor_and_a_given_result():
+    g = torch.Generator().manual_seed(1)
+    x, w = torch.randn(40, 300, generator=g).cuda()[:, 4:264], torch.randn(90, 520, generator=g).cuda()[:, 260:]
+    room = torch.full((40, 95), 7.0).cuda()
+    ops.float_gemm(x, w, room[:, 3:93])
+    assert _error(room[:, 3:93], x.double() @ w.double().t()) <= 5e-7 and (room[:, :3] == 7).all() and (room[:, 93:] == 7).all()
+    with pytest.raises(ops.KernelError):
+        ops.float_gemm(x[:, 1:], w[:, 1:])  # rows off their 16-byte boundaries
+    assert _error(gemm.linear(x[:, 1:], w[:, 1:]), x[:, 1:].double() @ w[:, 1:].double().t()) <= 2e-6  # the library takes them
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.4e38])
+@pytest.mark.parametrize("tile,splits", [(32, 1), (64, 4), (128, 1)])
+def test_numbers_that_are_not_finite_stay_in_their_row_and_column(value, tile, splits):
+    g = torch.Generator().manual_seed(2)
+    x, w = torch.randn(70, 320, generator=g).cuda(), torch.randn(140, 320, generator=g).cuda() * 0.1
+    x[5, 7], w[133, 300] = value, value
+    got, want = ops.float_gemm(x, w, tile=tile, splits=splits), (x.double() @ w.double().t()).float()
+    rest = torch.ones(70, 140, dtype=torch.bool)
+    rest[5], rest[:, 133] = False, False
+    assert _error(got[rest], want.double()[rest]) <= 5e-7
+    assert (got.isnan() == want.isnan()).all() and (got.isinf() == want.isinf()).all() and (got[want.isinf()] == want[want.isinf()]).all()
