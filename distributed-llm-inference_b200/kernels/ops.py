@@ -545,6 +545,7 @@ def device_wait_errors(clear: bool = True) -> dict[str, int]:
     for source, read, forget, defines in (("skinny_gemm.cu", "dli_skinny_gemm_error", "dli_skinny_gemm_clear_error", None),
                                           ("dense_gemm.cu", "dli_dense_gemm_error", "dli_dense_gemm_clear_error", None),
                                           ("float_gemm.cu", "dli_float_gemm_error", "dli_float_gemm_clear_error", None),
+                                          ("ssm_umma.cu", "dli_ssm_umma_error", "dli_ssm_umma_clear_error", None),
                                           ("recurrence_tiles.cu", "dli_recurrence_tiles_error", "dli_recurrence_tiles_clear_error", None),
                                           ("attention_tc.cu", "dli_paged_prefill_tc_error", "dli_paged_prefill_tc_clear_error", None),
                                           ("attention_tc.cu", "dli_paged_prefill_tc_error", "dli_paged_prefill_tc_clear_error", _BENT)):
@@ -1320,6 +1321,7 @@ def conv_state_update(state: torch.Tensor, u: torch.Tensor, col0: int, q_start: 
 SSM_SCAN_MAX_STATE = 512
 
 
+SSM_UMMA_MIN_STATE = 32  # of csrc/ssm_umma.cu, which takes multiples of 16
 SSM_CHUNK_MAX_STATE = 128  # the tensor-core form keeps a state column block in registers
 # Portions of up to a quarter tile are walked token after token.  That is on the safe side: us, walk / tiles, 64 heads, P 64, N 128: one portion of 4 tokens
 # 7.2 / 8.5, of 8 10.1 / 8.5, of 12 14.1 / 8.4, of 16 16.9 / 8.5; sixteen portions of 4 21 / 34, of 8 31 / 34, of 12 42 / 35, of 16 51 / 35; single tokens beside
@@ -1359,14 +1361,16 @@ def ssm_scan(y: torch.Tensor, xbc: torch.Tensor, u: torch.Tensor, dt_col: int, d
         if u.dtype != torch.bfloat16 or segments < 0:
             raise KernelError("ssm_scan: the tensor-core form takes bfloat16")
         count = state_slot.numel()
-        segments = segments or _fn("ssm_tc.cu", "dli_ssm_segments", [c_int] * 4)(count, heads, P, int(min(max_len, n)))
+        umma = SSM_UMMA_MIN_STATE <= N <= SSM_CHUNK_MAX_STATE and N % 16 == 0
+        source, name = ("ssm_umma.cu", "dli_ssm_umma") if umma else ("ssm_tc.cu", "dli_ssm_chunk")
+        segments = segments or _fn(source, "dli_ssm_umma_segments" if umma else "dli_ssm_segments", [c_int] * 4)(count, heads, P, int(min(max_len, n)))
         part = part_log = None
         if segments > 1:
             part = torch.empty(count * (segments - 1) * heads * P * N, dtype=torch.float32, device=y.device)
             part_log = torch.empty(count * (segments - 1) * heads, dtype=torch.float32, device=y.device)
-        f = _fn("ssm_tc.cu", "dli_ssm_chunk", [c_void_p, c_void_p, c_void_p, c_longlong, c_int] + [c_void_p] * 6 + [c_int] * 6 + [c_void_p] * 3)
+        f = _fn(source, name, [c_void_p, c_void_p, c_void_p, c_longlong, c_int] + [c_void_p] * 6 + [c_int] * (6 + umma) + [c_void_p] * 3)
         _check(f(_ptr(y), _ptr(xbc), _ptr(u), u.stride(0), dt_col, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(q_start),
-                 _ptr(state_slot), count, heads, P, N, groups, segments, _ptr(part), _ptr(part_log), _stream()), "ssm_scan")
+                 _ptr(state_slot), *([n] if umma else []), count, heads, P, N, groups, segments, _ptr(part), _ptr(part_log), _stream()), "ssm_scan")
         global launch_count
         launch_count += segments > 1  # two launches
         return
