@@ -37,12 +37,10 @@
 // 195 -> 80; 32 heads, N 64, prompts of 654, 981 and 1,310 67 -> 53.  The errors of y and S against 64 bits are smaller (1,500 tokens: 1.1e-7 and 7.8e-8, before 2.2e-7 and 1.9e-7).
 //
 // Every wait is bounded: after WAIT_LIMIT polls a code goes to *error_flag, and the CTA goes on to its end without another wait and without storing anything.
-#include <cuda.h>
-
-#include "common.cuh"
-#include "mma_split.cuh"
+#include "umma_tiles.cuh"
 
 using namespace dli;
+using namespace dli::umma;
 typedef __nv_bfloat16 bf16;
 
 namespace {
@@ -51,13 +49,9 @@ constexpr int TOKENS = 128;  // of a tile
 constexpr int COLS = 64;     // columns p of a CTA
 constexpr int WARPS = 16;
 constexpr int THREADS = (WARPS + 3) * 32;
-constexpr int SLAB = TOKENS * 128;  // bytes of 128 rows of 64 bfloat16 numbers, 128-byte swizzle
 constexpr float LOG_FLOOR = -1e4f;  // a log decay below this is 0 as a decay, and its sums stay finite
 constexpr double LOG2E = 1.4426950408889634074;
-constexpr unsigned WAIT_LIMIT = 1u << 24;
-// Sequences of up to SHORT tokens are walked, SHORT_HEADS heads by a CTA (the CTAs of the others leave): a CTA has an SM to itself, and with a head each 24
-// single tokens of 64 heads beside a portion of 100 took 44 us of 54.
-constexpr int SHORT = 4, SHORT_HEADS = 8;
+constexpr int SHORT = 4;  // sequences of up to so many tokens are walked
 
 struct Params {
   float* y;
@@ -72,6 +66,9 @@ struct Params {
   int segments;           // of a sequence; with more than one:
   float* part;            // [seqs][segments - 1][heads][P][N]: the state behind segment 0, then what each segment adds
   float* part_log;        // [seqs][segments - 1][heads]: the sum of its log decays
+  // Heads of a short sequence that a CTA walks (the CTAs of the others leave), 2^0 to 2^3: a CTA has an SM to itself, and with a head each 24 single tokens
+  // of 64 heads beside a portion of 100 took 44 us of 54; but eight heads take four times as long as one, and few short sequences had better spread.
+  int short_shift;
   int y_vec;              // sixteen read-outs side by side lie on a 16-byte boundary
   int* error_flag;
 };
@@ -148,21 +145,21 @@ __device__ __noinline__ void walk_again(const Params& p, int head, int col0, con
   }
 }
 
-// Few tokens of a head, thirty-two columns by a warp, eight at a time.
-__device__ __noinline__ void walk_short(const Params& p, int head, int from_col, float* state, int t_from, int t_end) {
+// Few tokens of columns from_col .. to_col - 1 of a head, by a warp, COUNT columns at a time.
+template <int COUNT> __device__ __noinline__ void walk_short(const Params& p, int head, int from_col, int to_col, float* state, int t_from, int t_end) {
   const int lane = threadIdx.x & 31, N = p.N, P = p.P, inner = p.heads * P, width = inner + 2 * p.groups * N;
   const float A = expf(p.A_log[head]), bias = p.dt_bias[head], Dh = p.D[head];
   const int g = head / (p.heads / p.groups);
-  for (int c0 = from_col; c0 < min(P, from_col + 32); c0 += 8) {  // (P is a multiple of 8)
-    float S[8][4];
+  for (int c0 = from_col; c0 < to_col; c0 += COUNT) {
+    float S[COUNT][4];
 #pragma unroll
-    for (int c = 0; c < 8; ++c)
+    for (int c = 0; c < COUNT; ++c)
 #pragma unroll
       for (int m = 0; m < 4; ++m) S[c][m] = lane + 32 * m < N ? state[(size_t)(c0 + c) * N + lane + 32 * m] : 0.f;
     for (int t = t_from; t < t_end; ++t) {
       const bf16* row = p.xbc + (size_t)t * width;
       const float dt = softplus(to_float(p.u[(size_t)t * p.u_stride + p.dt_col + head]) + bias), decay = expf(-A * dt);
-      float B[4], C[4], sum[8];
+      float B[4], C[4], sum[COUNT];
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
         const bool in = lane + 32 * m < N;
@@ -170,7 +167,7 @@ __device__ __noinline__ void walk_short(const Params& p, int head, int from_col,
         C[m] = in ? to_float(row[inner + (p.groups + g) * N + lane + 32 * m]) : 0.f;
       }
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
+      for (int c = 0; c < COUNT; ++c) {
         const float dtx = dt * to_float(row[head * P + c0 + c]);
         sum[c] = 0.f;
 #pragma unroll
@@ -180,133 +177,15 @@ __device__ __noinline__ void walk_short(const Params& p, int head, int from_col,
             sum[c] = fmaf(S[c][m], C[m], sum[c]);
           }
       }
-      // eight sums over the lanes: a lane keeps the half of its numbers that its bit names
-#pragma unroll
-      for (int half = 4, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
-        const bool upper = (lane & bit) != 0;
-#pragma unroll
-        for (int c = 0; c < half; ++c) {
-          const float give = upper ? sum[c] : sum[c + half], keep = upper ? sum[c + half] : sum[c];
-          sum[c] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
-        }
-      }
-      sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 2);
-      sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 1);
-      const int c = head * P + c0 + (lane >> 2);
-      if ((lane & 3) == 0) p.y[(size_t)t * inner + c] = fmaf(Dh, to_float(row[c]), sum[0]);
+      sum_over_lanes<COUNT>(sum, lane);
+      const int c = head * P + c0 + lane / (32 / COUNT);
+      if (lane % (32 / COUNT) == 0) p.y[(size_t)t * inner + c] = fmaf(Dh, to_float(row[c]), sum[0]);
     }
 #pragma unroll
-    for (int c = 0; c < 8; ++c)
+    for (int c = 0; c < COUNT; ++c)
 #pragma unroll
       for (int m = 0; m < 4; ++m)
         if (lane + 32 * m < N) state[(size_t)(c0 + c) * N + lane + 32 * m] = S[c][m];
-  }
-}
-
-__device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count)); }
-__device__ __forceinline__ void bar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool bar_done(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-  return done;
-}
-// Waits for a barrier's phase, `left` polls at most.  When they run out *failed says so, the caller polls once only from then on and goes on to the end;
-// nothing is stored behind it.  (A tight loop: the kernel's instructions should stay in the SM's cache.)
-__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, unsigned& left, volatile int* failed, int* error_flag, int code) {
-  uint32_t polls;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tmov.u32 %0, %3;\n"
-      "AGAIN_%=:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra DONE_%=;\n\t"
-      "sub.u32 %0, %0, 1;\n\tsetp.ne.u32 q, %0, 0;\n\t@q bra AGAIN_%=;\n"
-      "DONE_%=:\n\t}"
-      : "=&r"(polls) : "r"(bar), "r"(parity), "r"(left) : "memory");
-  if (polls == 0) {
-    left = 1;
-    if (!*failed) { *failed = code; atomicCAS(error_flag, 0, code); }
-  }
-  __syncwarp();
-}
-__device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-               ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
-}
-// Operand of 128-byte rows in 128-byte swizzle: 1,024 bytes between groups of eight rows; `slab`: bytes between runs of 64 of an operand whose rows are k
-__device__ __forceinline__ uint64_t operand(uint32_t addr, int slab = 0) {
-  return (uint64_t)((addr & 0x3FFFF) >> 4) | (uint64_t)(slab >> 4) << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
-}
-// kind::f16: float32 accumulator, bfloat16 operands, M = 128; a_rows_k / b_rows_k: the operand's rows in shared memory are k
-__device__ __forceinline__ uint32_t instruction(int n, bool a_rows_k, bool b_rows_k) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_rows_k << 15) | ((uint32_t)b_rows_k << 16) | ((uint32_t)(n >> 3) << 17) | (8u << 24);
-}
-// Products are issued by one lane of a warp that runs together, so that descriptors stay in uniform registers: by a thread in a branch of its own an
-// instruction took 100 to 180 clocks, more than the tensor cores need for it.
-__device__ __forceinline__ uint32_t elect_one() {
-  uint32_t one;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
-  return one;
-}
-__device__ __forceinline__ void product(uint32_t one, uint32_t sum, uint64_t a, uint64_t b, uint32_t idesc, bool add) {
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %5, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-               ::"r"(sum), "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)add), "r"(one) : "memory");
-}
-__device__ __forceinline__ void product_tmem(uint32_t one, uint32_t sum, uint32_t a, uint64_t b, uint32_t idesc, bool add) {  // A in tensor memory
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %5, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-               ::"r"(sum), "r"(a), "l"(b), "r"(idesc), "r"((uint32_t)add), "r"(one) : "memory");
-}
-__device__ __forceinline__ void commit(uint32_t one, uint32_t bar) {
-  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(one) : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
-                 "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-               : "r"(addr));
-}
-__device__ __forceinline__ void tmem_ld8(uint32_t addr, uint32_t (&v)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(addr));
-}
-__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&v)[16]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-               ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
-                 "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]));
-}
-__device__ __forceinline__ void tmem_st4(uint32_t addr, const uint32_t (&v)[4]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]));
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void st_shared16(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-__device__ __forceinline__ void ld_shared16(uint32_t addr, uint32_t (&v)[4]) {
-  asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ float lds(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-  return v;
-}
-__device__ __forceinline__ float4 lds4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-  return v;
-}
-// sixteen numbers in three terms to columns 16 part .. of row r of three slabs
-__device__ __forceinline__ void store_terms(uint32_t dst, int term_bytes, int r, int part, const float (&v)[16]) {
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    uint32_t t[3][4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) dli::split3(v[8 * h + 2 * e], v[8 * h + 2 * e + 1], t[0][e], t[1][e], t[2][e]);
-    const uint32_t at = dst + r * 128 + (((2 * part + h) ^ (r & 7)) << 4);
-#pragma unroll
-    for (int s = 0; s < 3; ++s) st_shared16(at + s * term_bytes, t[s][0], t[s][1], t[s][2], t[s][3]);
   }
 }
 
@@ -333,9 +212,12 @@ __global__ void __launch_bounds__(THREADS, 1) ssm_umma_kernel(const __grid_const
   const size_t block = (size_t)P * N;
   float* slot_state = p.state + ((size_t)p.state_slot[seq] * p.heads + head) * block;
   if (last - first <= SHORT) {  // (one tile, so it is segment 0)
-    const int mine = head + (warp >> 1);
-    if (head % SHORT_HEADS == 0 && warp < 2 * SHORT_HEADS && mine < p.heads)
-      walk_short(p, mine, col0 + (warp & 1) * 32, slot_state + (size_t)(warp >> 1) * block, t0, t1);
+    if (head & ((1 << p.short_shift) - 1)) return;
+    const int columns = 4 << p.short_shift, more = warp >> (4 - p.short_shift), from_col = col0 + (warp & ((WARPS >> p.short_shift) - 1)) * columns;
+    if (warp < WARPS && head + more < p.heads) {  // (P is a multiple of 8)
+      if (columns == 4) walk_short<4>(p, head + more, from_col, min(P, from_col + 4), slot_state + more * block, t0, t1);
+      else walk_short<8>(p, head + more, from_col, min(P, from_col + columns), slot_state + more * block, t0, t1);
+    }
     return;
   }
 
@@ -778,20 +660,15 @@ __global__ void __launch_bounds__(THREADS, 1) ssm_umma_kernel(const __grid_const
 
 inline int column_blocks(int P) { return (P + COLS - 1) / COLS; }
 
-typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiled encode_fn() {
-  static EncodeTiled fn = nullptr;
-  if (!fn) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess) fn = (EncodeTiled)ptr;
-  }
-  return fn;
-}
-
 int* error_flag_device = nullptr;
 int* error_flag_host = nullptr;
+
+// as many as leave every SM about one CTA of short sequences
+inline int short_shift(long long units) {
+  int s = 0;
+  while (s < 3 && units > ((long long)sm_count() << s) * 3 / 2) ++s;
+  return s;
+}
 
 template <int NB>
 int launch(const CUtensorMap& map, const CUtensorMap& map_y, const Params& p, cudaStream_t stream) {
@@ -834,29 +711,15 @@ DLI_EXPORT int dli_ssm_umma(float* y, const void* xbc, const void* u, long long 
     *error_flag_host = 0;
     if (cudaHostGetDevicePointer((void**)&error_flag_device, error_flag_host, 0) != cudaSuccess) return (int)cudaGetLastError();
   }
-  EncodeTiled fn = encode_fn();
-  if (!fn) return DLI_ERR_UNSUPPORTED;
-  const int width = heads * P + 2 * groups * N;
-  CUtensorMap map;
-  cuuint64_t dims[2] = {(cuuint64_t)width, (cuuint64_t)n};
-  cuuint64_t strides[1] = {(cuuint64_t)width * 2};
-  cuuint32_t box[2] = {64, TOKENS}, elem[2] = {1, 1};
-  if (fn(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(xbc), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return DLI_ERR_UNSUPPORTED;
-  const int y_vec = ((uintptr_t)y & 15) == 0;
-  CUtensorMap map_y = map;  // (not used where y is not aligned)
-  if (y_vec) {
-    cuuint64_t y_dims[2] = {(cuuint64_t)heads * P, (cuuint64_t)n}, y_strides[1] = {(cuuint64_t)heads * P * 4};
-    cuuint32_t y_box[2] = {32, 32};
-    if (fn(&map_y, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, y, y_dims, y_strides, y_box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-           CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return DLI_ERR_UNSUPPORTED;
-  }
+  const int width = heads * P + 2 * groups * N, y_vec = ((uintptr_t)y & 15) == 0;
+  CUtensorMap map, map_y;
+  if (!make_map(&map, xbc, false, n, width, width, TOKENS)) return DLI_ERR_UNSUPPORTED;
+  map_y = map;  // (not used where y is not aligned)
+  if (y_vec && !make_map(&map_y, y, true, n, (long long)heads * P, (long long)heads * P, 32)) return DLI_ERR_UNSUPPORTED;
   Params p;
   p.y = y; p.xbc = (const bf16*)xbc; p.u = (const bf16*)u; p.u_stride = u_stride; p.dt_col = dt_col; p.dt_bias = dt_bias; p.A_log = A_log; p.D = D;
   p.state = state; p.q_start = q_start; p.state_slot = state_slot; p.num_seqs = num_seqs; p.heads = heads; p.P = P; p.N = N; p.groups = groups;
-  p.segments = segments; p.part = part; p.part_log = part_log; p.y_vec = y_vec; p.error_flag = error_flag_device;
+  p.segments = segments; p.part = part; p.part_log = part_log; p.y_vec = y_vec; p.short_shift = short_shift((long long)column_blocks(P) * heads * num_seqs); p.error_flag = error_flag_device;
   return N <= 64 ? launch<1>(map, map_y, p, stream) : launch<2>(map, map_y, p, stream);
 }
 

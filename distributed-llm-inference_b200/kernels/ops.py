@@ -1321,7 +1321,8 @@ def conv_state_update(state: torch.Tensor, u: torch.Tensor, col0: int, q_start: 
 SSM_SCAN_MAX_STATE = 512
 
 
-SSM_UMMA_MIN_STATE = 32  # of csrc/ssm_umma.cu, which takes multiples of 16
+# Of csrc/ssm_umma.cu, which takes multiples of 16; tiles of 64 / 128 tokens, us, 64 heads, N 128: 17 tokens 9.4 / 10.2, 33 10.2 / 10.3, 100 17 / 11.
+SSM_UMMA_MIN_STATE, SSM_UMMA_MIN_TOKENS = 32, 33
 SSM_CHUNK_MAX_STATE = 128  # the tensor-core form keeps a state column block in registers
 # Portions of up to a quarter tile are walked token after token.  That is on the safe side: us, walk / tiles, 64 heads, P 64, N 128: one portion of 4 tokens
 # 7.2 / 8.5, of 8 10.1 / 8.5, of 12 14.1 / 8.4, of 16 16.9 / 8.5; sixteen portions of 4 21 / 34, of 8 31 / 34, of 12 42 / 35, of 16 51 / 35; single tokens beside
@@ -1361,7 +1362,7 @@ def ssm_scan(y: torch.Tensor, xbc: torch.Tensor, u: torch.Tensor, dt_col: int, d
         if u.dtype != torch.bfloat16 or segments < 0:
             raise KernelError("ssm_scan: the tensor-core form takes bfloat16")
         count = state_slot.numel()
-        umma = SSM_UMMA_MIN_STATE <= N <= SSM_CHUNK_MAX_STATE and N % 16 == 0
+        umma = SSM_UMMA_MIN_STATE <= N <= SSM_CHUNK_MAX_STATE and N % 16 == 0 and min(max_len, n) >= SSM_UMMA_MIN_TOKENS
         source, name = ("ssm_umma.cu", "dli_ssm_umma") if umma else ("ssm_tc.cu", "dli_ssm_chunk")
         segments = segments or _fn(source, "dli_ssm_umma_segments" if umma else "dli_ssm_segments", [c_int] * 4)(count, heads, P, int(min(max_len, n)))
         part = part_log = None
