@@ -545,6 +545,7 @@ def device_wait_errors(clear: bool = True) -> dict[str, int]:
     for source, read, forget, defines in (("skinny_gemm.cu", "dli_skinny_gemm_error", "dli_skinny_gemm_clear_error", None),
                                           ("dense_gemm.cu", "dli_dense_gemm_error", "dli_dense_gemm_clear_error", None),
                                           ("float_gemm.cu", "dli_float_gemm_error", "dli_float_gemm_clear_error", None),
+                                          ("matrix_memory_umma.cu", "dli_matrix_memory_umma_error", "dli_matrix_memory_umma_clear_error", None),
                                           ("ssm_umma.cu", "dli_ssm_umma_error", "dli_ssm_umma_clear_error", None),
                                           ("recurrence_tiles.cu", "dli_recurrence_tiles_error", "dli_recurrence_tiles_clear_error", None),
                                           ("attention_tc.cu", "dli_paged_prefill_tc_error", "dli_paged_prefill_tc_clear_error", None),
@@ -1931,6 +1932,9 @@ def channel_delta_scan(o: torch.Tensor, qkv: torch.Tensor, u: torch.Tensor, b_co
 
 MATRIX_MEMORY_MAX_HEAD_DIM = 512
 MATRIX_MEMORY_CHUNK_MAX_HEAD_DIM = 256  # the tensor-core kernel keeps a state column block in registers
+# From here on portions go in tiles of 128 tokens (csrc/matrix_memory_umma.cu).  Tiles of 64 / 128, us, heads of 128: 16 heads, 17 tokens 9.8 / 12.3, 44 beside two
+# single ones 12.7 / 12.3, 100 18 / 13; 8 heads, twice 21 beside two 10.2 / 12.3.
+MATRIX_MEMORY_UMMA_MIN_TOKENS = 49
 MATRIX_MEMORY_CHUNK_MIN_TOKENS = 17  # shorter portions are walked token after token
 
 
@@ -1969,15 +1973,18 @@ def matrix_memory_scan(o: torch.Tensor, divisor: torch.Tensor, u: torch.Tensor, 
     if form == "chunk":
         if u.dtype != torch.bfloat16 or d > MATRIX_MEMORY_CHUNK_MAX_HEAD_DIM:
             raise KernelError("matrix_memory_scan: the tensor-core form takes bfloat16 heads of at most 256")
-        lib = {"KEY_DIM": -(-d // 16) * 16}
+        count = state_slot.numel()
+        umma = 32 <= d <= 128 and d % 16 == 0 and dv % 8 == 0 and min(max_len, n) >= MATRIX_MEMORY_UMMA_MIN_TOKENS and u.data_ptr() % 16 == 0 and u.stride(0) % 8 == 0 and o.data_ptr() % 8 == 0
+        source, name, lib = ("matrix_memory_umma.cu", "dli_matrix_memory_umma", None) if umma else ("matrix_memory_tc.cu", "dli_matrix_memory_chunk", {"KEY_DIM": -(-d // 16) * 16})
         if segments < 1:
-            segments = _fn("matrix_memory_tc.cu", "dli_matrix_memory_segments", [c_int] * 4, lib)(state_slot.numel(), heads, dv, int(min(max_len, n)))
+            segments = _fn(source, name.replace("_chunk", "") + "_segments", [c_int] * 4, lib)(count, heads, dv, int(min(max_len, n)))
         part = part_m = None
         if segments > 1:
-            rows = state_slot.numel() * segments * heads * dv1
-            part, part_m = torch.empty(rows * d, dtype=torch.float32, device=o.device), torch.empty(rows * 2, dtype=torch.float32, device=o.device)
-        f = _fn("matrix_memory_tc.cu", "dli_matrix_memory_chunk", types + [c_int, c_void_p, c_void_p, c_void_p], lib)
-        _check(f(*args, segments, _ptr(part), _ptr(part_m), _stream()), "matrix_memory_scan")
+            rows = count * (segments - umma) * heads
+            part = torch.empty(rows * dv1 * d, dtype=torch.float32, device=o.device)
+            part_m = torch.empty(rows * (1 if umma else dv1) * 2, dtype=torch.float32, device=o.device)
+        f = _fn(source, name, types + [c_int] * (1 + umma) + [c_void_p, c_void_p, c_void_p], lib)
+        _check(f(*args, *([n] if umma else []), segments, _ptr(part), _ptr(part_m), _stream()), "matrix_memory_scan")
         global launch_count
         launch_count += segments > 1  # two launches
     elif form == "walk":
