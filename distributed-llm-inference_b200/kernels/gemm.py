@@ -76,6 +76,30 @@ def dense_product(x, features: int, epilogue: str) -> bool:
     raise ValueError(f"unknown epilogue {epilogue!r}")
 
 
+# Steps of more tokens than the decode product takes, up to here, go to the engine's product for some tokens (csrc/few_gemm.cu) where it beats the library.
+# Measured in chains of replayed products with cold weights, us, library / own at 9, 33 and 64 tokens: 2,048 features of K 2,048 5.5/3.6, 5.6/4.6, 5.7/4.9;
+# 2,048 of 8,192 13.1/9.6, 13.2/10.9, 13.4/11.3; 1,024 of 4,096 10.1/4.3, 7.9/5.4, 7.9/6.4; 4,096 of 4,096 9.7/8.5, 9.8/9.7, 9.9/10.0; but where all SMs have a
+# tile of their own anyway 10,304 of 2,048 10.7/9.7, 11.6/10.8, 9.7/11.1; 6,176 of 2,048 7.7/7.3, 7.6/8.2, 7.4/8.6.  gate|up with SiLU * up (8,192 each, of 2,048)
+# 16.4/13.1, 16.6/14.3, 16.7/15.4, at 96 and 128 tokens 18.2/16.6, 17.7/17.8.
+FEW_MAX_TOKENS, FEW_MAX_TOKENS_SWIGLU, FEW_MAX_TOKENS_ANY_WIDTH = 64, 96, 24
+FEW_MIN_SIZE = 1024  # of K and of the features
+
+
+def few_splits(features: int, K: int) -> int:
+    """CTAs that share a tile's K: the most for which clusters of them still fit the GPU at once and each has four steps of 128."""
+    tiles, steps = -(-features // 128), -(-K // 128)
+    return next((s for s, places in ((8, 112), (4, 132), (2, 148)) if tiles * s <= places and steps >= 4 * s), 1)
+
+
+def few_product(x: torch.Tensor, weight: torch.Tensor, swiglu: bool = False) -> bool:
+    """Whether the product of these activations with a [features, K] weight goes to the engine's product for some tokens."""
+    if not ops.few_gemm_supported(x, weight) or x.shape[0] <= SKINNY_MAX_TOKENS or min(weight.shape) < FEW_MIN_SIZE:
+        return False
+    if swiglu:
+        return x.shape[0] <= FEW_MAX_TOKENS_SWIGLU and weight.shape[0] % 128 == 0
+    return x.shape[0] <= (FEW_MAX_TOKENS if weight.shape[0] <= 33 * 128 else FEW_MAX_TOKENS_ANY_WIDTH)
+
+
 def project(x, weight: torch.Tensor, out_dtype: torch.dtype | None = None, max_tokens: int = SKINNY_MAX_TOKENS) -> torch.Tensor:
     """y = x W^T for a step's tokens, in x's dtype or in ``out_dtype`` (float32 for logits).  x may be
     ops.ScaledRows (rows that still lack their norm's factor): those only exist for token counts that
@@ -136,6 +160,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None = Non
         raise RuntimeError("linear: TF32 was switched on; the float32 path must stay true 32-bit")
     if out is None and float_product(x, weight):
         return ops.float_gemm(x, weight)
+    if out is None and few_product(x, weight):
+        return ops.few_gemm(x, weight, few_splits(*weight.shape))
     return torch.matmul(x, weight.t(), out=out)
 
 

@@ -544,6 +544,7 @@ def device_wait_errors(clear: bool = True) -> dict[str, int]:
     found = {}
     for source, read, forget, defines in (("skinny_gemm.cu", "dli_skinny_gemm_error", "dli_skinny_gemm_clear_error", None),
                                           ("dense_gemm.cu", "dli_dense_gemm_error", "dli_dense_gemm_clear_error", None),
+                                          ("few_gemm.cu", "dli_few_gemm_error", "dli_few_gemm_clear_error", None),
                                           ("float_gemm.cu", "dli_float_gemm_error", "dli_float_gemm_clear_error", None),
                                           ("matrix_memory_umma.cu", "dli_matrix_memory_umma_error", "dli_matrix_memory_umma_clear_error", None),
                                           ("ssm_umma.cu", "dli_ssm_umma_error", "dli_ssm_umma_clear_error", None),
@@ -979,6 +980,32 @@ def dense_gemm_error() -> int:
 def skinny_gemm_error() -> int:
     """0, or which bounded wait of the decode matrix product ran out since the library was loaded."""
     return _fn("skinny_gemm.cu", "dli_skinny_gemm_error", [])()
+
+
+# ------------------------------------------------------------------ products of some tokens
+
+FEW_GEMM_MAX_TOKENS = 256
+
+
+def few_gemm_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether ``few_gemm`` takes these operands: bfloat16, up to 256 rows of a multiple of 8 numbers on 16-byte boundaries."""
+    return (x.dtype == weight.dtype == torch.bfloat16 and x.dim() == 2 and 1 <= x.shape[0] <= FEW_GEMM_MAX_TOKENS and x.shape[1] % 8 == 0 and x.stride(1) == 1
+            and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and weight.is_contiguous() and weight.data_ptr() % 16 == 0 and weight.shape[0] % 4 == 0)
+
+
+def few_gemm(x: torch.Tensor, weight: torch.Tensor, splits: int, swiglu: bool = False) -> torch.Tensor:
+    """x [tokens, K] times weight [features, K] transposed for 1 to 256 tokens, float32 sums, on tcgen05: every weight tile is read once, and ``splits``
+    CTAs (1, 2, 4, 8: a cluster) share its K.  ``swiglu``: the weight's rows are blocks of 64 gate rows and the 64 up rows of the same
+    features; returned is silu(gate) * up [tokens, features / 2]."""
+    if not (x.is_cuda and weight.is_cuda):
+        raise KernelError("few_gemm: the engine has no CPU path")
+    if not few_gemm_supported(x, weight) or x.shape[1] != weight.shape[1] or (swiglu and weight.shape[0] % 128):
+        raise KernelError("few_gemm: sizes, types or alignment not supported")
+    features = weight.shape[0]
+    out = torch.empty((x.shape[0], features // 2 if swiglu else features), dtype=torch.bfloat16, device=x.device)
+    f = _fn("few_gemm.cu", "dli_few_gemm", [c_void_p] * 3 + [c_int] * 3 + [c_longlong] + [c_int] * 2 + [c_void_p])
+    _check(f(_ptr(out), _ptr(x), _ptr(weight), x.shape[0], features, x.shape[1], x.stride(0), int(swiglu), splits, _stream()), "few_gemm")
+    return out
 
 
 # ------------------------------------------------------------------ float32 products on the tensor cores

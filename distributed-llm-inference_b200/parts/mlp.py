@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch
 
 from ..kernels import ops
-from ..kernels.gemm import dense_product, fused_epilogue, last_product, project
+from ..kernels.gemm import dense_product, few_product, few_splits, fused_epilogue, last_product, project
 from ..weights.loader import TensorDecl
 from .base import Part, PendingMixture, build_part, register_part, tensor_name
 
@@ -62,6 +62,8 @@ class SwiGLU(Part):
             act = ops.skinny_gemm_swiglu(x, self.w_gate_up, self.activation, self.limit, self.up_shift)
         elif self.tiled and dense_product(x, 2 * self.inter, "swiglu"):
             act = ops.dense_gemm_swiglu(x, self.w_gate_up, self.activation, self.limit, self.up_shift)
+        elif self.tiled and self.activation == "silu" and not self.limit and not self.up_shift and few_product(x, self.w_gate_up, swiglu=True):
+            act = ops.few_gemm(x, self.w_gate_up, few_splits(*self.w_gate_up.shape), swiglu=True)
         else:
             gate_up = project(x, self.w_gate_up)
             act = torch.empty((x.shape[0], self.inter), dtype=x.dtype, device=x.device)

@@ -1,0 +1,46 @@
+"""The product of some tokens (csrc/few_gemm.cu) against float64, at the edges of its tiles, steps and splits, and which products it serves."""
+
+import pytest
+import torch
+
+from dli_b200.kernels import gemm, ops
+
+
+def _error(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("splits", [1, 2, 4, 8])
+@pytest.mark.parametrize("tokens,features,K", [(1, 4, 8), (9, 132, 120), (16, 128, 128), (17, 300, 136), (33, 128, 1032), (64, 260, 2048), (65, 124, 384), (129, 256, 256), (256, 12, 1024)])
+def test_products_at_the_edges_of_tiles(tokens, features, K, splits):
+    g = torch.Generator().manual_seed(tokens + K)
+    room, w = torch.randn(tokens, K + 24, generator=g).bfloat16().cuda(), torch.randn(features, K, generator=g).bfloat16().cuda()
+    x = room[:, 8 : 8 + K]  # rows of a wider tensor
+    got = ops.few_gemm(x, w, splits)
+    # one rounding to bfloat16, 2^-9 at most and 2^-9 / sqrt(3) in the mean; float32 sums add 1e-6
+    assert got.shape == (tokens, features) and _error(got, x.double() @ w.double().t()) <= 2.0**-9
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("splits", [1, 2, 4])
+@pytest.mark.parametrize("tokens,I,K", [(9, 64, 128), (50, 192, 520), (96, 128, 1024)])
+def test_the_activation_of_a_gated_feed_forward(tokens, I, K, splits):
+    g = torch.Generator().manual_seed(tokens)
+    x, gate, up = torch.randn(tokens, K, generator=g).bfloat16().cuda(), (torch.randn(I, K, generator=g) * 0.1).bfloat16().cuda(), (torch.randn(I, K, generator=g) * 0.1).bfloat16().cuda()
+    w = torch.stack([gate.view(-1, 64, K), up.view(-1, 64, K)], 1).reshape(2 * I, K).contiguous()
+    a, b = (x.double() @ gate.double().t()).bfloat16(), (x.double() @ up.double().t()).bfloat16()  # the sums as bfloat16 holds them
+    want = torch.nn.functional.silu(a.double()) * b.double()
+    # a sum near the middle between two bfloat16 numbers may be rounded the other way: some of them move by 2^-8, on top of the result's own 2^-9
+    assert _error(ops.few_gemm(x, w, splits, swiglu=True), want) <= 2.0**-8
+
+
+def test_which_products_go_there():
+    def takes(tokens, features, K, dtype=torch.bfloat16, swiglu=False):
+        return gemm.few_product(torch.empty(tokens, K, dtype=dtype), torch.empty(features, K, dtype=dtype), swiglu)
+
+    assert takes(9, 2048, 2048) and takes(64, 2048, 8192) and not takes(65, 2048, 8192) and not takes(8, 2048, 2048)
+    assert takes(24, 10304, 2048) and not takes(25, 10304, 2048) and not takes(16, 2048, 512) and not takes(16, 64, 2048)
+    assert takes(96, 16384, 2048, swiglu=True) and not takes(97, 16384, 2048, swiglu=True) and not takes(16, 2048, 2048, torch.float32)
+    assert not gemm.few_product(torch.empty(16, 2052, dtype=torch.bfloat16)[:, 4:], torch.empty(2048, 2048, dtype=torch.bfloat16))  # rows off 16 bytes
+    assert [gemm.few_splits(*s) for s in ((2048, 2048), (16384, 2048), (1024, 4096), (4240, 2048), (4096, 4096), (1024, 1024))] == [4, 1, 8, 2, 4, 2]
