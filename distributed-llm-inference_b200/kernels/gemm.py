@@ -80,9 +80,11 @@ def dense_product(x, features: int, epilogue: str) -> bool:
 # Measured in chains of replayed products with cold weights, us, library / own at 9, 33 and 64 tokens: 2,048 features of K 2,048 5.5/3.6, 5.6/4.6, 5.7/4.9;
 # 2,048 of 8,192 13.1/9.6, 13.2/10.9, 13.4/11.3; 1,024 of 4,096 10.1/4.3, 7.9/5.4, 7.9/6.4; 4,096 of 4,096 9.7/8.5, 9.8/9.7, 9.9/10.0; but where all SMs have a
 # tile of their own anyway 10,304 of 2,048 10.7/9.7, 11.6/10.8, 9.7/11.1; 6,176 of 2,048 7.7/7.3, 7.6/8.2, 7.4/8.6.  gate|up with SiLU * up (8,192 each, of 2,048)
-# 16.4/13.1, 16.6/14.3, 16.7/15.4, at 96 and 128 tokens 18.2/16.6, 17.7/17.8.
-FEW_MAX_TOKENS, FEW_MAX_TOKENS_SWIGLU, FEW_MAX_TOKENS_ANY_WIDTH = 64, 96, 24
-FEW_MIN_SIZE = 1024  # of K and of the features
+# 16.4/13.1, 16.6/14.3, 16.7/15.4, at 96 and 128 tokens 18.2/16.6, 17.7/17.8.  Between other kernels a product of the engine starts and ends later than the
+# library's by up to a microsecond: an attention layer of 2,048 with 40 single tokens 30.7 -> 32.8 us with both products here, with 16 28.7 both; four layers of a
+# Llama of 2,048 with 16 single tokens 333 -> 281 us.
+FEW_MAX_TOKENS, FEW_MAX_TOKENS_SWIGLU, FEW_MAX_TOKENS_SHORT_K = 64, 96, 24
+FEW_MIN_SIZE, FEW_LONG_K, FEW_MAX_FEATURES = 1024, 4096, 4224  # least K and features; from which K on, and up to which width, more than 24 tokens go there
 
 
 def few_splits(features: int, K: int) -> int:
@@ -97,7 +99,7 @@ def few_product(x: torch.Tensor, weight: torch.Tensor, swiglu: bool = False) -> 
         return False
     if swiglu:
         return x.shape[0] <= FEW_MAX_TOKENS_SWIGLU and weight.shape[0] % 128 == 0
-    return x.shape[0] <= (FEW_MAX_TOKENS if weight.shape[0] <= 33 * 128 else FEW_MAX_TOKENS_ANY_WIDTH)
+    return x.shape[0] <= (FEW_MAX_TOKENS if weight.shape[1] >= FEW_LONG_K and weight.shape[0] <= FEW_MAX_FEATURES else FEW_MAX_TOKENS_SHORT_K)
 
 
 def project(x, weight: torch.Tensor, out_dtype: torch.dtype | None = None, max_tokens: int = SKINNY_MAX_TOKENS) -> torch.Tensor:

@@ -39,7 +39,7 @@ def test_which_products_go_there():
     def takes(tokens, features, K, dtype=torch.bfloat16, swiglu=False):
         return gemm.few_product(torch.empty(tokens, K, dtype=dtype), torch.empty(features, K, dtype=dtype), swiglu)
 
-    assert takes(9, 2048, 2048) and takes(64, 2048, 8192) and not takes(65, 2048, 8192) and not takes(8, 2048, 2048)
+    assert takes(24, 2048, 2048) and not takes(25, 2048, 2048) and takes(64, 2048, 8192) and not takes(65, 2048, 8192) and not takes(8, 2048, 2048)
     assert takes(24, 10304, 2048) and not takes(25, 10304, 2048) and not takes(16, 2048, 512) and not takes(16, 64, 2048)
     assert takes(96, 16384, 2048, swiglu=True) and not takes(97, 16384, 2048, swiglu=True) and not takes(16, 2048, 2048, torch.float32)
     assert not gemm.few_product(torch.empty(16, 2052, dtype=torch.bfloat16)[:, 4:], torch.empty(2048, 2048, dtype=torch.bfloat16))  # rows off 16 bytes
