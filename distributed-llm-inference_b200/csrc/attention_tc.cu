@@ -1261,6 +1261,18 @@ bool make_pool_map(CUtensorMap* map, const void* base, long long rows, int page_
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+#if !BENT_SCORES
+// the same with d a multiple of 64, as [rows / 8][d / 64][8][64]; a box is a page of one head (or 64 rows of it) with all its columns
+bool make_row_map(CUtensorMap* map, const void* base, long long rows, int page_size, int d) {
+  EncodeTiled fn = encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[4] = {64, 8, (cuuint64_t)(d / 64), (cuuint64_t)(rows / 8)}, strides[3] = {(cuuint64_t)d * 2, 128, (cuuint64_t)d * 16};
+  cuuint32_t box[4] = {64, 8, (cuuint32_t)(d / 64), (cuuint32_t)(page_size < 64 ? page_size / 8 : 8)}, elem[4] = {1, 1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+#endif
+
 int* error_flag_device = nullptr;
 int* error_flag_host = nullptr;
 
@@ -1283,16 +1295,17 @@ int launch_tc2(const CUtensorMap& map_k, const CUtensorMap& map_v, const Params&
 #if !BENT_SCORES
 // ================================================================ one pool: a cached row is key and value
 // Prompt portions over rows of 136 to 256 numbers whose leading numbers are the values (attention over a cached latent: many query
-// heads on one KV head).  The products and roles are those of the kernel with two threads per row; a tile of 128 rows comes once, as
-// SLABS slabs of 64 columns, and is the K-major operand of S = Q K^T and the MN-major operand of O += P V (all value columns in
-// one instruction).  Q, two tiles and P fill shared memory (64 + 2 x 64 + 32 KB with 256 columns), S twice and O tensor memory (256 + 256
-// columns).  The thread that issues products takes whichever of S(t + 1) and O += P(t) V(t) is possible first: a tile's stage is only free
-// for the copies once both have read it, so neither should stand behind the other.
+// heads on one KV head).  A tile of 128 rows comes once and is the K-major operand of S = Q K^T and the MN-major operand of O += P V (all value columns in
+// one instruction); it is copied in halves of 64 tokens to a ring of 5 (rows to 256) or 7 (to 192), which with Q fills shared memory.  S twice and O are
+// tensor memory (256 + 256 columns); the probabilities go over the scores that they come from and are the products' operand from there.  Four threads a
+// row do the softmax.  The warp that issues products takes whichever of S(t + 1) and O += P(t) V(t) is possible first.
 //
-// What bounds it: the copies.  With clocks taken in a CTA (4,096 tokens, 16 heads, rows of 256, 192 value columns), a tile takes 4,320 clocks; 3,900 pass
-// from a tile's request to its arrival (64 KB: all SMs read the same rows from L2 at 4.7 TB/s together, the next stage's request waits for O of
-// the tile before the last), 1,000 are S, 2,200 the softmax threads, 800 to 1,700 O.  Measured against the mma.sync kernel, us: 4,096 tokens 797 -> 185
-// (650 TFLOP/s), with a window of 1,024 355 -> 115, 512 tokens 43 -> 21, 8 tokens behind 2,000 four times 149 -> 50, 2 behind 2,000 141 -> 46; portions that see one
+// What bounds it: the chain.  With clocks taken in a CTA (4,096 tokens, 16 heads, rows of 256, 192 value columns), a tile takes 4,150 clocks: a half can
+// only be asked for when O of two tiles before is done, 1,400 until it is there, 1,300 S, 2,600 the softmax, 1,200 O.  Before (a copy for every page and slab:
+// 32 of 2 KB a tile, two threads a row, probabilities by way of shared memory) a tile took 4,320 and a CTA 24,000 beside its tiles, 16,000 of them to bring
+// Q a piece at a time and to zero both stages; those take 1,000 now and the CTA 8,000.  us, before and now: 4,096 tokens 213 -> 168, with a window of 1,024 139 -> 104,
+// 512 tokens 31 -> 23, 8 tokens behind 2,000 four times 61 -> 47, 2 behind 2,000 55 -> 45, 2,048 tokens with rows of 200 (copies by slab)
+// 74 -> 59 (the mma.sync kernel: 4,096 tokens 797, with a window 355, 512 tokens 43, 8 behind 2,000 149, 2 behind 2,000 141); portions that see one
 // key tile of the other kernel stay there (portions_pay_for_tiles_of_rows in kernels/attention.py).
 struct RowParams {
   bf16* out;
@@ -1307,10 +1320,13 @@ struct RowParams {
   int* error_flag;
 };
 
+constexpr int ROW_SOFTMAX_THREADS = 4 * ROWS, ROW_THREADS = ROW_SOFTMAX_THREADS + 64;
+constexpr int HALF_KEYS = KEYS / 2;  // keys of a copied half tile
+
 template <int SLABS> struct RowCfg {
-  static constexpr int STAGE = SLABS * TILE_BYTES;  // one tile of rows; also the Q tile
-  static constexpr int AT_P = 3 * STAGE, AT_MAX = AT_P + 2 * TILE_BYTES, AT_BAR = AT_MAX + 4 * ROWS * 4, SMEM = AT_BAR + 128;
-  static_assert(SMEM <= 227 * 1024, "one CTA fits an SM");
+  static constexpr int Q = SLABS * TILE_BYTES, HALF = Q / 2, HALVES = (224 * 1024 - Q) / HALF;
+  static constexpr int AT_MAX = Q + HALVES * HALF, AT_BAR = AT_MAX + 4 * ROWS * 4, SMEM = AT_BAR + 256;
+  static_assert(SMEM <= 227 * 1024 && HALVES <= 8, "one CTA fits an SM, and its barriers their place");
 };
 
 __device__ __forceinline__ bool barrier_phase_done(uint32_t bar, uint32_t parity) {
@@ -1318,29 +1334,58 @@ __device__ __forceinline__ bool barrier_phase_done(uint32_t bar, uint32_t parity
   asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done;
 }
+// Products are issued by one lane of a warp that runs together, so that descriptors stay in uniform registers.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one;
+}
+__device__ __forceinline__ void umma_one(uint32_t one, uint32_t sum, uint64_t a, uint64_t b, uint32_t idesc, bool add) {
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %5, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+               ::"r"(sum), "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)add), "r"(one) : "memory");
+}
+__device__ __forceinline__ void umma_tmem(uint32_t one, uint32_t sum, uint32_t a, uint64_t b, uint32_t idesc, bool add) {  // A in tensor memory
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %5, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+               ::"r"(sum), "r"(a), "l"(b), "r"(idesc), "r"((uint32_t)add), "r"(one) : "memory");
+}
+__device__ __forceinline__ void umma_commit_one(uint32_t one, uint32_t bar) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(one) : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+                 "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+               : "r"(addr));
+}
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&v)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
+                 "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]));
+}
 
-template <int SLABS>
-__global__ void __launch_bounds__(THREADS, 1) paged_prefill_row_kernel(const __grid_constant__ CUtensorMap map, const RowParams p) {
+// WHOLE: rows of whole slabs; one copy brings a page (of 64 tokens at most), and half a tile is [8 tokens][slab][8][128 bytes], eight rows of a slab
+// in one swizzled piece.  Otherwise it is [slab][64 rows][128 bytes], a copy for every page and slab.
+template <int SLABS, bool WHOLE>
+__global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const __grid_constant__ CUtensorMap map, const RowParams p) {
   using Cfg = RowCfg<SLABS>;
+  constexpr int PIECES = WHOLE ? SLABS * 1024 : 1024, NEXT_SLAB = WHOLE ? 1024 : HALF_KEYS * 128;  // bytes from eight rows to the next eight, from a slab to the next
+  constexpr int HALVES = Cfg::HALVES, HALF = Cfg::HALF;
   pdl_launch_dependents();
   extern __shared__ __align__(1024) unsigned char smem[];
-  unsigned char* sQ = smem;
-  unsigned char* sK = sQ + Cfg::STAGE;  // two stages
-  unsigned char* sP = smem + Cfg::AT_P;  // keys 0..63 | keys 64..127
-  float* row_max = (float*)(smem + Cfg::AT_MAX);  // [2 (tile parity)][2 (half)][128]
+  float* row_max = (float*)(smem + Cfg::AT_MAX);  // [4 (quarter of the keys)][128]
   uint64_t* bars = (uint64_t*)(smem + Cfg::AT_BAR);
-  uint32_t* tmem_slot = (uint32_t*)(bars + 8);
+  uint32_t* tmem_slot = (uint32_t*)(bars + 24);
   volatile int* failed = (volatile int*)(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int r = tid & (ROWS - 1), half = (tid >> 7) & 1;
-  const uint32_t k_full = smem_u32(bars), s_done = smem_u32(bars + 2), o_done = smem_u32(bars + 4), p_ready = smem_u32(bars + 6);
+  const uint32_t sQ = smem_u32(smem), sK = sQ + Cfg::Q;
+  const uint32_t k_full = smem_u32(bars), s_done = smem_u32(bars + 8), o_done = smem_u32(bars + 10), p_ready = smem_u32(bars + 14), q_full = smem_u32(bars + 16);
 
   const int s = p.seq0 + blockIdx.y;
   const int tile = gridDim.z - 1 - blockIdx.z;  // the tiles that see the most keys start first
   const int kvh = blockIdx.x / p.head_chunks, hc = blockIdx.x - kvh * p.head_chunks;
   const int q0 = p.q_start[s], qlen = p.q_start[s + 1] - q0, tok0 = tile * p.tokens_per_tile;
   if (tok0 >= qlen) return;  // the whole CTA: nothing was set up yet
-  if (smem_u32(smem) & 1023) {  // the swizzled tiles need it; nothing else lies in front of them
+  if (sQ & 1023) {  // the swizzled tiles need it; nothing else lies in front of them
     if (tid == 0) atomicExch(p.error_flag, 21);
     return;
   }
@@ -1351,10 +1396,11 @@ __global__ void __launch_bounds__(THREADS, 1) paged_prefill_row_kernel(const __g
   const int hi = pos0 + ntok, lo = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
   const int t_begin = lo / KEYS, t_end = (hi + KEYS - 1) / KEYS, num_tiles = t_end - t_begin;
   const int vslabs = (p.dv + 63) >> 6;
+  const int unit_bits = 31 - __clz(min(p.page_size, HALF_KEYS)), unit = 1 << unit_bits, page_bits = 31 - __clz(p.page_size);  // tokens of a copy (powers of two)
 
   if (tid == 0) {
-    for (int i = 0; i < 6; ++i) mbar_init(k_full + 8 * i, 1);  // k_full, s_done, o_done
-    mbar_init(p_ready, SOFTMAX_THREADS);
+    for (int i = 0; i < 14; ++i) mbar_init(k_full + 8 * i, 1);  // k_full (8), s_done (2), o_done (4)
+    for (int i = 0; i < 3; ++i) mbar_init(p_ready + 8 * i, ROW_SOFTMAX_THREADS / 32);  // p_ready (2), q_full
     *failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1363,230 +1409,264 @@ __global__ void __launch_bounds__(THREADS, 1) paged_prefill_row_kernel(const __g
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  pdl_wait();  // queries and the cache are the work of the kernels before this one
-
-  // ---- Q, swizzled by hand (rows beyond the used ones and columns beyond the row are zero); both stages start as zeros: pages beyond the
-  //      sequence are never fetched, and their (masked) rows must not multiply garbage
-  for (int idx = tid; idx < ROWS * 8 * SLABS; idx += THREADS) {
-    const int rr = idx / (8 * SLABS), c = idx - rr * (8 * SLABS);
-    const int tok = rr / Gc, hd = rr - tok * Gc;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (rr < rows_used && hd < nheads && c * 8 < p.d)
-      v = *reinterpret_cast<const uint4*>(p.q + (size_t)(q0 + tok0 + tok) * p.q_stride + (size_t)(head0 + hd) * p.d + c * 8);
-    *reinterpret_cast<uint4*>(sQ + (c >> 3) * TILE_BYTES + rr * 128 + (((c & 7) ^ (rr & 7)) << 4)) = v;
-  }
-  for (int idx = tid; idx < 2 * Cfg::STAGE / 16; idx += THREADS) reinterpret_cast<uint4*>(sK)[idx] = make_uint4(0, 0, 0, 0);
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot, tmem_s = tmem, tmem_o = tmem + 2 * KEYS;
+  pdl_wait();  // queries and the cache are the work of the kernels before this one
 
-  if (warp == SOFTMAX_THREADS / 32 + 1) {
-    // ================================================================ the warp that copies: a page per lane, all its slabs
-    const int pages = KEYS / p.page_size, page_i = lane & 15;
-    auto lookup = [&](int t) -> int {
-      const int first = t * KEYS + page_i * p.page_size;
-      const bool need = lane < 16 && t < t_end && page_i < pages && first < hi && first + p.page_size > lo;
-      return need ? table[first / p.page_size] : -1;
+  if (warp == ROW_SOFTMAX_THREADS / 32 + 1) {
+    // ================================================================ the warp that copies: half a tile at a time, a page per lane
+    const int halves = 2 * num_tiles;
+    auto lookup = [&](int h) -> int {
+      const int first = t_begin * KEYS + h * HALF_KEYS + (lane << unit_bits);
+      const bool need = h < halves && (lane << unit_bits) < HALF_KEYS && first < hi && first + unit > lo;
+      return need ? table[first >> page_bits] : -1;
     };
-    int page = lookup(t_begin), asked = 0;  // tiles whose copies were asked for
-    for (int t = 0; t < num_tiles && !*failed; ++t) {
-      const int st = t & 1, cur = page;
-      page = lookup(t_begin + t + 1);
-      if (t >= 2) {
-        if (lane == 0) wait_or_fail(o_done + 8 * st, ((t - 2) >> 1) & 1, failed, 22, p.error_flag);  // P V(t - 2), the stage's last reader
+    int page = lookup(0), asked = 0, slot = 0;  // halves whose copies were asked for
+    for (int h = 0; h < halves && !*failed; ++h) {
+      const int cur = page;
+      page = lookup(h + 1);
+      const int before = h - HALVES;  // the half that lies in this slot; the last to read it is P V of its tile
+      if (before >= 0 && !(before & 1)) {
+        if (lane == 0) wait_or_fail(o_done + 8 * ((before >> 1) & 3), (before >> 3) & 1, failed, 22, p.error_flag);
         __syncwarp();
         if (*failed) break;
       }
+      const uint32_t full = k_full + 8 * slot;
       const int count = __popc(__ballot_sync(0xffffffffu, cur >= 0));
-      if (lane == 0) mbar_expect_tx(k_full + 8 * st, (uint32_t)(count * p.page_size * 128 * SLABS));
+      if (lane == 0) mbar_expect_tx(full, (uint32_t)(count * unit * 128 * SLABS));
       __syncwarp();
       if (cur >= 0) {
+        const int row = (cur * p.nkv + kvh) * p.page_size + (((h & 1) * HALF_KEYS + (lane << unit_bits)) & (p.page_size - 1));
 #pragma unroll
-        for (int sl = 0; sl < SLABS; ++sl)
-          tma_load_2d(smem_u32(sK + st * Cfg::STAGE + sl * TILE_BYTES + page_i * p.page_size * 128), &map, sl * 64, (cur * p.nkv + kvh) * p.page_size, k_full + 8 * st);
+        for (int sl = 0; sl < (WHOLE ? 1 : SLABS); ++sl) {
+          const uint32_t to = sK + slot * HALF + sl * NEXT_SLAB + (lane << unit_bits) * (PIECES / 8);
+          if (WHOLE)
+            asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %3, %3, %4}], [%2];"
+                         ::"r"(to), "l"(&map), "r"(full), "r"(0), "r"(row >> 3) : "memory");
+          else
+            tma_load_2d(to, &map, sl * 64, row, full);
+        }
       }
       ++asked;
+      if (++slot == HALVES) slot = 0;
     }
     if (*failed && lane == 0)
-      for (int t = max(0, asked - 2); t < asked; ++t) wait_for_last(k_full + 8 * (t & 1), (t >> 1) & 1);
-  } else if (warp == SOFTMAX_THREADS / 32) {
-    // ================================================================ the thread that issues the matrix products
-    if (lane == 0) {
-      const uint32_t idesc_s = instr_desc(ROWS, KEYS, 0), idesc_o = instr_desc(ROWS, vslabs * 64, 1);
-      const int k_steps = (p.d + 15) >> 4;
-      const uint64_t next_slab = (uint64_t)(TILE_BYTES >> 4) << 16;  // of the MN-major operand: bytes from 64 columns to the next 64
-      const uint32_t qa = smem_u32(sQ), pa = smem_u32(sP);
-      int s_next = 0, o_next = 0;
-      unsigned idle = 0;
-      while (o_next < num_tiles && !*failed) {
-        bool moved = false;
-        // O += P(t) V(t): the probabilities are written, the output rescaled where a row's maximum grew
-        if (o_next < s_next && barrier_phase_done(p_ready, o_next & 1)) {
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t v = smem_u32(sK + (o_next & 1) * Cfg::STAGE);
+      for (int h = max(0, asked - HALVES); h < asked; ++h) wait_for_last(k_full + 8 * (h % HALVES), (h / HALVES) & 1);
+  } else if (warp == ROW_SOFTMAX_THREADS / 32) {
+    // ================================================================ the warp that issues the matrix products (one lane of it, the warp together)
+    const uint32_t one = elect_one();
+    const uint32_t idesc_s = instr_desc(ROWS, KEYS, 0), idesc_half = instr_desc(ROWS, HALF_KEYS, 0), idesc_o = instr_desc(ROWS, vslabs * 64, 1);
+    const int k_steps = (p.d + 15) >> 4;
+    const uint64_t next_slab = (uint64_t)(NEXT_SLAB >> 4) << 16;  // of the MN-major operand: bytes from 64 columns to the next 64
+    auto rows_desc = [](uint32_t addr) { return (smem_desc_sw128(addr) & ~((uint64_t)0x3FFF << 32)) | (uint64_t)(PIECES >> 4) << 32; };
+    int s_next = 0, o_next = 0, s_slot = 0, s_phase = 0, o_slot = 0;  // the tiles' first halves lie in these slots
+    unsigned idle = 0;
+    if (!wait_or_fail(q_full, 0, failed, 25, p.error_flag)) *failed = 25;
+    __syncwarp();
+    while (o_next < num_tiles && !__any_sync(0xffffffffu, *failed != 0)) {
+      bool moved = false;
+      // O += P(t) V(t): the probabilities are written, the output rescaled where a row's maximum grew
+      if (o_next < s_next && __all_sync(0xffffffffu, barrier_phase_done(p_ready + 8 * (o_next & 1), (o_next >> 1) & 1))) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t pa = tmem_s + (o_next & 1) * KEYS;
+        uint32_t v = sK + o_slot * HALF;
 #pragma unroll
-          for (int k = 0; k < KEYS / 16; ++k)
-            umma(tmem_o, smem_desc_sw128(pa + (k >> 2) * TILE_BYTES + (k & 3) * 32), smem_desc_sw128(v + k * 2048) | next_slab, idesc_o, (o_next | k) != 0);
-          umma_commit(o_done + 8 * (o_next & 1));
-          ++o_next;
-          moved = true;
-        }
-        // S(t) = Q K(t)^T: the rows have arrived; the buffer held S(t - 2), which every thread had read when P(t - 2) was handed in
-        if (s_next < num_tiles && s_next <= o_next + 1 && barrier_phase_done(k_full + 8 * (s_next & 1), (s_next >> 1) & 1)) {
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t k = smem_u32(sK + (s_next & 1) * Cfg::STAGE);
+        for (int half = 0; half < 2; ++half) {
 #pragma unroll
-          for (int kk = 0; kk < SLABS * 4; ++kk)
-            if (kk < k_steps)
-              umma(tmem_s + (s_next & 1) * KEYS, smem_desc_sw128(qa + (kk >> 2) * TILE_BYTES + (kk & 3) * 32), smem_desc_sw128(k + (kk >> 2) * TILE_BYTES + (kk & 3) * 32), idesc_s, kk != 0);
-          umma_commit(s_done + 8 * (s_next & 1));
-          ++s_next;
-          moved = true;
+          for (int k = 0; k < HALF_KEYS / 16; ++k)  // sixteen keys: eight columns; a quarter's probabilities lie where its scores began
+            umma_tmem(one, tmem_o, pa + half * 64 + (k >> 1) * 32 + (k & 1) * 8, rows_desc(v + k * 2 * PIECES) | next_slab, idesc_o, (o_next | half | k) != 0);
+          o_slot = o_slot + 1 == HALVES ? 0 : o_slot + 1;
+          v = sK + o_slot * HALF;
         }
-        if (moved) {
-          idle = 0;
-        } else if (++idle > WAIT_LIMIT) {
-          *failed = 23;
-          atomicExch(p.error_flag, 23);
-        } else {
-          __nanosleep(20);
-        }
+        umma_commit_one(one, o_done + 8 * (o_next & 3));
+        ++o_next;
+        moved = true;
       }
-      if (o_next < num_tiles) {
-        for (int t = max(0, s_next - 2); t < s_next; ++t) wait_for_last(s_done + 8 * (t & 1), (t >> 1) & 1);
-        for (int t = max(0, o_next - 2); t < o_next; ++t) wait_for_last(o_done + 8 * (t & 1), (t >> 1) & 1);
+      // S(t) = Q K(t)^T: the rows have arrived; the buffer held S(t - 2) and P(t - 2), which O has taken
+      const int slot2 = s_slot + 1 == HALVES ? 0 : s_slot + 1, phase2 = slot2 ? s_phase : s_phase ^ 1;
+      if (s_next < num_tiles && (s_next < 2 || __all_sync(0xffffffffu, barrier_phase_done(o_done + 8 * ((s_next - 2) & 3), ((s_next - 2) >> 2) & 1)))
+          && __all_sync(0xffffffffu, barrier_phase_done(k_full + 8 * s_slot, s_phase) && barrier_phase_done(k_full + 8 * slot2, phase2))) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t k = sK + s_slot * HALF, k2 = sK + slot2 * HALF, to = tmem_s + (s_next & 1) * KEYS;
+        const bool joined = WHOLE && slot2 != 0;  // the pieces of both halves have the same distance
+#pragma unroll
+        for (int kk = 0; kk < SLABS * 4; ++kk)
+          if (kk < k_steps) {
+            const uint64_t q = smem_desc_sw128(sQ + (kk >> 2) * TILE_BYTES + (kk & 3) * 32);
+            const uint32_t at = (kk >> 2) * NEXT_SLAB + (kk & 3) * 32;
+            umma_one(one, to, q, rows_desc(k + at), joined ? idesc_s : idesc_half, kk != 0);
+            if (!joined) umma_one(one, to + HALF_KEYS, q, rows_desc(k2 + at), idesc_half, kk != 0);
+          }
+        umma_commit_one(one, s_done + 8 * (s_next & 1));
+        ++s_next;
+        s_slot = slot2 + 1 == HALVES ? 0 : slot2 + 1;
+        s_phase = s_slot ? phase2 : phase2 ^ 1;
+        moved = true;
       }
+      if (moved) {
+        idle = 0;
+      } else if (++idle > WAIT_LIMIT) {
+        *failed = 23;
+        if (lane == 0) atomicExch(p.error_flag, 23);
+      }
+    }
+    if (o_next < num_tiles) {
+      for (int t = max(0, s_next - 2); t < s_next; ++t) wait_for_last(s_done + 8 * (t & 1), (t >> 1) & 1);
+      for (int t = max(0, o_next - 4); t < o_next; ++t) wait_for_last(o_done + 8 * (t & 3), (t >> 2) & 1);
     }
     __syncwarp();
   } else {
-    // ================================================================ softmax threads: two a row, 64 keys and half of the value columns each
+    // ================================================================ softmax threads: four a row, 32 keys and a quarter of the value columns each
+    const int r = tid & (ROWS - 1), quarter = tid >> 7, rows_bar = 1 + (warp & 3);
+    // ---- Q, a row a warp, all of a thread's pieces under way at once (rows beyond the used ones and columns beyond the row are zeros)
+    {
+      const int by_heads = 65536 / Gc + 1;  // rr / Gc = rr * by_heads >> 16 for rr < 128, as rr / 65536 < 1 / Gc
+#pragma unroll
+      for (int i = 0; i < ROWS / (ROW_SOFTMAX_THREADS / 32); ++i) {
+        const int rr = i * (ROW_SOFTMAX_THREADS / 32) + warp, tok = rr * by_heads >> 16, hd = rr - tok * Gc;
+        const bool there = rr < rows_used && hd < nheads && lane * 8 < p.d;
+        const bf16* from = p.q + (there ? (size_t)(q0 + tok0 + tok) * p.q_stride + (size_t)(head0 + hd) * p.d + lane * 8 : 0);
+        if (lane < 8 * SLABS)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                       ::"r"(sQ + (lane >> 3) * TILE_BYTES + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4)), "l"(from), "r"(there ? 16 : 0) : "memory");
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(q_full);
+    }
     const int rtok = r / Gc;
     const bool rvalid = r < rows_used && (r - rtok * Gc) < nheads;
     const int rpos = pos0 + rtok;
     const uint32_t lane_bits = (uint32_t)((warp & 3) * 32) << 16;
-    const int col0 = half * 64, half_cols = vslabs * 32;
+    const int col0 = quarter * 32, my_cols = vslabs * 16;
     float m = -CUDART_INF_F, l = 0.f;
     bool ok = true;
-    const int group = r >> 6;
-    const uint32_t my_o = tmem_o + lane_bits + half * half_cols;
-    const uint32_t pchunk = smem_u32(sP) + half * TILE_BYTES + r * 128 + ((r & 7) << 4);  // chunk c: with c added to bits 4..6
+    const uint32_t my_o = tmem_o + lane_bits + quarter * my_cols;
+    const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2);
 
     for (int it = 0; it < num_tiles; ++it) {
       const int b = it & 1, base = (t_begin + it) * KEYS;
+      const uint32_t my_s = tmem_s + b * KEYS + lane_bits + col0;
       ok = wait_or_fail(s_done + 8 * b, (it >> 1) & 1, failed, 24, p.error_flag) && ok;
+      __syncwarp();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const bool full = base + KEYS - 1 <= pos0 && (p.window <= 0 || base >= hi - p.window);  // every row sees all of the tile
-      float sc[64];
-      {
-        uint32_t v0[32], v1[32];
-        tmem_ld32_nowait(tmem_s + b * KEYS + lane_bits + col0, v0);
-        tmem_ld32_nowait(tmem_s + b * KEYS + lane_bits + col0 + 32, v1);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      uint32_t packed[32];
+      tmem_ld32_nowait(my_s, packed);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      float sc[32];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) { sc[j] = __uint_as_float(v0[j]); sc[32 + j] = __uint_as_float(v1[j]); }
-      }
+      for (int j = 0; j < 32; ++j) sc[j] = __uint_as_float(packed[j]);
       if (!full) {
         const int first = base + col0;
         const int hi_j = rpos - first, lo_j = p.window > 0 ? rpos - p.window - first : -1;
 #pragma unroll
-        for (int j = 0; j < 64; ++j) sc[j] = (j <= hi_j && j > lo_j) ? sc[j] : -CUDART_INF_F;
+        for (int j = 0; j < 32; ++j) sc[j] = (j <= hi_j && j > lo_j) ? sc[j] : -CUDART_INF_F;
       }
-      float mx[8];
+      float mx[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) mx[j] = max3(sc[j], sc[j + 8], sc[j + 16]);
-#pragma unroll
-      for (int j = 24; j < 56; j += 16)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) mx[i] = max3(mx[i], sc[j + i], sc[j + 8 + i]);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) mx[i] = fmaxf(mx[i], sc[56 + i]);
-      float* rm = row_max + b * 2 * ROWS;  // by parity: a fast thread's next tile writes the other buffer
-      rm[half * ROWS + r] = max3(max3(mx[0], mx[1], mx[2]), max3(mx[3], mx[4], mx[5]), fmaxf(mx[6], mx[7]));
-      if (group == 0) asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_THREADS / 2) : "memory");  // the two halves of this row's 64-row group
-      else asm volatile("bar.sync 2, %0;" ::"n"(SOFTMAX_THREADS / 2) : "memory");
+      for (int i = 0; i < 4; ++i) mx[i] = max3(max3(sc[i], sc[i + 4], sc[i + 8]), max3(sc[i + 12], sc[i + 16], sc[i + 20]), fmaxf(sc[i + 24], sc[i + 28]));
+      asm volatile("bar.sync %0, 128;" ::"r"(rows_bar) : "memory");  // the four threads of each of these 32 rows: the last tile's maxima have been read
+      row_max[quarter * ROWS + r] = fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]);
+      asm volatile("bar.sync %0, 128;" ::"r"(rows_bar) : "memory");
       // probabilities are relative to the exact maximum so far: the largest one is then 1 and bfloat16 holds it as it is (following the maximum
-      // only when it has grown by 2^8 took 175 us instead of 185 for 4,096 tokens, but an error 2 to 23 % larger)
+      // only when it has grown by 2^8 gave an error 2 to 23 % larger)
       const float before = m;
-      m = max3(m, rm[r], rm[ROWS + r]);
+      m = max3(max3(m, row_max[r], row_max[ROWS + r]), row_max[2 * ROWS + r], row_max[3 * ROWS + r]);
       const bool grown = m > before;  // also the first finite maximum (before = -inf)
       const float corr = grown ? ex2((before - m) * p.scale_log2) : 1.f;
       const float neg = (m == -CUDART_INF_F) ? 0.f : -m * p.scale_log2;
+      const uint64_t neg2 = pack_f32x2(neg, neg);
+      uint64_t sum[2] = {0, 0};
+      uint32_t probs[16];
 #pragma unroll
-      for (int j = 0; j < 64; ++j) sc[j] = ex2(fmaf(sc[j], p.scale_log2, neg));  // masked: ex2(-inf) = 0
-      // P and O are free once the product of the tile before has finished
-      if (it > 0) {
-        ok = wait_or_fail(o_done + 8 * (b ^ 1), ((it - 1) >> 1) & 1, failed, 22, p.error_flag) && ok;
+      for (int j = 0; j < 16; ++j) {
+        float x0, x1;
+        unpack_f32x2(fma_f32x2(pack_f32x2(sc[2 * j], sc[2 * j + 1]), scale2, neg2), x0, x1);  // masked: ex2(-inf) = 0
+        __nv_bfloat162 b2 = __floats2bfloat162_rn(ex2(x0), ex2(x1));
+        probs[j] = *reinterpret_cast<uint32_t*>(&b2);
+        sum[j & 1] = add_f32x2(sum[j & 1], pack_f32x2(__uint_as_float(probs[j] << 16), __uint_as_float(probs[j] & 0xffff0000u)));  // of the rounded numbers, the weights the values get
+      }
+      tmem_st16(my_s, probs);  // over this thread's own scores
+      float sum0, sum1;
+      unpack_f32x2(add_f32x2(sum[0], sum[1]), sum0, sum1);
+      l = l * corr + (sum0 + sum1);
+      // O is free once the product of the tile before has finished
+      if (it > 0 && __any_sync(0xffffffffu, grown)) {
+        ok = wait_or_fail(o_done + 8 * ((it - 1) & 3), ((it - 1) >> 2) & 1, failed, 22, p.error_flag) && ok;
         ok = __all_sync(0xffffffffu, ok);
-        if (__any_sync(0xffffffffu, grown)) {
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          if (ok) {
-            for (int c = 0; c < half_cols; c += 32) {
-              uint32_t v[32];
-              tmem_ld32_nowait(my_o + c, v);
-              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (ok) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * corr);
-              tmem_st32(my_o + c, v);
-            }
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          for (int half = 0; half < 2; ++half) {
+            uint32_t v[2][16];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+              if (2 * half + i < vslabs) tmem_ld16(my_o + 32 * half + 16 * i, v[i]);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+              if (2 * half + i < vslabs) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[i][j] = __float_as_uint(__uint_as_float(v[i][j]) * corr);
+                tmem_st16(my_o + 32 * half + 16 * i, v[i]);
+              }
           }
         }
       }
-      float sum[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int j = 0; j < 64; j += 8) {
-        uint32_t packed[4];
-#pragma unroll
-        for (int e = 0; e < 8; e += 2) {
-          __nv_bfloat162 b2 = __floats2bfloat162_rn(sc[j + e], sc[j + e + 1]);
-          packed[e >> 1] = *reinterpret_cast<uint32_t*>(&b2);
-          sum[(e >> 1) & 3] += __uint_as_float(packed[e >> 1] << 16) + __uint_as_float(packed[e >> 1] & 0xffff0000u);  // of the rounded numbers, the weights the values get
+      // rows that were not fetched, and those of the last page that hold no token: S has been taken, as values they must not multiply garbage
+      const int from = max(((lo >> unit_bits) << unit_bits) - base, 0), to = min(min(((hi + unit - 1) >> unit_bits) << unit_bits, kvlen) - base, KEYS);
+      if (from > 0 || to < KEYS) {
+        const int empty = from + KEYS - to;
+        for (int i = tid; i < empty * 32; i += ROW_SOFTMAX_THREADS) {
+          const int row = (i >> 5) < from ? i >> 5 : (i >> 5) - from + to, c = lane;
+          const int slot = (2 * it + (row >> 6)) % HALVES, at = slot * HALF + (c >> 3) * NEXT_SLAB + ((row >> 3) & 7) * PIECES + (row & 7) * 128 + ((c & 7) << 4);
+          if (c < 8 * vslabs) *reinterpret_cast<uint4*>(smem + Cfg::Q + at) = make_uint4(0, 0, 0, 0);
         }
-        st_shared_v4(pchunk ^ ((j >> 3) << 4), packed[0], packed[1], packed[2], packed[3]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       }
-      l = l * corr + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
-      if (base + KEYS > kvlen) {  // rows of the last page that hold no token: S has been taken, as values they must not multiply garbage
-        const int from = max(kvlen - base, 0);
-        for (int i = tid; i < (KEYS - from) * 8 * vslabs; i += SOFTMAX_THREADS) {
-          const int row = from + i / (8 * vslabs), c = i % (8 * vslabs);
-          *reinterpret_cast<uint4*>(sK + b * Cfg::STAGE + (c >> 3) * TILE_BYTES + row * 128 + ((c & 7) << 4)) = make_uint4(0, 0, 0, 0);
-        }
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // P is read by the tensor cores
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      mbar_arrive(p_ready);  // P is written, the output rescaled and S read
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_ready + 8 * b);  // P is written, the output rescaled and S read
     }
-    // ---- the finished output, once the last product is done; the row sum is the two halves' sums
-    ok = wait_or_fail(o_done + 8 * ((num_tiles - 1) & 1), ((num_tiles - 1) >> 1) & 1, failed, 22, p.error_flag) && ok;
+    // ---- the finished output, once the last product is done; the row sum is the four quarters' sums
+    ok = wait_or_fail(o_done + 8 * ((num_tiles - 1) & 3), ((num_tiles - 1) >> 2) & 1, failed, 22, p.error_flag) && ok;
     ok = __all_sync(0xffffffffu, ok);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    float* rl = row_max + (num_tiles & 1) * 2 * ROWS;  // not the buffer of the last tile's maxima
-    rl[half * ROWS + r] = l;
-    if (group == 0) asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_THREADS / 2) : "memory");
-    else asm volatile("bar.sync 2, %0;" ::"n"(SOFTMAX_THREADS / 2) : "memory");
+    asm volatile("bar.sync %0, 128;" ::"r"(rows_bar) : "memory");
+    row_max[quarter * ROWS + r] = l;
+    asm volatile("bar.sync %0, 128;" ::"r"(rows_bar) : "memory");
     const int head = head0 + (r - rtok * Gc);
-    const float inv = 1.f / (rl[r] + rl[ROWS + r] + sink_term(rvalid ? sink_of(p.sink_heads, p.sink_log2, head) : -CUDART_INF_F, m * p.scale_log2));
-    const size_t row = (size_t)(q0 + tok0 + rtok) * p.nh + head;
-    for (int c = 0; c < half_cols; c += 32) {
-      uint32_t v[32];
+    const float total = (row_max[r] + row_max[ROWS + r]) + (row_max[2 * ROWS + r] + row_max[3 * ROWS + r]);
+    const float inv = 1.f / (total + sink_term(rvalid ? sink_of(p.sink_heads, p.sink_log2, head) : -CUDART_INF_F, m * p.scale_log2));
+    const bool store = ok && !*failed && rvalid;
+    bf16* out = p.out + (store ? ((size_t)(q0 + tok0 + rtok) * p.nh + head) * p.out_row + quarter * my_cols : 0);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      uint32_t v[2][16];
       if (ok) {
-        tmem_ld32_nowait(my_o + c, v);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          if (2 * half + i < vslabs) tmem_ld16(my_o + 32 * half + 16 * i, v[i]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       }
-      if (ok && !*failed && rvalid) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 8) {
-          const int col = half * half_cols + c + j;
-          if (col >= p.dv) break;
-          uint4 w;
-          __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&w);
+      for (int i = 0; i < 2; ++i)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) h2[e] = __floats2bfloat162_rn(__uint_as_float(v[j + 2 * e]) * inv, __uint_as_float(v[j + 2 * e + 1]) * inv);
-          *reinterpret_cast<uint4*>(p.out + row * p.out_row + col) = w;
+        for (int j = 0; j < 16; j += 8) {
+          const int col = 32 * half + 16 * i + j;
+          if (store && 2 * half + i < vslabs && quarter * my_cols + col < p.dv) {
+            uint4 w;
+            __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&w);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) h2[e] = __floats2bfloat162_rn(__uint_as_float(v[i][j + 2 * e]) * inv, __uint_as_float(v[i][j + 2 * e + 1]) * inv);
+            *reinterpret_cast<uint4*>(out + col) = w;
+          }
         }
-      }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1594,17 +1674,17 @@ __global__ void __launch_bounds__(THREADS, 1) paged_prefill_row_kernel(const __g
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
 }
 
-template <int SLABS> int launch_rows(const CUtensorMap& map, const RowParams& p, int num_seqs, int max_q_len, cudaStream_t stream) {
+template <int SLABS, bool WHOLE> int launch_rows(const CUtensorMap& map, const RowParams& p, int num_seqs, int max_q_len, cudaStream_t stream) {
   using Cfg = RowCfg<SLABS>;
   static OncePerDevice configured;
   if (!configured.here()) {
-    cudaError_t e = cudaFuncSetAttribute(paged_prefill_row_kernel<SLABS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(paged_prefill_row_kernel<SLABS, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
     if (e != cudaSuccess) return (int)e;
     configured.here() = true;
   }
   const int tiles = (max_q_len + p.tokens_per_tile - 1) / p.tokens_per_tile;
   if (tiles > 65535 || num_seqs > 65535) return DLI_ERR_UNSUPPORTED;  // the grid's y and z
-  return (int)launch_pdl((paged_prefill_row_kernel<SLABS>), dim3(p.nkv * p.head_chunks, num_seqs, tiles), dim3(THREADS), (size_t)Cfg::SMEM, stream, 1, map, p);
+  return (int)launch_pdl((paged_prefill_row_kernel<SLABS, WHOLE>), dim3(p.nkv * p.head_chunks, num_seqs, tiles), dim3(ROW_THREADS), (size_t)Cfg::SMEM, stream, 1, map, p);
 }
 #endif
 
@@ -1721,7 +1801,9 @@ DLI_EXPORT int dli_paged_prefill_rows(void* out, const void* q, long long q_stri
     if (cudaHostGetDevicePointer((void**)&error_flag_device, error_flag_host, 0) != cudaSuccess) return (int)cudaGetLastError();
   }
   CUtensorMap map;
-  if (!make_pool_map(&map, pool, num_pages * nkv * page_size, page_size, head_dim)) return DLI_ERR_UNSUPPORTED;
+  const bool whole = head_dim % 64 == 0;  // (elsewhere the last slab's rows would end in the next row, and behind the pool)
+  const long long rows = num_pages * nkv * page_size;
+  if (!(whole ? make_row_map(&map, pool, rows, page_size, head_dim) : make_pool_map(&map, pool, rows, page_size < HALF_KEYS ? page_size : HALF_KEYS, head_dim))) return DLI_ERR_UNSUPPORTED;
   RowParams p;
   p.out = (bf16*)out; p.q = (const bf16*)q; p.q_stride = q_stride; p.block_tables = block_tables; p.max_blocks = max_blocks; p.q_start = q_start;
   p.kv_len = kv_len; p.seq0 = seq0; p.nh = nh; p.nkv = nkv; p.page_size = page_size; p.window = window;
@@ -1734,7 +1816,8 @@ DLI_EXPORT int dli_paged_prefill_rows(void* out, const void* q, long long q_stri
   p.tokens_per_tile = ROWS / p.heads_per_chunk;
   p.d = head_dim; p.dv = value_dim; p.out_row = head_dim;
   p.error_flag = error_flag_device;
-  return head_dim <= 192 ? launch_rows<3>(map, p, num_seqs, max_q_len, stream) : launch_rows<4>(map, p, num_seqs, max_q_len, stream);
+  if (whole) return head_dim == 192 ? launch_rows<3, true>(map, p, num_seqs, max_q_len, stream) : launch_rows<4, true>(map, p, num_seqs, max_q_len, stream);
+  return head_dim <= 192 ? launch_rows<3, false>(map, p, num_seqs, max_q_len, stream) : launch_rows<4, false>(map, p, num_seqs, max_q_len, stream);
 }
 #endif
 

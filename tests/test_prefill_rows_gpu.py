@@ -131,3 +131,27 @@ def test_which_rows_have_the_kernel():
     assert ok(256, 16) and ok(136, 8) and ok(192, 128)
     assert not ok(128, 16) and not ok(264, 16) and not ok(140, 16) and not ok(256, 4) and not ok(256, 48)
     assert attention._slab_kernels(64, True) and not attention._slab_kernels(256, True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("page", [8, 16, 64])
+@pytest.mark.parametrize("lens,heads,nkv,row,dv,window", [
+    ([(300, 77), (1, 130)], 16, 1, 192, 128, None), ([(9, 118), (7, 121), (260, 0)], 16, 2, 256, 192, None), ([(140, 260)], 16, 1, 192, 192, 20), ([(64, 191)], 20, 1, 256, 8, 133)])
+def test_pages_that_come_whole(lens, heads, nkv, row, dv, page, window):
+    """Rows of whole slabs come as one box a page, whatever its size; the same numbers as with pages of 128."""
+    outs = []
+    for size in (page, 128):
+        pool, tables, rows, q, start, kv_len = _case(lens, heads, nkv, row, size)
+        g = torch.Generator().manual_seed(11)
+        values = [torch.randn(*r.shape, generator=g).to(torch.bfloat16) for r in rows]
+        for s, value in enumerate(values):  # [tokens, nkv, row], the same tokens in either paging
+            for t in range(value.shape[0]):
+                pool[tables[s, t // size], :, t % size] = value[t].to(pool.dtype)
+        out = torch.zeros((q.shape[0], heads * row), dtype=torch.bfloat16, device="cuda")
+        q = torch.randn(*q.shape, generator=torch.Generator().manual_seed(12)).to(torch.bfloat16)
+        ops.paged_prefill_rows(out, q.cuda(), pool.cuda(), tables.cuda(), start.cuda(), kv_len.cuda(), 0, len(lens), max(c for c, _ in lens), heads, row**-0.5, window, value_dim=dv)
+        outs.append(out.view(-1, heads, row)[..., :dv].cpu())
+    want = _exact(lens, values, q, start, heads, nkv, row, dv, row**-0.5, window, None)
+    for got in outs:  # probabilities and outputs are rounded to bfloat16 (2^-9 each) on the way, the products' sums are float32
+        assert (got.double() - want).norm() <= 6e-3 * want.norm() and (got.double() - want).abs().max() <= 3e-2 * max(1.0, want.abs().max())
+    assert ops.device_wait_errors() == {}
