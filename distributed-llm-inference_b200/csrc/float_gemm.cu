@@ -119,7 +119,6 @@ __device__ __forceinline__ bool finite(float v) { return fabsf(v) <= 3.402823466
 template <int NT>
 __global__ void __launch_bounds__(THREADS, 1) float_gemm_kernel(const __grid_constant__ FloatParams p) {
   using Z = Shape<NT>;
-  pdl_launch_dependents();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Z::STAGES * Z::STAGE);  // full[STAGES], empty[STAGES], sum_full[LARGE], sum_empty[LARGE]
@@ -332,6 +331,9 @@ __global__ void __launch_bounds__(THREADS, 1) float_gemm_kernel(const __grid_con
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // nobody leaves while its sums are read
   }
+  // Not before: a CTA has an SM's shared memory, and what is launched meanwhile, such as the attention behind the rotary embedding, which only waits, would all
+  // lie on the SMs that have none (81 tokens with 16 heads: the attention 58 us, 122 with the kernels behind this one launched at its start).
+  pdl_launch_dependents();
   if (warp == CONVERTERS / 32) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Z::COLUMNS) : "memory");
