@@ -139,6 +139,14 @@ __device__ __forceinline__ void bend_row(float (&sc)[N], const ScoreBend& b, flo
   }
 }
 #endif
+// Queries go to shared memory without waiting for one another: with a load and a store at a time the prologue of a CTA of 128 rows of 256 numbers took
+// 16,000 clocks.  bytes 0: zeros
+__device__ __forceinline__ void query_piece(uint32_t to, const void* from, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void query_pieces_there() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// row / heads = row * heads_inverse(heads) >> 16 for rows below 128: what is too much is row / 65536 < 1 / heads
+__device__ __forceinline__ int heads_inverse(int heads) { return 65536 / heads + 1; }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -240,15 +248,15 @@ __global__ void __launch_bounds__(THREADS, 1) paged_prefill_tc_kernel(const __gr
   // ---- Q tile, swizzled by hand: 16-byte chunk c of row r lies at r * 128 + ((c ^ (r & 7)) * 16);
   //      rows beyond the used ones are zero.  Both value stages start as zeros: pages beyond the
   //      sequence are never fetched, and their (masked) columns must not multiply garbage.
+  const int by_heads = heads_inverse(Gc);
   for (int idx = tid; idx < ROWS * 8; idx += THREADS) {
     const int rr = idx >> 3, c = idx & 7;
-    const int tok = rr / Gc, hd = rr - tok * Gc;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (rr < rows_used && hd < nheads)
-      v = *reinterpret_cast<const uint4*>(p.q + (size_t)(q0 + tok0 + tok) * p.q_stride + (size_t)(head0 + hd) * D + c * 8);
-    *reinterpret_cast<uint4*>(sQ + rr * 128 + ((c ^ (rr & 7)) << 4)) = v;
+    const int tok = rr * by_heads >> 16, hd = rr - tok * Gc;
+    const bool there = rr < rows_used && hd < nheads;
+    query_piece(smem_u32(sQ + rr * 128 + ((c ^ (rr & 7)) << 4)), p.q + (there ? (size_t)(q0 + tok0 + tok) * p.q_stride + (size_t)(head0 + hd) * D + c * 8 : 0), there ? 16 : 0);
   }
   for (int idx = tid; idx < 2 * TILE_BYTES / 16; idx += THREADS) reinterpret_cast<uint4*>(sV)[idx] = make_uint4(0, 0, 0, 0);
+  query_pieces_there();
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -601,15 +609,16 @@ __global__ void __launch_bounds__(T2Cfg<HD, HV>::THREADS, 1) paged_prefill_tc2_k
   pdl_wait();  // queries and the cache are the work of the kernels before this one
 
   // ---- both Q tiles, swizzled by hand (rows beyond the used ones are zero); the value stages start as zeros
+  const int by_heads = heads_inverse(Gc);
   for (int idx = tid; idx < QT * ROWS * (D / 8); idx += T2_THREADS) {
     const int rr = idx / (D / 8), c = idx - rr * (D / 8);  // rr: row among those of all tiles; c: 16-byte chunk of the row
-    const int rt = rr & (ROWS - 1), tok = (rr >> 7) * tpt + rt / Gc, hd = rt % Gc;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (rt / Gc < tpt && tok < ntok && hd < nheads && c * 8 < p.d)
-      v = *reinterpret_cast<const uint4*>(p.q + (size_t)(q0 + tok0 + tok) * p.q_stride + (size_t)(head0 + hd) * p.d + c * 8);
-    *reinterpret_cast<uint4*>(sQ + (rr >> 7) * K_BYTES + (c >> 3) * TILE_BYTES + rt * 128 + (((c & 7) ^ (rt & 7)) << 4)) = v;
+    const int rt = rr & (ROWS - 1), nth = rt * by_heads >> 16, tok = (rr >> 7) * tpt + nth, hd = rt - nth * Gc;
+    const bool there = nth < tpt && tok < ntok && hd < nheads && c * 8 < p.d;
+    query_piece(smem_u32(sQ + (rr >> 7) * K_BYTES + (c >> 3) * TILE_BYTES + rt * 128 + (((c & 7) ^ (rt & 7)) << 4)),
+                p.q + (there ? (size_t)(q0 + tok0 + tok) * p.q_stride + (size_t)(head0 + hd) * p.d + c * 8 : 0), there ? 16 : 0);
   }
   for (int idx = tid; idx < 2 * V_BYTES / 16; idx += T2_THREADS) reinterpret_cast<uint4*>(sV)[idx] = make_uint4(0, 0, 0, 0);
+  query_pieces_there();
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -950,15 +959,16 @@ __global__ void __launch_bounds__(DIFF_THREADS, 1) paged_prefill_diff_kernel(con
   pdl_wait();  // queries and the cache are the work of the kernels before this one
 
   // ---- both Q tiles, swizzled by hand (rows beyond the used ones are zero); the value stages start as zeros
+  const int by_heads = heads_inverse(Gc);
   for (int idx = tid; idx < QT * ROWS * (D / 8); idx += DIFF_THREADS) {
     const int rr = idx / (D / 8), c = idx - rr * (D / 8);  // rr: row among those of all tiles; c: 16-byte chunk of the row
-    const int rt = rr & (ROWS - 1), tok = rt / Gc, hd = rt % Gc;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (tok < ntok && hd < nheads)
-      v = *reinterpret_cast<const uint4*>(p.q + (size_t)(q0 + tok0 + tok) * p.q_stride + (size_t)(head0 + hd) * 2 * D + (rr >> 7) * D + c * 8);
-    *reinterpret_cast<uint4*>(sQ + (rr >> 7) * TILE_BYTES + rt * 128 + ((c ^ (rt & 7)) << 4)) = v;
+    const int rt = rr & (ROWS - 1), tok = rt * by_heads >> 16, hd = rt - tok * Gc;
+    const bool there = tok < ntok && hd < nheads;
+    query_piece(smem_u32(sQ + (rr >> 7) * TILE_BYTES + rt * 128 + ((c ^ (rt & 7)) << 4)),
+                p.q + (there ? (size_t)(q0 + tok0 + tok) * p.q_stride + (size_t)(head0 + hd) * 2 * D + (rr >> 7) * D + c * 8 : 0), there ? 16 : 0);
   }
   for (int idx = tid; idx < 2 * V_BYTES / 16; idx += DIFF_THREADS) reinterpret_cast<uint4*>(sV)[idx] = make_uint4(0, 0, 0, 0);
+  query_pieces_there();
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -1522,17 +1532,16 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
     const int r = tid & (ROWS - 1), quarter = tid >> 7, rows_bar = 1 + (warp & 3);
     // ---- Q, a row a warp, all of a thread's pieces under way at once (rows beyond the used ones and columns beyond the row are zeros)
     {
-      const int by_heads = 65536 / Gc + 1;  // rr / Gc = rr * by_heads >> 16 for rr < 128, as rr / 65536 < 1 / Gc
+      const int by_heads = heads_inverse(Gc);
 #pragma unroll
       for (int i = 0; i < ROWS / (ROW_SOFTMAX_THREADS / 32); ++i) {
         const int rr = i * (ROW_SOFTMAX_THREADS / 32) + warp, tok = rr * by_heads >> 16, hd = rr - tok * Gc;
         const bool there = rr < rows_used && hd < nheads && lane * 8 < p.d;
         const bf16* from = p.q + (there ? (size_t)(q0 + tok0 + tok) * p.q_stride + (size_t)(head0 + hd) * p.d + lane * 8 : 0);
         if (lane < 8 * SLABS)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
-                       ::"r"(sQ + (lane >> 3) * TILE_BYTES + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4)), "l"(from), "r"(there ? 16 : 0) : "memory");
+          query_piece(sQ + (lane >> 3) * TILE_BYTES + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4), from, there ? 16 : 0);
       }
-      asm volatile("cp.async.wait_all;" ::: "memory");
+      query_pieces_there();
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(q_full);
