@@ -896,6 +896,7 @@ struct DiffParams {
   int tokens_per_tile, heads_per_chunk, head_chunks;
   int dv;
   int* error_flag;
+  int tiles, singles;  // tiles of the longest portion; single tokens beside the portions: the sequences in front of seq0
 };
 
 constexpr int DIFF_THREADS = 2 * ROWS + 128;
@@ -922,8 +923,13 @@ __global__ void __launch_bounds__(DIFF_THREADS, 1) paged_prefill_diff_kernel(con
                  s_done = smem_u32(bars + 8), s_read = smem_u32(bars + 10), p_ready = smem_u32(bars + 12), o_done = smem_u32(bars + 14);
 
   // the tiles that see the most keys start first
-  const int s = p.seq0 + blockIdx.y;
-  const int tile = gridDim.z - 1 - blockIdx.z;
+  // (the single tokens come last, as many a layer of the grid as there are portions: where the portions' last wave leaves SMs idle they cost no time of
+  // their own)
+  const int nth = ((int)blockIdx.z - p.tiles) * (int)gridDim.y + (int)blockIdx.y;
+  const bool single = (int)blockIdx.z >= p.tiles;
+  if (single && nth >= p.singles) return;
+  const int s = single ? p.seq0 - p.singles + nth : p.seq0 + (int)blockIdx.y;
+  const int tile = single ? 0 : p.tiles - 1 - (int)blockIdx.z;
   const int kvh = blockIdx.x / p.head_chunks, hc = blockIdx.x - kvh * p.head_chunks;
   const int q0 = p.q_start[s];
   const int qlen = p.q_start[s + 1] - q0;
@@ -1756,10 +1762,11 @@ DLI_EXPORT int dli_paged_prefill_tc(void* out, const void* q, long long q_stride
 #if !BENT_SCORES
 // Differential attention of sequences [seq0, seq0 + num_seqs): k_pool [pages, nkv, page_size, 128] (two maps of 64), v_pool [.., value_dim].
 DLI_EXPORT int dli_paged_prefill_diff(void* out, const void* q, long long q_stride, const void* k_pool, const void* v_pool, long long num_pages,
-                                      const int* block_tables, int max_blocks, const int* q_start, const int* kv_len, int seq0, int num_seqs,
+                                      const int* block_tables, int max_blocks, const int* q_start, const int* kv_len, int seq0, int num_seqs, int singles,
                                       int max_q_len, const void* gate, int gate_stride, int nh, int nkv, int value_dim, int page_size, int window,
                                       int keep_first, float scale, float lambda, float post, float eps, cudaStream_t stream) {
   if (num_seqs == 0) return 0;
+  if (singles < 0 || singles > seq0) return DLI_ERR_UNSUPPORTED;
   if (value_dim < 8 || value_dim > 128 || value_dim % 8 || nkv < 1 || nh % nkv || page_size < 8 || page_size > 128 || (KEYS % page_size) != 0) return DLI_ERR_UNSUPPORTED;
   if ((((uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)q | (uintptr_t)out) & 15) || q_stride % 8) return DLI_ERR_UNSUPPORTED;
   if (!error_flag_host) {
@@ -1788,8 +1795,10 @@ DLI_EXPORT int dli_paged_prefill_diff(void* out, const void* q, long long q_stri
   p.dv = value_dim;
   p.error_flag = error_flag_device;
   const int tiles = (max_q_len + p.tokens_per_tile - 1) / p.tokens_per_tile;
-  if (tiles > 65535 || num_seqs > 65535) return DLI_ERR_UNSUPPORTED;  // the grid's y and z
-  return (int)launch_pdl(paged_prefill_diff_kernel, dim3(nkv * p.head_chunks, num_seqs, tiles), dim3(DIFF_THREADS), (size_t)DIFF_SMEM, stream, 1, map_k, map_v, p);
+  const int layers = tiles + (singles + num_seqs - 1) / num_seqs;
+  if (layers > 65535 || num_seqs > 65535) return DLI_ERR_UNSUPPORTED;  // the grid's y and z
+  p.tiles = tiles; p.singles = singles;
+  return (int)launch_pdl(paged_prefill_diff_kernel, dim3(nkv * p.head_chunks, num_seqs, layers), dim3(DIFF_THREADS), (size_t)DIFF_SMEM, stream, 1, map_k, map_v, p);
 }
 #endif
 

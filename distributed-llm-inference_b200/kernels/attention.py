@@ -176,6 +176,30 @@ def diff_portions_apart(batch, tokens: int, num_heads: int, nkv: int, window: in
     return two <= 0.85 * one
 
 
+def diff_singles_beside(batch, num_heads: int, nkv: int, window: int | None, keep_first: int) -> bool:
+    """Whether the single tokens of a step go to the launch of its portions (``ops.paged_prefill_diff``), whose last CTAs they are, or to their own.
+
+    Where the portions' last wave of CTAs leaves places for all of them they start when the last portion CTAs have started, and what they see beyond those takes the
+    launch longer, 17 us for 1,000 keys.  A launch of their own and the merge of its partial results behind it take 11 us and 5 to 20 for 1,000 keys.  Measured, us: 9 tokens at
+    1,500 keys (a window of 1,024) beside 1,535 behind 1,024, 16 heads on 4: 93 apart, 78 beside.  A recorded step (its portions have no lengths yet) keeps them apart."""
+    singles, lens, starts = batch.num_single, getattr(batch, "q_lens", [])[batch.num_single :], getattr(batch, "starts", [])[batch.num_single :]
+    if not lens or min(lens) < 1 or len(starts) != len(lens):
+        return False
+
+    def seen(keys: int) -> float:  # thousands of keys that a query reads
+        return (min(keys, window + keep_first + 64) if window else keys) / 1000
+
+    group, sms = num_heads // nkv, sm_count()
+    heads = min(group, 128)  # of a CTA's rows
+    wide = nkv * -(-group // heads)
+    ctas = wide * sum(-(-q // (128 // heads)) for q in lens)
+    if wide * singles > -ctas % sms:
+        return False
+    last = seen(_portion_keys(batch)) if ctas <= sms else seen(min(starts))
+    alone = seen(batch.max_kv_len_single)
+    return 17 * (alone - last) <= 0.6 * (11 + alone * 20 * max(0.26, singles * nkv / sms))
+
+
 def diff_attention(out: torch.Tensor, q: torch.Tensor, cache, batch, gate: torch.Tensor | None, num_heads: int, scale: float,
                    window: int | None, keep_first: int, lam: float, post: float, eps: float) -> None:
     """Differential attention of every token of the step over its sequence's pages (``ops.diff_attention_simt`` says what is
@@ -187,9 +211,10 @@ def diff_attention(out: torch.Tensor, q: torch.Tensor, cache, batch, gate: torch
         vdim, singles, seqs, longest, seen = cache.v.shape[3], batch.num_single, batch.num_seqs, batch.max_q_len, batch.max_kv_len
         if (seqs > singles and ops.prefill_diff_supported(d2 // 2, vdim, cache.page_size) and diff_portions_apart(batch, q.shape[0], num_heads, nkv, window, keep_first)
                 and (out.data_ptr() | q.data_ptr() | cache.k.data_ptr() | cache.v.data_ptr()) % 16 == 0):
+            beside = singles if singles and diff_singles_beside(batch, num_heads, nkv, window, keep_first) else 0
             ops.paged_prefill_diff(out, q, cache.k, cache.v, group.block_tables, batch.q_start, batch.kv_len, singles, seqs - singles, longest, gate, num_heads,
-                                   scale, window, keep_first, lam, post, eps)
-            if not singles:
+                                   scale, window, keep_first, lam, post, eps, beside)
+            if beside == singles:
                 return
             seqs, longest, seen = singles, 1, batch.max_kv_len_single
         splits, scratch = 1, None

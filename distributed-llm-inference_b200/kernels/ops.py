@@ -1750,8 +1750,9 @@ def prefill_diff_supported(dim: int, vdim: int, page_size: int) -> bool:
 
 def paged_prefill_diff(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, block_tables: torch.Tensor, q_start: torch.Tensor,
                        kv_len: torch.Tensor, seq0: int, num_seqs: int, max_q_len: int, gate: torch.Tensor | None, num_heads: int, scale: float,
-                       window: int | None, keep_first: int, lam: float, post: float, eps: float) -> None:
-    """``diff_attention_tc`` for the prompt portions of sequences seq0 .. seq0 + num_seqs - 1, on tcgen05 tensor cores (maps of 64, values of up to 128)."""
+                       window: int | None, keep_first: int, lam: float, post: float, eps: float, singles: int = 0) -> None:
+    """``diff_attention_tc`` for the prompt portions of sequences seq0 .. seq0 + num_seqs - 1, on tcgen05 tensor cores (maps of 64, values of up to 128), and
+    for the ``singles`` single tokens of the sequences in front of them."""
     for t, name in ((out, "out"), (q, "q"), (k_pool, "k_pool"), (v_pool, "v_pool")):
         _need(t, name, torch.bfloat16)
     _need(block_tables, "block_tables", torch.int32), _need(q_start, "q_start", torch.int32), _need(kv_len, "kv_len", torch.int32)
@@ -1763,12 +1764,12 @@ def paged_prefill_diff(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor,
         raise KernelError("paged_prefill_diff: shapes do not agree or sizes not supported")
     if gate is not None and (gate.dtype != out.dtype or gate.shape != (n, num_heads) or gate.stride(1) != 1 or not gate.is_cuda):
         raise KernelError("paged_prefill_diff: gate must be [n, heads] with unit column stride")
-    if seq0 + num_seqs > kv_len.numel() or q_start.numel() != kv_len.numel() + 1:
+    if seq0 + num_seqs > kv_len.numel() or q_start.numel() != kv_len.numel() + 1 or not 0 <= singles <= seq0:
         raise KernelError("paged_prefill_diff: sequence range outside the batch")
     f = _fn("attention_tc.cu", "dli_paged_prefill_diff", [c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p]
-            + [c_int] * 3 + [c_void_p] + [c_int] * 7 + [c_float] * 4 + [c_void_p])
+            + [c_int] * 4 + [c_void_p] + [c_int] * 7 + [c_float] * 4 + [c_void_p])
     _check(f(_ptr(out), _ptr(q), q.shape[1], _ptr(k_pool), _ptr(v_pool), pages, _ptr(block_tables), block_tables.shape[1], _ptr(q_start), _ptr(kv_len), seq0,
-             num_seqs, int(max_q_len), _ptr(gate), 0 if gate is None else gate.stride(0), num_heads, nkv, vdim, page_size, int(window or 0), int(keep_first),
+             num_seqs, int(singles), int(max_q_len), _ptr(gate), 0 if gate is None else gate.stride(0), num_heads, nkv, vdim, page_size, int(window or 0), int(keep_first),
              float(scale), float(lam), float(post), float(eps), _stream()), "paged_prefill_diff")
 
 

@@ -49,3 +49,15 @@ def test_single_tokens_beside_a_scan(heads, singles, portions, apart):
     batch = types.SimpleNamespace(num_single=singles, num_seqs=singles + len(portions), n=singles + sum(portions), max_q_len=max(portions, default=1))
     assert ssm.scan_singles_apart(batch, 64, 128, heads, torch.bfloat16) == apart
     assert ssm.scan_singles_apart(batch, 64, 128, heads, torch.float32) == 0
+
+
+@pytest.mark.parametrize("portions,singles,context,window,beside", [
+    ([(1535, 1024)], 9, 1500, 1024, True), ([(1535, 1024)], 9, 1500, None, True), ([(1535, 0)], 9, 1500, None, False), ([(1535, 0)], 9, 300, None, True),
+    ([(1024, 0)], 4, 900, None, True), ([(1024, 0)], 4, 3000, None, False), ([(1535, 1024)], 64, 1500, 1024, False), ([(0, 0)], 4, 100, None, False)])
+def test_single_tokens_beside_portions_of_differential_attention(portions, singles, context, window, beside, monkeypatch):
+    """In the portions' launch where its last wave has places for all and they see little more than its last CTAs; a recorded step keeps them apart."""
+    monkeypatch.setattr(attention, "sm_count", lambda: 148)
+    lens, starts = [1] * singles + [q for q, _ in portions], [context - 1] * singles + [before for _, before in portions]
+    batch = types.SimpleNamespace(num_single=singles, num_seqs=len(lens), q_lens=lens, starts=starts, max_kv_len_single=context, max_kv_len=max(q + b for q, b in zip(lens, starts)),
+                                  max_kv_len_portion=max(q + b for q, b in portions))
+    assert attention.diff_singles_beside(batch, 16, 4, window, 16 if window else 0) == beside

@@ -145,3 +145,22 @@ def test_which_sizes_have_the_kernel():
     ok = ops.prefill_diff_supported
     assert ok(64, 128, 16) and ok(64, 24, 8) and ok(64, 64, 128)
     assert not ok(128, 128, 16) and not ok(64, 136, 16) and not ok(64, 20, 16) and not ok(64, 128, 4) and not ok(48, 96, 16)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens,singles", [([(1, 0), (1, 300), (1, 40), (1, 127), (1, 128), (150, 20), (31, 0)], 5), ([(1, 700), (40, 0)], 1), ([(1, 9), (1, 64), (2, 0), (3, 500), (130, 7)], 2),
+                                          ([(1, 5), (1, 255), (1, 256), (60, 0)], 2)])
+@pytest.mark.parametrize("window,keep", [(None, 0), (100, 16)])
+def test_single_tokens_in_the_portions_launch(lens, singles, window, keep):
+    """The sequences in front of the portions as layers of the same launch, more of them than portions and fewer; what is not asked for stays."""
+    portions = sum(1 for q, _ in lens if q > 1)
+    seq0 = len(lens) - portions
+    k, v, tables, rows, q, gate, start, kv_len = _case(lens, 8, 2, 128, 16, seed=9)
+    want = _exact(lens, rows, q, gate, start, 8, 2, 128, 0.125, window, keep, 0.7, 0.3, 1e-6)
+    out = torch.full((q.shape[0], 8 * 128), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.paged_prefill_diff(out, q.cuda(), k.cuda(), v.cuda(), tables.cuda(), start.cuda(), kv_len.cuda(), seq0, portions, max(c for c, _ in lens), gate.cuda()[:, :8], 8, 0.125,
+                           window, keep, 0.7, 0.3, 1e-6, singles)
+    left = seq0 - singles
+    assert (out[:left] == 7.0).all()
+    _near(out[left:].cpu(), want[left:])
+    assert ops.device_wait_errors() == {}
