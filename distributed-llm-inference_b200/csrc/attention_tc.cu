@@ -532,6 +532,11 @@ __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
   return d;
 }
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
 __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
   uint64_t d;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
@@ -1311,18 +1316,21 @@ int launch_tc2(const CUtensorMap& map_k, const CUtensorMap& map_v, const Params&
 #if !BENT_SCORES
 // ================================================================ one pool: a cached row is key and value
 // Prompt portions over rows of 136 to 256 numbers whose leading numbers are the values (attention over a cached latent: many query
-// heads on one KV head).  A tile of 128 rows comes once and is the K-major operand of S = Q K^T and the MN-major operand of O += P V (all value columns in
-// one instruction); it is copied in halves of 64 tokens to a ring of 5 (rows to 256) or 7 (to 192), which with Q fills shared memory.  S twice and O are
-// tensor memory (256 + 256 columns); the probabilities go over the scores that they come from and are the products' operand from there.  Four threads a
-// row do the softmax.  The warp that issues products takes whichever of S(t + 1) and O += P(t) V(t) is possible first.
+// heads on one KV head).  A tile of 64 rows comes once and is the K-major operand of S = Q K^T and the MN-major operand of O += P V (all value columns in
+// one instruction); six of them fill shared memory, so that copies are never waited for.  Q lies in tensor memory (SLABS x 32 columns) beside the scores of
+// three tiles (two where the output has more than 192 columns) and the output; the probabilities go over the scores that they come from and are the
+// products' operand from there.  Two groups of 256 threads do the softmax of a tile each in turns, two threads a row; a group reads the other's maxima of
+// the tile before from shared memory.  S and O are issued by a warp each.
 //
-// What bounds it: the chain.  With clocks taken in a CTA (4,096 tokens, 16 heads, rows of 256, 192 value columns), a tile takes 4,150 clocks: a half can
-// only be asked for when O of two tiles before is done, 1,400 until it is there, 1,300 S, 2,600 the softmax, 1,200 O.  Before (a copy for every page and slab:
-// 32 of 2 KB a tile, two threads a row, probabilities by way of shared memory) a tile took 4,320 and a CTA 24,000 beside its tiles, 16,000 of them to bring
-// Q a piece at a time and to zero both stages; those take 1,000 now and the CTA 8,000.  us, before and now: 4,096 tokens 213 -> 168, with a window of 1,024 139 -> 104,
-// 512 tokens 31 -> 23, 8 tokens behind 2,000 four times 61 -> 47, 2 behind 2,000 55 -> 45, 2,048 tokens with rows of 200 (copies by slab)
-// 74 -> 59 (the mma.sync kernel: 4,096 tokens 797, with a window 355, 512 tokens 43, 8 behind 2,000 149, 2 behind 2,000 141); portions that see one
-// key tile of the other kernel stay there (portions_pay_for_tiles_of_rows in kernels/attention.py).
+// What bounds it: the chain from O of a tile over the rescaling of the output for the next tile, whose maximum nearly always grows in some row of a warp, to the
+// next O.  With clocks taken in a CTA (4,096 tokens, 16 heads, rows of 256, 192 value columns), a tile of 64 keys takes 1,690 clocks: 600 until O is seen to be
+// done, 870 to rescale 192 columns while the tensor cores are at the next S, 200 until the next O is issued; the tensor cores' work is 930 of it, and a CTA takes 8,000 beside its tiles.
+// Tiles of 128 keys in two stages with Q in shared memory took 4,320 for 128 keys (3,900 between a copy's request and its arrival) and 24,000 beside them, the
+// same with half tiles in a ring 4,150; Q in tensor memory, one warp for both products 2,430 for 64; a warp each 1,790; no condition between
+// instructions 1,690.  us, before all that and now: 4,096 tokens 213 -> 142, with a window of 1,024 139 -> 93, 512 tokens 31 -> 22, 8 tokens behind 2,000 four times
+// 61 -> 40, 2 behind 2,000 55 -> 37, 2,048 tokens with rows of 200 (copies by slab) 74 -> 53, 700 of 128 heads behind 3,000 416 -> 280 (the mma.sync kernel: 4,096
+// tokens 797, with a window 355, 512 tokens 43, 8 behind 2,000 149, 2 behind 2,000 141); portions that see one key tile of the other
+// kernel stay there (portions_pay_for_tiles_of_rows in kernels/attention.py).
 struct RowParams {
   bf16* out;
   const bf16* q;
@@ -1336,29 +1344,20 @@ struct RowParams {
   int* error_flag;
 };
 
-constexpr int ROW_SOFTMAX_THREADS = 4 * ROWS, ROW_THREADS = ROW_SOFTMAX_THREADS + 64;
-constexpr int HALF_KEYS = KEYS / 2;  // keys of a copied half tile
+constexpr int ROW_SOFTMAX_THREADS = 4 * ROWS, ROW_THREADS = ROW_SOFTMAX_THREADS + 96;
+constexpr int ROW_KEYS = 64, ROW_STAGES = 6;  // keys of a tile, tiles in shared memory
 
 template <int SLABS> struct RowCfg {
-  static constexpr int Q = SLABS * TILE_BYTES, HALF = Q / 2, HALVES = (224 * 1024 - Q) / HALF;
-  static constexpr int AT_MAX = Q + HALVES * HALF, AT_BAR = AT_MAX + 4 * ROWS * 4, SMEM = AT_BAR + 256;
-  static_assert(SMEM <= 227 * 1024 && HALVES <= 8, "one CTA fits an SM, and its barriers their place");
+  static constexpr int STAGE = SLABS * ROW_KEYS * 128, AT_Q = (ROW_STAGES - 2) * STAGE;  // Q passes through the last two stages
+  static constexpr int AT_MAX = ROW_STAGES * STAGE, AT_BAR = AT_MAX + 8 * ROWS * 4, SMEM = AT_BAR + 256;
+  static_assert(SMEM <= 227 * 1024 && 2 * STAGE == SLABS * TILE_BYTES, "one CTA fits an SM, Q two stages");
 };
 
-__device__ __forceinline__ bool barrier_phase_done(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-  return done;
-}
 // Products are issued by one lane of a warp that runs together, so that descriptors stay in uniform registers.
 __device__ __forceinline__ uint32_t elect_one() {
   uint32_t one;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
   return one;
-}
-__device__ __forceinline__ void umma_one(uint32_t one, uint32_t sum, uint64_t a, uint64_t b, uint32_t idesc, bool add) {
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %5, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-               ::"r"(sum), "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)add), "r"(one) : "memory");
 }
 __device__ __forceinline__ void umma_tmem(uint32_t one, uint32_t sum, uint32_t a, uint64_t b, uint32_t idesc, bool add) {  // A in tensor memory
   asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %5, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
@@ -1379,29 +1378,32 @@ __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&v)[16]
                  "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]));
 }
 
-// WHOLE: rows of whole slabs; one copy brings a page (of 64 tokens at most), and half a tile is [8 tokens][slab][8][128 bytes], eight rows of a slab
-// in one swizzled piece.  Otherwise it is [slab][64 rows][128 bytes], a copy for every page and slab.
-template <int SLABS, bool WHOLE>
+// WHOLE: rows of whole slabs; one copy brings a page (of 64 tokens at most), and a tile is [8 tokens][slab][8][128 bytes], eight rows of a slab
+// in one swizzled piece.  Otherwise it is [slab][64 rows][128 bytes], a copy for every page and slab.  SB: scores in tensor memory at once.
+template <int SLABS, bool WHOLE, int SB>
 __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const __grid_constant__ CUtensorMap map, const RowParams p) {
   using Cfg = RowCfg<SLABS>;
-  constexpr int PIECES = WHOLE ? SLABS * 1024 : 1024, NEXT_SLAB = WHOLE ? 1024 : HALF_KEYS * 128;  // bytes from eight rows to the next eight, from a slab to the next
-  constexpr int HALVES = Cfg::HALVES, HALF = Cfg::HALF;
+  constexpr int PIECES = WHOLE ? SLABS * 1024 : 1024, NEXT_SLAB = WHOLE ? 1024 : ROW_KEYS * 128;  // bytes from eight rows to the next eight, from a slab to the next
+  constexpr int STAGE = Cfg::STAGE, STAGES = ROW_STAGES;
+  constexpr int AT_O = SB * ROW_KEYS, AT_Q = TMEM_COLS - SLABS * 32;  // columns: scores, output (192 with three, 256 with two), queries
+  static_assert(SB == 3 ? AT_O + 192 <= AT_Q : AT_O + 256 <= AT_Q, "tensor memory");
   pdl_launch_dependents();
   extern __shared__ __align__(1024) unsigned char smem[];
-  float* row_max = (float*)(smem + Cfg::AT_MAX);  // [4 (quarter of the keys)][128]
+  float* row_max = (float*)(smem + Cfg::AT_MAX);  // [4 (tile)][2 (half of the keys)][128]; at the end [4 (part)][128] sums and maxima
   uint64_t* bars = (uint64_t*)(smem + Cfg::AT_BAR);
-  uint32_t* tmem_slot = (uint32_t*)(bars + 24);
+  uint32_t* tmem_slot = (uint32_t*)(bars + 28);
   volatile int* failed = (volatile int*)(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t sQ = smem_u32(smem), sK = sQ + Cfg::Q;
-  const uint32_t k_full = smem_u32(bars), s_done = smem_u32(bars + 8), o_done = smem_u32(bars + 10), p_ready = smem_u32(bars + 14), q_full = smem_u32(bars + 16);
+  const uint32_t sK = smem_u32(smem);
+  const uint32_t k_full = smem_u32(bars), k_free = smem_u32(bars + 6), s_done = smem_u32(bars + 12), o_done = smem_u32(bars + 16), p_ready = smem_u32(bars + 20),
+                 q_full = smem_u32(bars + 24);
 
   const int s = p.seq0 + blockIdx.y;
   const int tile = gridDim.z - 1 - blockIdx.z;  // the tiles that see the most keys start first
   const int kvh = blockIdx.x / p.head_chunks, hc = blockIdx.x - kvh * p.head_chunks;
   const int q0 = p.q_start[s], qlen = p.q_start[s + 1] - q0, tok0 = tile * p.tokens_per_tile;
   if (tok0 >= qlen) return;  // the whole CTA: nothing was set up yet
-  if (sQ & 1023) {  // the swizzled tiles need it; nothing else lies in front of them
+  if (sK & 1023) {  // the swizzled tiles need it; nothing else lies in front of them
     if (tid == 0) atomicExch(p.error_flag, 21);
     return;
   }
@@ -1410,13 +1412,14 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
   const int pos0 = kvlen - qlen + tok0, rows_used = ntok * Gc;
   const int* table = p.block_tables + (size_t)s * p.max_blocks;
   const int hi = pos0 + ntok, lo = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
-  const int t_begin = lo / KEYS, t_end = (hi + KEYS - 1) / KEYS, num_tiles = t_end - t_begin;
+  const int t_begin = lo / ROW_KEYS, t_end = (hi + ROW_KEYS - 1) / ROW_KEYS, num_tiles = t_end - t_begin;
   const int vslabs = (p.dv + 63) >> 6;
-  const int unit_bits = 31 - __clz(min(p.page_size, HALF_KEYS)), unit = 1 << unit_bits, page_bits = 31 - __clz(p.page_size);  // tokens of a copy (powers of two)
+  const int unit_bits = 31 - __clz(min(p.page_size, ROW_KEYS)), unit = 1 << unit_bits, page_bits = 31 - __clz(p.page_size);  // tokens of a copy (powers of two)
 
   if (tid == 0) {
-    for (int i = 0; i < 14; ++i) mbar_init(k_full + 8 * i, 1);  // k_full (8), s_done (2), o_done (4)
-    for (int i = 0; i < 3; ++i) mbar_init(p_ready + 8 * i, ROW_SOFTMAX_THREADS / 32);  // p_ready (2), q_full
+    for (int i = 0; i < 20; ++i) mbar_init(k_full + 8 * i, 1);  // k_full (6), k_free (6), s_done (4), o_done (4)
+    for (int i = 0; i < 4; ++i) mbar_init(p_ready + 8 * i, ROW_SOFTMAX_THREADS / 64);  // the warps of a tile's group
+    mbar_init(q_full, ROW_SOFTMAX_THREADS / 32);
     *failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1428,24 +1431,22 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot, tmem_s = tmem, tmem_o = tmem + 2 * KEYS;
+  const uint32_t tmem_s = *tmem_slot, tmem_o = tmem_s + AT_O, tmem_q = tmem_s + AT_Q;
   pdl_wait();  // queries and the cache are the work of the kernels before this one
 
   if (warp == ROW_SOFTMAX_THREADS / 32 + 1) {
-    // ================================================================ the warp that copies: half a tile at a time, a page per lane
-    const int halves = 2 * num_tiles;
-    auto lookup = [&](int h) -> int {
-      const int first = t_begin * KEYS + h * HALF_KEYS + (lane << unit_bits);
-      const bool need = h < halves && (lane << unit_bits) < HALF_KEYS && first < hi && first + unit > lo;
+    // ================================================================ the warp that copies: a tile at a time, a page per lane
+    auto lookup = [&](int t) -> int {
+      const int first = (t_begin + t) * ROW_KEYS + (lane << unit_bits);
+      const bool need = t < num_tiles && (lane << unit_bits) < ROW_KEYS && first < hi && first + unit > lo;
       return need ? table[first >> page_bits] : -1;
     };
-    int page = lookup(0), asked = 0, slot = 0;  // halves whose copies were asked for
-    for (int h = 0; h < halves && !*failed; ++h) {
+    int page = lookup(0), asked = 0, slot = 0, turn = 0;  // tiles whose copies were asked for
+    for (int t = 0; t < num_tiles && !*failed; ++t) {
       const int cur = page;
-      page = lookup(h + 1);
-      const int before = h - HALVES;  // the half that lies in this slot; the last to read it is P V of its tile
-      if (before >= 0 && !(before & 1)) {
-        if (lane == 0) wait_or_fail(o_done + 8 * ((before >> 1) & 3), (before >> 3) & 1, failed, 22, p.error_flag);
+      page = lookup(t + 1);
+      if (turn > 0 || slot >= STAGES - 2) {  // O of the tile that lies in this stage, its last reader; the first time there Q
+        if (lane == 0) turn > 0 ? wait_or_fail(k_free + 8 * slot, (turn - 1) & 1, failed, 22, p.error_flag) : wait_or_fail(q_full, 0, failed, 25, p.error_flag);
         __syncwarp();
         if (*failed) break;
       }
@@ -1454,10 +1455,10 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
       if (lane == 0) mbar_expect_tx(full, (uint32_t)(count * unit * 128 * SLABS));
       __syncwarp();
       if (cur >= 0) {
-        const int row = (cur * p.nkv + kvh) * p.page_size + (((h & 1) * HALF_KEYS + (lane << unit_bits)) & (p.page_size - 1));
+        const int row = (cur * p.nkv + kvh) * p.page_size + (((t_begin + t) * ROW_KEYS + (lane << unit_bits)) & (p.page_size - 1));
 #pragma unroll
         for (int sl = 0; sl < (WHOLE ? 1 : SLABS); ++sl) {
-          const uint32_t to = sK + slot * HALF + sl * NEXT_SLAB + (lane << unit_bits) * (PIECES / 8);
+          const uint32_t to = sK + slot * STAGE + sl * NEXT_SLAB + (lane << unit_bits) * (PIECES / 8);
           if (WHOLE)
             asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %3, %3, %4}], [%2];"
                          ::"r"(to), "l"(&map), "r"(full), "r"(0), "r"(row >> 3) : "memory");
@@ -1466,77 +1467,69 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
         }
       }
       ++asked;
-      if (++slot == HALVES) slot = 0;
+      if (++slot == STAGES) slot = 0, ++turn;
     }
     if (*failed && lane == 0)
-      for (int h = max(0, asked - HALVES); h < asked; ++h) wait_for_last(k_full + 8 * (h % HALVES), (h / HALVES) & 1);
-  } else if (warp == ROW_SOFTMAX_THREADS / 32) {
-    // ================================================================ the warp that issues the matrix products (one lane of it, the warp together)
+      for (int t = max(0, asked - STAGES); t < asked; ++t) wait_for_last(k_full + 8 * (t % STAGES), (t / STAGES) & 1);
+  } else if (warp >= ROW_SOFTMAX_THREADS / 32) {
+    // ================================================================ the warps that issue the matrix products (one lane of each, the warp together): one S, one O, so that
+    //                                                                  O, on which the next tile waits, does not stand behind a whole S
     const uint32_t one = elect_one();
-    const uint32_t idesc_s = instr_desc(ROWS, KEYS, 0), idesc_half = instr_desc(ROWS, HALF_KEYS, 0), idesc_o = instr_desc(ROWS, vslabs * 64, 1);
-    const int k_steps = (p.d + 15) >> 4;
-    const uint64_t next_slab = (uint64_t)(NEXT_SLAB >> 4) << 16;  // of the MN-major operand: bytes from 64 columns to the next 64
-    auto rows_desc = [](uint32_t addr) { return (smem_desc_sw128(addr) & ~((uint64_t)0x3FFF << 32)) | (uint64_t)(PIECES >> 4) << 32; };
-    int s_next = 0, o_next = 0, s_slot = 0, s_phase = 0, o_slot = 0;  // the tiles' first halves lie in these slots
-    unsigned idle = 0;
-    if (!wait_or_fail(q_full, 0, failed, 25, p.error_flag)) *failed = 25;
-    __syncwarp();
-    while (o_next < num_tiles && !__any_sync(0xffffffffu, *failed != 0)) {
-      bool moved = false;
-      // O += P(t) V(t): the probabilities are written, the output rescaled where a row's maximum grew
-      if (o_next < s_next && __all_sync(0xffffffffu, barrier_phase_done(p_ready + 8 * (o_next & 1), (o_next >> 1) & 1))) {
+    const uint64_t rows = (smem_desc_sw128(sK) & ~((uint64_t)0x3FFF << 32)) | (uint64_t)(PIECES >> 4) << 32;  // of the first stage (a descriptor counts 16 bytes)
+    int slot = 0, phase = 0, buf = 0, t = 0;
+    bool good = wait_or_fail(q_full, 0, failed, 25, p.error_flag);
+    if (warp == ROW_SOFTMAX_THREADS / 32) {
+      const uint32_t idesc = instr_desc(ROWS, ROW_KEYS, 0);
+      const int k_steps = (p.d + 15) >> 4;
+      for (; t < num_tiles; ++t) {  // S(t) = Q K(t)^T: the rows have arrived; the buffer held S(t - SB) and P(t - SB), which O has taken
+        good = good && wait_or_fail(k_full + 8 * slot, phase, failed, 17, p.error_flag);
+        if (t >= SB) good = good && wait_or_fail(o_done + 8 * ((t - SB) & 3), ((t - SB) >> 2) & 1, failed, 23, p.error_flag);
+        if (!__all_sync(0xffffffffu, good)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t pa = tmem_s + (o_next & 1) * KEYS;
-        uint32_t v = sK + o_slot * HALF;
+        const uint64_t k = rows + (uint32_t)(slot * (STAGE >> 4));
+        const uint32_t to = tmem_s + buf * ROW_KEYS;
+        if (WHOLE) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
+          for (int kk = 0; kk < SLABS * 4; ++kk) umma_tmem(one, to, tmem_q + kk * 8, k + (((kk >> 2) * NEXT_SLAB + (kk & 3) * 32) >> 4), idesc, kk != 0);
+        } else {
 #pragma unroll
-          for (int k = 0; k < HALF_KEYS / 16; ++k)  // sixteen keys: eight columns; a quarter's probabilities lie where its scores began
-            umma_tmem(one, tmem_o, pa + half * 64 + (k >> 1) * 32 + (k & 1) * 8, rows_desc(v + k * 2 * PIECES) | next_slab, idesc_o, (o_next | half | k) != 0);
-          o_slot = o_slot + 1 == HALVES ? 0 : o_slot + 1;
-          v = sK + o_slot * HALF;
+          for (int kk = 0; kk < SLABS * 4; ++kk)
+            if (kk < k_steps) umma_tmem(one, to, tmem_q + kk * 8, k + (((kk >> 2) * NEXT_SLAB + (kk & 3) * 32) >> 4), idesc, kk != 0);
         }
-        umma_commit_one(one, o_done + 8 * (o_next & 3));
-        ++o_next;
-        moved = true;
+        umma_commit_one(one, s_done + 8 * (t & 3));
+        if (++slot == STAGES) slot = 0, phase ^= 1;
+        if (++buf == SB) buf = 0;
       }
-      // S(t) = Q K(t)^T: the rows have arrived; the buffer held S(t - 2) and P(t - 2), which O has taken
-      const int slot2 = s_slot + 1 == HALVES ? 0 : s_slot + 1, phase2 = slot2 ? s_phase : s_phase ^ 1;
-      if (s_next < num_tiles && (s_next < 2 || __all_sync(0xffffffffu, barrier_phase_done(o_done + 8 * ((s_next - 2) & 3), ((s_next - 2) >> 2) & 1)))
-          && __all_sync(0xffffffffu, barrier_phase_done(k_full + 8 * s_slot, s_phase) && barrier_phase_done(k_full + 8 * slot2, phase2))) {
+      if (t < num_tiles)
+        for (int i = max(0, t - 4); i < t; ++i) wait_for_last(s_done + 8 * (i & 3), (i >> 2) & 1);
+    } else {
+      const uint32_t idesc = instr_desc(ROWS, vslabs * 64, 1);
+      const uint64_t next_slab = (uint64_t)(NEXT_SLAB >> 4) << 16;  // of the MN-major operand: bytes from 64 columns to the next 64
+      for (; t < num_tiles; ++t) {  // O += P(t) V(t): the probabilities are written, the output rescaled where a row's maximum grew
+        good = good && wait_or_fail(p_ready + 8 * (t & 3), (t >> 2) & 1, failed, 19, p.error_flag);
+        if (!__all_sync(0xffffffffu, good)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t k = sK + s_slot * HALF, k2 = sK + slot2 * HALF, to = tmem_s + (s_next & 1) * KEYS;
-        const bool joined = WHOLE && slot2 != 0;  // the pieces of both halves have the same distance
+        const uint32_t pa = tmem_s + buf * ROW_KEYS;
+        const uint64_t v = (rows | next_slab) + (uint32_t)(slot * (STAGE >> 4));
 #pragma unroll
-        for (int kk = 0; kk < SLABS * 4; ++kk)
-          if (kk < k_steps) {
-            const uint64_t q = smem_desc_sw128(sQ + (kk >> 2) * TILE_BYTES + (kk & 3) * 32);
-            const uint32_t at = (kk >> 2) * NEXT_SLAB + (kk & 3) * 32;
-            umma_one(one, to, q, rows_desc(k + at), joined ? idesc_s : idesc_half, kk != 0);
-            if (!joined) umma_one(one, to + HALF_KEYS, q, rows_desc(k2 + at), idesc_half, kk != 0);
-          }
-        umma_commit_one(one, s_done + 8 * (s_next & 1));
-        ++s_next;
-        s_slot = slot2 + 1 == HALVES ? 0 : slot2 + 1;
-        s_phase = s_slot ? phase2 : phase2 ^ 1;
-        moved = true;
+        for (int k = 0; k < ROW_KEYS / 16; ++k)  // sixteen keys: eight columns; a half's probabilities lie where its scores began
+          umma_tmem(one, tmem_o, pa + (k >> 1) * 32 + (k & 1) * 8, v + (k * 2 * PIECES >> 4), idesc, (t | k) != 0);
+        umma_commit_one(one, o_done + 8 * (t & 3));
+        umma_commit_one(one, k_free + 8 * slot);
+        if (++slot == STAGES) slot = 0;
+        if (++buf == SB) buf = 0;
       }
-      if (moved) {
-        idle = 0;
-      } else if (++idle > WAIT_LIMIT) {
-        *failed = 23;
-        if (lane == 0) atomicExch(p.error_flag, 23);
-      }
-    }
-    if (o_next < num_tiles) {
-      for (int t = max(0, s_next - 2); t < s_next; ++t) wait_for_last(s_done + 8 * (t & 1), (t >> 1) & 1);
-      for (int t = max(0, o_next - 4); t < o_next; ++t) wait_for_last(o_done + 8 * (t & 3), (t >> 2) & 1);
+      if (t < num_tiles)
+        for (int i = max(0, t - 4); i < t; ++i) wait_for_last(o_done + 8 * (i & 3), (i >> 2) & 1);
     }
     __syncwarp();
   } else {
-    // ================================================================ softmax threads: four a row, 32 keys and a quarter of the value columns each
-    const int r = tid & (ROWS - 1), quarter = tid >> 7, rows_bar = 1 + (warp & 3);
-    // ---- Q, a row a warp, all of a thread's pieces under way at once (rows beyond the used ones and columns beyond the row are zeros)
+    // ================================================================ softmax threads: two groups of 256 in turns, a tile each; two threads a row, 32 keys and half of
+    //                                                                  the value columns each
+    const int r = tid & (ROWS - 1), part = tid >> 7, group = part >> 1, half = part & 1;
+    const uint32_t lane_bits = (uint32_t)((warp & 3) * 32) << 16;
+    // ---- Q, a row a warp, all of a thread's pieces under way at once (rows beyond the used ones and columns beyond the row are zeros), then, a row a thread
+    //      and a slab a warp, to tensor memory
     {
       const int by_heads = heads_inverse(Gc);
 #pragma unroll
@@ -1545,36 +1538,52 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
         const bool there = rr < rows_used && hd < nheads && lane * 8 < p.d;
         const bf16* from = p.q + (there ? (size_t)(q0 + tok0 + tok) * p.q_stride + (size_t)(head0 + hd) * p.d + lane * 8 : 0);
         if (lane < 8 * SLABS)
-          query_piece(sQ + (lane >> 3) * TILE_BYTES + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4), from, there ? 16 : 0);
+          query_piece(sK + Cfg::AT_Q + (lane >> 3) * TILE_BYTES + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4), from, there ? 16 : 0);
       }
       query_pieces_there();
+      asm volatile("bar.sync 13, %0;" ::"n"(ROW_SOFTMAX_THREADS) : "memory");
+      if (part < SLABS) {
+        uint32_t v[32];
+        const uint32_t from = sK + Cfg::AT_Q + part * TILE_BYTES + r * 128;
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[4 * c]), "=r"(v[4 * c + 1]), "=r"(v[4 * c + 2]), "=r"(v[4 * c + 3]) : "r"(from + ((c ^ (r & 7)) << 4)) : "memory");
+        tmem_st32(tmem_q + lane_bits + part * 32, v);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(q_full);
     }
     const int rtok = r / Gc;
     const bool rvalid = r < rows_used && (r - rtok * Gc) < nheads;
     const int rpos = pos0 + rtok;
-    const uint32_t lane_bits = (uint32_t)((warp & 3) * 32) << 16;
-    const int col0 = quarter * 32, my_cols = vslabs * 16;
-    float m = -CUDART_INF_F, l = 0.f;
+    const int col0 = half * 32;
+    float m = -CUDART_INF_F, l = 0.f;  // the maximum of what this group and the other have seen up to this group's last tile; the sum of this thread's keys
     bool ok = true;
-    const uint32_t my_o = tmem_o + lane_bits + quarter * my_cols;
+    const uint32_t my_o = tmem_o + lane_bits + half * vslabs * 32;
     const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2);
+    // Rows 32 i .. are four warps, two a group.  Barrier t (three of them in turns): the tile's group waits for its own maxima of tile t, and the other group has left those of tile t - 1
+    // (one that would be used for t + 3 meanwhile waits for O(t) first: its scores' place)
+    const int rows_bar = 1 + (warp & 3) * 3;
+    if (group == 1) asm volatile("bar.arrive %0, 128;" ::"r"(rows_bar) : "memory");
+    int buf = group % SB, turn = group, next_turn = group + 1;  // of this group's tile: t % SB; t % 3, (t + 1) % 3
+    const int first_row = lo >> unit_bits << unit_bits, end_row = min((hi + unit - 1) >> unit_bits << unit_bits, kvlen);  // what lies in shared memory
 
-    for (int it = 0; it < num_tiles; ++it) {
-      const int b = it & 1, base = (t_begin + it) * KEYS;
-      const uint32_t my_s = tmem_s + b * KEYS + lane_bits + col0;
-      ok = wait_or_fail(s_done + 8 * b, (it >> 1) & 1, failed, 24, p.error_flag) && ok;
+    for (int it = group; it < num_tiles; it += 2) {
+      const int base = (t_begin + it) * ROW_KEYS;
+      const uint32_t my_s = tmem_s + buf * ROW_KEYS + lane_bits + col0;
+      ok = wait_or_fail(s_done + 8 * (it & 3), (it >> 2) & 1, failed, 24, p.error_flag) && ok;
       __syncwarp();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const bool full = base + KEYS - 1 <= pos0 && (p.window <= 0 || base >= hi - p.window);  // every row sees all of the tile
-      uint32_t packed[32];
-      tmem_ld32_nowait(my_s, packed);
+      const bool full = base + ROW_KEYS - 1 <= pos0 && (p.window <= 0 || base >= hi - p.window);  // every row sees all of the tile
+      uint32_t raw[32];
+      tmem_ld32_nowait(my_s, raw);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       float sc[32];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) sc[j] = __uint_as_float(packed[j]);
+      for (int j = 0; j < 32; ++j) sc[j] = __uint_as_float(raw[j]);
       if (!full) {
         const int first = base + col0;
         const int hi_j = rpos - first, lo_j = p.window > 0 ? rpos - p.window - first : -1;
@@ -1584,13 +1593,17 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
       float mx[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) mx[i] = max3(max3(sc[i], sc[i + 4], sc[i + 8]), max3(sc[i + 12], sc[i + 16], sc[i + 20]), fmaxf(sc[i + 24], sc[i + 28]));
-      asm volatile("bar.sync %0, 128;" ::"r"(rows_bar) : "memory");  // the four threads of each of these 32 rows: the last tile's maxima have been read
-      row_max[quarter * ROWS + r] = fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]);
-      asm volatile("bar.sync %0, 128;" ::"r"(rows_bar) : "memory");
+      float* now = row_max + (it & 3) * 2 * ROWS + r;
+      const float* last = row_max + ((it - 1) & 3) * 2 * ROWS + r;
+      now[half * ROWS] = fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]);
+      if (it + 1 < num_tiles) asm volatile("bar.arrive %0, 128;" ::"r"(rows_bar + next_turn) : "memory");
+      asm volatile("bar.sync %0, 128;" ::"r"(rows_bar + turn) : "memory");
       // probabilities are relative to the exact maximum so far: the largest one is then 1 and bfloat16 holds it as it is (following the maximum
       // only when it has grown by 2^8 gave an error 2 to 23 % larger)
-      const float before = m;
-      m = max3(max3(m, row_max[r], row_max[ROWS + r]), row_max[2 * ROWS + r], row_max[3 * ROWS + r]);
+      const float mine = m;
+      float before = m;
+      if (it > 0) before = max3(m, last[0], last[ROWS]);  // that of the tile before, to which the output is relative
+      m = max3(before, now[0], now[ROWS]);
       const bool grown = m > before;  // also the first finite maximum (before = -inf)
       const float corr = grown ? ex2((before - m) * p.scale_log2) : 1.f;
       const float neg = (m == -CUDART_INF_F) ? 0.f : -m * p.scale_log2;
@@ -1608,98 +1621,110 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
       tmem_st16(my_s, probs);  // over this thread's own scores
       float sum0, sum1;
       unpack_f32x2(add_f32x2(sum[0], sum[1]), sum0, sum1);
-      l = l * corr + (sum0 + sum1);
-      // O is free once the product of the tile before has finished
+      l = l * (m > mine ? ex2((mine - m) * p.scale_log2) : 1.f) + (sum0 + sum1);
+      // rows that were not fetched, and those of the last page that hold no token: S has been taken, as values they must not multiply garbage
+      if (base < first_row || base + ROW_KEYS > end_row) {
+        const int from = max(first_row - base, 0), to = min(end_row - base, ROW_KEYS);
+        const int empty = from + ROW_KEYS - to, at = (it % STAGES) * STAGE + (lane >> 3) * NEXT_SLAB + ((lane & 7) << 4);
+        for (int i = (tid & 255) >> 5; i < empty; i += 8) {
+          const int row = i < from ? i : i - from + to;
+          if (lane < 8 * vslabs) *reinterpret_cast<uint4*>(smem + at + (row >> 3) * PIECES + (row & 7) * 128) = make_uint4(0, 0, 0, 0);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      }
+      // O is free once the product of the tile before has finished.  From here to the arrival below is what a tile waits on: two pieces of 32 columns under way
+      // at once, and nothing else.
       if (it > 0 && __any_sync(0xffffffffu, grown)) {
         ok = wait_or_fail(o_done + 8 * ((it - 1) & 3), ((it - 1) >> 2) & 1, failed, 22, p.error_flag) && ok;
         ok = __all_sync(0xffffffffu, ok);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (ok) {
+          const uint64_t corr2 = pack_f32x2(corr, corr);
+          auto scaled = [&](uint32_t at, uint32_t (&v)[32]) {
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            uint32_t v[2][16];
+            for (int j = 0; j < 32; j += 2) {
+              float x, y;
+              unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), corr2), x, y);
+              v[j] = __float_as_uint(x), v[j + 1] = __float_as_uint(y);
+            }
+            tmem_st32(at, v);
+          };
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
-              if (2 * half + i < vslabs) tmem_ld16(my_o + 32 * half + 16 * i, v[i]);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-              if (2 * half + i < vslabs) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) v[i][j] = __float_as_uint(__uint_as_float(v[i][j]) * corr);
-                tmem_st16(my_o + 32 * half + 16 * i, v[i]);
-              }
-          }
+          for (int i = 0; i < 4; i += 2)
+            if (i < vslabs) {
+              uint32_t v0[32], v1[32];
+              tmem_ld32_nowait(my_o + 32 * i, v0);
+              if (i + 1 < vslabs) tmem_ld32_nowait(my_o + 32 * i + 32, v1);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+              scaled(my_o + 32 * i, v0);
+              if (i + 1 < vslabs) scaled(my_o + 32 * i + 32, v1);
+            }
         }
-      }
-      // rows that were not fetched, and those of the last page that hold no token: S has been taken, as values they must not multiply garbage
-      const int from = max(((lo >> unit_bits) << unit_bits) - base, 0), to = min(min(((hi + unit - 1) >> unit_bits) << unit_bits, kvlen) - base, KEYS);
-      if (from > 0 || to < KEYS) {
-        const int empty = from + KEYS - to;
-        for (int i = tid; i < empty * 32; i += ROW_SOFTMAX_THREADS) {
-          const int row = (i >> 5) < from ? i >> 5 : (i >> 5) - from + to, c = lane;
-          const int slot = (2 * it + (row >> 6)) % HALVES, at = slot * HALF + (c >> 3) * NEXT_SLAB + ((row >> 3) & 7) * PIECES + (row & 7) * 128 + ((c & 7) << 4);
-          if (c < 8 * vslabs) *reinterpret_cast<uint4*>(smem + Cfg::Q + at) = make_uint4(0, 0, 0, 0);
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_ready + 8 * b);  // P is written, the output rescaled and S read
+      if (lane == 0) mbar_arrive(p_ready + 8 * (it & 3));  // P is written, the output rescaled and S read
+      buf += 2;
+      if (buf >= SB) buf -= SB;
+      turn = next_turn == 2 ? 0 : next_turn + 1;
+      next_turn = turn == 2 ? 0 : turn + 1;
     }
-    // ---- the finished output, once the last product is done; the row sum is the four quarters' sums
+    // ---- the finished output, once the last product is done (then no barrier above is still waited at); the row sum is that of the four threads' sums, each
+    //      relative to the maximum that its group knew last
     ok = wait_or_fail(o_done + 8 * ((num_tiles - 1) & 3), ((num_tiles - 1) >> 2) & 1, failed, 22, p.error_flag) && ok;
     ok = __all_sync(0xffffffffu, ok);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("bar.sync %0, 128;" ::"r"(rows_bar) : "memory");
-    row_max[quarter * ROWS + r] = l;
+    row_max[part * ROWS + r] = l;
+    row_max[(4 + part) * ROWS + r] = m;
     asm volatile("bar.sync %0, 128;" ::"r"(rows_bar) : "memory");
-    const int head = head0 + (r - rtok * Gc);
-    const float total = (row_max[r] + row_max[ROWS + r]) + (row_max[2 * ROWS + r] + row_max[3 * ROWS + r]);
+    m = max3(row_max[4 * ROWS + r], row_max[6 * ROWS + r], -CUDART_INF_F);  // (a group's threads know the same)
+    float total = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float known = row_max[(4 + i) * ROWS + r];
+      total += row_max[i * ROWS + r] * (m > known ? ex2((known - m) * p.scale_log2) : 1.f);
+    }
+    const int head = head0 + (r - rtok * Gc), my_cols = vslabs * 16;
     const float inv = 1.f / (total + sink_term(rvalid ? sink_of(p.sink_heads, p.sink_log2, head) : -CUDART_INF_F, m * p.scale_log2));
     const bool store = ok && !*failed && rvalid;
-    bf16* out = p.out + (store ? ((size_t)(q0 + tok0 + rtok) * p.nh + head) * p.out_row + quarter * my_cols : 0);
+    bf16* out = p.out + (store ? ((size_t)(q0 + tok0 + rtok) * p.nh + head) * p.out_row + part * my_cols : 0);
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      uint32_t v[2][16];
+    for (int i = 0; i < 4; ++i) {
+      if (i >= vslabs) break;
+      uint32_t v[16];
       if (ok) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-          if (2 * half + i < vslabs) tmem_ld16(my_o + 32 * half + 16 * i, v[i]);
+        tmem_ld16(tmem_o + lane_bits + part * my_cols + 16 * i, v);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       }
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+      for (int j = 0; j < 16; j += 8)
+        if (store && part * my_cols + 16 * i + j < p.dv) {
+          uint4 w;
+          __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&w);
 #pragma unroll
-        for (int j = 0; j < 16; j += 8) {
-          const int col = 32 * half + 16 * i + j;
-          if (store && 2 * half + i < vslabs && quarter * my_cols + col < p.dv) {
-            uint4 w;
-            __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&w);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) h2[e] = __floats2bfloat162_rn(__uint_as_float(v[i][j + 2 * e]) * inv, __uint_as_float(v[i][j + 2 * e + 1]) * inv);
-            *reinterpret_cast<uint4*>(out + col) = w;
-          }
+          for (int e = 0; e < 4; ++e) h2[e] = __floats2bfloat162_rn(__uint_as_float(v[j + 2 * e]) * inv, __uint_as_float(v[j + 2 * e + 1]) * inv);
+          *reinterpret_cast<uint4*>(out + 16 * i + j) = w;
         }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_s), "r"(TMEM_COLS) : "memory");
 }
 
-template <int SLABS, bool WHOLE> int launch_rows(const CUtensorMap& map, const RowParams& p, int num_seqs, int max_q_len, cudaStream_t stream) {
+template <int SLABS, bool WHOLE, int SB> int launch_rows(const CUtensorMap& map, const RowParams& p, int num_seqs, int max_q_len, cudaStream_t stream) {
   using Cfg = RowCfg<SLABS>;
   static OncePerDevice configured;
   if (!configured.here()) {
-    cudaError_t e = cudaFuncSetAttribute(paged_prefill_row_kernel<SLABS, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(paged_prefill_row_kernel<SLABS, WHOLE, SB>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
     if (e != cudaSuccess) return (int)e;
     configured.here() = true;
   }
   const int tiles = (max_q_len + p.tokens_per_tile - 1) / p.tokens_per_tile;
   if (tiles > 65535 || num_seqs > 65535) return DLI_ERR_UNSUPPORTED;  // the grid's y and z
-  return (int)launch_pdl((paged_prefill_row_kernel<SLABS, WHOLE>), dim3(p.nkv * p.head_chunks, num_seqs, tiles), dim3(ROW_THREADS), (size_t)Cfg::SMEM, stream, 1, map, p);
+  return (int)launch_pdl((paged_prefill_row_kernel<SLABS, WHOLE, SB>), dim3(p.nkv * p.head_chunks, num_seqs, tiles), dim3(ROW_THREADS), (size_t)Cfg::SMEM, stream, 1, map, p);
 }
 #endif
 
@@ -1821,7 +1846,7 @@ DLI_EXPORT int dli_paged_prefill_rows(void* out, const void* q, long long q_stri
   CUtensorMap map;
   const bool whole = head_dim % 64 == 0;  // (elsewhere the last slab's rows would end in the next row, and behind the pool)
   const long long rows = num_pages * nkv * page_size;
-  if (!(whole ? make_row_map(&map, pool, rows, page_size, head_dim) : make_pool_map(&map, pool, rows, page_size < HALF_KEYS ? page_size : HALF_KEYS, head_dim))) return DLI_ERR_UNSUPPORTED;
+  if (!(whole ? make_row_map(&map, pool, rows, page_size, head_dim) : make_pool_map(&map, pool, rows, page_size < ROW_KEYS ? page_size : ROW_KEYS, head_dim))) return DLI_ERR_UNSUPPORTED;
   RowParams p;
   p.out = (bf16*)out; p.q = (const bf16*)q; p.q_stride = q_stride; p.block_tables = block_tables; p.max_blocks = max_blocks; p.q_start = q_start;
   p.kv_len = kv_len; p.seq0 = seq0; p.nh = nh; p.nkv = nkv; p.page_size = page_size; p.window = window;
@@ -1834,8 +1859,10 @@ DLI_EXPORT int dli_paged_prefill_rows(void* out, const void* q, long long q_stri
   p.tokens_per_tile = ROWS / p.heads_per_chunk;
   p.d = head_dim; p.dv = value_dim; p.out_row = head_dim;
   p.error_flag = error_flag_device;
-  if (whole) return head_dim == 192 ? launch_rows<3, true>(map, p, num_seqs, max_q_len, stream) : launch_rows<4, true>(map, p, num_seqs, max_q_len, stream);
-  return head_dim <= 192 ? launch_rows<3, false>(map, p, num_seqs, max_q_len, stream) : launch_rows<4, false>(map, p, num_seqs, max_q_len, stream);
+  // three tiles' scores fit tensor memory beside outputs of up to 192 columns
+  if (head_dim <= 192) return whole ? launch_rows<3, true, 3>(map, p, num_seqs, max_q_len, stream) : launch_rows<3, false, 3>(map, p, num_seqs, max_q_len, stream);
+  if (value_dim <= 192) return whole ? launch_rows<4, true, 3>(map, p, num_seqs, max_q_len, stream) : launch_rows<4, false, 3>(map, p, num_seqs, max_q_len, stream);
+  return whole ? launch_rows<4, true, 2>(map, p, num_seqs, max_q_len, stream) : launch_rows<4, false, 2>(map, p, num_seqs, max_q_len, stream);
 }
 #endif
 
