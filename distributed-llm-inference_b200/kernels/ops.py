@@ -2132,7 +2132,7 @@ def moe_products(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_up
     partial = torch.empty((rows, W), dtype=torch.float32, device=x.device)
     f = _fn("moe_sort.cu", "dli_moe_sort_gather", [c_void_p] * 4 + [c_int] * 5 + [c_void_p])
     _check(f(_ptr(xs), _ptr(x), _ptr(ids), _ptr(ints), n, W, E, top, MOE_TILE_ROWS, _stream()), "moe_products")
-    launch_count += 1 if pairs <= 2048 else 4  # two kernels a call (one block sorts up to 2,048 pairs), else five
+    launch_count += 1 if pairs <= 2048 else 3  # two kernels a call (one block sorts up to 2,048 pairs), else four
     g = _fn("dense_gemm.cu", "dli_dense_gemm_grouped", [c_void_p] * 6 + [c_int] * 6 + [c_void_p])
     maps = (_ptr(used), _ptr(tile_expert), _ptr(row_pair))
     _check(g(_ptr(hidden), _ptr(xs), _ptr(w_up), *maps, rows, (2 if gated else 1) * ff, W, E, 1 if gated else 0, act if gated else act + 1, _stream()), "moe_products")
