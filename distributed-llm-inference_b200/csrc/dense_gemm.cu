@@ -14,7 +14,7 @@
 //     share few weight tiles).
 //   * One thread of each CTA issues its TMA copies (cp.async.bulk.tensor, 128-byte swizzle) of a [128 x 64] tile of
 //     x and a [128 x 64] half tile of W per k step, six steps ahead; rows beyond the matrices arrive as zeros.
-//   * One thread of the first CTA issues tcgen05.mma (M = 2 x 128, N = 256, K = 16; four per k step) into one of TWO
+//   * One lane of a warp of the first CTA issues tcgen05.mma (M = 2 x 128, N = 256, K = 16; four per k step) into one of TWO
 //     accumulators in tensor memory (2 x 256 columns in each CTA), so the products of the next tile run while
 //   * four warps of each CTA read the finished accumulator with tcgen05.ld (lane = token, column = feature), apply
 //     the epilogue and store.
@@ -319,16 +319,21 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
   asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                ::"r"(dst), "l"(map), "r"(bar & PEER_BIT_MASK), "r"(x), "r"(y) : "memory");
 }
-__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one;
+}
+__device__ __forceinline__ void umma_pair(uint32_t one, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %5, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(one) : "memory");
 }
 // arrives, once the products issued so far have finished, on the barrier at this offset in both CTAs of the pair
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(bar), "h"((uint16_t)3) : "memory");
+__device__ __forceinline__ void umma_commit_pair(uint32_t one, uint32_t bar) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+               ::"r"(bar), "h"((uint16_t)3), "r"(one) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_at(uint32_t bar, uint32_t cta) {
   asm volatile("{\n\t.reg .b32 remote;\n\tmapa.shared::cluster.u32 remote, %0, %1;\n\tmbarrier.arrive.shared::cluster.b64 _, [remote];\n\t}"
@@ -403,36 +408,36 @@ __global__ void __launch_bounds__(THREADS, 1) dense_gemm_pair_kernel(const __gri
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ---- products: the first CTA's thread issues them for both
-    if (lane == 0 && rank == 0) {
-      const uint32_t idesc = instr_desc(2 * BM, BN);
+    // ---- products: the first CTA's warp issues them for both, by one lane but together, so that descriptors stay in uniform registers
+    if (rank == 0) {
+      const uint32_t one = elect_one(), idesc = instr_desc(2 * BM, BN);
       if (GROUPED) pdl_wait();
       const int tiles = m_pairs_of() * p.n_tiles;
-      int it = 0, local = 0;
-      for (int tile = pair; tile < tiles && !*failed; tile += pairs, ++local) {
+      const uint64_t a = smem_desc_sw128(smem_u32(smem)), b = a + (A_BYTES >> 4);  // of the first stage (a descriptor counts 16 bytes)
+      int s = 0, phase = 0, local = 0;
+      for (int tile = pair; tile < tiles && !__any_sync(0xffffffffu, *failed != 0); tile += pairs, ++local) {
         const int buf = local & 1;
-        if (local >= 2 && !mbar_wait(acc_empty0 + 8 * buf, ((local >> 1) - 1) & 1, p.wait_limit, failed)) {
+        if (local >= 2 && !__all_sync(0xffffffffu, mbar_wait(acc_empty0 + 8 * buf, ((local >> 1) - 1) & 1, p.wait_limit, failed))) {
           if (!*failed) { *failed = 2; atomicCAS(p.error_flag, 0, 2); }
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         bool ok = true;
-        for (int kt = 0; kt < p.k_tiles; ++kt, ++it) {
-          const int s = it % PAIR_STAGES;
-          if (!mbar_wait(full0 + 8 * s, (it / PAIR_STAGES) & 1, p.wait_limit, failed)) {
+        for (int kt = 0; kt < p.k_tiles; ++kt) {
+          if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, phase, p.wait_limit, failed))) {
             if (!*failed) { *failed = 3; atomicCAS(p.error_flag, 0, 3); }
             ok = false;
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a = smem_u32(smem + (size_t)s * PAIR_STAGE_BYTES);
+          const uint32_t at = s * (PAIR_STAGE_BYTES >> 4);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            umma_pair(tmem + buf * BN, smem_desc_sw128(a + k * 32), smem_desc_sw128(a + A_BYTES + k * 32), idesc, (kt | k) != 0);
-          umma_commit_pair(empty0 + 8 * s);  // arrives in both CTAs once these products have read the stage
+          for (int k = 0; k < BK / 16; ++k) umma_pair(one, tmem + buf * BN, a + (at + 2 * k), b + (at + 2 * k), idesc, (kt | k) != 0);
+          umma_commit_pair(one, empty0 + 8 * s);  // arrives in both CTAs once these products have read the stage
+          if (++s == PAIR_STAGES) s = 0, phase ^= 1;
         }
         if (!ok) break;
-        umma_commit_pair(acc_full0 + 8 * buf);  // arrives in both CTAs once every product of the tile has finished
+        umma_commit_pair(one, acc_full0 + 8 * buf);  // arrives in both CTAs once every product of the tile has finished
       }
     }
     __syncwarp();
