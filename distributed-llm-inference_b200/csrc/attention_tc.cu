@@ -87,6 +87,19 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t b
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// Products are issued by one lane of a warp that runs together, so that descriptors stay in uniform registers.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one;
+}
+__device__ __forceinline__ void umma_one(uint32_t one, uint32_t sum, uint64_t a, uint64_t b, uint32_t idesc, bool add) {
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %5, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+               ::"r"(sum), "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)add), "r"(one) : "memory");
+}
+__device__ __forceinline__ void umma_commit_one(uint32_t one, uint32_t bar) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(one) : "memory");
+}
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -673,15 +686,16 @@ __global__ void __launch_bounds__(T2Cfg<HD, HV>::THREADS, 1) paged_prefill_tc2_k
       }
     }
   } else if (warp == QT * ROWS / 32 || (QT == 2 && warp == QT * ROWS / 32 + 2)) {
-    // ================================================================ the warps that issue the matrix products (their first lanes):
-    // one per query tile.  A single thread that served both tiles spent its time on issuing and became what every
+    // ================================================================ the warps that issue the matrix products (one lane, the warp together: 2,048 tokens of 32 heads
+    // 40.4 us by a lane in a branch of its own, 38.0 so): one per query tile.  A single thread that served both tiles spent its time on issuing and became what every
     // softmax group waited for.  A tile's products become possible in a fixed order, S(t + 1) (its threads have S(t) in
     // registers) before O += P(t) V(t) (the same threads have written P(t)), so the thread waits for each in turn and
     // sleeps in the barrier meanwhile: a polling loop takes issue slots from the softmax warps of its scheduler.  A stage
     // of keys or values is handed back to the copies when both threads have committed their products with it (those
     // barriers count QT arrivals).
     const int q = warp == QT * ROWS / 32 ? 0 : 1;  // this thread's query tile
-    if (lane == 0) {
+    {
+      const uint32_t one = elect_one();
       const uint32_t idesc_s = instr_desc(ROWS, KEYS, 0), idesc_o = instr_desc(ROWS, 64, 1);
       const int k_steps = (p.d + 15) >> 4;  // (the columns of a last half step are zeros)
       const uint32_t qa = smem_u32(sQ + q * K_BYTES), pa = smem_u32(sP + q * 2 * TILE_BYTES);
@@ -690,20 +704,22 @@ __global__ void __launch_bounds__(T2Cfg<HD, HV>::THREADS, 1) paged_prefill_tc2_k
         const uint32_t k = smem_u32(sK + (t & 1) * K_BYTES);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          if (kk < k_steps) umma(tmem_s + q * KEYS, smem_desc_sw128(qa + (kk >> 2) * TILE_BYTES + (kk & 3) * 32), smem_desc_sw128(k + (kk >> 2) * TILE_BYTES + (kk & 3) * 32), idesc_s, kk != 0);
-        umma_commit(s_done + 8 * q);
-        umma_commit(k_free + 8 * (t & 1));  // this tile's product with K(t) is issued
+          if (kk < k_steps) umma_one(one, tmem_s + q * KEYS, smem_desc_sw128(qa + (kk >> 2) * TILE_BYTES + (kk & 3) * 32), smem_desc_sw128(k + (kk >> 2) * TILE_BYTES + (kk & 3) * 32), idesc_s, kk != 0);
+        umma_commit_one(one, s_done + 8 * q);
+        umma_commit_one(one, k_free + 8 * (t & 1));  // this tile's product with K(t) is issued
       };
-      bool ok = num_tiles > 0 && wait_or_fail(k_full, 0, failed, 17, p.error_flag);
+      bool ok = num_tiles > 0 && __all_sync(0xffffffffu, wait_or_fail(k_full, 0, failed, 17, p.error_flag));
       if (ok) scores(0);
       for (int t = 0; t < num_tiles && ok; ++t) {
         if (t + 1 < num_tiles) {  // the keys are there and the thread of every row has S_q(t) in registers
           ok = wait_or_fail(k_full + 8 * ((t + 1) & 1), ((t + 1) >> 1) & 1, failed, 17, p.error_flag) && wait_or_fail(s_read + 8 * q, t & 1, failed, 18, p.error_flag);
+          ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           scores(t + 1);
         }
         // O_q += P_q(t) V(t)
         ok = wait_or_fail(p_ready + 8 * q, t & 1, failed, 19, p.error_flag) && wait_or_fail(v_full + 8 * (t & 1), (t >> 1) & 1, failed, 20, p.error_flag);
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t v = smem_u32(sV + (t & 1) * V_BYTES);
@@ -711,9 +727,9 @@ __global__ void __launch_bounds__(T2Cfg<HD, HV>::THREADS, 1) paged_prefill_tc2_k
         for (int sl = 0; sl < VSLABS; ++sl)  // 64 output columns at a time: the values' slab is the MN-major operand
 #pragma unroll
           for (int k = 0; k < KEYS / 16; ++k)
-            umma(tmem_o + q * HV + sl * 64, smem_desc_sw128(pa + (k >> 2) * TILE_BYTES + (k & 3) * 32), smem_desc_sw128(v + sl * TILE_BYTES + k * 2048), idesc_o, (t | k) != 0);
-        umma_commit(o_done + 8 * q);
-        umma_commit(v_free + 8 * (t & 1));  // this tile's product with V(t) is issued
+            umma_one(one, tmem_o + q * HV + sl * 64, smem_desc_sw128(pa + (k >> 2) * TILE_BYTES + (k & 3) * 32), smem_desc_sw128(v + sl * TILE_BYTES + k * 2048), idesc_o, (t | k) != 0);
+        umma_commit_one(one, o_done + 8 * q);
+        umma_commit_one(one, v_free + 8 * (t & 1));  // this tile's product with V(t) is issued
       }
     }
     __syncwarp();
@@ -1028,9 +1044,10 @@ __global__ void __launch_bounds__(DIFF_THREADS, 1) paged_prefill_diff_kernel(con
     if (*failed && lane == 0)
       for (int t = max(0, asked - 2); t < asked; ++t) wait_for_last(full + 8 * (t & 1), (t >> 1) & 1);
   } else if (warp == QT * ROWS / 32 || warp == QT * ROWS / 32 + 2) {
-    // ================================================================ the warps that issue the matrix products (their first lanes): one per map
+    // ================================================================ the warps that issue the matrix products (one lane, the warp together): one per map
     const int q = warp == QT * ROWS / 32 ? 0 : 1;
-    if (lane == 0) {
+    {
+      const uint32_t one = elect_one();
       const uint32_t idesc_s = instr_desc(ROWS, KEYS, 0), idesc_o = instr_desc(ROWS, HV, 1);
       const uint64_t next_slab = (uint64_t)(TILE_BYTES >> 4) << 16;  // of the MN-major operand: bytes from 64 columns to the next 64
       const uint32_t qa = smem_u32(sQ + q * TILE_BYTES), pa = smem_u32(sP + q * 2 * TILE_BYTES);
@@ -1039,30 +1056,32 @@ __global__ void __launch_bounds__(DIFF_THREADS, 1) paged_prefill_diff_kernel(con
         const uint32_t k = smem_u32(sK + (t & 1) * K_BYTES + q * TILE_BYTES);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          umma(tmem_s + q * KEYS, smem_desc_sw128(qa + kk * 32), smem_desc_sw128(k + kk * 32), idesc_s, kk != 0);
-        umma_commit(s_done + 8 * q);
-        umma_commit(k_free + 8 * (t & 1));  // this tile's product with K(t) is issued
+          umma_one(one, tmem_s + q * KEYS, smem_desc_sw128(qa + kk * 32), smem_desc_sw128(k + kk * 32), idesc_s, kk != 0);
+        umma_commit_one(one, s_done + 8 * q);
+        umma_commit_one(one, k_free + 8 * (t & 1));  // this tile's product with K(t) is issued
       };
-      bool ok = num_tiles > 0 && wait_or_fail(k_full, 0, failed, 17, p.error_flag);
+      bool ok = num_tiles > 0 && __all_sync(0xffffffffu, wait_or_fail(k_full, 0, failed, 17, p.error_flag));
       int scored = 0, summed = 0;  // tiles whose products were issued
       if (ok) { scores(0); ++scored; }
       for (int t = 0; t < num_tiles && ok; ++t) {
         if (t + 1 < num_tiles) {  // the keys are there and the thread of every row has S_q(t) in registers
           ok = wait_or_fail(k_full + 8 * ((t + 1) & 1), ((t + 1) >> 1) & 1, failed, 17, p.error_flag) && wait_or_fail(s_read + 8 * q, t & 1, failed, 18, p.error_flag);
+          ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           scores(t + 1);
           ++scored;
         }
         // O_q += P_q(t) V(t)
         ok = wait_or_fail(p_ready + 8 * q, t & 1, failed, 19, p.error_flag) && wait_or_fail(v_full + 8 * (t & 1), (t >> 1) & 1, failed, 20, p.error_flag);
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t v = smem_u32(sV + (t & 1) * V_BYTES);
 #pragma unroll
         for (int k = 0; k < KEYS / 16; ++k)
-          umma(tmem_o + q * HV, smem_desc_sw128(pa + (k >> 2) * TILE_BYTES + (k & 3) * 32), smem_desc_sw128(v + k * 2048) | next_slab, idesc_o, (t | k) != 0);
-        umma_commit(o_done + 8 * q);
-        umma_commit(v_free + 8 * (t & 1));  // this tile's product with V(t) is issued
+          umma_one(one, tmem_o + q * HV, smem_desc_sw128(pa + (k >> 2) * TILE_BYTES + (k & 3) * 32), smem_desc_sw128(v + k * 2048) | next_slab, idesc_o, (t | k) != 0);
+        umma_commit_one(one, o_done + 8 * q);
+        umma_commit_one(one, v_free + 8 * (t & 1));  // this tile's product with V(t) is issued
         ++summed;
       }
       if (!ok) {
@@ -1353,18 +1372,9 @@ template <int SLABS> struct RowCfg {
   static_assert(SMEM <= 227 * 1024 && 2 * STAGE == SLABS * TILE_BYTES, "one CTA fits an SM, Q two stages");
 };
 
-// Products are issued by one lane of a warp that runs together, so that descriptors stay in uniform registers.
-__device__ __forceinline__ uint32_t elect_one() {
-  uint32_t one;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
-  return one;
-}
 __device__ __forceinline__ void umma_tmem(uint32_t one, uint32_t sum, uint32_t a, uint64_t b, uint32_t idesc, bool add) {  // A in tensor memory
   asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %5, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
                ::"r"(sum), "r"(a), "l"(b), "r"(idesc), "r"((uint32_t)add), "r"(one) : "memory");
-}
-__device__ __forceinline__ void umma_commit_one(uint32_t one, uint32_t bar) {
-  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(one) : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
