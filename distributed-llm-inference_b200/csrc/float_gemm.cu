@@ -103,9 +103,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
                  "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
                : "r"(addr));
 }
-__device__ __forceinline__ float4 load4(const float* p, bool in) {  // (pinned: the loads of a step stay in front of the wait that hides them)
+// (Pinned: the loads of a step stay in front of the wait that hides them.  Plain loads: .nc wants memory that nobody writes while the kernel runs, but with a
+// programmatic launch the kernel in front, which writes x, may still run when this one starts, and the wait for it orders ordinary loads only.)
+__device__ __forceinline__ float4 load4(const float* p, bool in) {
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (in) asm volatile("ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  if (in) asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ float plain_dot(const float* a, const float* b, int K) {

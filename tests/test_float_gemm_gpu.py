@@ -1,8 +1,11 @@
 """The float32 product on the tensor cores (csrc/float_gemm.cu) against float64, at the edges of its tiles, steps and splits."""
 
+from pathlib import Path
+
 import pytest
 import torch
 
+from dli_b200.csrc import build
 from dli_b200.kernels import gemm, ops
 
 
@@ -45,3 +48,10 @@ def test_numbers_that_are_not_finite_stay_in_their_row_and_column(value, tile, s
     rest[5], rest[:, 133] = False, False
     assert _error(got[rest], want.double()[rest]) <= 5e-7
     assert (got.isnan() == want.isnan()).all() and (got.isinf() == want.isinf()).all() and (got[want.isinf()] == want[want.isinf()]).all()
+
+
+def test_no_kernel_loads_by_the_non_coherent_path():
+    """Kernels start while the one in front still runs (programmatic launches), and its end orders ordinary loads only."""
+    sources = sorted(p for p in Path(build.__file__).parent.iterdir() if p.suffix in (".cu", ".cuh", ".h"))
+    assert len(sources) > 20
+    assert [p.name for p in sources if "ld.global.nc" in p.read_text() or "__ldg(" in p.read_text()] == []
