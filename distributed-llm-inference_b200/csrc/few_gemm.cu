@@ -15,7 +15,8 @@
 // and the end, about 3 us (1 to 2 more at 64 tokens).  Figures against the library's products stand beside the rule (kernels/gemm.py).  Before a copy
 // brought 128 k, K 8,192 on sixteen SMs took 27 us instead of 18.
 //
-// Every wait on an mbarrier is bounded: after WAIT_LIMIT polls a code goes to *error_flag, nothing more is issued or stored, and the CTA ends when its copies have landed.
+// Every wait on an mbarrier is bounded: after `wait_limit` polls a code goes to *error_flag, no CTA of the cluster stores anything (the others hear of it in front of
+// the barrier behind which sums are added), and the CTA ends when its copies have landed.
 #include "umma_tiles.cuh"
 #include <type_traits>
 
@@ -35,6 +36,8 @@ struct FewParams {
   int tokens, features, K, splits, mode;
   int wide;  // K is a multiple of 128: one copy brings both slabs
   int* error_flag;
+  unsigned wait_limit;
+  int skip_step;  // -1 in every launch of the engine: the step whose copies of x a test leaves out (dli_few_gemm_wait_test)
 };
 
 template <int NT> struct Shape {  // NT: room for tokens
@@ -77,10 +80,10 @@ __global__ void __launch_bounds__(THREADS, 1) few_gemm_kernel(const __grid_const
   const uint32_t tmem = *tmem_slot;
   const int f0 = blockIdx.x * BF, split = blockIdx.y, all = (p.K + BK - 1) / BK, share = (all + p.splits - 1) / p.splits;
   const int first = min(all, split * share), steps = min(all, first + share) - first;  // (a last split may be empty)
+  unsigned left = p.wait_limit;
 
   if (warp == 0) {
     const uint32_t one = elect_one();
-    unsigned left = WAIT_LIMIT;
     const int ahead = min(steps, Z::STAGES);
     auto load = [&](uint32_t dst, const CUtensorMap* map, int step, int row, int slab, uint32_t bar) {
       if (p.wide) {
@@ -100,7 +103,8 @@ __global__ void __launch_bounds__(THREADS, 1) few_gemm_kernel(const __grid_const
     __syncwarp();
     pdl_wait();
     if (one)
-      for (int s = 0; s < ahead; ++s) load(sm + s * Z::STAGE + Z::B, &map_x, first + s, 0, Z::B_SLAB, full0 + 8 * s);
+      for (int s = 0; s < ahead; ++s)
+        if (first + s != p.skip_step) load(sm + s * Z::STAGE + Z::B, &map_x, first + s, 0, Z::B_SLAB, full0 + 8 * s);
     __syncwarp();
     int asked = ahead;
     for (int s = ahead; s < steps; ++s) {
@@ -117,11 +121,10 @@ __global__ void __launch_bounds__(THREADS, 1) few_gemm_kernel(const __grid_const
     }
     if (*failed)  // what is still on its way lands here, not in the next CTA's shared memory
       for (int s = max(0, asked - Z::STAGES); s < asked; ++s)
-        for (unsigned i = 0; i < WAIT_LIMIT && !bar_done(full0 + 8 * (s % Z::STAGES), (s / Z::STAGES) & 1); ++i) {}
+        for (unsigned i = 0; i < p.wait_limit && !bar_done(full0 + 8 * (s % Z::STAGES), (s / Z::STAGES) & 1); ++i) {}
   } else if (warp == 1) {
     const uint32_t one = elect_one(), tm = __shfl_sync(0xffffffffu, tmem, 0), idesc = instruction((p.tokens + 15) / 16 * 16, false, false);
     const uint64_t stages = operand(sm);  // (a descriptor counts 16 bytes)
-    unsigned left = WAIT_LIMIT;
     for (int s = 0; s < steps; ++s) {
       const int stage = s % Z::STAGES;
       bar_wait(full0 + 8 * stage, (s / Z::STAGES) & 1, left, failed, p.error_flag, 2);
@@ -137,7 +140,6 @@ __global__ void __launch_bounds__(THREADS, 1) few_gemm_kernel(const __grid_const
     __syncwarp();
   } else {
     // ---- the sums to shared memory: lane = feature, column = token
-    unsigned left = WAIT_LIMIT;
     bar_wait(done, 0, left, failed, p.error_flag, 3);
     tmem_after();
     const int quad = warp & 3;
@@ -156,6 +158,9 @@ __global__ void __launch_bounds__(THREADS, 1) few_gemm_kernel(const __grid_const
     }
     tmem_before();
   }
+  if (left == 1 && lane < p.splits)  // a wait of this warp ran out: every CTA of the cluster would add what is not there
+    asm volatile("{\n\t.reg .b32 remote;\n\tmapa.shared::cluster.u32 remote, %0, %1;\n\tst.shared::cluster.u32 [remote], %2;\n\t}"
+                 ::"r"(smem_u32(tmem_slot + 1)), "r"(lane), "r"(*failed) : "memory");
   if (p.splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   else __syncthreads();
   pdl_wait();  // (every thread that writes: the output may alias memory that the kernel in front still reads)
@@ -250,9 +255,8 @@ template <int NT> int launch(const CUtensorMap& map_x, const CUtensorMap& map_w,
 
 }  // namespace
 
-// out [tokens][features], or (swiglu) [tokens][features / 2] = silu(gate) * up for weights whose rows are interleaved in blocks of 64 gate rows and the 64 up
-// rows of the same features.  x: rows x_row numbers apart.  splits (1, 2, 4 or 8): CTAs that share a tile's k.
-DLI_EXPORT int dli_few_gemm(void* out, const void* x, const void* w, int tokens, int features, int K, long long x_row, int swiglu, int splits, cudaStream_t stream) {
+static int run(void* out, const void* x, const void* w, int tokens, int features, int K, long long x_row, int swiglu, int splits, unsigned wait_limit, int skip_step,
+               cudaStream_t stream) {
   if (tokens < 1 || tokens > 256 || features < 4 || features % 4 || K < 8 || K % 8 || x_row % 8 || (((uintptr_t)x | (uintptr_t)w) & 15) || ((uintptr_t)out & 7) ||
       (swiglu && features % 128) || (splits != 1 && splits != 2 && splits != 4 && splits != 8))
     return DLI_ERR_UNSUPPORTED;
@@ -269,10 +273,27 @@ DLI_EXPORT int dli_few_gemm(void* out, const void* x, const void* w, int tokens,
   if (!made) return DLI_ERR_UNSUPPORTED;
   FewParams p;
   p.out = (bf16*)out; p.tokens = tokens; p.features = features; p.K = K; p.splits = splits; p.mode = swiglu ? SWIGLU : STORE; p.wide = wide; p.error_flag = error_flag_device;
+  p.wait_limit = wait_limit; p.skip_step = skip_step;
   if (room == 16) return launch<16>(map_x, map_w, p, stream);
   if (room == 32) return launch<32>(map_x, map_w, p, stream);
   if (room == 64) return launch<64>(map_x, map_w, p, stream);
   return room == 128 ? launch<128>(map_x, map_w, p, stream) : launch<256>(map_x, map_w, p, stream);
+}
+
+// out [tokens][features], or (swiglu) [tokens][features / 2] = silu(gate) * up for weights whose rows are interleaved in blocks of 64 gate rows and the 64 up
+// rows of the same features.  x: rows x_row numbers apart.  splits (1, 2, 4 or 8): CTAs that share a tile's k.
+DLI_EXPORT int dli_few_gemm(void* out, const void* x, const void* w, int tokens, int features, int K, long long x_row, int swiglu, int splits, cudaStream_t stream) {
+  return run(out, x, w, tokens, features, K, x_row, swiglu, splits, WAIT_LIMIT, -1, stream);
+}
+
+// For tests: the copies of x of step `skip_step` (of 128 k) are left out and every wait gives up after `wait_limit` polls: the wait for that step runs out (code 2), and
+// the one for the sums that depend on it (3).  Every step has a stage of its own.
+DLI_EXPORT int dli_few_gemm_wait_test(void* out, const void* x, const void* w, int tokens, int features, int K, int splits, unsigned wait_limit, int skip_step,
+                                      cudaStream_t stream) {
+  const int steps = (K + BK - 1) / BK;
+  if (wait_limit < 2 || wait_limit > WAIT_LIMIT || tokens > 32 || splits < 1 || (steps + splits - 1) / splits > Shape<32>::STAGES || skip_step < 0 || skip_step >= steps)
+    return DLI_ERR_UNSUPPORTED;
+  return run(out, x, w, tokens, features, K, K, 0, splits, wait_limit, skip_step, stream);
 }
 
 // 0, or the code of the first wait that ran out (1 stages, 2 copies, 3 sums)

@@ -29,7 +29,8 @@
 // 127; 10,304 features, K 2,048 77 / 156 / 420 -> 48 / 74 / 194.  Errors against 64 bits 0.7e-7 to 1.5e-7 of the result (the library 0.9e-7 to 1.6e-6, larger at each of
 // these sizes; with 256 k in one accumulator 2.4e-7).
 //
-// Every wait is bounded: after `wait_limit` polls a code goes to *error_flag and the CTA ends early; it has no copies in flight.
+// Every wait is bounded: after `wait_limit` polls a code goes to *error_flag and the CTA ends early (it has no copies in flight).  A warp stores only sums that it has seen
+// finished; in a cluster none of the CTAs stores anything (the others hear of it in front of the barrier behind which sums are added).
 #include "common.cuh"
 #include "mma_split.cuh"
 
@@ -51,6 +52,7 @@ struct FloatParams {
   int tokens, features, K, splits, token_tiles;
   int* error_flag;
   unsigned wait_limit;
+  int skip_step;  // -1 in every launch of the engine: the step whose terms a test does not hand in (dli_float_gemm_wait_test)
 };
 
 template <int NT> struct Shape {  // NT: tokens of a tile
@@ -157,13 +159,13 @@ __global__ void __launch_bounds__(THREADS, 1) float_gemm_kernel(const __grid_con
   const float* x = p.x + batch * p.x_batch;
   const float* w = p.w + batch * p.w_batch;
   float* out = p.out + batch * p.out_batch;
+  bool ok = true;
   pdl_wait();
 
   if (warp == CONVERTERS / 32) {
     // ---- products
     const uint32_t one = elect_one(), tm = __shfl_sync(0xffffffffu, tmem, 0), small = tm + Z::SMALL;
     const uint64_t stages = operand(smem_u32(smem));  // (a descriptor counts 16 bytes)
-    bool ok = true;
     auto wait = [&](uint32_t bar, uint32_t parity, int code) { ok = __all_sync(0xffffffffu, ok && bar_wait(bar, parity, p, failed, code)); };
     for (int s = 0; s < steps; ++s) {
       const int stage = s % Z::STAGES, chunk = s / Z::CHUNK, buf = chunk % Z::LARGE;
@@ -218,7 +220,6 @@ __global__ void __launch_bounds__(THREADS, 1) float_gemm_kernel(const __grid_con
         for (int e = 0; e < 16; ++e) acc[j + e] += __uint_as_float(v[e]);
       }
     };
-    bool ok = true;
     auto take_chunk = [&](int chunk) {
       const int buf = chunk % Z::LARGE;
       ok = __all_sync(0xffffffffu, ok && bar_wait(sum_full0 + 8 * buf, (chunk / Z::LARGE) & 1, p, failed, 3));
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(THREADS, 1) float_gemm_kernel(const __grid_con
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // (in front of the loads: it waits for those under way)
       __syncwarp();
-      if (lane == 0) bar_arrive(full0 + 8 * stage);
+      if (lane == 0 && first + s != p.skip_step) bar_arrive(full0 + 8 * stage);
       if (s + Z::AHEAD < steps) fetch(first + s + Z::AHEAD, lo, hi);
     };
 #pragma unroll
@@ -300,6 +301,9 @@ __global__ void __launch_bounds__(THREADS, 1) float_gemm_kernel(const __grid_con
       for (int j = 0; j < NT / 2; ++j) part[j * BF] = acc[j];
     }
   }
+  if (!ok && p.splits > 1 && lane < p.splits)
+    asm volatile("{\n\t.reg .b32 remote;\n\tmapa.shared::cluster.u32 remote, %0, %1;\n\tst.shared::cluster.u32 [remote], %2;\n\t}"
+                 ::"r"(smem_u32(tmem_slot + 1)), "r"(lane), "r"(*failed) : "memory");
   __syncthreads();
   if (p.splits > 1) {
     // ---- every CTA of the cluster adds all sums of its share of the tile's tokens
@@ -377,9 +381,8 @@ void choose(int tokens, int features, int batches, int steps, int& tile, int& sp
 
 }  // namespace
 
-// tile: tokens of a tile (32, 64 or 128), splits: CTAs that share a tile's k (1, 2, 4 or 8); 0 and 0: chosen here.
-DLI_EXPORT int dli_float_gemm(float* out, const float* x, const float* w, int batches, int tokens, int features, int K, long long x_row, long long w_row,
-                              long long out_row, long long x_batch, long long w_batch, long long out_batch, int tile, int splits, cudaStream_t stream) {
+static int run(float* out, const float* x, const float* w, int batches, int tokens, int features, int K, long long x_row, long long w_row, long long out_row,
+               long long x_batch, long long w_batch, long long out_batch, int tile, int splits, unsigned wait_limit, int skip_step, cudaStream_t stream) {
   if (batches == 0 || tokens == 0 || features == 0) return 0;
   if (batches < 0 || tokens < 0 || features < 0 || K < 4 || K % 4 || x_row % 4 || w_row % 4 || x_batch % 4 || w_batch % 4 || (((uintptr_t)x | (uintptr_t)w) & 15) ||
       (tile != 0 && tile != 32 && tile != 64 && tile != 128) || (splits != 0 && splits != 1 && splits != 2 && splits != 4 && splits != 8))
@@ -393,10 +396,24 @@ DLI_EXPORT int dli_float_gemm(float* out, const float* x, const float* w, int ba
   FloatParams p;
   p.x = x; p.w = w; p.out = out; p.x_row = x_row; p.w_row = w_row; p.out_row = out_row; p.x_batch = x_batch; p.w_batch = w_batch; p.out_batch = out_batch;
   p.tokens = tokens; p.features = features; p.K = K; p.splits = splits; p.token_tiles = (tokens + tile - 1) / tile;
-  p.error_flag = error_flag_device; p.wait_limit = WAIT_LIMIT;
+  p.error_flag = error_flag_device; p.wait_limit = wait_limit; p.skip_step = skip_step;
   if ((long long)p.token_tiles * batches > 65535) return DLI_ERR_UNSUPPORTED;
   if (tile == 32) return launch<32>(p, batches, stream);
   return tile == 64 ? launch<64>(p, batches, stream) : launch<128>(p, batches, stream);
+}
+
+// tile: tokens of a tile (32, 64 or 128), splits: CTAs that share a tile's k (1, 2, 4 or 8); 0 and 0: chosen here.
+DLI_EXPORT int dli_float_gemm(float* out, const float* x, const float* w, int batches, int tokens, int features, int K, long long x_row, long long w_row,
+                              long long out_row, long long x_batch, long long w_batch, long long out_batch, int tile, int splits, cudaStream_t stream) {
+  return run(out, x, w, batches, tokens, features, K, x_row, w_row, out_row, x_batch, w_batch, out_batch, tile, splits, WAIT_LIMIT, -1, stream);
+}
+
+// For tests: the terms of step `skip_step` (of 64 k) are never handed in and every wait gives up after `wait_limit` polls: the products' wait for them runs out (code 2),
+// and those for sums and stages that depend on it (3, 4).
+DLI_EXPORT int dli_float_gemm_wait_test(float* out, const float* x, const float* w, int tokens, int features, int K, int tile, int splits, unsigned wait_limit, int skip_step,
+                                        cudaStream_t stream) {
+  if (wait_limit < 1 || wait_limit > WAIT_LIMIT || tile == 0 || splits == 0 || skip_step < 0 || skip_step >= (K + BK - 1) / BK) return DLI_ERR_UNSUPPORTED;
+  return run(out, x, w, 1, tokens, features, K, K, K, features, 0, 0, 0, tile, splits, wait_limit, skip_step, stream);
 }
 
 // 0, or the code of the first wait that ran out (1 accumulators, 2 terms, 3 sums, 4 stages)

@@ -1008,6 +1008,13 @@ def few_gemm(x: torch.Tensor, weight: torch.Tensor, splits: int, swiglu: bool = 
     return out
 
 
+def few_gemm_wait_test(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, splits: int, wait_limit: int, skip_step: int) -> None:
+    """For tests: ``few_gemm`` into ``out``, with the copies of x of step ``skip_step`` (128 columns of K) left out and every wait given up after
+    ``wait_limit`` polls.  The kernel records a code, stores nothing and returns."""
+    f = _fn("few_gemm.cu", "dli_few_gemm_wait_test", [c_void_p] * 3 + [c_int] * 4 + [ctypes.c_uint, c_int, c_void_p])
+    _check(f(_ptr(out), _ptr(x), _ptr(weight), x.shape[0], weight.shape[0], x.shape[1], splits, wait_limit, skip_step, _stream()), "few_gemm_wait_test")
+
+
 # ------------------------------------------------------------------ float32 products on the tensor cores
 
 
@@ -1039,6 +1046,13 @@ def float_gemm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None =
     _check(f(_ptr(out), _ptr(x), _ptr(weight), batches, x.shape[-2], weight.shape[-2], x.shape[-1], x.stride(-2), weight.stride(-2), out.stride(-2),
              *between, tile, splits, _stream()), "float_gemm")
     return out
+
+
+def float_gemm_wait_test(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, tile: int, splits: int, wait_limit: int, skip_step: int) -> None:
+    """For tests: ``float_gemm`` of contiguous operands into ``out``, with the terms of step ``skip_step`` (64 columns of K) never handed in and every wait
+    given up after ``wait_limit`` polls.  The kernel records a code and returns; a cluster stores nothing."""
+    f = _fn("float_gemm.cu", "dli_float_gemm_wait_test", [c_void_p] * 3 + [c_int] * 5 + [ctypes.c_uint, c_int, c_void_p])
+    _check(f(_ptr(out), _ptr(x), _ptr(weight), x.shape[0], weight.shape[0], x.shape[1], tile, splits, wait_limit, skip_step, _stream()), "float_gemm_wait_test")
 
 
 # ------------------------------------------------------------------ layer norm around the residual stream

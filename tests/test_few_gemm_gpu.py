@@ -35,6 +35,23 @@ def test_the_activation_of_a_gated_feed_forward(tokens, I, K, splits):
     assert _error(ops.few_gemm(x, w, splits, swiglu=True), want) <= 2.0**-8
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("splits,skip", [(1, 2), (2, 5), (2, 0), (4, 7)])
+def test_a_wait_that_runs_out(splits, skip):
+    """One CTA of each cluster misses a step's copies: none of the cluster's CTAs stores what it would add up, the code is read once, the next product is right."""
+    g = torch.Generator().manual_seed(skip)
+    K = 512 if splits == 1 else 1024
+    x, w = torch.randn(17, K, generator=g).bfloat16().cuda(), torch.randn(300, K, generator=g).bfloat16().cuda()
+    assert ops.device_wait_errors() == {}
+    out = torch.full((17, 300), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.few_gemm_wait_test(out, x, w, splits, wait_limit=4000, skip_step=skip)
+    torch.cuda.synchronize()  # returns: the kernel ended by itself
+    assert (out == 7).all()
+    assert ops.device_wait_errors()["few_gemm.cu"] in (2, 3) and ops.device_wait_errors() == {}
+    assert _error(ops.few_gemm(x, w, splits), x.double() @ w.double().t()) <= 2.0**-9
+    assert ops.device_wait_errors() == {}
+
+
 def test_which_products_go_there():
     def takes(tokens, features, K, dtype=torch.bfloat16, swiglu=False):
         return gemm.few_product(torch.empty(tokens, K, dtype=dtype), torch.empty(features, K, dtype=dtype), swiglu)

@@ -50,6 +50,22 @@ def test_numbers_that_are_not_finite_stay_in_their_row_and_column(value, tile, s
     assert (got.isnan() == want.isnan()).all() and (got.isinf() == want.isinf()).all() and (got[want.isinf()] == want[want.isinf()]).all()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("tile,splits,skip", [(32, 2, 7), (64, 4, 0), (128, 2, 3), (32, 1, 7)])
+def test_a_wait_that_runs_out(tile, splits, skip):
+    """One CTA of each cluster waits for terms that are never handed in: none of the cluster's CTAs stores what it would add up."""
+    g = torch.Generator().manual_seed(skip)
+    x, w = torch.randn(40, 512, generator=g).cuda(), torch.randn(140, 512, generator=g).cuda()
+    assert ops.device_wait_errors() == {}
+    out = torch.full((40, 140), 7.0, device="cuda")
+    ops.float_gemm_wait_test(out, x, w, tile, splits, wait_limit=4000, skip_step=skip)
+    torch.cuda.synchronize()  # returns: the kernel ended by itself
+    assert (out == 7).all()
+    assert ops.device_wait_errors()["float_gemm.cu"] in (1, 2, 3, 4) and ops.device_wait_errors() == {}
+    assert _error(ops.float_gemm(x, w, tile=tile, splits=splits), x.double() @ w.double().t()) <= 5e-7
+    assert ops.device_wait_errors() == {}
+
+
 def test_no_kernel_loads_by_the_non_coherent_path():
     """Kernels start while the one in front still runs (programmatic launches), and its end orders ordinary loads only."""
     sources = sorted(p for p in Path(build.__file__).parent.iterdir() if p.suffix in (".cu", ".cuh", ".h"))
