@@ -18,7 +18,8 @@
 // beside 300 109 -> 57.  A tile takes 6.1 us where n goes along, 4.4 elsewhere.  Errors against 64 bits (mean of six seeds, 200 tokens): o 2.9e-7, S 3.1e-7, o over its
 // divisor 3.9e-7 (before 5.4e-7, 5.7e-7 and 8.3e-7).
 //
-// Every wait is bounded: after WAIT_LIMIT polls a code goes to *error_flag, and the CTA goes on to its end without another wait and without storing anything.
+// Every wait is bounded: after `wait_limit` polls a code goes to *error_flag, and the CTA goes on to its end without another wait; from then on it stores no read-outs, and
+// states and maxima not at all.
 #include "matrix_memory.cuh"
 #include <math_constants.h>
 #include "umma_tiles.cuh"
@@ -54,6 +55,8 @@ struct Params {
   int short_shift;        // heads of a short sequence that a CTA walks, as a power of two (as in ssm_umma.cu)
   int o_vec;              // read-outs lie on 16-byte boundaries
   int* error_flag;
+  unsigned wait_limit;
+  int skip_tile;          // -1 in every launch of the engine: the tile of every CTA whose copies of q and k a test leaves out
 };
 
 // Per tile, floats: g_t and a_j in log2 units (two terms each) | exp(m0 - g_t) | exp(a_j - g_C) | exp(a_j - A) with A the largest a of the block of 32 | exp(-m_t) |
@@ -222,6 +225,7 @@ __global__ void __launch_bounds__(THREADS, 1) matrix_memory_umma_kernel(const __
   };
   float fin = 0.f;  // 0 while every result was finite, NaN from the first one on that was not
   float S[16], S0_n = 0.f;  // .. and of n (warps 0..3)
+  float m_end = 0.f, forgot_end = 0.f;  // (the warp of the tables) the maximum behind the last tile, the sum of the log forget gates
   const int quad = warp & 3, cg = (warp >> 2) & 3, row = quad * 32 + lane;  // this thread's row, and which sixteen columns
   auto each_state = [&](auto&& fn) {  // fn(number e of S, its offset in a [P][N] block) for those that exist
     if (row < N) {
@@ -237,7 +241,7 @@ __global__ void __launch_bounds__(THREADS, 1) matrix_memory_umma_kernel(const __
     // ---- products
     const uint32_t one = elect_one();
     const int k16 = N / 16;
-    unsigned left = WAIT_LIMIT;
+    unsigned left = p.wait_limit;
     auto wait = [&](uint32_t bar, uint32_t parity, int code) { bar_wait(bar, parity, left, failed, p.error_flag, code); };
     const uint64_t c_desc = operand(sm + Z::C), b_desc = operand(sm + Z::B), bt_desc = operand(sm + Z::B, SLAB), wx_desc = operand(sm + Z::WX), s0_desc = operand(sm + Z::S0),
                    x_desc = operand(sm + Z::X);  // (a descriptor counts 16 bytes)
@@ -303,7 +307,7 @@ __global__ void __launch_bounds__(THREADS, 1) matrix_memory_umma_kernel(const __
   } else if (warp == WARPS + 2) {
     // ---- copies
     const uint32_t one = elect_one();
-    unsigned left = WAIT_LIMIT;
+    unsigned left = p.wait_limit;
     auto wait = [&](uint32_t bar, uint32_t parity, int code) { bar_wait(bar, parity, left, failed, p.error_flag, code); };
     int xs = 0, cbs = 0;  // copies asked for
     for (int i = 0; i < tiles; ++i) {
@@ -318,11 +322,11 @@ __global__ void __launch_bounds__(THREADS, 1) matrix_memory_umma_kernel(const __
         wait(emit ? yb_done : d_done, (i - 1) & 1, 8);
         if (with_n) wait(qk_read, (i - 1) & 1, 17);
       }
-      if (left == 1) break;
+      if (left == 1 || *failed) break;
       if (one) {
         bar_expect(cb_full, (emit ? 2 : 1) * NB * SLAB);
 #pragma unroll
-        for (int b = 0; b < NB; ++b) {
+        for (int b = 0; b < NB && i != p.skip_tile; ++b) {
           tma_load(sm + Z::B + b * SLAB, &map, (p.heads + head) * N + b * 64, t0 + i * TOKENS, cb_full);
           if (emit) tma_load(sm + Z::C + b * SLAB, &map, head * N + b * 64, t0 + i * TOKENS, cb_full);
         }
@@ -330,14 +334,14 @@ __global__ void __launch_bounds__(THREADS, 1) matrix_memory_umma_kernel(const __
       ++cbs;
     }
     if (*failed) {  // what is still on its way lands here, not in the next CTA's shared memory
-      for (unsigned i = 0; cbs > 0 && i < WAIT_LIMIT && !bar_done(cb_full, (cbs - 1) & 1); ++i) {}
+      for (unsigned i = 0; cbs > 0 && i < p.wait_limit && !bar_done(cb_full, (cbs - 1) & 1); ++i) {}
       for (int b = 0; b < 2 && b < xs; ++b)
-        for (unsigned i = 0; i < WAIT_LIMIT && !bar_done(x_full + 8 * ((xs - 1 - b) & 1), ((xs - 1 - b) >> 1) & 1); ++i) {}
+        for (unsigned i = 0; i < p.wait_limit && !bar_done(x_full + 8 * ((xs - 1 - b) & 1), ((xs - 1 - b) >> 1) & 1); ++i) {}
     }
   } else if (warp == WARPS + 1) {
     // ---- tables: four tokens a lane
     const float bias_i = p.bias[head], bias_f = p.bias[p.heads + head];
-    unsigned left = WAIT_LIMIT;
+    unsigned left = p.wait_limit;
     double m0 = (double)start_top([](float, float, int) {}) * LOG2E, forgot = 0.0;  // (log2 units)
     float gi[4], gf[4];
     auto load_raw = [&](int base) {
@@ -414,17 +418,8 @@ __global__ void __launch_bounds__(THREADS, 1) matrix_memory_umma_kernel(const __
       __syncwarp();
       if (lane == 0) bar_arrive(tab_full + 8 * (i & 1));
     }
-    if (!*failed) {
-      const float m = (float)(m0 / LOG2E);
-      if (t1 == last) {  // a copy for each of this CTA's columns
-        for (int c = lane; c < COLS; c += 32)
-          if (col0 + c < P) slot_top[col0 + c] = m;
-        if (with_n && lane == 0) slot_top[P] = m;
-      } else if (!SECOND && lane == 0 && with_n) {
-        p.part_m[pbase(seg) * 2] = m;
-        p.part_m[pbase(seg) * 2 + 1] = (float)(forgot / LOG2E);
-      }
-    }
+    m_end = (float)(m0 / LOG2E);
+    forgot_end = (float)(forgot / LOG2E);
   } else {
     // ---- the sixteen warps
 #pragma unroll
@@ -442,7 +437,7 @@ __global__ void __launch_bounds__(THREADS, 1) matrix_memory_umma_kernel(const __
     }
     const float scale = 1.f / sqrtf((float)N);
     const uint32_t lanes = (uint32_t)(quad * 32) << 16;
-    unsigned left = WAIT_LIMIT;
+    unsigned left = p.wait_limit;
     auto wait = [&](uint32_t bar, uint32_t parity, int code) { bar_wait(bar, parity, left, failed, p.error_flag, code); };
     const bool storer = cg == 0;  // the warp of a quarter of the rows that asks for their way out
     // The weighted values of tile i, and the state at its start, in three terms (their readers of the tile before have ended: d_done, yb_done)
@@ -616,7 +611,7 @@ __global__ void __launch_bounds__(THREADS, 1) matrix_memory_umma_kernel(const __
           n_own = fmaf(lds(tab + Table::END * 4), n_own, (shares[4 * TOKENS + row] + shares[5 * TOKENS + row]) + (shares[6 * TOKENS + row] + shares[7 * TOKENS + row]));
           if (emit) {
             const float all = (shares[row] + shares[TOKENS + row]) + (shares[2 * TOKENS + row] + shares[3 * TOKENS + row]);
-            if (row < len && left > 1) {
+            if (row < len && left > 1 && !*failed) {
               fin = fmaf(all, 0.f, fin);
               p.divisor[(size_t)(base + row) * p.heads + head] = fmaxf(fabsf(all * scale), lds(tab + (Table::FLOOR + row) * 4)) + 1e-6f;
             }
@@ -671,7 +666,7 @@ __global__ void __launch_bounds__(THREADS, 1) matrix_memory_umma_kernel(const __
                       __float_as_uint(v[4 * e + 3]));
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("bar.sync %0, 128;" ::"r"(1 + quad) : "memory");
-        const bool whole = p.o_vec && quad * 32 + 32 <= len, ok = left > 1;  // 32 rows of this sequence
+        const bool whole = p.o_vec && quad * 32 + 32 <= len, ok = left > 1 && !*failed;  // 32 rows of this sequence
         if (ok && whole && storer) {
           if (lane < 2 && P - col0 >= 32 * (lane + 1))
             asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
@@ -716,6 +711,16 @@ __global__ void __launch_bounds__(THREADS, 1) matrix_memory_umma_kernel(const __
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T_ALL) : "memory");
   }
   if (*failed) return;
+  if (warp == WARPS + 1) {
+    if (t1 == last) {  // a copy for each of this CTA's columns (a second walk stores its own)
+      for (int c = lane; c < COLS; c += 32)
+        if (!again && col0 + c < P) slot_top[col0 + c] = m_end;
+      if (!again && with_n && lane == 0) slot_top[P] = m_end;
+    } else if (!SECOND && lane == 0 && with_n) {
+      p.part_m[pbase(seg) * 2] = m_end;
+      p.part_m[pbase(seg) * 2 + 1] = forgot_end;
+    }
+  }
   if (again) {
     int second = 0, end = 0;  // segments behind the first start again from the state behind it, the last one that was walked from the slot's
     if (SECOND) segment_tiles((last - first + TOKENS - 1) / TOKENS, p.segments, 1, second, end);
@@ -770,10 +775,9 @@ DLI_EXPORT int dli_matrix_memory_umma_segments(int num_seqs, int heads, int dv, 
   return fill < 2 ? 1 : (fill > 32 ? 33 : (int)fill + 1);
 }
 
-// n: rows of u.  segments > 1: part [num_seqs (segments - 1) heads (dv + 1) d] and part_m [num_seqs (segments - 1) heads 2] are scratch.
-DLI_EXPORT int dli_matrix_memory_umma(float* o, float* divisor, const void* u, long long u_stride, const float* gates, const float* bias, float cap, float* state,
-                                      float* top, const int* q_start, const int* state_slot, int num_seqs, int heads, int d, int dv, int n, int segments, float* part,
-                                      float* part_m, cudaStream_t stream) {
+static int run(float* o, float* divisor, const void* u, long long u_stride, const float* gates, const float* bias, float cap, float* state, float* top, const int* q_start,
+               const int* state_slot, int num_seqs, int heads, int d, int dv, int n, int segments, float* part, float* part_m, unsigned wait_limit, int skip_tile,
+               cudaStream_t stream) {
   if (num_seqs == 0 || n == 0) return 0;
   if (n < 0 || heads < 1 || heads > 65535 || d < 32 || d > 128 || d % 16 || dv < 8 || dv % 8 || segments < 1 || (long long)num_seqs * segments > 65535 || !(cap > 0.f) ||
       ((uintptr_t)u & 15) || u_stride % 8 || ((uintptr_t)o & 7) || (segments > 1 && (!part || !part_m)))
@@ -792,7 +796,23 @@ DLI_EXPORT int dli_matrix_memory_umma(float* o, float* divisor, const void* u, l
   p.o = o; p.divisor = divisor; p.u = (const bf16*)u; p.u_stride = u_stride; p.gates = gates; p.bias = bias; p.cap = cap; p.state = state; p.top = top;
   p.q_start = q_start; p.state_slot = state_slot; p.num_seqs = num_seqs; p.heads = heads; p.d = d; p.dv = dv; p.segments = segments; p.part = part;
   p.part_m = part_m; p.o_vec = o_vec; p.short_shift = short_shift((long long)column_blocks(dv) * heads * num_seqs); p.error_flag = error_flag_device;
+  p.wait_limit = wait_limit; p.skip_tile = skip_tile;
   return d <= 64 ? launch<1>(map, map_o, p, stream) : launch<2>(map, map_o, p, stream);
+}
+
+// n: rows of u.  segments > 1: part [num_seqs (segments - 1) heads (dv + 1) d] and part_m [num_seqs (segments - 1) heads 2] are scratch.
+DLI_EXPORT int dli_matrix_memory_umma(float* o, float* divisor, const void* u, long long u_stride, const float* gates, const float* bias, float cap, float* state,
+                                      float* top, const int* q_start, const int* state_slot, int num_seqs, int heads, int d, int dv, int n, int segments, float* part,
+                                      float* part_m, cudaStream_t stream) {
+  return run(o, divisor, u, u_stride, gates, bias, cap, state, top, q_start, state_slot, num_seqs, heads, d, dv, n, segments, part, part_m, WAIT_LIMIT, -1, stream);
+}
+
+// For tests: in one segment, with every CTA's copies of q and k of tile `skip_tile` left out and every wait given up after `wait_limit` polls.
+DLI_EXPORT int dli_matrix_memory_umma_wait_test(float* o, float* divisor, const void* u, long long u_stride, const float* gates, const float* bias, float cap, float* state,
+                                                float* top, const int* q_start, const int* state_slot, int num_seqs, int heads, int d, int dv, int n, unsigned wait_limit,
+                                                int skip_tile, cudaStream_t stream) {
+  if (wait_limit < 2 || wait_limit > WAIT_LIMIT || skip_tile < 0) return DLI_ERR_UNSUPPORTED;
+  return run(o, divisor, u, u_stride, gates, bias, cap, state, top, q_start, state_slot, num_seqs, heads, d, dv, n, 1, nullptr, nullptr, wait_limit, skip_tile, stream);
 }
 
 // 0, or the code of the first wait that ran out since the library was loaded or the code was last cleared

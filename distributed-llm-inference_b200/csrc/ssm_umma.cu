@@ -36,7 +36,8 @@
 // prompts of 666, 1,000 and 1,335 tokens 160 -> 73, one of 4,096 207 -> 108, of 600 48 -> 28, of 300 38 -> 19, of 33 10 -> 10; 128 heads, one of 2,048
 // 195 -> 80; 32 heads, N 64, prompts of 654, 981 and 1,310 67 -> 53.  The errors of y and S against 64 bits are smaller (1,500 tokens: 1.1e-7 and 7.8e-8, before 2.2e-7 and 1.9e-7).
 //
-// Every wait is bounded: after WAIT_LIMIT polls a code goes to *error_flag, and the CTA goes on to its end without another wait and without storing anything.
+// Every wait is bounded: after `wait_limit` polls a code goes to *error_flag, and the CTA goes on to its end without another wait; from then on it stores no read-outs, and
+// states not at all.
 #include "umma_tiles.cuh"
 
 using namespace dli;
@@ -71,6 +72,8 @@ struct Params {
   int short_shift;
   int y_vec;              // sixteen read-outs side by side lie on a 16-byte boundary
   int* error_flag;
+  unsigned wait_limit;
+  int skip_tile;          // -1 in every launch of the engine: the tile of every CTA whose copies of B and C a test leaves out
 };
 
 // Per tile, floats: l in log2 units (two terms) | dt | exp(l) | exp(l_last - l) dt | exp(l_e - l) dt with e the last token of the block of 32, and exp(l_last)
@@ -269,7 +272,7 @@ __global__ void __launch_bounds__(THREADS, 1) ssm_umma_kernel(const __grid_const
     // ---- products
     const uint32_t one = elect_one();
     const int k16 = N / 16;
-    unsigned left = WAIT_LIMIT;
+    unsigned left = p.wait_limit;
     auto wait = [&](uint32_t bar, uint32_t parity, int code) { bar_wait(bar, parity, left, failed, p.error_flag, code); };
     const uint64_t c_desc = operand(sm + Z::C), b_desc = operand(sm + Z::B), bt_desc = operand(sm + Z::B, SLAB), wx_desc = operand(sm + Z::WX), s0_desc = operand(sm + Z::S0),
                    x_desc = operand(sm + Z::X);  // (a descriptor counts 16 bytes)
@@ -335,7 +338,7 @@ __global__ void __launch_bounds__(THREADS, 1) ssm_umma_kernel(const __grid_const
   } else if (warp == WARPS + 2) {
     // ---- copies
     const uint32_t one = elect_one();
-    unsigned left = WAIT_LIMIT;
+    unsigned left = p.wait_limit;
     auto wait = [&](uint32_t bar, uint32_t parity, int code) { bar_wait(bar, parity, left, failed, p.error_flag, code); };
     int xs = 0, cbs = 0;  // copies asked for
     for (int i = 0; i < tiles; ++i) {
@@ -347,11 +350,11 @@ __global__ void __launch_bounds__(THREADS, 1) ssm_umma_kernel(const __grid_const
       }
       ++xs;
       if (i >= 1) wait(emit ? yb_done : d_done, (i - 1) & 1, 8);  // C and B have been read
-      if (left == 1) break;
+      if (left == 1 || *failed) break;
       if (one) {
         bar_expect(cb_full, (emit ? 2 : 1) * NB * SLAB);
 #pragma unroll
-        for (int b = 0; b < NB; ++b) {
+        for (int b = 0; b < NB && i != p.skip_tile; ++b) {
           tma_load(sm + Z::B + b * SLAB, &map, inner + g * N + b * 64, t0 + i * TOKENS, cb_full);
           if (emit) tma_load(sm + Z::C + b * SLAB, &map, inner + (p.groups + g) * N + b * 64, t0 + i * TOKENS, cb_full);
         }
@@ -359,14 +362,14 @@ __global__ void __launch_bounds__(THREADS, 1) ssm_umma_kernel(const __grid_const
       ++cbs;
     }
     if (*failed) {  // what is still on its way lands here, not in the next CTA's shared memory
-      for (unsigned i = 0; cbs > 0 && i < WAIT_LIMIT && !bar_done(cb_full, (cbs - 1) & 1); ++i) {}
+      for (unsigned i = 0; cbs > 0 && i < p.wait_limit && !bar_done(cb_full, (cbs - 1) & 1); ++i) {}
       for (int b = 0; b < 2 && b < xs; ++b)
-        for (unsigned i = 0; i < WAIT_LIMIT && !bar_done(x_full + 8 * ((xs - 1 - b) & 1), ((xs - 1 - b) >> 1) & 1); ++i) {}
+        for (unsigned i = 0; i < p.wait_limit && !bar_done(x_full + 8 * ((xs - 1 - b) & 1), ((xs - 1 - b) >> 1) & 1); ++i) {}
     }
   } else if (warp == WARPS + 1) {
     // ---- tables: four tokens a lane
     const float A = expf(p.A_log[head]), bias = p.dt_bias[head];
-    unsigned left = WAIT_LIMIT;
+    unsigned left = p.wait_limit;
     double total = 0.0;
     float raw[4];
     auto load_raw = [&](int base) {
@@ -433,7 +436,7 @@ __global__ void __launch_bounds__(THREADS, 1) ssm_umma_kernel(const __grid_const
     }
     const float Dh = p.D[head];
     const uint32_t lanes = (uint32_t)(quad * 32) << 16;
-    unsigned left = WAIT_LIMIT;
+    unsigned left = p.wait_limit;
     auto wait = [&](uint32_t bar, uint32_t parity, int code) { bar_wait(bar, parity, left, failed, p.error_flag, code); };
     const bool storer = cg == 0;  // the warp of a quarter of the rows that asks for their way out
     // The weighted values of tile i and the state at its start, in three terms (their readers of the tile before have ended: d_done).
@@ -608,7 +611,7 @@ __global__ void __launch_bounds__(THREADS, 1) ssm_umma_kernel(const __grid_const
                       __float_as_uint(v[4 * e + 3]));
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("bar.sync %0, 128;" ::"r"(1 + quad) : "memory");
-        const bool whole = p.y_vec && quad * 32 + 32 <= len, ok = left > 1;  // 32 rows of this sequence
+        const bool whole = p.y_vec && quad * 32 + 32 <= len, ok = left > 1 && !*failed;  // 32 rows of this sequence
         if (ok && whole && storer) {
           if (lane < 2 && P - col0 >= 32 * (lane + 1))
             asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
@@ -698,10 +701,9 @@ DLI_EXPORT int dli_ssm_umma_segments(int num_seqs, int heads, int P, int max_len
   return fill < 2 ? 1 : (fill > 32 ? 33 : (int)fill + 1);
 }
 
-// n: rows of xbc.  segments > 1: part [num_seqs (segments - 1) heads P N] and part_log [num_seqs (segments - 1) heads] are scratch.
-DLI_EXPORT int dli_ssm_umma(float* y, const void* xbc, const void* u, long long u_stride, int dt_col, const float* dt_bias, const float* A_log, const float* D,
-                            float* state, const int* q_start, const int* state_slot, int n, int num_seqs, int heads, int P, int N, int groups, int segments,
-                            float* part, float* part_log, cudaStream_t stream) {
+static int run(float* y, const void* xbc, const void* u, long long u_stride, int dt_col, const float* dt_bias, const float* A_log, const float* D, float* state,
+               const int* q_start, const int* state_slot, int n, int num_seqs, int heads, int P, int N, int groups, int segments, float* part, float* part_log,
+               unsigned wait_limit, int skip_tile, cudaStream_t stream) {
   if (num_seqs == 0 || n == 0) return 0;
   if (n < 0 || heads < 1 || heads > 65535 || groups < 1 || heads % groups || P < 8 || P % 8 || N < 32 || N % 16 || N > 128 || segments < 1 ||
       (long long)num_seqs * segments > 65535 || ((uintptr_t)xbc & 15) || ((uintptr_t)y & 7) || ((uintptr_t)state & 7) || (segments > 1 && (!part || !part_log)))
@@ -720,7 +722,23 @@ DLI_EXPORT int dli_ssm_umma(float* y, const void* xbc, const void* u, long long 
   p.y = y; p.xbc = (const bf16*)xbc; p.u = (const bf16*)u; p.u_stride = u_stride; p.dt_col = dt_col; p.dt_bias = dt_bias; p.A_log = A_log; p.D = D;
   p.state = state; p.q_start = q_start; p.state_slot = state_slot; p.num_seqs = num_seqs; p.heads = heads; p.P = P; p.N = N; p.groups = groups;
   p.segments = segments; p.part = part; p.part_log = part_log; p.y_vec = y_vec; p.short_shift = short_shift((long long)column_blocks(P) * heads * num_seqs); p.error_flag = error_flag_device;
+  p.wait_limit = wait_limit; p.skip_tile = skip_tile;
   return N <= 64 ? launch<1>(map, map_y, p, stream) : launch<2>(map, map_y, p, stream);
+}
+
+// n: rows of xbc.  segments > 1: part [num_seqs (segments - 1) heads P N] and part_log [num_seqs (segments - 1) heads] are scratch.
+DLI_EXPORT int dli_ssm_umma(float* y, const void* xbc, const void* u, long long u_stride, int dt_col, const float* dt_bias, const float* A_log, const float* D,
+                            float* state, const int* q_start, const int* state_slot, int n, int num_seqs, int heads, int P, int N, int groups, int segments,
+                            float* part, float* part_log, cudaStream_t stream) {
+  return run(y, xbc, u, u_stride, dt_col, dt_bias, A_log, D, state, q_start, state_slot, n, num_seqs, heads, P, N, groups, segments, part, part_log, WAIT_LIMIT, -1, stream);
+}
+
+// For tests: in one segment, with every CTA's copies of B and C of tile `skip_tile` left out and every wait given up after `wait_limit` polls.
+DLI_EXPORT int dli_ssm_umma_wait_test(float* y, const void* xbc, const void* u, long long u_stride, int dt_col, const float* dt_bias, const float* A_log, const float* D,
+                                      float* state, const int* q_start, const int* state_slot, int n, int num_seqs, int heads, int P, int N, int groups,
+                                      unsigned wait_limit, int skip_tile, cudaStream_t stream) {
+  if (wait_limit < 2 || wait_limit > WAIT_LIMIT || skip_tile < 0) return DLI_ERR_UNSUPPORTED;
+  return run(y, xbc, u, u_stride, dt_col, dt_bias, A_log, D, state, q_start, state_slot, n, num_seqs, heads, P, N, groups, 1, nullptr, nullptr, wait_limit, skip_tile, stream);
 }
 
 // 0, or the code of the first wait that ran out since the library was loaded or the code was last cleared

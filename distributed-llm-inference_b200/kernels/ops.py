@@ -1425,6 +1425,15 @@ def ssm_scan(y: torch.Tensor, xbc: torch.Tensor, u: torch.Tensor, dt_col: int, d
              _ptr(state_slot), state_slot.numel(), heads, P, N, groups, int(max_len), DT_CODE[u.dtype], _stream()), "ssm_scan")
 
 
+def ssm_umma_wait_test(y: torch.Tensor, xbc: torch.Tensor, u: torch.Tensor, dt_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
+                       state: torch.Tensor, q_start: torch.Tensor, state_slot: torch.Tensor, groups: int, wait_limit: int, skip_tile: int) -> None:
+    """For tests: ``ssm_scan`` in tiles of 128 tokens, with the copies of B and C of tile ``skip_tile`` left out and every wait given up after ``wait_limit`` polls."""
+    _, heads, P, N = state.shape
+    f = _fn("ssm_umma.cu", "dli_ssm_umma_wait_test", [c_void_p] * 3 + [c_longlong, c_int] + [c_void_p] * 6 + [c_int] * 6 + [ctypes.c_uint, c_int, c_void_p])
+    _check(f(_ptr(y), _ptr(xbc), _ptr(u), u.stride(0), dt_col, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(q_start), _ptr(state_slot), xbc.shape[0],
+             state_slot.numel(), heads, P, N, groups, wait_limit, skip_tile, _stream()), "ssm_umma_wait_test")
+
+
 def gated_group_rmsnorm(out: torch.Tensor, y: torch.Tensor, u: torch.Tensor, z_col: int, weight: torch.Tensor, parts: int, eps: float,
                         gate_after: bool = False, gate: str = "silu", divisor: torch.Tensor | None = None) -> None:
     """out = g / sqrt(mean(g^2) + eps) * weight with g = y * silu(z), the mean taken over each of ``parts`` equal runs
@@ -1971,6 +1980,16 @@ def channel_delta_scan(o: torch.Tensor, qkv: torch.Tensor, u: torch.Tensor, b_co
 
 
 # ------------------------------------------------------------------ matrix memory with exponential gates
+
+def matrix_memory_umma_wait_test(o: torch.Tensor, divisor: torch.Tensor, u: torch.Tensor, gates: torch.Tensor, gate_bias: torch.Tensor, cap: float, state: torch.Tensor,
+                                 top: torch.Tensor, q_start: torch.Tensor, state_slot: torch.Tensor, wait_limit: int, skip_tile: int) -> None:
+    """For tests: ``matrix_memory_scan`` in tiles of 128 tokens, with the copies of q and k of tile ``skip_tile`` left out and every wait given up after ``wait_limit`` polls."""
+    _, heads, dv1, d = state.shape
+    f = _fn("matrix_memory_umma.cu", "dli_matrix_memory_umma_wait_test",
+            [c_void_p] * 3 + [c_longlong, c_void_p, c_void_p, c_float] + [c_void_p] * 4 + [c_int] * 5 + [ctypes.c_uint, c_int, c_void_p])
+    _check(f(_ptr(o), _ptr(divisor), _ptr(u), u.stride(0), _ptr(gates), _ptr(gate_bias), float(cap), _ptr(state), _ptr(top), _ptr(q_start), _ptr(state_slot),
+             state_slot.numel(), heads, d, dv1 - 1, u.shape[0], wait_limit, skip_tile, _stream()), "matrix_memory_umma_wait_test")
+
 
 MATRIX_MEMORY_MAX_HEAD_DIM = 512
 MATRIX_MEMORY_CHUNK_MAX_HEAD_DIM = 256  # the tensor-core kernel keeps a state column block in registers

@@ -87,3 +87,26 @@ def test_infinities_and_nans_stay_where_the_recurrence_has_them(where, value, ba
     for segments in (1, 3):
         for a, b in zip(_run(inputs, lens, torch.arange(2), form="chunk", segments=segments), want):
             assert _same_kind(a, b, 4e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("skip", [0, 1])
+def test_a_wait_that_runs_out(skip):
+    """The copies of q and k of one tile never come: no read-outs or divisors of that tile or a later one, no states and no maxima are stored, the next step is right."""
+    H, d, dv, lens = 2, 48, 72, [300, 290]
+    inputs = _inputs(H, d, dv, lens, 5)
+    want = _exact(inputs[0], inputs[1], inputs[2], inputs[3].clone(), inputs[4], lens)
+    q_start, slot = torch.tensor([0, 300, 590], dtype=torch.int32).cuda(), torch.arange(2, dtype=torch.int32).cuda()
+    assert ops.device_wait_errors() == {}
+    u, gates, bias, state, top = [x.cuda() for x in inputs]
+    o, div = torch.full((590, H * dv), 7.0).cuda(), torch.full((590, H), 7.0).cuda()
+    ops.matrix_memory_umma_wait_test(o, div, u, gates, bias, CAP, state, top, q_start, slot, wait_limit=20000, skip_tile=skip)
+    torch.cuda.synchronize()  # returns: the kernel ended by itself
+    assert torch.equal(state.cpu(), inputs[3]) and torch.equal(top.cpu(), inputs[4])
+    for first, last in ((0, 300), (300, 590)):
+        for got, exact in ((o, want[0]), (div, want[1])):
+            assert _same_kind(got[first : first + 128 * skip].cpu(), exact[first : first + 128 * skip], 4e-6) and (got[first + 128 * skip : last] == 7).all()
+    assert "matrix_memory_umma.cu" in ops.device_wait_errors() and ops.device_wait_errors() == {}
+    for a, b in zip(_run(inputs, lens, torch.arange(2), form="chunk", segments=1), want):
+        assert _same_kind(a, b, 4e-6)
+    assert ops.device_wait_errors() == {}

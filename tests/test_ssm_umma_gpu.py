@@ -52,3 +52,26 @@ def test_infinities_and_nans_stay_where_the_recurrence_has_them(where, value, ba
         y, st = torch.zeros(n, H * P).cuda(), state.cuda()
         ops.ssm_scan(y, xbc.cuda(), u.cuda(), 0, vec[0], vec[1] * 0.1, vec[2], st, q_start, slot, 1, max_len=300, form="chunk", segments=segments)
         assert _same_kind(y, want[0], 1e-6) and _same_kind(st, want[1], 1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("skip", [0, 1])
+def test_a_wait_that_runs_out(skip):
+    """The copies of B and C of one tile never come: no read-outs of that tile or a later one and no states are stored, the code is read once, the next scan is right."""
+    H, P, N, lens = 3, 72, 48, [300, 290]
+    n, g = sum(lens), torch.Generator().manual_seed(5)
+    xbc, u, state = torch.randn(n, H * P + 2 * N, generator=g).bfloat16(), torch.randn(n, H, generator=g).bfloat16(), torch.randn(2, H, P, N, generator=g)
+    vec = torch.randn(3, H, generator=g)
+    vec[0] -= 3.0
+    want = _exact(xbc, u, 0, *vec, state.clone(), lens, 1)
+    q_start, slot, vec = torch.tensor([0, 300, 590], dtype=torch.int32).cuda(), torch.arange(2, dtype=torch.int32).cuda(), vec.cuda()
+    assert ops.device_wait_errors() == {}
+    y, st = torch.full((n, H * P), 7.0).cuda(), state.cuda()
+    ops.ssm_umma_wait_test(y, xbc.cuda(), u.cuda(), 0, *vec, st, q_start, slot, 1, wait_limit=20000, skip_tile=skip)
+    torch.cuda.synchronize()  # returns: the kernel ended by itself
+    assert torch.equal(st.cpu(), state)
+    for first, last in ((0, 300), (300, 590)):
+        assert _same_kind(y[first : first + 128 * skip], want[0][first : first + 128 * skip], 1e-6) and (y[first + 128 * skip : last] == 7).all()
+    assert "ssm_umma.cu" in ops.device_wait_errors() and ops.device_wait_errors() == {}
+    ops.ssm_scan(y, xbc.cuda(), u.cuda(), 0, *vec, st, q_start, slot, 1, max_len=300, form="chunk", segments=1)
+    assert _same_kind(y, want[0], 1e-6) and _same_kind(st, want[1], 1e-6) and ops.device_wait_errors() == {}
