@@ -76,30 +76,56 @@ def dense_product(x, features: int, epilogue: str) -> bool:
     raise ValueError(f"unknown epilogue {epilogue!r}")
 
 
-# Steps of more tokens than the decode product takes, up to here, go to the engine's product for some tokens (csrc/few_gemm.cu) where it beats the library.
-# Measured in chains of replayed products with cold weights, us, library / own at 9, 33 and 64 tokens: 2,048 features of K 2,048 5.5/3.6, 5.6/4.6, 5.7/4.9;
-# 2,048 of 8,192 13.1/9.6, 13.2/10.9, 13.4/11.3; 1,024 of 4,096 10.1/4.3, 7.9/5.4, 7.9/6.4; 4,096 of 4,096 9.7/8.5, 9.8/9.7, 9.9/10.0; but where all SMs have a
-# tile of their own anyway 10,304 of 2,048 10.7/9.7, 11.6/10.8, 9.7/11.1; 6,176 of 2,048 7.7/7.3, 7.6/8.2, 7.4/8.6.  gate|up with SiLU * up (8,192 each, of 2,048)
-# 16.4/13.1, 16.6/14.3, 16.7/15.4, at 96 and 128 tokens 18.2/16.6, 17.7/17.8.  Between other kernels a product of the engine starts and ends later than the
-# library's by up to a microsecond: an attention layer of 2,048 with 40 single tokens 30.7 -> 32.8 us with both products here, with 16 28.7 both; four layers of a
-# Llama of 2,048 with 16 single tokens 333 -> 281 us.
+# Steps of more tokens than the decode product takes go to the engine's product for some tokens (csrc/few_gemm.cu) where it beats the library.  Measured with cold weights
+# between a norm and an activation (us, library / own), and in chains of whole layers (norm, layer, norm, ..: own minus library, a layer).
+# As a rule up to 24 tokens: at 9 and 24 of them 2,048 features of K 2,048 9.3/7.4 and 9.6/8.1, 10,304 of 2,048 14.3/12.3 and 14.5/12.8, 4,096 of 1,024 8.5/7.3 and
+# 8.7/7.7; layers of 2,048 with 16 tokens: the products in front -2.1 (grouped-query), -0.7 (latent), -1.2 (Mamba-2), behind -2.0, -1.7, -1.9.
+#   * Long sums with few features, up to 64: at 33 and 64 tokens 2,048 of 8,192 15.4/12.4 and 15.7/12.2, 1,024 of 4,096 10.3/6.7 and 10.3/7.9.  4,096 of 4,096 only up to 40:
+#     the product behind a layer of 4,096, at 32 / 48 / 64 tokens: grouped-query -3.0 / -1.9 / -0.2, differential -2.0 / -0.7 / -0.3, latent -0.6 / -0.3 / +1.9,
+#     matrix memory 0.0 / +1.7 / +2.0.
+#   * Where two CTAs share K (few_splits) they stay behind: 6,176 of 2,048 in front of a gated delta rule -0.4 / +1.1 / +1.9 at 12 / 16 / 20 tokens, 8,192 of 2,048 of a
+#     matrix memory +0.4 at 12; of 4,096, 6,144 to 8,480 features: -0.3 to -2.6 at 16 tokens, -0.3 to +1.0 at 20 and 24.
+#   * Small products up to 16: 1,024 of 1,024 behind a gated delta rule 0.0 / +0.7 / +0.7 at 16 / 20 / 24 tokens.
+#   * A CTA has an SM, so a tile more than SMs is a second wave: 18,944 features (148 tiles) of 2,048 19.7/18.7, 19,072 19.7/23.7, 24,576 24.0/25.4, 28,672 (three quarters of
+#     two waves) 27.2/26.4, of 1,024 16.9/17.5.
+# gate|up with SiLU * up up to 96: 16,384 of 2,048 at 9 / 64 / 96 tokens 16.4/13.1, 16.7/15.4, 18.2/16.6; but 11,264 of 8,192 (88 CTAs, each all of K) at 96 42.0/44.3, and
+# in a second wave 28,672 of 4,096 at 9 / 64 / 96 44.2/41.3, 48.0/48.2, 54.6/55.9, of 1,024 at 64 18.7/19.9, 57,344 of 4,096 at 24 / 48 86.5/84.6, 87.4/91.5.
 FEW_MAX_TOKENS, FEW_MAX_TOKENS_SWIGLU, FEW_MAX_TOKENS_SHORT_K = 64, 96, 24
 FEW_MIN_SIZE, FEW_LONG_K, FEW_MAX_FEATURES = 1024, 4096, 4224  # least K and features; from which K on, and up to which width, more than 24 tokens go there
+FEW_WAVE_FILL = 0.75
 
 
 def few_splits(features: int, K: int) -> int:
-    """CTAs that share a tile's K: the most for which clusters of them still fit the GPU at once and each has four steps of 128."""
+    """CTAs that share a tile's K: the most for which clusters of them still fit the GPU at once (of a B200's 148 SMs, clusters of four fill 132, of eight 112)
+    and each has four steps of 128."""
     tiles, steps = -(-features // 128), -(-K // 128)
     return next((s for s, places in ((8, 112), (4, 132), (2, 148)) if tiles * s <= places and steps >= 4 * s), 1)
 
 
+def few_max_tokens(features: int, K: int, swiglu: bool = False) -> int:
+    """The most tokens whose product with a [features, K] weight goes to the engine's product for some tokens (0: none)."""
+    tiles, sms, splits = -(-features // 128), sm_count(), few_splits(features, K)
+    waves = -(-tiles // sms)
+    if waves > 1:
+        if tiles < FEW_WAVE_FILL * waves * sms or (K < 2048 and not swiglu):
+            return 0
+        return FEW_MAX_TOKENS if swiglu and waves == 2 and K >= 2048 else FEW_MAX_TOKENS_SHORT_K
+    if swiglu:
+        return FEW_MAX_TOKENS_SWIGLU if splits > 1 or K < 4096 or tiles >= FEW_WAVE_FILL * sms else FEW_MAX_TOKENS
+    if K >= FEW_LONG_K and features <= FEW_MAX_FEATURES:
+        return FEW_MAX_TOKENS if features <= 3200 or K >= 8192 else 40
+    if K < 2048 and features <= 3200:
+        return 16
+    if splits == 2 and 2048 <= K < 8192:
+        return 16 if K >= 3072 or features <= 5400 else 12 if features <= 7168 else 0
+    return FEW_MAX_TOKENS_SHORT_K
+
+
 def few_product(x: torch.Tensor, weight: torch.Tensor, swiglu: bool = False) -> bool:
     """Whether the product of these activations with a [features, K] weight goes to the engine's product for some tokens."""
-    if not ops.few_gemm_supported(x, weight) or x.shape[0] <= SKINNY_MAX_TOKENS or min(weight.shape) < FEW_MIN_SIZE:
+    if not SKINNY_MAX_TOKENS < x.shape[0] <= FEW_MAX_TOKENS_SWIGLU or not ops.few_gemm_supported(x, weight) or min(weight.shape) < FEW_MIN_SIZE or (swiglu and weight.shape[0] % 128):
         return False
-    if swiglu:
-        return x.shape[0] <= FEW_MAX_TOKENS_SWIGLU and weight.shape[0] % 128 == 0
-    return x.shape[0] <= (FEW_MAX_TOKENS if weight.shape[1] >= FEW_LONG_K and weight.shape[0] <= FEW_MAX_FEATURES else FEW_MAX_TOKENS_SHORT_K)
+    return x.shape[0] <= few_max_tokens(*weight.shape, swiglu)
 
 
 def project(x, weight: torch.Tensor, out_dtype: torch.dtype | None = None, max_tokens: int = SKINNY_MAX_TOKENS) -> torch.Tensor:

@@ -61,3 +61,14 @@ def test_which_products_go_there():
     assert takes(96, 16384, 2048, swiglu=True) and not takes(97, 16384, 2048, swiglu=True) and not takes(16, 2048, 2048, torch.float32)
     assert not gemm.few_product(torch.empty(16, 2052, dtype=torch.bfloat16)[:, 4:], torch.empty(2048, 2048, dtype=torch.bfloat16))  # rows off 16 bytes
     assert [gemm.few_splits(*s) for s in ((2048, 2048), (16384, 2048), (1024, 4096), (4240, 2048), (4096, 4096), (1024, 1024))] == [4, 1, 8, 2, 4, 2]
+
+
+@pytest.mark.parametrize("features,K,swiglu,most", [
+    (18944, 2048, False, 24), (19072, 2048, False, 0), (20608, 4096, False, 0), (28672, 2048, False, 24), (28672, 1024, False, 0), (38016, 2048, False, 0), (37888, 4096, False, 24),
+    (19200, 4096, True, 0), (28672, 4096, True, 64), (28672, 1024, True, 24), (57344, 4096, True, 24), (11264, 8192, True, 64), (18944, 8192, True, 96), (16384, 2048, True, 96),
+    (4096, 4096, False, 40), (2048, 4096, False, 64), (4096, 8192, False, 64), (1024, 4096, False, 64), (6144, 4096, False, 16), (12352, 4096, False, 24),
+    (5376, 2048, False, 16), (6176, 2048, False, 12), (8192, 2048, False, 0), (10304, 2048, False, 24), (4096, 2048, False, 24), (4096, 1024, False, 24), (1024, 1024, False, 16)])
+def test_up_to_how_many_tokens(features, K, swiglu, most, monkeypatch):
+    """The lines lie where both sides were measured: a second wave of tiles, CTAs that share K in pairs, and wide products of some more tokens cost more than the library's."""
+    monkeypatch.setattr(gemm, "sm_count", lambda: 148)
+    assert gemm.few_max_tokens(features, K, swiglu) == most
