@@ -152,11 +152,13 @@ __global__ void __launch_bounds__(ROUTE_THREADS) moe_route_kernel(int* __restric
   if (warp == 0) choose_experts(ids + t * top, weights + t * top, score, choice, mark, picked, correction, E, top, groups, keep, scale, mode, lane);
 }
 
-// A portion of many tokens: a block takes eight of them, a warp four experts' rows with four of the tokens at a time, so that a number of either,
-// once read, serves four products, and the next numbers are under way meanwhile.  Every sum is added up in the order of the kernel above.  W a
-// multiple of 8, 16-byte aligned rows.  What bounds it: the rows' latency; four tokens a block and nothing under way ahead took (cold, launch
-// included, us) 24.6 for 2,048 tokens of 2,048 and 16 experts, now 22.5; 59.4 for 3,825 of 4,096, now 51.2; 63.5 for 2,048 of 2,048 and 64 experts, now 51.2.
-constexpr int ROUTE_TOKENS = 8, ROUTE_ROWS = 4, ROUTE_HALF = 4;  // tokens of a block, experts and tokens of a warp
+// A portion of many tokens: a block takes four of them and a warp four experts' rows at a time, so that a number of either, once read,
+// serves four products.  Every sum is added up in the order of the kernel above.  W a multiple of 8, 16-byte aligned rows.
+// What bounds it: the rows' latency, so the next numbers can be under way meanwhile (AHEAD): 44.6 us instead of 55.3 for 2,048 tokens of 2,048 and 64 experts, 16.3 instead of 19.7
+// for 16, 67 instead of 93 for 64 of width 4,096; float32, 1,184 tokens, 39 instead of 47.  That takes registers, so that fewer blocks lie on an SM, four instead of six (float32:
+// two instead of five), and a launch just above a wave of them takes two: 2,500 tokens 80 us ahead, 57 not; 5,000 127 and 95; 4,736 88 and 93; float32, 2,048 tokens, 74 and 63.  A
+// wave ahead takes 0.76 of one without (float32: 0.55 to 0.75), and the waves are counted.
+constexpr int ROUTE_TOKENS = 4, ROUTE_ROWS = 4;
 template <typename T> struct Run8;  // eight numbers as they lie in memory
 template <> struct Run8<__nv_bfloat16> {
   uint4 v;
@@ -170,59 +172,78 @@ template <> struct Run8<float> {
   float4 a, b;
   __device__ __forceinline__ void get(float (&f)[8]) const { f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w; }
 };
-template <typename T>
-__global__ void __launch_bounds__(256) moe_route_many_kernel(int* __restrict__ ids, float* __restrict__ weights, const T* __restrict__ x,
-                                                             const float* __restrict__ router, const float* __restrict__ correction, int n,
-                                                             int W, int E, int top, int groups, int keep, float scale, int mode) {
+template <typename T> constexpr int route_blocks(bool ahead) { return sizeof(T) == 2 ? (ahead ? 4 : 6) : (ahead ? 2 : 5); }  // on an SM, by registers
+template <typename T, bool AHEAD>
+__global__ void __launch_bounds__(AHEAD ? 256 : ROUTE_TOKENS * 32)
+    moe_route_many_kernel(int* __restrict__ ids, float* __restrict__ weights, const T* __restrict__ x, const float* __restrict__ router,
+                          const float* __restrict__ correction, int n, int W, int E, int top, int groups, int keep, float scale, int mode) {
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ float sm[];  // per token: score [E] | choice [E] | mark [groups]
   __shared__ int picked[ROUTE_TOKENS][MAX_TOP];
   const int per_token = 2 * E + groups;
   const size_t t0 = (size_t)blockIdx.x * ROUTE_TOKENS;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = warp >> 2;
-  const T* rows[ROUTE_HALF];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const T* rows[ROUTE_TOKENS];
 #pragma unroll
-  for (int j = 0; j < ROUTE_HALF; ++j) rows[j] = x + min(t0 + half * ROUTE_HALF + j, (size_t)n - 1) * W;
-  for (int e0 = (warp & 3) * ROUTE_ROWS; e0 < E; e0 += 4 * ROUTE_ROWS) {
-    float acc[ROUTE_ROWS][ROUTE_HALF];
+  for (int j = 0; j < ROUTE_TOKENS; ++j) {  // (a bound of 256 threads and the two forms of one index: what gives ptxas' better code, 126 and 80 registers, float32 184 and 92)
+    if constexpr (AHEAD) rows[j] = x + min(t0 + j, (size_t)n - 1) * W;
+    else rows[j] = x + (t0 + j < (size_t)n ? t0 + j : (size_t)n - 1) * W;
+  }
+  for (int e0 = warp * ROUTE_ROWS; e0 < E; e0 += ROUTE_TOKENS * ROUTE_ROWS) {
+    float acc[ROUTE_ROWS][ROUTE_TOKENS];
 #pragma unroll
     for (int r = 0; r < ROUTE_ROWS; ++r)
 #pragma unroll
-      for (int j = 0; j < ROUTE_HALF; ++j) acc[r][j] = 0.f;
+      for (int j = 0; j < ROUTE_TOKENS; ++j) acc[r][j] = 0.f;
     const float* w[ROUTE_ROWS];
 #pragma unroll
     for (int r = 0; r < ROUTE_ROWS; ++r) w[r] = router + (size_t)min(e0 + r, E - 1) * W;
-    Run8<T> xr[ROUTE_HALF];
-    Run8<float> wr[ROUTE_ROWS];
-    auto fetch = [&](int i) {
+    if constexpr (AHEAD) {
+      Run8<T> xr[ROUTE_TOKENS];
+      Run8<float> wr[ROUTE_ROWS];
+      auto fetch = [&](int i) {
 #pragma unroll
-      for (int j = 0; j < ROUTE_HALF; ++j) xr[j] = *reinterpret_cast<const Run8<T>*>(rows[j] + i);
+        for (int j = 0; j < ROUTE_TOKENS; ++j) xr[j] = *reinterpret_cast<const Run8<T>*>(rows[j] + i);
 #pragma unroll
-      for (int r = 0; r < ROUTE_ROWS; ++r) wr[r] = *reinterpret_cast<const Run8<float>*>(w[r] + i);
-    };
-    if (lane * 8 < W) fetch(lane * 8);
-    for (int i = lane * 8; i < W; i += 256) {
-      float xv[ROUTE_HALF][8], wv[ROUTE_ROWS][8];
+        for (int r = 0; r < ROUTE_ROWS; ++r) wr[r] = *reinterpret_cast<const Run8<float>*>(w[r] + i);
+      };
+      if (lane * 8 < W) fetch(lane * 8);
+      for (int i = lane * 8; i < W; i += 256) {
+        float xv[ROUTE_TOKENS][8], wv[ROUTE_ROWS][8];
 #pragma unroll
-      for (int j = 0; j < ROUTE_HALF; ++j) xr[j].get(xv[j]);
+        for (int j = 0; j < ROUTE_TOKENS; ++j) xr[j].get(xv[j]);
 #pragma unroll
-      for (int r = 0; r < ROUTE_ROWS; ++r) wr[r].get(wv[r]);
-      fetch(i + 256 < W ? i + 256 : i);
+        for (int r = 0; r < ROUTE_ROWS; ++r) wr[r].get(wv[r]);
+        fetch(i + 256 < W ? i + 256 : i);
 #pragma unroll
-      for (int r = 0; r < ROUTE_ROWS; ++r)
+        for (int r = 0; r < ROUTE_ROWS; ++r)
 #pragma unroll
-        for (int j = 0; j < ROUTE_HALF; ++j)
+          for (int j = 0; j < ROUTE_TOKENS; ++j)
 #pragma unroll
-          for (int k = 0; k < 8; ++k) acc[r][j] = fmaf(wv[r][k], xv[j][k], acc[r][j]);
+            for (int k = 0; k < 8; ++k) acc[r][j] = fmaf(wv[r][k], xv[j][k], acc[r][j]);
+      }
+    }
+    for (int i = lane * 8; !AHEAD && i < W; i += 256) {
+      float xv[ROUTE_TOKENS][8];
+#pragma unroll
+      for (int j = 0; j < ROUTE_TOKENS; ++j) load8(rows[j] + i, xv[j]);
+#pragma unroll
+      for (int r = 0; r < ROUTE_ROWS; ++r) {
+        float wv[8];
+        load8(w[r] + i, wv);
+#pragma unroll
+        for (int j = 0; j < ROUTE_TOKENS; ++j)
+#pragma unroll
+          for (int k = 0; k < 8; ++k) acc[r][j] = fmaf(wv[k], xv[j][k], acc[r][j]);
+      }
     }
 #pragma unroll
     for (int r = 0; r < ROUTE_ROWS; ++r)
 #pragma unroll
-      for (int j = 0; j < ROUTE_HALF; ++j) {
+      for (int j = 0; j < ROUTE_TOKENS; ++j) {
         const float z = warp_sum(acc[r][j]);
-        float* score = sm + (half * ROUTE_HALF + j) * per_token;
-        if (lane == 0 && e0 + r < E) put_score(score, score + E, e0 + r, z, correction, mode);
+        if (lane == 0 && e0 + r < E) put_score(sm + j * per_token, sm + j * per_token + E, e0 + r, z, correction, mode);
       }
   }
   __syncthreads();
@@ -318,12 +339,15 @@ DLI_EXPORT int dli_moe_route(int* ids, float* weights, const void* x, const floa
   cudaError_t e;
   const size_t many_smem = (size_t)ROUTE_TOKENS * (2 * E + groups) * sizeof(float);
   if (n > ROUTE_MANY_TOKENS && (W % 8) == 0 && ((((uintptr_t)x) | ((uintptr_t)router)) & 15) == 0 && many_smem <= 48 * 1024 - ROUTE_TOKENS * MAX_TOP * sizeof(int)) {
-    const dim3 grid((n + ROUTE_TOKENS - 1) / ROUTE_TOKENS), block(ROUTE_TOKENS * 32);
+    const int blocks = (n + ROUTE_TOKENS - 1) / ROUTE_TOKENS, sms = sm_count();
+    auto ahead = [&](int with, int without) { return 0.76f * ((blocks + with * sms - 1) / (with * sms)) <= (blocks + without * sms - 1) / (without * sms); };
+    const dim3 grid(blocks), block(ROUTE_TOKENS * 32);
     if (dtype == DLI_F32)
-      return (int)launch_pdl((moe_route_many_kernel<float>), grid, block, many_smem, stream, 1, ids, weights, (const float*)x, router, correction, n, W, E, top,
-                             groups, keep, scale, mode);
-    return (int)launch_pdl((moe_route_many_kernel<__nv_bfloat16>), grid, block, many_smem, stream, 1, ids, weights, (const __nv_bfloat16*)x, router, correction,
-                           n, W, E, top, groups, keep, scale, mode);
+      return (int)launch_pdl(ahead(route_blocks<float>(true), route_blocks<float>(false)) ? moe_route_many_kernel<float, true> : moe_route_many_kernel<float, false>, grid, block,
+                             many_smem, stream, 1, ids, weights, (const float*)x, router, correction, n, W, E, top, groups, keep, scale, mode);
+    return (int)launch_pdl(ahead(route_blocks<__nv_bfloat16>(true), route_blocks<__nv_bfloat16>(false)) ? moe_route_many_kernel<__nv_bfloat16, true>
+                                                                                                        : moe_route_many_kernel<__nv_bfloat16, false>,
+                           grid, block, many_smem, stream, 1, ids, weights, (const __nv_bfloat16*)x, router, correction, n, W, E, top, groups, keep, scale, mode);
   }
   if (dtype == DLI_F32) {
     static MaxPerDevice set;
