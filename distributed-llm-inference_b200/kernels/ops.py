@@ -1363,7 +1363,7 @@ def conv_state_update(state: torch.Tensor, u: torch.Tensor, col0: int, q_start: 
 SSM_SCAN_MAX_STATE = 512
 
 
-# Of csrc/ssm_umma.cu, which takes multiples of 16; tiles of 64 / 128 tokens, us, 64 heads, N 128: 17 tokens 9.4 / 10.2, 33 10.2 / 10.3, 100 17 / 11.
+# csrc/ssm_umma.cu (tiles of 128 tokens; states of multiples of 16 numbers) takes a step from these on, csrc/ssm_tc.cu (tiles of 64) the others.
 SSM_UMMA_MIN_STATE, SSM_UMMA_MIN_TOKENS = 32, 33
 SSM_CHUNK_MAX_STATE = 128  # the tensor-core form keeps a state column block in registers
 # Portions of up to a quarter tile are walked token after token.  That is on the safe side: us, walk / tiles, 64 heads, P 64, N 128: one portion of 4 tokens
@@ -1380,14 +1380,51 @@ def ssm_scan_form(dtype: torch.dtype, P: int, N: int, max_len: int, aligned: boo
     return "walk"
 
 
+def _waves(ctas: int) -> int:
+    """0, 1 or 2: CTAs of which an SM holds one fit the GPU at once, in two waves, or take more."""
+    from .attention import sm_count
+
+    return 0 if ctas <= sm_count() else 1 if ctas <= 2 * sm_count() else 2
+
+
+def _portions(n: int, count: int, longest: int) -> tuple[int, float]:
+    """Of a step's ``count`` sequences with ``n`` tokens, the longest with ``longest``: how many bring more than one token, and how many in the mean, if the host does not say."""
+    portions = max(1, min(count, 1 + (n - longest) // 2))
+    return portions, n / portions
+
+
+# The fewest tokens of a portion in the mean from which on tiles of 128 are faster, for (up to one wave of their CTAs, up to two, more): such a CTA has an SM to
+# itself, so short portions of many heads queue, while four to eight CTAs with tiles of 64 share an SM, the more the smaller the state.  From 1,950 steps (8 to 128 heads, P 32 to 128, 1
+# to 16 portions of together 33 to 6,000 tokens beside 0 to 48 single ones).  Tiles of 64 / 128, us, one portion of 64 heads (N 128) of 17 tokens 9.4 / 10.2, 33 10.2 / 10.3,
+# 100 17 / 11, 600 48 / 28; 4 portions of 46 tokens, 32 heads of 128 columns, N 64 10.6 / 18.1; 5 of 24, 128 heads, N 128 28.8 / 45.7; 5 of 60, 128 heads, N 64 27.5 / 41.1; 24 single tokens and 3
+# portions of 154, 32 heads of 128 columns, N 32 33 / 44.  With it 25 of the 1,950 take over 5 % longer than tiles of 64, with a line at 33 tokens alone 577.
+SSM_UMMA_MEAN = {32: (90, 250, 400), 64: (60, 150, 220), 128: (33, 60, 75)}
+SSM_UMMA_MEAN_SINGLES = {32: (180, 250, 400), 64: (100, 150, 220), 128: (33, 33, 40)}  # beside ten single tokens or more, each of which takes a tile of 64
+
+
+def ssm_tile(heads: int, P: int, N: int, n: int, count: int, portions: tuple[int, float] | None, longest: int) -> int:
+    """Tokens of a tile with which the tensor-core scan takes a step of ``count`` sequences: 64 or 128.  ``portions``: how many of them bring more than one
+    token, and how many in the mean (None: not known)."""
+    longest = min(longest, n)
+    if not (SSM_UMMA_MIN_STATE <= N <= SSM_CHUNK_MAX_STATE and N % 16 == 0 and longest >= SSM_UMMA_MIN_TOKENS):
+        return 64
+    portions, mean = portions or _portions(n, count, longest)
+    ctas, singles, size = -(-P // 64) * heads * portions, count - portions, 32 if N <= 32 else 64 if N <= 64 else 128
+    # few CTAs with long portions: tiles of 64 are cut into more segments (1,177 tokens of 32 heads, N 64 34 / 41, 1,330 of 8, N 32 26 / 40, but 616 of 32 29 / 24, 2,718 of 64 94 / 71)
+    if size <= 64 and _waves(4 * ctas) == 0 and 700 <= mean <= 2100 and (not singles or (size == 32 and ctas <= 16)):
+        return 64
+    return 128 if mean >= (SSM_UMMA_MEAN_SINGLES if singles >= 10 else SSM_UMMA_MEAN)[size][_waves(ctas)] else 64
+
+
 def ssm_scan(y: torch.Tensor, xbc: torch.Tensor, u: torch.Tensor, dt_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
              state: torch.Tensor, q_start: torch.Tensor, state_slot: torch.Tensor, groups: int, max_len: int = 1 << 30,
-             form: str | None = None, segments: int = 0) -> None:
+             form: str | None = None, segments: int = 0, portions: tuple[int, float] | None = None, tile: int = 0) -> None:
     """The selective scan of every sequence's tokens of this step, from and to its slot of ``state`` [slots, heads, P, N]
     (float32; S transposed, so that a column's N values are contiguous).  xbc [n, heads P + 2 groups N] holds x | B | C; dt_raw is column dt_col + head of u.  Per head:
     dt = softplus(dt_raw + dt_bias), S <- exp(-exp(a_log) dt) S + dt B x^T, y = S^T C + d_skip x.  y [n, heads P] float32.
     ``max_len``: the most tokens a sequence brings, if the host knows (a launch hint).  ``form``: ``"walk"``, ``"chunk"``, or None (chosen:
-    ``ssm_scan_form``).  ``segments`` (of the form ``"chunk"``; 0: chosen): into how many runs of tiles a sequence is cut."""
+    ``ssm_scan_form``).  ``segments`` (of the form ``"chunk"``; 0: chosen): into how many runs of tiles a sequence is cut.  ``portions``: how many
+    of the sequences bring more than one token and how many in the mean, if the host knows (a launch hint); ``tile`` (of the form ``"chunk"``; 64 or 128, 0: chosen, ``ssm_tile``)."""
     _columns(u, "ssm_scan"), _need(xbc, "xbc", u.dtype), _need(y, "y", torch.float32), _need(state, "state", torch.float32)
     for t, name in ((dt_bias, "dt_bias"), (a_log, "a_log"), (d_skip, "d_skip")):
         _need(t, name, torch.float32)
@@ -1404,7 +1441,7 @@ def ssm_scan(y: torch.Tensor, xbc: torch.Tensor, u: torch.Tensor, dt_col: int, d
         if u.dtype != torch.bfloat16 or segments < 0:
             raise KernelError("ssm_scan: the tensor-core form takes bfloat16")
         count = state_slot.numel()
-        umma = SSM_UMMA_MIN_STATE <= N <= SSM_CHUNK_MAX_STATE and N % 16 == 0 and min(max_len, n) >= SSM_UMMA_MIN_TOKENS
+        umma = (tile or ssm_tile(heads, P, N, n, count, portions, max_len)) == 128
         source, name = ("ssm_umma.cu", "dli_ssm_umma") if umma else ("ssm_tc.cu", "dli_ssm_chunk")
         segments = segments or _fn(source, "dli_ssm_umma_segments" if umma else "dli_ssm_segments", [c_int] * 4)(count, heads, P, int(min(max_len, n)))
         part = part_log = None
@@ -1993,8 +2030,7 @@ def matrix_memory_umma_wait_test(o: torch.Tensor, divisor: torch.Tensor, u: torc
 
 MATRIX_MEMORY_MAX_HEAD_DIM = 512
 MATRIX_MEMORY_CHUNK_MAX_HEAD_DIM = 256  # the tensor-core kernel keeps a state column block in registers
-# From here on portions go in tiles of 128 tokens (csrc/matrix_memory_umma.cu).  Tiles of 64 / 128, us, heads of 128: 16 heads, 17 tokens 9.8 / 12.3, 44 beside two
-# single ones 12.7 / 12.3, 100 18 / 13; 8 heads, twice 21 beside two 10.2 / 12.3.
+# csrc/matrix_memory_umma.cu (tiles of 128 tokens) takes a step from these on, csrc/matrix_memory_tc.cu (tiles of 64) the others.
 MATRIX_MEMORY_UMMA_MIN_TOKENS = 49
 MATRIX_MEMORY_CHUNK_MIN_TOKENS = 17  # shorter portions are walked token after token
 
@@ -2007,16 +2043,36 @@ def matrix_memory_form(dtype: torch.dtype, d: int, max_len: int) -> str:
     return "walk"
 
 
+# As SSM_UMMA_MEAN (up to one wave of CTAs, up to two, more), beside up to one, up to nine and more single tokens, for key sizes of up to 32, 64, 128; from 1,950 steps of 4 to
+# 32 heads.  Tiles of 64 / 128, us, heads of 128: 16 heads, 17 tokens 9.8 / 12.3, 44 beside two single ones 12.7 / 12.3, 100 18 / 13; 8 heads, twice 21 beside two 10.2 / 12.3; 16
+# heads, 6 portions of 28 14.7 / 23.6, of 89 26.9 / 23.9; heads of 64: 32, 5 portions of 51 19.2 / 21.8.  With it 16 of the 1,950 take over 5 % longer than tiles of
+# 64, with a line at 49 tokens alone 98.
+_NEVER = 1 << 30
+MATRIX_MEMORY_UMMA_MEAN = {32: ((60, 180, _NEVER),) * 3, 64: ((45, 60, 110), (45, 60, 110), (0, 0, 40)), 128: ((0, 60, 70), (0, 45, 50), (0, 0, 0))}
+
+
+def matrix_memory_tile(heads: int, d: int, dv: int, n: int, count: int, portions: tuple[int, float] | None, longest: int) -> int:
+    """Tokens of a tile with which the tensor-core form of the matrix memory takes a step (of sizes that both tiles take): 64 or 128.  ``portions``: as in ``ssm_tile``."""
+    longest = min(longest, n)
+    if longest < MATRIX_MEMORY_UMMA_MIN_TOKENS:
+        return 64
+    portions, mean = portions or _portions(n, count, longest)
+    ctas, singles = -(-dv // 64) * heads * portions, count - portions
+    least = MATRIX_MEMORY_UMMA_MEAN[32 if d <= 32 else 64 if d <= 64 else 128][0 if singles < 2 else 1 if singles < 10 else 2]
+    return 128 if mean >= least[_waves(ctas)] else 64
+
+
 def matrix_memory_scan(o: torch.Tensor, divisor: torch.Tensor, u: torch.Tensor, gates: torch.Tensor, gate_bias: torch.Tensor, cap: float,
                        state: torch.Tensor, top: torch.Tensor, q_start: torch.Tensor, state_slot: torch.Tensor, max_len: int = 1 << 30,
-                       form: str | None = None, segments: int = 0) -> None:
+                       form: str | None = None, segments: int = 0, portions: tuple[int, float] | None = None, tile: int = 0) -> None:
     """A matrix memory with exponential gates over every sequence's tokens of this step, from and to its slot of ``state``
     [slots, heads, dv + 1, d] (float32; S transposed, the last row is n) and ``top`` [slots, heads, dv + 1] (m, a copy per column).
     u [n, .]: q | k | v in its leading columns (heads of d, d, dv); gates [n, 2 heads] float32: the input gates' sums, then the
     forget gates'; ``gate_bias`` [2 heads].  Per head i = cap tanh((gate + bias) / cap), f = logsigmoid(cap tanh(...)),
     m' = max(f + m, i), S <- exp(f + m - m') S + exp(i - m') k v^T, n likewise with k alone.  Left: o [n, heads dv] = S^T q / sqrt(d)
     and divisor [n, heads] = max(|n . q| / sqrt(d), exp(-m)) + 1e-6, both float32.  ``form``: ``"walk"``, ``"chunk"``, or None (chosen).
-    ``segments`` (of the form ``"chunk"``; 0: chosen): into how many runs of tiles a sequence is cut that are walked side by side."""
+    ``segments`` (of the form ``"chunk"``; 0: chosen): into how many runs of tiles a sequence is cut that are walked side by side.  ``portions``: how many of the
+    sequences bring more than one token and how many in the mean, if the host knows (a launch hint); ``tile`` (of the form ``"chunk"``; 64 or 128, 0: chosen, ``matrix_memory_tile``)."""
     _columns(u, "matrix_memory_scan"), _need(o, "o", torch.float32), _need(divisor, "divisor", torch.float32)
     _need(gates, "gates", torch.float32), _need(gate_bias, "gate_bias", torch.float32)
     _need(state, "state", torch.float32), _need(top, "top", torch.float32)
@@ -2035,7 +2091,8 @@ def matrix_memory_scan(o: torch.Tensor, divisor: torch.Tensor, u: torch.Tensor, 
         if u.dtype != torch.bfloat16 or d > MATRIX_MEMORY_CHUNK_MAX_HEAD_DIM:
             raise KernelError("matrix_memory_scan: the tensor-core form takes bfloat16 heads of at most 256")
         count = state_slot.numel()
-        umma = 32 <= d <= 128 and d % 16 == 0 and dv % 8 == 0 and min(max_len, n) >= MATRIX_MEMORY_UMMA_MIN_TOKENS and u.data_ptr() % 16 == 0 and u.stride(0) % 8 == 0 and o.data_ptr() % 8 == 0
+        umma = (32 <= d <= 128 and d % 16 == 0 and dv % 8 == 0 and u.data_ptr() % 16 == 0 and u.stride(0) % 8 == 0 and u.stride(0) >= heads * (2 * d + dv) and o.data_ptr() % 8 == 0
+                and (tile or matrix_memory_tile(heads, d, dv, n, count, portions, max_len)) == 128)
         source, name, lib = ("matrix_memory_umma.cu", "dli_matrix_memory_umma", None) if umma else ("matrix_memory_tc.cu", "dli_matrix_memory_chunk", {"KEY_DIM": -(-d // 16) * 16})
         if segments < 1:
             segments = _fn(source, name.replace("_chunk", "") + "_segments", [c_int] * 4, lib)(count, heads, dv, int(min(max_len, n)))

@@ -44,6 +44,18 @@ def scan_singles_apart(batch, P: int, N: int, heads: int, dtype: torch.dtype) ->
     return s if batch.num_seqs * heads * -(-P // 64) > 4 * 148 else 0
 
 
+def tile_hint(batch) -> dict:
+    """The option ``portions`` of a call in tiles: how many of the step's sequences bring more than one token, and how many in the mean, if the step says so.  A
+    recorded step knows the tokens of all together, and behind its portions, whose lengths it does not know yet, has a sequence that stays empty."""
+    lens = getattr(batch, "q_lens", [])[batch.num_single :]
+    if not lens or not batch.q_start.is_cuda:
+        return {}
+    if min(lens) > 0:
+        return {"portions": (len(lens), sum(lens) / len(lens))}
+    portions = max(1, len(lens) - 1)
+    return {"portions": (portions, (batch.n - batch.num_single) / portions)}
+
+
 def scan_calls(batch, s: int, form: str | None = None, tiles: str = "tiles") -> list[tuple]:
     """A recurrence's calls for a step whose first ``s`` single tokens are taken apart: (rows, q_start, state_slot, options) of each.  ``form``: of a
     single call; ``tiles``: of the portions' one."""
@@ -126,7 +138,7 @@ class Mamba2Mixer(Part):
         y = torch.empty((n, self.inner), dtype=torch.float32, device=x.device)
         for rows, q_start, slots, options in scan_calls(batch, scan_singles_apart(batch, self.P, self.N, self.heads, x.dtype), tiles=None):
             ops.ssm_scan(y[:rows], xbc[:rows], u[:rows], self.inner + self.channels, w["dt_bias"], w["A_log"], w["D"], ssm_state, q_start, slots, self.groups,
-                         **options)
+                         **tile_hint(batch), **options)
         gated = torch.empty((n, self.inner), dtype=x.dtype, device=x.device)
         ops.gated_group_rmsnorm(gated, y, u, 0, w["norm"], self.parts, self.eps)
         return project(gated, w["o"])
@@ -496,7 +508,8 @@ class MatrixMemory(Part):
         gates = project(x, w["gates"], out_dtype=torch.float32)  # i | f
         o = torch.empty((n, self.inner), dtype=torch.float32, device=x.device)
         divisor = torch.empty((n, self.heads), dtype=torch.float32, device=x.device)
-        ops.matrix_memory_scan(o, divisor, u, gates, w["gate_bias"], self.cap, state, top, batch.q_start, batch.state_slot, max_len=batch.max_q_len)
+        ops.matrix_memory_scan(o, divisor, u, gates, w["gate_bias"], self.cap, state, top, batch.q_start, batch.state_slot, max_len=batch.max_q_len,
+                               **tile_hint(batch))
         gated = torch.empty((n, self.inner), dtype=x.dtype, device=x.device)
         ops.gated_group_rmsnorm(gated, o, u, self.g_col, w["norm"], self.heads, self.eps, gate_after=True, gate="sigmoid", divisor=divisor)
         return project(gated, w["o"])

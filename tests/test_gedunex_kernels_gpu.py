@@ -125,7 +125,7 @@ def test_matrix_memory(sizes, dtype, form):
         return o, div, s, m
 
     want = run(ref, "cpu")
-    for more in ({},) if form == "walk" else ({}, {"segments": 1}, {"segments": 2}, {"segments": 7}):  # (seven: more than a sequence has tiles)
+    for more in ({},) if form == "walk" else ({}, {"tile": 64}, *({"segments": s, "tile": t} for s in (1, 2, 7) for t in (64, 128))):  # (seven: more than a sequence has tiles)
         for a, b, what in zip(run(ops, "cuda", form, **more), want, ("o", "divisor", "state", "top")):
             _close(a, b, 2e-5, f"{what} {more}")
     if form == "walk":
@@ -142,7 +142,7 @@ def test_matrix_memory_with_gates_at_their_extremes():
     gates[50:120, heads:] = -60.0
     q_start, slots = _i32([0, n]), _i32([2])
     out = []
-    for module, where, more in ((ref, "cpu", {}), (ops, "cuda", {"segments": 1}), (ops, "cuda", {"segments": 3}), (ops, "cuda", {"form": "walk"})):
+    for module, where, more in ((ref, "cpu", {}), *((ops, "cuda", {"segments": s, "tile": t}) for s in (1, 3) for t in (64, 128)), (ops, "cuda", {"form": "walk"})):
         o, div = torch.zeros(n, heads * dv, device=where), torch.zeros(n, heads, device=where)
         s, m = state.clone().to(where), top.clone().to(where)
         module.matrix_memory_scan(o, div, u.to(where), gates.to(where), bias.to(where), 15.0, s, m, q_start.to(where), slots.to(where), max_len=n, **more)

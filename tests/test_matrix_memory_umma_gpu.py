@@ -59,7 +59,7 @@ def test_tiles_of_128_tokens(H, d, dv, lens):
     inputs[0][sum(lens) :] = float("nan")  # rows behind the last token belong to no sequence
     want = _exact(inputs[0], inputs[1], inputs[2], inputs[3].clone(), inputs[4], lens)
     order, n, walked = torch.arange(len(lens) - 1, -1, -1), sum(lens), None
-    for how in ({"form": "walk"}, {"form": "chunk"}, {"form": "chunk", "segments": 1}, {"form": "chunk", "segments": 3}, {"form": "chunk", "segments": 9}):
+    for how in ({"form": "walk"}, *({"form": "chunk", "segments": s, "tile": 128} for s in (0, 1, 3, 9))):
         o, div, state, top = _run(inputs, lens, order, **how)
         errors = [float((a.double() - b).norm() / b.norm()) for a, b in ((o[:n], want[0]), (div[:n], want[1]), (state, want[2]), (top, want[3]))]
         walked = walked or errors
@@ -85,7 +85,7 @@ def test_infinities_and_nans_stay_where_the_recurrence_has_them(where, value, ba
         u[bad, {"q": d, "k": (H + 1) * d, "v": 2 * H * d + dv}[where] + 3] = value
     want = _exact(inputs[0], inputs[1], inputs[2], state.clone(), inputs[4], lens)
     for segments in (1, 3):
-        for a, b in zip(_run(inputs, lens, torch.arange(2), form="chunk", segments=segments), want):
+        for a, b in zip(_run(inputs, lens, torch.arange(2), form="chunk", segments=segments, tile=128), want):
             assert _same_kind(a, b, 4e-6)
 
 
@@ -107,6 +107,6 @@ def test_a_wait_that_runs_out(skip):
         for got, exact in ((o, want[0]), (div, want[1])):
             assert _same_kind(got[first : first + 128 * skip].cpu(), exact[first : first + 128 * skip], 4e-6) and (got[first + 128 * skip : last] == 7).all()
     assert "matrix_memory_umma.cu" in ops.device_wait_errors() and ops.device_wait_errors() == {}
-    for a, b in zip(_run(inputs, lens, torch.arange(2), form="chunk", segments=1), want):
+    for a, b in zip(_run(inputs, lens, torch.arange(2), form="chunk", segments=1, tile=128), want):
         assert _same_kind(a, b, 4e-6)
     assert ops.device_wait_errors() == {}

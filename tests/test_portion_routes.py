@@ -61,3 +61,30 @@ def test_single_tokens_beside_portions_of_differential_attention(portions, singl
     batch = types.SimpleNamespace(num_single=singles, num_seqs=len(lens), q_lens=lens, starts=starts, max_kv_len_single=context, max_kv_len=max(q + b for q, b in zip(lens, starts)),
                                   max_kv_len_portion=max(q + b for q, b in portions))
     assert attention.diff_singles_beside(batch, 16, 4, window, 16 if window else 0) == beside
+
+
+@pytest.mark.parametrize("heads,P,N,singles,portions,tile", [
+    (64, 64, 128, 0, [33], 128), (64, 64, 128, 0, [32], 64), (64, 64, 128, 0, [1000, 666, 1335], 128), (32, 128, 64, 0, [13, 55, 58, 58], 64), (128, 64, 128, 0, [25, 18, 11, 32, 36], 64),
+    (128, 32, 64, 0, [73, 66, 51, 63, 43], 64), (32, 128, 32, 24, [151, 153, 159], 64), (32, 64, 64, 4, [35, 24, 44, 49], 64), (64, 64, 128, 24, [100], 128), (32, 64, 64, 0, [1177], 64),
+    (32, 64, 64, 0, [616], 128), (32, 64, 64, 0, [3057], 128), (8, 64, 32, 3, [1330], 64), (8, 64, 128, 0, [1330], 128), (64, 64, 40, 0, [600], 64), (64, 64, 16, 0, [600], 64)])
+def test_tiles_of_the_scan(heads, P, N, singles, portions, tile):
+    """Tiles of 128 tokens where their CTAs, each with an SM to itself, do not queue with short portions."""
+    n, count = singles + sum(portions), singles + len(portions)
+    assert ops.ssm_tile(heads, P, N, n, count, (len(portions), sum(portions) / len(portions)), max(portions)) == tile
+
+
+@pytest.mark.parametrize("heads,d,singles,portions,tile", [
+    (16, 128, 0, [48], 64), (16, 128, 7, [600], 128), (16, 128, 0, [28] * 5 + [49], 64), (16, 128, 0, [89] * 6, 128), (16, 128, 16, [30, 60], 128), (32, 64, 0, [54, 69, 21, 82, 30], 64),
+    (32, 64, 0, [200] * 5, 128), (32, 32, 0, [100] * 8, 64), (16, 32, 0, [100], 128), (16, 64, 48, [37, 50], 128)])
+def test_tiles_of_the_matrix_memory(heads, d, singles, portions, tile):
+    n, count = singles + sum(portions), singles + len(portions)
+    assert ops.matrix_memory_tile(heads, d, d, n, count, (len(portions), sum(portions) / len(portions)), max(portions)) == tile
+
+
+def test_what_a_step_says_of_its_portions():
+    """As it is; a recorded one (its portions have no lengths yet, one of its sequences stays empty) the tokens of all together; without word the longest bounds the others."""
+    start = types.SimpleNamespace(is_cuda=True)
+    assert ssm.tile_hint(types.SimpleNamespace(q_lens=[1, 1, 30, 10], num_single=2, n=42, q_start=start)) == {"portions": (2, 20.0)}
+    assert ssm.tile_hint(types.SimpleNamespace(q_lens=[1, 1, 0, 0, 0], num_single=2, n=66, q_start=start)) == {"portions": (2, 32.0)}
+    assert ssm.tile_hint(types.SimpleNamespace(num_single=0, n=42, q_start=start)) == {}
+    assert ops.ssm_tile(64, 64, 128, 600, 1, None, 1 << 30) == 128 and ops.ssm_tile(64, 64, 128, 100, 10, None, 40) == 64

@@ -41,7 +41,7 @@ def test_tiles_and_segments(H, P, N, groups, lens, dt_shift):
     walked = None
     for form, segments in (("walk", 0), ("chunk", 0), ("chunk", 1), ("chunk", 2), ("chunk", 3), ("chunk", 7)):  # (seven: more than a sequence has tiles)
         y, st = torch.full((n, H * P), float("nan"), device="cuda"), state.flip(0).cuda()
-        ops.ssm_scan(y, xbc.cuda(), u.cuda(), dt_col, dt_bias.cuda(), a_log.cuda(), d_skip.cuda(), st, q_start, slot, groups, max_len=max(lens), form=form, segments=segments)
+        ops.ssm_scan(y, xbc.cuda(), u.cuda(), dt_col, dt_bias.cuda(), a_log.cuda(), d_skip.cuda(), st, q_start, slot, groups, max_len=max(lens), form=form, segments=segments, tile=64)
         errors = [float((a.cpu().double() - b).norm() / b.norm()) for a, b in ((y, y_ref), (st.flip(0), st_ref))]
         # float32: some four roundings of 2^-24 a token that add up at random over at most 500 tokens, 2.7e-6, and twice that for scatter
         assert all(e <= 5.4e-6 for e in errors), (form, segments, errors)
@@ -66,7 +66,7 @@ def test_a_gate_that_is_not_a_number_stays_one(where):
     q_start, slot = torch.tensor([0, n], dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda()
     for form, segments in (("walk", 0), ("chunk", 1), ("chunk", 3)):
         y, state = torch.zeros(n, H, P).cuda(), torch.zeros(1, H, P, N).cuda()
-        ops.ssm_scan(y.view(n, -1), xbc, u.cuda(), 0, zero.cuda(), a_log.cuda(), zero.cuda(), state, q_start, slot, 1, max_len=n, form=form, segments=segments)
+        ops.ssm_scan(y.view(n, -1), xbc, u.cuda(), 0, zero.cuda(), a_log.cuda(), zero.cuda(), state, q_start, slot, 1, max_len=n, form=form, segments=segments, tile=64)
         assert y[bad:, 1].isnan().all() and state[:, 1].isnan().all(), (form, segments)
         assert y[:bad].isfinite().all() and y[:, 0].isfinite().all() and state[:, 0].isfinite().all(), (form, segments)
 
@@ -101,7 +101,7 @@ def test_infinities_and_nans_stay_where_the_recurrence_has_them(where, value, ba
     q_start, slot, vec = torch.tensor([0, n], dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda(), vec.cuda()
     for segments in (1, 3):
         y, st = torch.zeros(n, H * P).cuda(), state.cuda()
-        ops.ssm_scan(y, xbc.cuda(), u.cuda(), 0, vec[0], vec[1] * 0.1, vec[2], st, q_start, slot, 1, max_len=n, form="chunk", segments=segments)
+        ops.ssm_scan(y, xbc.cuda(), u.cuda(), 0, vec[0], vec[1] * 0.1, vec[2], st, q_start, slot, 1, max_len=n, form="chunk", segments=segments, tile=64)
         if value == 3.0e38:  # (sums of such numbers may leave float32 on the way in one order and not in another: only tokens in front of it are compared)
             assert where == "state" or _same_kind(y[:bad], want[0][:bad], 1e-6)
         else:
@@ -170,8 +170,9 @@ def test_a_tile_may_be_replayed_from_a_graph():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("tile", [64, 128])
 @pytest.mark.parametrize("segments", [1, 3])
-def test_a_recorded_step_takes_other_sequences(segments):
+def test_a_recorded_step_takes_other_sequences(segments, tile):
     """Recorded once and replayed with other sequences: empty ones in the middle and at the end, and rows behind the last token that belong to none."""
     H, P, N, rows, steps = 2, 24, 32, 210, ([1, 63, 65, 0, 71], [0, 200, 1, 9, 0], [64, 0, 0, 2, 128], [0, 0, 0, 0, 0])
     S, g = len(steps[0]), torch.Generator().manual_seed(19)
@@ -181,7 +182,7 @@ def test_a_recorded_step_takes_other_sequences(segments):
     y, state = torch.zeros(rows, H * P).cuda(), start.cuda()
 
     def run():
-        ops.ssm_scan(y, x[0], x[1], 0, x[2], x[3], x[4], state, q_start, slot, 1, max_len=rows, form="chunk", segments=segments)
+        ops.ssm_scan(y, x[0], x[1], 0, x[2], x[3], x[4], state, q_start, slot, 1, max_len=rows, form="chunk", segments=segments, tile=tile)
 
     run()
     graph = torch.cuda.CUDAGraph()

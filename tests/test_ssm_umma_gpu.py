@@ -22,7 +22,7 @@ def test_tiles_of_128_tokens(H, P, N, groups, lens, dt_shift):
     errors = {}
     for form, segments in (("walk", 0), ("chunk", 0), ("chunk", 1), ("chunk", 3), ("chunk", 9)):
         y, st = torch.full((n + 5, H * P), 7.0, device="cuda"), state.flip(0).cuda()
-        ops.ssm_scan(y, xbc.cuda(), u.cuda(), 1, *[v.cuda() for v in vec], st, q_start, slot, groups, max_len=max(lens), form=form, segments=segments)
+        ops.ssm_scan(y, xbc.cuda(), u.cuda(), 1, *[v.cuda() for v in vec], st, q_start, slot, groups, max_len=max(lens), form=form, segments=segments, tile=128)
         errors[form, segments] = [float((a.cpu().double() - b).norm() / b.norm()) for a, b in ((y[:n], want[0]), (st.flip(0), want[1]))]
         # float32: some four roundings of 2^-24 a token that add up at random over at most 700 tokens, 6.3e-6 with twice that for scatter; tiles no worse than the walk
         assert all(e <= min(6.3e-6, max(4e-7, 2 * w)) for e, w in zip(errors[form, segments], errors["walk", 0])), errors
@@ -50,7 +50,7 @@ def test_infinities_and_nans_stay_where_the_recurrence_has_them(where, value, ba
     q_start, slot, vec = torch.tensor([0, 300, 320], dtype=torch.int32).cuda(), torch.arange(2, dtype=torch.int32).cuda(), vec.cuda()
     for segments in (1, 3):
         y, st = torch.zeros(n, H * P).cuda(), state.cuda()
-        ops.ssm_scan(y, xbc.cuda(), u.cuda(), 0, vec[0], vec[1] * 0.1, vec[2], st, q_start, slot, 1, max_len=300, form="chunk", segments=segments)
+        ops.ssm_scan(y, xbc.cuda(), u.cuda(), 0, vec[0], vec[1] * 0.1, vec[2], st, q_start, slot, 1, max_len=300, form="chunk", segments=segments, tile=128)
         assert _same_kind(y, want[0], 1e-6) and _same_kind(st, want[1], 1e-6)
 
 
@@ -73,5 +73,5 @@ def test_a_wait_that_runs_out(skip):
     for first, last in ((0, 300), (300, 590)):
         assert _same_kind(y[first : first + 128 * skip], want[0][first : first + 128 * skip], 1e-6) and (y[first + 128 * skip : last] == 7).all()
     assert "ssm_umma.cu" in ops.device_wait_errors() and ops.device_wait_errors() == {}
-    ops.ssm_scan(y, xbc.cuda(), u.cuda(), 0, *vec, st, q_start, slot, 1, max_len=300, form="chunk", segments=1)
+    ops.ssm_scan(y, xbc.cuda(), u.cuda(), 0, *vec, st, q_start, slot, 1, max_len=300, form="chunk", segments=1, tile=128)
     assert _same_kind(y, want[0], 1e-6) and _same_kind(st, want[1], 1e-6) and ops.device_wait_errors() == {}
