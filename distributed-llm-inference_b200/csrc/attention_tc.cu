@@ -937,6 +937,7 @@ __global__ void __launch_bounds__(DIFF_THREADS, 1) paged_prefill_diff_kernel(con
   uint64_t* bars = (uint64_t*)(sP + QT * 2 * TILE_BYTES);
   uint32_t* tmem_slot = (uint32_t*)(bars + 16);
   volatile int* failed = (volatile int*)(tmem_slot + 1);
+  int* first_token = (int*)(tmem_slot + 2);     // (a register less in the loop)
   float* row_sum = (float*)(bars + 32);         // of map 2
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -976,6 +977,7 @@ __global__ void __launch_bounds__(DIFF_THREADS, 1) paged_prefill_diff_kernel(con
     for (int i = 10; i < 14; ++i) mbar_init(k_full + 8 * i, ROWS);  // s_read, p_ready
     for (int i = 14; i < 16; ++i) mbar_init(k_full + 8 * i, 1);  // o_done
     *failed = 0;
+    *first_token = q0 + tok0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -1209,7 +1211,7 @@ __global__ void __launch_bounds__(DIFF_THREADS, 1) paged_prefill_diff_kernel(con
       l = l * corr + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
       if (base > last_whole) {  // rows of the last page that hold no token must not multiply garbage (either map's threads see to it)
         ok = wait_or_fail(v_full + 8 * (t & 1), (t >> 1) & 1, failed, 20, p.error_flag) && ok;
-        const int from = max(p.kv_len[s] - base, 0);
+        const int from = max(last_whole + KEYS - base, 0);
         for (int i = r; i < (KEYS - from) * 16; i += ROWS)
           *reinterpret_cast<uint4*>(sV + (t & 1) * V_BYTES + ((i >> 3) & 1) * TILE_BYTES + (from + (i >> 4)) * 128 + ((i & 7) << 4)) = make_uint4(0, 0, 0, 0);
       }
@@ -1245,7 +1247,7 @@ __global__ void __launch_bounds__(DIFF_THREADS, 1) paged_prefill_diff_kernel(con
 #pragma unroll
         for (int j = 0; j < 32; ++j) ss = c + j < p.dv ? fmaf(o[j], o[j], ss) : ss;
       }
-      const size_t token = q0 + tok0 + rtok;
+      const size_t token = *first_token + rtok;
       const int head = head0 + (r % Gc);
       float f = p.post / sqrtf(ss / (float)p.dv + p.eps);
       if (p.gate && rvalid) f *= 1.f / (1.f + expf(-__bfloat162float(p.gate[token * p.gate_stride + head])));

@@ -1394,7 +1394,7 @@ def _portions(n: int, count: int, longest: int) -> tuple[int, float]:
 
 
 # The fewest tokens of a portion in the mean from which on tiles of 128 are faster, for (up to one wave of their CTAs, up to two, more): such a CTA has an SM to
-# itself, so short portions of many heads queue, while four to eight CTAs with tiles of 64 share an SM, the more the smaller the state.  From 1,950 steps (8 to 128 heads, P 32 to 128, 1
+# itself, so short portions of many heads queue, while two CTAs or more with tiles of 64 share an SM, the more the smaller the state.  From 1,950 steps (8 to 128 heads, P 32 to 128, 1
 # to 16 portions of together 33 to 6,000 tokens beside 0 to 48 single ones).  Tiles of 64 / 128, us, one portion of 64 heads (N 128) of 17 tokens 9.4 / 10.2, 33 10.2 / 10.3,
 # 100 17 / 11, 600 48 / 28; 4 portions of 46 tokens, 32 heads of 128 columns, N 64 10.6 / 18.1; 5 of 24, 128 heads, N 128 28.8 / 45.7; 5 of 60, 128 heads, N 64 27.5 / 41.1; 24 single tokens and 3
 # portions of 154, 32 heads of 128 columns, N 32 33 / 44.  With it 25 of the 1,950 take over 5 % longer than tiles of 64, with a line at 33 tokens alone 577.
