@@ -106,7 +106,7 @@ __device__ __forceinline__ void unpack(const Raw8<float>& r, float (&v)[8]) {
 constexpr int CONV_TOKS = 8;
 
 template <typename T, int TAPS>
-__global__ void __launch_bounds__(128, sizeof(T) == 2 ? 4 : 3)
+__global__ void __launch_bounds__(128, sizeof(T) == 2 || TAPS == 2 ? 4 : 3)
     causal_conv_silu_window_kernel(T* __restrict__ out, const T* __restrict__ u, long long u_stride, int col0,
                                                const float* __restrict__ w, const float* __restrict__ bias, const T* __restrict__ state,
                                                const int* __restrict__ seq_of_token, const int* __restrict__ q_start,
