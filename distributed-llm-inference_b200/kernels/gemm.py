@@ -170,14 +170,29 @@ def last_product(x: torch.Tensor, weight: torch.Tensor, defer: bool):
 
 # From this many tokens and this inner size on a float32 product goes to the engine's own kernel on the tensor cores (csrc/float_gemm.cu: three
 # bfloat16 terms a number, true float32 results).  Library / own, us: 2,048 x 2,048, 1 / 4 / 8 / 100 / 512 tokens 12/21, 32/23, 32/22, 57/27, 94/45; 8,192 x 2,048
-# 23/35, 37/35, 57/35, 94/49, 315/137; K 192, 8 / 512 tokens 12/12, 18/14; K 64 8/10 up to 200 tokens.
+# 23/35, 37/35, 57/35, 94/49, 315/137; K 192, 8 / 512 tokens 12/12, 18/14; K 64 8/10 up to 200 tokens.  From 17 tokens on every size of K 256 and more gains, 4 to 128,256 features
+# (64 features of K 2,048 at 24 tokens 33/12, of K 256 6.8/6.0; a few of K 256 lose up to 0.8 of 7).  Up to 16 the library has kernels of its own for small products: 512
+# features of K 256 3.6/5.9, of K 384 4.5/7.3, of K 512 8.2/7.0; 320 of K 768 6.6/7.3, 384 8.8/7.1; and for few features with long sums, which the own one puts on one cluster a tile: 64 of K
+# 4,096 12.8/12.3, of 8,192 13.4/19.5, 256 of 8,192 19.4/25.8 (but 32 of 4,096 39/12); at 8 also for the widest, 32,768 of 4,096 167/174, 16,384 of 8,192 201/172.
 FLOAT_MIN_TOKENS, FLOAT_MIN_K = 8, 256
+FLOAT_FEW_TOKENS, FLOAT_FEW_MIN_SIZE = 16, 1 << 18  # (size: numbers of a weight)
 
 
 def float_product(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether x [.., n, in] times weight [.., out, in] transposed goes to the engine's float32 product."""
-    return (x.dtype == torch.float32 and x.is_cuda and x.dim() in (2, 3) and x.shape[-2] >= FLOAT_MIN_TOKENS and x.shape[-1] >= FLOAT_MIN_K
-            and ops.float_gemm_supported(x, weight))
+    if not (x.dtype == torch.float32 and x.is_cuda and x.dim() in (2, 3) and x.shape[-2] >= FLOAT_MIN_TOKENS and x.shape[-1] >= FLOAT_MIN_K
+            and ops.float_gemm_supported(x, weight)):
+        return False
+    return x.shape[-2] > FLOAT_FEW_TOKENS or _float_few(x.shape[-2], weight.numel() // x.shape[-1], x.shape[-1])
+
+
+def _float_few(tokens: int, features: int, K: int) -> bool:
+    """Whether a float32 product of FLOAT_MIN_TOKENS to FLOAT_FEW_TOKENS tokens goes there."""
+    if K < 1024:
+        return features * K >= FLOAT_FEW_MIN_SIZE
+    if K <= 2048:
+        return True
+    return features <= 24576 or tokens >= 12 if features > 256 else features <= 32 and K <= 6144
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:

@@ -66,6 +66,15 @@ def test_a_wait_that_runs_out(tile, splits, skip):
     assert ops.device_wait_errors() == {}
 
 
+@pytest.mark.parametrize("tokens,features,K,own", [
+    (8, 512, 256, False), (8, 1024, 256, True), (16, 512, 384, False), (8, 512, 512, True), (12, 320, 768, False), (16, 384, 768, True), (8, 64, 1024, True), (16, 64, 2048, True),
+    (8, 64, 8192, False), (16, 256, 8192, False), (8, 320, 8192, True), (8, 32768, 2048, True), (8, 32768, 4096, False), (12, 32768, 4096, True), (8, 8192, 2048, True),
+    (8, 16384, 8192, True), (16, 32, 4096, True), (16, 32, 8192, False)])
+def test_which_products_of_few_tokens_go_there(tokens, features, K, own):
+    """Small products and few features with long sums stay with the library up to 16 tokens."""
+    assert gemm._float_few(tokens, features, K) == own
+
+
 def test_no_kernel_loads_by_the_non_coherent_path():
     """Kernels start while the one in front still runs (programmatic launches), and its end orders ordinary loads only."""
     sources = sorted(p for p in Path(build.__file__).parent.iterdir() if p.suffix in (".cu", ".cuh", ".h"))
