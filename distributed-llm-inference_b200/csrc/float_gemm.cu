@@ -371,12 +371,13 @@ void choose(int tokens, int features, int batches, int steps, int& tile, int& sp
   for (int nt = 32; nt <= 128; nt *= 2)
     for (int s = 1; s <= MAX_SPLITS && s <= steps; s *= 2) {
       if ((fixed_tile && nt != fixed_tile) || (fixed_splits && s != fixed_splits)) continue;
+      if (!fixed_tile && (long long)((tokens + nt - 1) / nt) * batches > 65535) continue;  // (the grid's z)
       const long long ctas = feature_tiles * ((tokens + nt - 1) / nt) * batches * s, places = s == 8 ? 112 : s == 4 ? 132 : sm_count();
       const double step = nt == 128 ? 1.8 : nt == 64 ? 1.5 : 1.2, around = (nt == 128 ? 7.5 : nt == 64 ? 6. : 4.5) + (s > 1 ? 1.5 : 0.);
       const double us = (double)((ctas + places - 1) / places) * ((steps + s - 1) / s * step + around);
       if (best < 0. || us < best) { best = us; tile = nt; splits = s; }
     }
-  if (best < 0.) { tile = fixed_tile ? fixed_tile : 32; splits = 1; }  // (more splits asked for than steps: one)
+  if (best < 0.) { tile = fixed_tile ? fixed_tile : 128; splits = 1; }  // (more splits asked for than steps: one)
 }
 
 }  // namespace

@@ -988,9 +988,11 @@ FEW_GEMM_MAX_TOKENS = 256
 
 
 def few_gemm_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
-    """Whether ``few_gemm`` takes these operands: bfloat16, up to 256 rows of a multiple of 8 numbers on 16-byte boundaries."""
-    return (x.dtype == weight.dtype == torch.bfloat16 and x.dim() == 2 and 1 <= x.shape[0] <= FEW_GEMM_MAX_TOKENS and x.shape[1] % 8 == 0 and x.stride(1) == 1
-            and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and weight.is_contiguous() and weight.data_ptr() % 16 == 0 and weight.shape[0] % 4 == 0)
+    """Whether ``few_gemm`` takes these operands: bfloat16 on one device, up to 256 rows of a multiple of 8 numbers on 16-byte boundaries that lie behind one another (a tensor
+    map's do; an expanded row's or a sliding window's do not)."""
+    return (x.dtype == weight.dtype == torch.bfloat16 and x.device == weight.device and x.dim() == weight.dim() == 2 and 1 <= x.shape[0] <= FEW_GEMM_MAX_TOKENS
+            and x.shape[1] == weight.shape[1] and x.shape[1] % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.stride(0) >= x.shape[1] and x.data_ptr() % 16 == 0
+            and weight.is_contiguous() and weight.data_ptr() % 16 == 0 and weight.shape[0] % 4 == 0)
 
 
 def few_gemm(x: torch.Tensor, weight: torch.Tensor, splits: int, swiglu: bool = False) -> torch.Tensor:
@@ -1019,8 +1021,10 @@ def few_gemm_wait_test(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor,
 
 
 def float_gemm_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
-    """Whether ``float_gemm`` takes these operands: float32, rows of a multiple of 4 numbers that start on 16-byte boundaries."""
-    if x.dtype != torch.float32 or weight.dtype != torch.float32 or x.dim() != weight.dim() or x.dim() not in (2, 3):
+    """Whether ``float_gemm`` takes these operands: float32 on one device, rows of a multiple of 4 numbers that start on 16-byte boundaries, at most 65,535 tiles of 128 tokens."""
+    if x.dtype != torch.float32 or weight.dtype != torch.float32 or x.device != weight.device or x.dim() != weight.dim() or x.dim() not in (2, 3):
+        return False
+    if -(-x.shape[-2] // 128) * (x.shape[0] if x.dim() == 3 else 1) > 65535:
         return False
     if x.shape[-1] != weight.shape[-1] or x.shape[-1] < 4 or x.shape[-1] % 4 or (x.dim() == 3 and x.shape[0] != weight.shape[0]):
         return False
@@ -2091,7 +2095,7 @@ def matrix_memory_scan(o: torch.Tensor, divisor: torch.Tensor, u: torch.Tensor, 
         if u.dtype != torch.bfloat16 or d > MATRIX_MEMORY_CHUNK_MAX_HEAD_DIM:
             raise KernelError("matrix_memory_scan: the tensor-core form takes bfloat16 heads of at most 256")
         count = state_slot.numel()
-        umma = (32 <= d <= 128 and d % 16 == 0 and dv % 8 == 0 and u.data_ptr() % 16 == 0 and u.stride(0) % 8 == 0 and u.stride(0) >= heads * (2 * d + dv) and o.data_ptr() % 8 == 0
+        umma = (32 <= d <= 128 and d % 16 == 0 and dv % 8 == 0 and u.data_ptr() % 16 == 0 and u.stride(0) % 8 == 0 and o.data_ptr() % 8 == 0
                 and (tile or matrix_memory_tile(heads, d, dv, n, count, portions, max_len)) == 128)
         source, name, lib = ("matrix_memory_umma.cu", "dli_matrix_memory_umma", None) if umma else ("matrix_memory_tc.cu", "dli_matrix_memory_chunk", {"KEY_DIM": -(-d // 16) * 16})
         if segments < 1:

@@ -72,3 +72,17 @@ def test_up_to_how_many_tokens(features, K, swiglu, most, monkeypatch):
     """The lines lie where both sides were measured: a second wave of tiles, CTAs that share K in pairs, and wide products of some more tokens cost more than the library's."""
     monkeypatch.setattr(gemm, "sm_count", lambda: 148)
     assert gemm.few_max_tokens(features, K, swiglu) == most
+
+
+def test_rows_that_do_not_lie_behind_one_another_stay_with_the_library():
+    w = torch.empty(2048, 2048, dtype=torch.bfloat16)
+    assert gemm.few_product(torch.empty(16, 2056, dtype=torch.bfloat16)[:, :2048], w) and not gemm.few_product(torch.empty(1, 2048, dtype=torch.bfloat16).expand(16, -1), w)
+    assert not gemm.few_product(torch.empty(4096, dtype=torch.bfloat16).as_strided((16, 2048), (8, 1)), w)
+    assert not ops.few_gemm_supported(torch.empty(16, 2048, dtype=torch.bfloat16), torch.empty(2048, 2048, dtype=torch.bfloat16, device="meta"))  # on another device
+
+
+@pytest.mark.gpu
+def test_an_expanded_row():
+    g = torch.Generator().manual_seed(3)
+    x, w = torch.randn(1, 2048, generator=g).bfloat16().cuda().expand(16, -1), torch.randn(1024, 2048, generator=g).bfloat16().cuda()
+    assert _error(gemm.linear(x, w), x.double() @ w.double().t()) <= 2.0**-9

@@ -75,6 +75,20 @@ def test_which_products_of_few_tokens_go_there(tokens, features, K, own):
     assert gemm._float_few(tokens, features, K) == own
 
 
+def test_more_tiles_than_a_grid_has_stay_with_the_library():
+    x, w = torch.empty(256), torch.empty(8, 256)
+    assert ops.float_gemm_supported(x.expand(65535 * 128, 256), w) and not ops.float_gemm_supported(x.expand(65535 * 128 + 1, 256), w)
+    assert ops.float_gemm_supported(x.expand(65535, 8, 256), w.expand(65535, 8, 256)) and not ops.float_gemm_supported(x.expand(65536, 8, 256), w.expand(65536, 8, 256))
+    assert not ops.float_gemm_supported(x.expand(8, 256), w.to("meta"))
+
+
+@pytest.mark.gpu
+def test_as_many_products_as_a_grid_has():
+    x, w = torch.ones(1, 1, 256, device="cuda").expand(65535, 33, 256), torch.full((1, 1, 256), 0.5, device="cuda").expand(65535, 3, 256)
+    out = ops.float_gemm(x, w)  # in tiles of 32 there would be twice as many
+    assert out.shape == (65535, 33, 3) and (out == 128).all()
+
+
 def test_no_kernel_loads_by_the_non_coherent_path():
     """Kernels start while the one in front still runs (programmatic launches), and its end orders ordinary loads only."""
     sources = sorted(p for p in Path(build.__file__).parent.iterdir() if p.suffix in (".cu", ".cuh", ".h"))
