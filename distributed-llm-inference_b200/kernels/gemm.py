@@ -201,10 +201,12 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None = Non
         raise RuntimeError("linear: the engine has no CPU path")
     if torch.backends.cuda.matmul.allow_tf32:
         raise RuntimeError("linear: TF32 was switched on; the float32 path must stay true 32-bit")
-    if out is None and float_product(x, weight):
-        return ops.float_gemm(x, weight)
-    if out is None and few_product(x, weight):
-        return ops.few_gemm(x, weight, few_splits(*weight.shape))
+    if out is None:  # (a step that is launched kernel by kernel waits for the host: what most products need not ask is asked first)
+        if x.dtype == torch.float32:
+            if float_product(x, weight):
+                return ops.float_gemm(x, weight)
+        elif x.shape[0] <= FEW_MAX_TOKENS_SWIGLU and few_product(x, weight):
+            return ops.few_gemm(x, weight, few_splits(*weight.shape))
     return torch.matmul(x, weight.t(), out=out)
 
 
