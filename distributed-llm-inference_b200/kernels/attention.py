@@ -180,8 +180,11 @@ def diff_singles_beside(batch, num_heads: int, nkv: int, window: int | None, kee
     """Whether the single tokens of a step go to the launch of its portions (``ops.paged_prefill_diff``), whose last CTAs they are, or to their own.
 
     Where the portions' last wave of CTAs leaves places for all of them they start when the last portion CTAs have started, and what they see beyond those takes the
-    launch longer, 17 us for 1,000 keys.  A launch of their own and the merge of its partial results behind it take 11 us and 5 to 20 for 1,000 keys.  Measured, us: 9 tokens at
-    1,500 keys (a window of 1,024) beside 1,535 behind 1,024, 16 heads on 4: 93 apart, 78 beside.  A recorded step (its portions have no lengths yet) keeps them apart."""
+    launch longer, 17 us for 1,000 keys.  A launch of their own and the merge of its partial results behind it take 11 us and 5 to 20 for 1,000 keys (both slopes as in
+    ``diff_portions_apart``).  Measured, us, apart / beside, 16 heads on 4: 9 tokens at 1,500 keys (a window of 1,024) beside 1,535 behind 1,024 93 / 78, 24 at 3,000 beside 1,200 behind
+    1,024 126 / 120, 1 at 1,000 beside 1,200 49 / 40, 2 at 1,500 beside 500 behind 512 48 / 38; 8 heads on 2: 1 at 8,000 beside 200 64 / 123, 40 at 8,000 beside 200 behind 1,024 166 / 181; 32 on
+    8: 2 at 3,000 beside 200 behind 1,024 55 / 66.  Of 120 steps (1 to 64 tokens at 100 to 8,000 keys, 1 to 4 portions, windows of 512 and 1,024) none takes over 3 % longer for this rule than
+    apart, and six that it keeps apart could save 3 to 20 %.  A recorded step (its portions have no lengths yet) keeps them apart."""
     singles, lens, starts = batch.num_single, getattr(batch, "q_lens", [])[batch.num_single :], getattr(batch, "starts", [])[batch.num_single :]
     if not lens or min(lens) < 1 or len(starts) != len(lens):
         return False
@@ -195,7 +198,7 @@ def diff_singles_beside(batch, num_heads: int, nkv: int, window: int | None, kee
     ctas = wide * sum(-(-q // (128 // heads)) for q in lens)
     if wide * singles > -ctas % sms:
         return False
-    last = seen(_portion_keys(batch)) if ctas <= sms else seen(min(starts))
+    last = seen(max(q + before for q, before in zip(lens, starts))) if ctas <= sms else seen(min(starts))
     alone = seen(batch.max_kv_len_single)
     return 17 * (alone - last) <= 0.6 * (11 + alone * 20 * max(0.26, singles * nkv / sms))
 

@@ -51,6 +51,17 @@ def test_numbers_that_are_not_finite_stay_in_their_row_and_column(value, tile, s
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("x_power,w_power", [(-118, 0), (-126, 0), (0, -126), (-140, 60), (60, -140), (-70, -50), (90, -90), (110, -60), (40, 60)])
+@pytest.mark.parametrize("splits", [1, 4])
+def test_numbers_of_any_size(x_power, w_power, splits):
+    """The third term of a float32 number, 2^-17 and less of it, counts down to the smallest numbers; what is too large for the terms is computed again."""
+    g = torch.Generator().manual_seed(4)
+    x, w = (torch.randn(40, 320, generator=g).double() * 2.0**x_power).float().cuda(), (torch.randn(130, 320, generator=g).double() * 2.0**w_power).float().cuda()
+    # as above 5e-7; computed again by 320 additions one after another, of which the sum's last bits see some sqrt(320) 2^-24, 1.1e-6, twice that for scatter
+    assert _error(ops.float_gemm(x, w, tile=32, splits=splits), x.double() @ w.double().t()) <= (2.2e-6 if x_power > 100 or x_power + w_power > 75 else 5e-7)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("tile,splits,skip", [(32, 2, 7), (64, 4, 0), (128, 2, 3), (32, 1, 7)])
 def test_a_wait_that_runs_out(tile, splits, skip):
     """One CTA of each cluster waits for terms that are never handed in: none of the cluster's CTAs stores what it would add up."""

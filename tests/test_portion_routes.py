@@ -63,6 +63,16 @@ def test_single_tokens_beside_portions_of_differential_attention(portions, singl
     assert attention.diff_singles_beside(batch, 16, 4, window, 16 if window else 0) == beside
 
 
+@pytest.mark.parametrize("portions,singles,context,nh,nkv,beside", [([(200, 0)], 1, 8000, 8, 2, False), ([(200, 1024)], 40, 8000, 8, 2, False), ([(500, 1024)], 1, 8000, 32, 8, False),
+                                                                  ([(200, 1024)], 2, 3000, 32, 8, False), ([(500, 512)], 1, 700, 16, 4, True)])
+def test_long_single_tokens_stay_apart_whatever_the_step_says_of_its_portions(portions, singles, context, nh, nkv, beside, monkeypatch):
+    """A step that names only its longest sequence: the portions' keys follow from their lengths, not from the single tokens' context."""
+    monkeypatch.setattr(attention, "sm_count", lambda: 148)
+    lens, starts = [1] * singles + [q for q, _ in portions], [context - 1] * singles + [before for _, before in portions]
+    batch = types.SimpleNamespace(num_single=singles, num_seqs=len(lens), q_lens=lens, starts=starts, max_kv_len_single=context, max_kv_len=max(context, *(q + b for q, b in portions)))
+    assert attention.diff_singles_beside(batch, nh, nkv, None, 0) == beside
+
+
 @pytest.mark.parametrize("heads,P,N,singles,portions,tile", [
     (64, 64, 128, 0, [33], 128), (64, 64, 128, 0, [32], 64), (64, 64, 128, 0, [1000, 666, 1335], 128), (32, 128, 64, 0, [13, 55, 58, 58], 64), (128, 64, 128, 0, [25, 18, 11, 32, 36], 64),
     (128, 32, 64, 0, [73, 66, 51, 63, 43], 64), (32, 128, 32, 24, [151, 153, 159], 64), (32, 64, 64, 4, [35, 24, 44, 49], 64), (64, 64, 128, 24, [100], 128), (32, 64, 64, 0, [1177], 64),
