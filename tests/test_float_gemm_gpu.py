@@ -62,6 +62,17 @@ def test_numbers_of_any_size(x_power, w_power, splits):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("x_power,w_power", [(-110, 0), (0, -110), (-118, 0), (60, -118), (-126, 40), (-60, -60), (90, -90), (40, 60)])
+@pytest.mark.parametrize("splits", [1, 4])
+def test_numbers_of_any_size(x_power, w_power, splits):
+    """The three terms are the number down to 2^-110, from there on but for 2^-134."""
+    g = torch.Generator().manual_seed(4)
+    x, w = (torch.randn(40, 320, generator=g).double() * 2.0**x_power).float().cuda(), (torch.randn(130, 320, generator=g).double() * 2.0**w_power).float().cuda()
+    # as above 5e-7; beside it up to 2^-134 of numbers around 2^power
+    assert _error(ops.float_gemm(x, w, tile=32, splits=splits), x.double() @ w.double().t()) <= 5e-7 + 2.0 ** (-134 - min(x_power, w_power))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("tile,splits,skip", [(32, 2, 7), (64, 4, 0), (128, 2, 3), (32, 1, 7)])
 def test_a_wait_that_runs_out(tile, splits, skip):
     """One CTA of each cluster waits for terms that are never handed in: none of the cluster's CTAs stores what it would add up."""
