@@ -1,4 +1,4 @@
-// out[t, f] = sum over k of x[t, k] * W[f, k] for a step of some tokens (9 to 256), bfloat16 in and out, float32 sums, on tcgen05; or the activation of a
+// out[t, f] = sum over k of x[t, k] * W[f, k] for a step of some tokens (up to 128; the engine asks for 9 to 96, kernels/gemm.py: few_max_tokens), bfloat16 in and out, float32 sums, on tcgen05; or the activation of a
 // gated feed-forward on such sums.
 //
 // A step of so few tokens is the reading of the weights: features take the 128-row side of the instruction, all tokens its columns, and every weight
@@ -42,7 +42,7 @@ struct FewParams {
 
 template <int NT> struct Shape {  // NT: room for tokens
   static constexpr int A_SLAB = BF * 128, B_SLAB = NT * 128, B = 2 * A_SLAB, STAGE = 2 * (A_SLAB + B_SLAB);
-  static constexpr int STAGES = NT <= 32 ? 5 : NT == 64 ? 4 : NT == 128 ? 3 : 2;
+  static constexpr int STAGES = NT <= 32 ? 5 : NT == 64 ? 4 : 3;
   static constexpr int COLUMNS = NT < 32 ? 32 : NT;
   static constexpr int SUMS = NT * BF * 4;  // a CTA's sums [tokens][features], in the stages' place
   static constexpr int SMEM = STAGES * STAGE + 256 + 1024;
@@ -257,7 +257,7 @@ template <int NT> int launch(const CUtensorMap& map_x, const CUtensorMap& map_w,
 
 static int run(void* out, const void* x, const void* w, int tokens, int features, int K, long long x_row, int swiglu, int splits, unsigned wait_limit, int skip_step,
                cudaStream_t stream) {
-  if (tokens < 1 || tokens > 256 || features < 4 || features % 4 || K < 8 || K % 8 || x_row % 8 || (((uintptr_t)x | (uintptr_t)w) & 15) || ((uintptr_t)out & 7) ||
+  if (tokens < 1 || tokens > 128 || features < 4 || features % 4 || K < 8 || K % 8 || x_row % 8 || (((uintptr_t)x | (uintptr_t)w) & 15) || ((uintptr_t)out & 7) ||
       (swiglu && features % 128) || (splits != 1 && splits != 2 && splits != 4 && splits != 8))
     return DLI_ERR_UNSUPPORTED;
   if (!error_flag_host) {
@@ -265,7 +265,7 @@ static int run(void* out, const void* x, const void* w, int tokens, int features
     *error_flag_host = 0;
     if (cudaHostGetDevicePointer((void**)&error_flag_device, error_flag_host, 0) != cudaSuccess) return (int)cudaGetLastError();
   }
-  const int room = tokens <= 16 ? 16 : tokens <= 32 ? 32 : tokens <= 64 ? 64 : tokens <= 128 ? 128 : 256;
+  const int room = tokens <= 16 ? 16 : tokens <= 32 ? 32 : tokens <= 64 ? 64 : 128;
   CUtensorMap map_x, map_w;
   const int wide = K % BK == 0;
   const bool made = wide ? make_wide_map(&map_x, x, tokens, K, x_row, room) && make_wide_map(&map_w, w, features, K, K, BF)
@@ -276,8 +276,7 @@ static int run(void* out, const void* x, const void* w, int tokens, int features
   p.wait_limit = wait_limit; p.skip_step = skip_step;
   if (room == 16) return launch<16>(map_x, map_w, p, stream);
   if (room == 32) return launch<32>(map_x, map_w, p, stream);
-  if (room == 64) return launch<64>(map_x, map_w, p, stream);
-  return room == 128 ? launch<128>(map_x, map_w, p, stream) : launch<256>(map_x, map_w, p, stream);
+  return room == 64 ? launch<64>(map_x, map_w, p, stream) : launch<128>(map_x, map_w, p, stream);
 }
 
 // out [tokens][features], or (swiglu) [tokens][features / 2] = silu(gate) * up for weights whose rows are interleaved in blocks of 64 gate rows and the 64 up

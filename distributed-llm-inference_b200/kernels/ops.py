@@ -984,11 +984,11 @@ def skinny_gemm_error() -> int:
 
 # ------------------------------------------------------------------ products of some tokens
 
-FEW_GEMM_MAX_TOKENS = 256
+FEW_GEMM_MAX_TOKENS = 128
 
 
 def few_gemm_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
-    """Whether ``few_gemm`` takes these operands: bfloat16 on one device, up to 256 rows of a multiple of 8 numbers on 16-byte boundaries that lie behind one another (a tensor
+    """Whether ``few_gemm`` takes these operands: bfloat16 on one device, up to 128 rows of a multiple of 8 numbers on 16-byte boundaries that lie behind one another (a tensor
     map's do; an expanded row's or a sliding window's do not)."""
     return (x.dtype == weight.dtype == torch.bfloat16 and x.device == weight.device and x.dim() == weight.dim() == 2 and 1 <= x.shape[0] <= FEW_GEMM_MAX_TOKENS
             and x.shape[1] == weight.shape[1] and x.shape[1] % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.stride(0) >= x.shape[1] and x.data_ptr() % 16 == 0
@@ -996,7 +996,7 @@ def few_gemm_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
 
 
 def few_gemm(x: torch.Tensor, weight: torch.Tensor, splits: int, swiglu: bool = False) -> torch.Tensor:
-    """x [tokens, K] times weight [features, K] transposed for 1 to 256 tokens, float32 sums, on tcgen05: every weight tile is read once, and ``splits``
+    """x [tokens, K] times weight [features, K] transposed for 1 to 128 tokens, float32 sums, on tcgen05: every weight tile is read once, and ``splits``
     CTAs (1, 2, 4, 8: a cluster) share its K.  ``swiglu``: the weight's rows are blocks of 64 gate rows and the 64 up rows of the same
     features; returned is silu(gate) * up [tokens, features / 2]."""
     if not (x.is_cuda and weight.is_cuda):
