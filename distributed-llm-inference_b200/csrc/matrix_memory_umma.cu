@@ -765,8 +765,8 @@ int launch(const CUtensorMap& map, const CUtensorMap& map_o, const Params& p, cu
 
 }  // namespace
 
-// Into how many segments the sequences of a step are cut: a launch (of one segment fewer) gives every SM a CTA, and no segment is shorter than three
-// tiles.  Two segments would follow one another: three is the fewest that gain.
+// Into how many segments the sequences of a step are cut: a launch (of one segment fewer) gives every SM a CTA, and behind the first there is at most one for every
+// three tiles of the longest sequence: those have about three tiles or more, the last of them what is left, and the first what they leave, often one (segment_tiles).  Two segments would follow one another: three is the fewest that gain.
 DLI_EXPORT int dli_matrix_memory_umma_segments(int num_seqs, int heads, int dv, int max_len) {
   const long long units = (long long)column_blocks(dv) * heads * (num_seqs > 0 ? num_seqs : 1);
   long long fill = sm_count() / (units > 0 ? units : 1);

@@ -690,8 +690,8 @@ int launch(const CUtensorMap& map, const CUtensorMap& map_y, const Params& p, cu
 
 }  // namespace
 
-// Into how many segments the sequences of a step are cut: a launch (of one segment fewer) gives every SM a CTA, and no segment is shorter than four
-// tiles.  Two segments would follow one another: three is the fewest that gain.  Measured (us at segments 1 / 3 / 4 / 5, 64 heads, P 64, N 128): one
+// Into how many segments the sequences of a step are cut: a launch (of one segment fewer) gives every SM a CTA, and behind the first there is at most one for every
+// four tiles of the longest sequence: those have about four tiles or more, the last of them what is left, and the first what they leave, often one (segment_tiles).  Two segments would follow one another: three is the fewest that gain.  Measured (us at segments 1 / 3 / 4 / 5, 64 heads, P 64, N 128): one
 // prompt of 4,096 tokens 143 / 108 / 144 / 130 (four and five: more CTAs than SMs), of 600 28 / 32 / 27 / 27; three prompts (192 CTAs of one segment) 73 / 104.
 DLI_EXPORT int dli_ssm_umma_segments(int num_seqs, int heads, int P, int max_len) {
   const long long units = (long long)column_blocks(P) * heads * (num_seqs > 0 ? num_seqs : 1);

@@ -1,7 +1,10 @@
 """Matrix products y = x W^T.
 
 The reference's engine uses a library for every linear layer (nn.Linear, i.e.
-cuBLAS: src/dli/model/llama.py:72-74,95,190,305); so does this wrapper.  The
+cuBLAS: src/dli/model/llama.py:72-74,95,190,305).  Here a product goes to one of the
+engine's own tcgen05 kernels where the rules below say that it beats the library:
+few tokens (csrc/skinny_gemm.cu), some (few_gemm.cu), many with their elementwise step
+(dense_gemm.cu), float32 (float_gemm.cu); the others stay with the library.  The
 float32 path is true 32-bit: TF32 and reduced-precision accumulation are switched
 off for the process when this module is imported, and checked at every call.
 """
@@ -19,9 +22,10 @@ torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
 torch.backends.cuda.matmul.allow_fp16_reduced_precision_reduction = False
 
 
-# Up to this many tokens a layer's bfloat16 products go to the engine's own tcgen05 kernel, which
+# Up to this many tokens a layer's bfloat16 products go to the engine's decode product, which
 # there beats the library on three of the four shapes and fuses the next elementwise step;
-# measured on B200 at Llama-3.2-1B sizes, the library's kernels win from about 12 tokens on.
+# measured on B200 at Llama-3.2-1B sizes, the library's kernels beat it from about 12 tokens on
+# (steps of 9 tokens and more: few_max_tokens).
 # The head's product (float32 logits straight from the accumulator) stays with it up to 64.
 SKINNY_MAX_TOKENS = 8
 SKINNY_MAX_TOKENS_HEAD = 64
