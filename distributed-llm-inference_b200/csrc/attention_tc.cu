@@ -164,8 +164,8 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // bounded wait that also gives up as soon as another thread has recorded a failure
-__device__ __forceinline__ bool wait_or_fail(uint32_t bar, uint32_t parity, volatile int* failed, int code, int* error_flag) {
-  for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
+__device__ __forceinline__ bool wait_or_fail(uint32_t bar, uint32_t parity, volatile int* failed, int code, int* error_flag, unsigned limit = WAIT_LIMIT) {
+  for (unsigned i = 0; i < limit; ++i) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -179,8 +179,8 @@ __device__ __forceinline__ bool wait_or_fail(uint32_t bar, uint32_t parity, vola
 }
 
 // For a kernel that gives up: what it still has under way on this barrier may not land in shared or tensor memory that is no longer its own.
-__device__ __forceinline__ void wait_for_last(uint32_t bar, uint32_t parity) {
-  for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
+__device__ __forceinline__ void wait_for_last(uint32_t bar, uint32_t parity, unsigned limit = WAIT_LIMIT) {
+  for (unsigned i = 0; i < limit; ++i) {
     uint32_t done;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(done) : "r"(bar), "r"(parity) : "memory");
@@ -1363,6 +1363,8 @@ struct RowParams {
   int tokens_per_tile, heads_per_chunk, head_chunks;
   int d, dv, out_row;  // columns of a cached row, of the values that are wanted, of the output's rows
   int* error_flag;
+  unsigned wait_limit;
+  int skip_tile;  // -1 in every launch of the engine: the tile of every CTA whose copies a test leaves out
 };
 
 constexpr int ROW_SOFTMAX_THREADS = 4 * ROWS, ROW_THREADS = ROW_SOFTMAX_THREADS + 96;
@@ -1370,7 +1372,7 @@ constexpr int ROW_KEYS = 64, ROW_STAGES = 6;  // keys of a tile, tiles in shared
 
 template <int SLABS> struct RowCfg {
   static constexpr int STAGE = SLABS * ROW_KEYS * 128, AT_Q = (ROW_STAGES - 2) * STAGE;  // Q passes through the last two stages
-  static constexpr int AT_MAX = ROW_STAGES * STAGE, AT_BAR = AT_MAX + 8 * ROWS * 4, SMEM = AT_BAR + 256;
+  static constexpr int AT_MAX = ROW_STAGES * STAGE, AT_BAR = AT_MAX + 8 * ROWS * 4, SMEM = AT_BAR + 256 + 32;
   static_assert(SMEM <= 227 * 1024 && 2 * STAGE == SLABS * TILE_BYTES, "one CTA fits an SM, Q two stages");
 };
 
@@ -1405,6 +1407,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
   uint64_t* bars = (uint64_t*)(smem + Cfg::AT_BAR);
   uint32_t* tmem_slot = (uint32_t*)(bars + 28);
   volatile int* failed = (volatile int*)(tmem_slot + 1);
+  volatile int* passed = (volatile int*)(bars + 32);  // [4 (rows 32 i ..)][2 (group)] the last tile at whose barrier they met
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t sK = smem_u32(smem);
   const uint32_t k_full = smem_u32(bars), k_free = smem_u32(bars + 6), s_done = smem_u32(bars + 12), o_done = smem_u32(bars + 16), p_ready = smem_u32(bars + 20),
@@ -1432,6 +1435,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
     for (int i = 0; i < 20; ++i) mbar_init(k_full + 8 * i, 1);  // k_full (6), k_free (6), s_done (4), o_done (4)
     for (int i = 0; i < 4; ++i) mbar_init(p_ready + 8 * i, ROW_SOFTMAX_THREADS / 64);  // the warps of a tile's group
     mbar_init(q_full, ROW_SOFTMAX_THREADS / 32);
+    for (int i = 0; i < 8; ++i) passed[i] = -1;
     *failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1458,7 +1462,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
       const int cur = page;
       page = lookup(t + 1);
       if (turn > 0 || slot >= STAGES - 2) {  // O of the tile that lies in this stage, its last reader; the first time there Q
-        if (lane == 0) turn > 0 ? wait_or_fail(k_free + 8 * slot, (turn - 1) & 1, failed, 22, p.error_flag) : wait_or_fail(q_full, 0, failed, 25, p.error_flag);
+        if (lane == 0) turn > 0 ? wait_or_fail(k_free + 8 * slot, (turn - 1) & 1, failed, 22, p.error_flag, p.wait_limit) : wait_or_fail(q_full, 0, failed, 25, p.error_flag, p.wait_limit);
         __syncwarp();
         if (*failed) break;
       }
@@ -1466,7 +1470,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
       const int count = __popc(__ballot_sync(0xffffffffu, cur >= 0));
       if (lane == 0) mbar_expect_tx(full, (uint32_t)(count * unit * 128 * SLABS));
       __syncwarp();
-      if (cur >= 0) {
+      if (cur >= 0 && t != p.skip_tile) {
         const int row = (cur * p.nkv + kvh) * p.page_size + (((t_begin + t) * ROW_KEYS + (lane << unit_bits)) & (p.page_size - 1));
 #pragma unroll
         for (int sl = 0; sl < (WHOLE ? 1 : SLABS); ++sl) {
@@ -1482,20 +1486,20 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
       if (++slot == STAGES) slot = 0, ++turn;
     }
     if (*failed && lane == 0)
-      for (int t = max(0, asked - STAGES); t < asked; ++t) wait_for_last(k_full + 8 * (t % STAGES), (t / STAGES) & 1);
+      for (int t = max(0, asked - STAGES); t < asked; ++t) wait_for_last(k_full + 8 * (t % STAGES), (t / STAGES) & 1, p.wait_limit);
   } else if (warp >= ROW_SOFTMAX_THREADS / 32) {
     // ================================================================ the warps that issue the matrix products (one lane of each, the warp together): one S, one O, so that
     //                                                                  O, on which the next tile waits, does not stand behind a whole S
     const uint32_t one = elect_one();
     const uint64_t rows = (smem_desc_sw128(sK) & ~((uint64_t)0x3FFF << 32)) | (uint64_t)(PIECES >> 4) << 32;  // of the first stage (a descriptor counts 16 bytes)
     int slot = 0, phase = 0, buf = 0, t = 0;
-    bool good = wait_or_fail(q_full, 0, failed, 25, p.error_flag);
+    bool good = wait_or_fail(q_full, 0, failed, 25, p.error_flag, p.wait_limit);
     if (warp == ROW_SOFTMAX_THREADS / 32) {
       const uint32_t idesc = instr_desc(ROWS, ROW_KEYS, 0);
       const int k_steps = (p.d + 15) >> 4;
       for (; t < num_tiles; ++t) {  // S(t) = Q K(t)^T: the rows have arrived; the buffer held S(t - SB) and P(t - SB), which O has taken
-        good = good && wait_or_fail(k_full + 8 * slot, phase, failed, 17, p.error_flag);
-        if (t >= SB) good = good && wait_or_fail(o_done + 8 * ((t - SB) & 3), ((t - SB) >> 2) & 1, failed, 23, p.error_flag);
+        good = good && wait_or_fail(k_full + 8 * slot, phase, failed, 17, p.error_flag, p.wait_limit);
+        if (t >= SB) good = good && wait_or_fail(o_done + 8 * ((t - SB) & 3), ((t - SB) >> 2) & 1, failed, 23, p.error_flag, p.wait_limit);
         if (!__all_sync(0xffffffffu, good)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint64_t k = rows + (uint32_t)(slot * (STAGE >> 4));
@@ -1513,12 +1517,12 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
         if (++buf == SB) buf = 0;
       }
       if (t < num_tiles)
-        for (int i = max(0, t - 4); i < t; ++i) wait_for_last(s_done + 8 * (i & 3), (i >> 2) & 1);
+        for (int i = max(0, t - 4); i < t; ++i) wait_for_last(s_done + 8 * (i & 3), (i >> 2) & 1, p.wait_limit);
     } else {
       const uint32_t idesc = instr_desc(ROWS, vslabs * 64, 1);
       const uint64_t next_slab = (uint64_t)(NEXT_SLAB >> 4) << 16;  // of the MN-major operand: bytes from 64 columns to the next 64
       for (; t < num_tiles; ++t) {  // O += P(t) V(t): the probabilities are written, the output rescaled where a row's maximum grew
-        good = good && wait_or_fail(p_ready + 8 * (t & 3), (t >> 2) & 1, failed, 19, p.error_flag);
+        good = good && wait_or_fail(p_ready + 8 * (t & 3), (t >> 2) & 1, failed, 19, p.error_flag, p.wait_limit);
         if (!__all_sync(0xffffffffu, good)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t pa = tmem_s + buf * ROW_KEYS;
@@ -1532,7 +1536,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
         if (++buf == SB) buf = 0;
       }
       if (t < num_tiles)
-        for (int i = max(0, t - 4); i < t; ++i) wait_for_last(o_done + 8 * (i & 3), (i >> 2) & 1);
+        for (int i = max(0, t - 4); i < t; ++i) wait_for_last(o_done + 8 * (i & 3), (i >> 2) & 1, p.wait_limit);
     }
     __syncwarp();
   } else {
@@ -1577,7 +1581,8 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
     const uint32_t my_o = tmem_o + lane_bits + half * vslabs * 32;
     const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2);
     // Rows 32 i .. are four warps, two a group.  Barrier t (three of them in turns): the tile's group waits for its own maxima of tile t, and the other group has left those of tile t - 1
-    // (one that would be used for t + 3 meanwhile waits for O(t) first: its scores' place)
+    // (one that would be used for t + 3 meanwhile waits for O(t) first: its scores' place.  Where a wait ran out nothing else keeps it back, and a warp that came to the barrier of
+    // tile t + 3 while one is still on its way to that of tile t would leave the other there: it looks how far the other group has come)
     const int rows_bar = 1 + (warp & 3) * 3;
     if (group == 1) asm volatile("bar.arrive %0, 128;" ::"r"(rows_bar) : "memory");
     int buf = group % SB, turn = group, next_turn = group + 1;  // of this group's tile: t % SB; t % 3, (t + 1) % 3
@@ -1586,7 +1591,9 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
     for (int it = group; it < num_tiles; it += 2) {
       const int base = (t_begin + it) * ROW_KEYS;
       const uint32_t my_s = tmem_s + buf * ROW_KEYS + lane_bits + col0;
-      ok = wait_or_fail(s_done + 8 * (it & 3), (it >> 2) & 1, failed, 24, p.error_flag) && ok;
+      ok = wait_or_fail(s_done + 8 * (it & 3), (it >> 2) & 1, failed, 24, p.error_flag, p.wait_limit) && ok;
+      if (!ok)
+        for (unsigned i = 0; i < 1u << 28 && passed[(warp & 3) * 2 + (group ^ 1)] < it - 3; ++i) {}
       __syncwarp();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const bool full = base + ROW_KEYS - 1 <= pos0 && (p.window <= 0 || base >= hi - p.window);  // every row sees all of the tile
@@ -1610,6 +1617,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
       now[half * ROWS] = fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]);
       if (it + 1 < num_tiles) asm volatile("bar.arrive %0, 128;" ::"r"(rows_bar + next_turn) : "memory");
       asm volatile("bar.sync %0, 128;" ::"r"(rows_bar + turn) : "memory");
+      if (lane == 0) passed[(warp & 3) * 2 + group] = it;
       // probabilities are relative to the exact maximum so far: the largest one is then 1 and bfloat16 holds it as it is (following the maximum
       // only when it has grown by 2^8 gave an error 2 to 23 % larger)
       const float mine = m;
@@ -1647,7 +1655,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
       // O is free once the product of the tile before has finished.  From here to the arrival below is what a tile waits on: two pieces of 32 columns under way
       // at once, and nothing else.
       if (it > 0 && __any_sync(0xffffffffu, grown)) {
-        ok = wait_or_fail(o_done + 8 * ((it - 1) & 3), ((it - 1) >> 2) & 1, failed, 22, p.error_flag) && ok;
+        ok = wait_or_fail(o_done + 8 * ((it - 1) & 3), ((it - 1) >> 2) & 1, failed, 22, p.error_flag, p.wait_limit) && ok;
         ok = __all_sync(0xffffffffu, ok);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (ok) {
@@ -1682,15 +1690,15 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) paged_prefill_row_kernel(const
       turn = next_turn == 2 ? 0 : next_turn + 1;
       next_turn = turn == 2 ? 0 : turn + 1;
     }
-    // ---- the finished output, once the last product is done (then no barrier above is still waited at); the row sum is that of the four threads' sums, each
-    //      relative to the maximum that its group knew last
-    ok = wait_or_fail(o_done + 8 * ((num_tiles - 1) & 3), ((num_tiles - 1) >> 2) & 1, failed, 22, p.error_flag) && ok;
+    // ---- the finished output, once the last product is done; the row sum is that of the four threads' sums, each relative to the maximum that its group knew last
+    ok = wait_or_fail(o_done + 8 * ((num_tiles - 1) & 3), ((num_tiles - 1) >> 2) & 1, failed, 22, p.error_flag, p.wait_limit) && ok;
     ok = __all_sync(0xffffffffu, ok);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("bar.sync %0, 128;" ::"r"(rows_bar) : "memory");
+    // (a barrier of its own: where a wait ran out one group may be here while the other is still at those of the tiles)
+    asm volatile("bar.sync 13, %0;" ::"n"(ROW_SOFTMAX_THREADS) : "memory");
     row_max[part * ROWS + r] = l;
     row_max[(4 + part) * ROWS + r] = m;
-    asm volatile("bar.sync %0, 128;" ::"r"(rows_bar) : "memory");
+    asm volatile("bar.sync 13, %0;" ::"n"(ROW_SOFTMAX_THREADS) : "memory");
     m = max3(row_max[4 * ROWS + r], row_max[6 * ROWS + r], -CUDART_INF_F);  // (a group's threads know the same)
     float total = 0.f;
 #pragma unroll
@@ -1842,10 +1850,9 @@ DLI_EXPORT int dli_paged_prefill_diff(void* out, const void* q, long long q_stri
 #if !BENT_SCORES
 // One pool whose rows (136 to 256 numbers, a multiple of 8) are keys and, in their first value_dim numbers (a multiple of 8), values; the
 // output's rows have head_dim numbers a head, of which the first value_dim are written.
-DLI_EXPORT int dli_paged_prefill_rows(void* out, const void* q, long long q_stride, const void* pool, long long num_pages, const int* block_tables,
-                                      int max_blocks, const int* q_start, const int* kv_len, int seq0, int num_seqs, int max_q_len, int nh, int nkv,
-                                      int head_dim, int value_dim, int page_size, int window, float scale, float sink, const float* sink_heads,
-                                      cudaStream_t stream) {
+static int run_rows(void* out, const void* q, long long q_stride, const void* pool, long long num_pages, const int* block_tables, int max_blocks, const int* q_start,
+                    const int* kv_len, int seq0, int num_seqs, int max_q_len, int nh, int nkv, int head_dim, int value_dim, int page_size, int window, float scale, float sink,
+                    const float* sink_heads, unsigned wait_limit, int skip_tile, cudaStream_t stream) {
   if (num_seqs == 0) return 0;
   if (head_dim <= 128 || head_dim > 256 || head_dim % 8 || value_dim < 8 || value_dim > head_dim || value_dim % 8) return DLI_ERR_UNSUPPORTED;
   if (nkv < 1 || nh % nkv || page_size < 8 || page_size > 128 || (KEYS % page_size) != 0) return DLI_ERR_UNSUPPORTED;
@@ -1871,10 +1878,28 @@ DLI_EXPORT int dli_paged_prefill_rows(void* out, const void* q, long long q_stri
   p.tokens_per_tile = ROWS / p.heads_per_chunk;
   p.d = head_dim; p.dv = value_dim; p.out_row = head_dim;
   p.error_flag = error_flag_device;
+  p.wait_limit = wait_limit; p.skip_tile = skip_tile;
   // three tiles' scores fit tensor memory beside outputs of up to 192 columns
   if (head_dim <= 192) return whole ? launch_rows<3, true, 3>(map, p, num_seqs, max_q_len, stream) : launch_rows<3, false, 3>(map, p, num_seqs, max_q_len, stream);
   if (value_dim <= 192) return whole ? launch_rows<4, true, 3>(map, p, num_seqs, max_q_len, stream) : launch_rows<4, false, 3>(map, p, num_seqs, max_q_len, stream);
   return whole ? launch_rows<4, true, 2>(map, p, num_seqs, max_q_len, stream) : launch_rows<4, false, 2>(map, p, num_seqs, max_q_len, stream);
+}
+
+DLI_EXPORT int dli_paged_prefill_rows(void* out, const void* q, long long q_stride, const void* pool, long long num_pages, const int* block_tables,
+                                      int max_blocks, const int* q_start, const int* kv_len, int seq0, int num_seqs, int max_q_len, int nh, int nkv,
+                                      int head_dim, int value_dim, int page_size, int window, float scale, float sink, const float* sink_heads,
+                                      cudaStream_t stream) {
+  return run_rows(out, q, q_stride, pool, num_pages, block_tables, max_blocks, q_start, kv_len, seq0, num_seqs, max_q_len, nh, nkv, head_dim, value_dim, page_size, window,
+                  scale, sink, sink_heads, WAIT_LIMIT, -1, stream);
+}
+
+// For tests: without window and sink, with every CTA's copies of tile `skip_tile` (of 64 keys) left out and every wait given up after `wait_limit` polls.
+DLI_EXPORT int dli_paged_prefill_rows_wait_test(void* out, const void* q, long long q_stride, const void* pool, long long num_pages, const int* block_tables, int max_blocks,
+                                                const int* q_start, const int* kv_len, int num_seqs, int max_q_len, int nh, int nkv, int head_dim, int page_size, float scale,
+                                                unsigned wait_limit, int skip_tile, cudaStream_t stream) {
+  if (wait_limit < 1 || wait_limit > WAIT_LIMIT || skip_tile < 0) return DLI_ERR_UNSUPPORTED;
+  return run_rows(out, q, q_stride, pool, num_pages, block_tables, max_blocks, q_start, kv_len, 0, num_seqs, max_q_len, nh, nkv, head_dim, head_dim, page_size, 0, scale,
+                  -INFINITY, nullptr, wait_limit, skip_tile, stream);
 }
 #endif
 

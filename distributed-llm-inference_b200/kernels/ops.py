@@ -409,6 +409,16 @@ def paged_prefill_rows(out: torch.Tensor, q: torch.Tensor, pool: torch.Tensor, b
            "paged_prefill_rows")
 
 
+def paged_prefill_rows_wait_test(out: torch.Tensor, q: torch.Tensor, pool: torch.Tensor, block_tables: torch.Tensor, q_start: torch.Tensor, kv_len: torch.Tensor,
+                                 max_q_len: int, num_heads: int, scale: float, wait_limit: int, skip_tile: int) -> None:
+    """For tests: ``paged_prefill_rows`` with the copies of tile ``skip_tile`` (64 keys) left out and every wait given up after ``wait_limit`` polls."""
+    pages, nkv, page_size, row = pool.shape
+    f = _fn("attention_tc.cu", "dli_paged_prefill_rows_wait_test", [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p]
+            + [c_int] * 6 + [c_float, ctypes.c_uint, c_int, c_void_p])
+    _check(f(_ptr(out), _ptr(q), q.shape[1], _ptr(pool), pages, _ptr(block_tables), block_tables.shape[1], _ptr(q_start), _ptr(kv_len), kv_len.numel(), max_q_len, num_heads, nkv,
+             row, page_size, scale, wait_limit, skip_tile, _stream()), "paged_prefill_rows_wait_test")
+
+
 def paged_prefill_tc(
     out: torch.Tensor,
     qkv: torch.Tensor,

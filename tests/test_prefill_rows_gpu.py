@@ -155,3 +155,28 @@ def test_pages_that_come_whole(lens, heads, nkv, row, dv, page, window):
     for got in outs:  # probabilities and outputs are rounded to bfloat16 (2^-9 each) on the way, the products' sums are float32
         assert (got.double() - want).norm() <= 6e-3 * want.norm() and (got.double() - want).abs().max() <= 3e-2 * max(1.0, want.abs().max())
     assert ops.device_wait_errors() == {}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("row,skip", [(256, 0), (256, 7), (192, 3), (200, 1)])
+def test_a_wait_that_runs_out(row, skip):
+    """The copies of one tile never come: the CTAs that see it store nothing, the others their rows, the code is read once, the next call is right."""
+    lens, heads = [(300, 250), (20, 40)], 16
+    pool, tables, rows, q, start, kv_len = _case(lens, heads, 1, row, 16)
+    want = _exact(lens, rows, q, start, heads, 1, row, row, row**-0.5, None, None)
+    args = [x.cuda() for x in (q, pool, tables, start, kv_len)]
+    out = torch.full((q.shape[0], heads * row), 7.0, dtype=torch.bfloat16, device="cuda")
+    assert ops.device_wait_errors() == {}
+    ops.paged_prefill_rows_wait_test(out, *args, 300, heads, row**-0.5, wait_limit=20000, skip_tile=skip)
+    torch.cuda.synchronize()  # returns: the kernel ended by itself
+    got, tokens = out.view(-1, heads, row).cpu(), 128 // heads  # of a CTA
+    for first, count, before in ((0, 300, 250), (300, 20, 40)):
+        for t in range(0, count, tokens):
+            part = slice(first + t, first + min(t + tokens, count))
+            if before + min(t + tokens, count) > 64 * skip:
+                assert (got[part] == 7).all()
+            else:
+                assert (got[part].double() - want[part]).norm() <= 6e-3 * want[part].norm()
+    assert "attention_tc.cu" in ops.device_wait_errors() and ops.device_wait_errors() == {}
+    ops.paged_prefill_rows(out, *args, 0, 2, 300, heads, row**-0.5)
+    assert (out.view(-1, heads, row).cpu().double() - want).norm() <= 6e-3 * want.norm() and ops.device_wait_errors() == {}
